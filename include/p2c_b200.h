@@ -123,11 +123,11 @@ typedef struct p2c_certify_stats {
   uint64_t nodes_evaluated;                /* interval nodes whose mid sample was evaluated */
   uint64_t distance_evals;                 /* distance evaluations (3 per root + 1 per child) */
   uint64_t fp64_ops;                       /* counted FP64 add/sub/mul/div/sqrt (census launches only) */
-  uint64_t donations;                      /* subtrees handed between lanes of a warp */
+  uint64_t donations;                      /* nodes published to other warps */
   uint64_t queries;                        /* queries certified */
   uint64_t error_word;                     /* nonzero if a bounded wait or a capacity check failed */
-  uint64_t max_warp_iterations;            /* longest warp loop (one distance sample per lane per iteration) */
-  uint64_t busy_lane_iterations;           /* sum over iterations of lanes holding work */
+  uint64_t max_warp_iterations;            /* longest warp loop (up to 32 nodes per iteration) */
+  uint64_t busy_lane_iterations;           /* sum over iterations of lanes whose node counted */
 } p2c_certify_stats;
 
 /* ---- library ------------------------------------------------------------ */

@@ -54,7 +54,6 @@ struct RecordProblem {
   }
 };
 
-template <bool kShare, bool kCount>
 __global__ void __launch_bounds__(kCertifyThreads, kCertifyMinBlocks)
     certify_records_kernel(const __grid_constant__ RecordProblem prob, const __grid_constant__ CertParams prm,
                            int fetch_pt, int fetch_ee, const __grid_constant__ EnginePools pools,
@@ -66,9 +65,37 @@ __global__ void __launch_bounds__(kCertifyThreads, kCertifyMinBlocks)
   // odd warps take the edge-edge queue first, so that the tail of one family
   // overlaps the bulk of the other
   const bool ee_first = ((blockIdx.x * kCertifyWarps + (threadIdx.x >> 5)) & 1u) != 0u;
-  const bool ok = run_engine<kShare, kShare, kCount>(prob, prm, fetch_pt, fetch_ee, ee_first, sh, st,
-                                                     &scratch->engine, pools, t_start);
+  const bool ok = run_engine<true>(prob, prm, fetch_pt, fetch_ee, ee_first, sh, st, &scratch->engine, pools, t_start);
   flush_stats(st, ok, scratch);
+}
+
+// The census: every query walked alone in the reference's order.
+__global__ void __launch_bounds__(kCertifyThreads)
+    census_kernel(const __grid_constant__ RecordProblem prob, const __grid_constant__ CertParams prm,
+                  CertifyScratch* scratch) {
+  CensusStats st;
+  const unsigned long long t_start = global_ns();
+  const long long n1 = prob.n(1), n = n1 + prob.n(2);
+  bool ok = true;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; ok && i < n;
+       i += (long long)gridDim.x * blockDim.x) {
+    const int f = i < n1 ? 1 : 2;
+    const long long q = i < n1 ? i : i - n1;
+    Geo g;
+    double T0, T1;
+    int bad = 0;
+    prob.load(f, q, g, T0, T1, bad);
+    if (bad != 0) {
+      prob.invalid(f, q, bad, T0, T1);
+      continue;
+    }
+    st.queries += 1;
+    Outcome o;
+    ok = walk_tree(g, f, T0, T1, prm, t_start, o, st);
+    if (ok) prob.finish(f, q, o);
+  }
+  __syncwarp();
+  flush_census(st, ok, scratch);
 }
 
 }  // namespace
@@ -86,8 +113,7 @@ int launch_certify_records(const void* pt, long long n_pt, const void* ee, long 
   P2C_CUDA(reset_scratch(sc, stream, !census));
   if (n_pt + n_ee == 0) return P2C_OK;
   LaunchShape shape;
-  int rc = census ? certify_shape(certify_records_kernel<false, true>, &shape)
-                  : certify_shape(certify_records_kernel<true, false>, &shape);
+  int rc = certify_shape(certify_records_kernel, &shape);
   if (rc != P2C_OK) return rc;
   const CertParams ppt = make_params(cfg, shape, n_pt);
   const CertParams pee = make_params(cfg, shape, n_ee);
@@ -102,13 +128,11 @@ int launch_certify_records(const void* pt, long long n_pt, const void* ee, long 
   prob.T0 = T0;
   prob.T1 = T1;
   const EnginePools pools = pools_at(sc);
-  if (census) {
-    certify_records_kernel<false, true><<<shape.grid, kCertifyThreads, shape.smem, stream>>>(
-        prob, ppt, ppt.fetch_limit, pee.fetch_limit, pools, sc);
-  } else {
-    certify_records_kernel<true, false><<<shape.grid, kCertifyThreads, shape.smem, stream>>>(
-        prob, ppt, ppt.fetch_limit, pee.fetch_limit, pools, sc);
-  }
+  if (census)
+    census_kernel<<<shape.grid, kCertifyThreads, 0, stream>>>(prob, ppt, sc);
+  else
+    certify_records_kernel<<<shape.grid, kCertifyThreads, shape.smem, stream>>>(prob, ppt, ppt.fetch_limit,
+                                                                                 pee.fetch_limit, pools, sc);
   P2C_CUDA(cudaGetLastError());
   return P2C_OK;
 }

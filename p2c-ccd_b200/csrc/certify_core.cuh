@@ -9,20 +9,7 @@
 //  * std::clamp/min/max are restated with the same comparisons (NaN and signed
 //    zero behave as in libstdc++).
 //
-// Engine: one persistent loop per warp.  A lane owns one interval node at a
-// time and walks its subtree depth-first, left child first, with no stack: the
-// node is (path bits, depth) and its endpoints are recomputed from the root by
-// replaying the bisections (the same 0.5*(a+b) roundings the reference
-// recursion performs).  Every non-root node needs only its midpoint sample:
-// its endpoints are midpoints or endpoints of ancestors, already known to be
-// farther than eps_space (otherwise the ancestor would be a collision leaf).
-// When the query queue is empty, idle lanes take the shallowest pending right
-// subtree of a busy lane ("donation"), so one grazing query is bisected by up
-// to 32 lanes.  Per-query reduction in shared memory reproduces the recursion's
-// result exactly: the leftmost collision leaf in depth-first order (smallest
-// left-aligned path key) wins; else any undecided leaf makes the query
-// undecided; else separation with the minimum leaf margin.  Nodes right of a
-// known collision are pruned (the serial recursion never visits them).
+// The warp engine that walks the interval trees is in certify_engine.cuh.
 #pragma once
 
 #include <cmath>
@@ -280,8 +267,8 @@ struct Geo {
 };
 
 // Query geometry held in a warp's shared slot (struct-of-arrays [k][slot]):
-// lanes read their own slot's 24 coordinates per sample instead of keeping
-// them in registers, which halves the engine's register footprint.
+// lanes read a slot's 24 coordinates per sample instead of keeping them in
+// registers.
 template <class Slots>
 struct SlotGeo {
   const Slots& ws;
@@ -336,20 +323,6 @@ P2C_HD double motion_radius(const double nrm[4], double t0, double t1, C& c) {
 
 // ---- path arithmetic -------------------------------------------------------
 // Level l (1-based) of a node's path is bit (64 - l); bit 1 = went right.
-__device__ __forceinline__ unsigned long long top_bits(int k) {  // levels 1..k
-  return k <= 0 ? 0ull : (k >= 64 ? ~0ull : (~0ull << (64 - k)));
-}
-__device__ __forceinline__ unsigned long long level_bit(int l) { return 1ull << (64 - l); }
-
-// Pending right siblings of the current node inside the lane's subtree:
-// levels in (sub_depth, depth] where the path went left and that were not
-// handed to another lane.
-__device__ __forceinline__ unsigned long long pending_levels(unsigned long long path,
-                                                             unsigned long long donated, int depth,
-                                                             int sub_depth) {
-  return top_bits(depth) & ~top_bits(sub_depth) & ~path & ~donated;
-}
-
 // Endpoints of the node (path, depth) under root [T0, T1], recomputed with the
 // recursion's own roundings.  Under the root [0, 1] every bisection is exact:
 // the endpoints at depth d are multiples of 2^-d, so a + b needs at most d + 1
@@ -427,26 +400,18 @@ struct CertParams {
   double eps_time;
   double eps_space;
   int max_depth;
-  int fetch_limit;               // queries a warp keeps in flight (1..32)
+  int fetch_limit;               // queries a warp keeps in flight (1..32; the engine's slots bound it)
   unsigned long long budget_ns;  // device time budget of one launch (0 = none)
 };
 
-// Per-warp shared state: 32 query slots, struct-of-arrays so that lanes
-// reading their own slot hit distinct banks.  A slot caches one query's
-// geometry for the lanes of this warp that work on it; the query's reduction
-// lives in global memory (QueryAgg) so that other warps can share its tree.
-struct WarpSlots {
-  double p0[12][32];
-  double p1[12][32];
-  double T0[32], T1[32];
-  unsigned long long coll_key[32];  // this warp's view of the leftmost collision (pruning)
-  long long qidx[32];
-  int family[32];
-  double nrm[4][32];                // motion norms of the slot's primitive (MotionRadius factors)
+// Counters of one warp's loop (warp-uniform).
+struct WarpStats {
+  unsigned nodes = 0, evals = 0, donations = 0, queries = 0, iters = 0, busy = 0;
 };
 
-struct WarpStats {
-  unsigned long long nodes = 0, evals = 0, donations = 0, queries = 0, ops = 0, iters = 0, busy = 0;
+// Counters of the census launch (per thread).
+struct CensusStats {
+  unsigned long long nodes = 0, evals = 0, queries = 0, ops = 0;
 };
 
 // Position of the (r+1)-th set bit of m (r counts from 0); m has > r set bits.

@@ -1,30 +1,48 @@
 // certify_engine.cuh — the persistent warp engine of the interval certifier.
 //
-// A query is one interval tree (one primitive over one interval).  A lane
-// walks a subtree depth-first, left child first, with no stack: a node is
-// (path bits, depth) and its endpoints are recomputed from the root by
-// replaying the bisections (the same 0.5*(a+b) roundings the reference
-// recursion performs, certificate_engine.cpp:311).  Every non-root node needs
+// A query is one interval tree (one primitive over one interval).  A warp
+// keeps up to kSlots queries in shared memory and ONE stack of their pending
+// nodes.  Every iteration pops up to 32 nodes, one per lane, takes each node's
+// midpoint sample, and pushes the two children of every node that splits,
+// left child on top: lanes are never tied to a tree, so none idles while the
+// warp holds 32 nodes, and nothing is handed from lane to lane.  A node needs
 // only its midpoint sample: its endpoints are midpoints or endpoints of
 // ancestors, already known to be farther than eps_space (otherwise the
-// ancestor would be a collision leaf and would not have been split).
+// ancestor would be a collision leaf and would not have been split).  A root
+// takes three samples (t0, t1, mid) on three lanes.
 //
-// Work sharing, in three levels:
-//   * queries: warps take queries from per-family queues (at most
-//     fetch_limit in flight, so small batches leave lanes free to help);
-//   * lanes: an idle lane takes the shallowest pending right subtree of a
-//     busy lane of its warp (donation);
-//   * warps (kExport): when some warp has nothing to do, busy warps publish
-//     pending subtrees to a global pool that idle warps drain, so one deep
-//     tree is bisected by many warps.
+// When the stack holds few nodes, the idle lanes sample the nodes' descendants
+// in the same iteration: one node and its next four levels fill 31 lanes, two
+// nodes and three levels 30, and so on.  A descendant counts only if every
+// ancestor in the group turns out to split (a ballot and at most four bit
+// tests), so results are unchanged, and the chain of dependent samples of a
+// deep tree shortens by up to five: a warp's instructions cost the same
+// whether one lane or all take part.
+//
+// Across warps (kExport): when some warp has nothing to do, a warp holding
+// more nodes than one iteration takes publishes its shallowest ones to a
+// global pool that idle warps drain, so one deep tree is bisected by many
+// warps.
+//
 // The reduction of a tree reproduces the recursion's result exactly: the
 // leftmost collision leaf in depth-first order wins (keys are left-aligned
 // paths with a sentinel bit below the last level, so disjoint nodes compare
 // in depth-first order and the key encodes the leaf), else any undecided leaf
 // makes the tree undecided, else separation with the minimum leaf margin.  A
-// tree's reduction lives in its warp's shared slot until one of its subtrees
-// leaves the warp, then in a pooled global record.  Nodes right of a known
+// tree's reduction lives in its warp's slot; once one of its nodes leaves the
+// warp, every warp that held part of it adds its slot's reduction to a pooled
+// record, and the last one writes the result.  Nodes right of a known
 // collision are pruned: the recursion never reaches them.
+//
+// Bound by issue and by dependent FP64 chains, not by memory (128 x 128 cloth
+// certification: 750 instructions per 32 nodes, DRAM idle, 4 warps per
+// scheduler).  Against the engine that tied a lane to a subtree and handed
+// subtrees between lanes (one sample, then donation, per iteration), on a
+// B200: two 40,960-triangle spheres 75 -> 33 us (12 iterations on the longest
+// warp instead of 27), 20,000 plain queries 365 -> 190 us, a 60,000-triangle
+// cloth's 295,000 self candidates 780 -> 470 us, 64 uneven scenes 283 -> 200 us.
+// Idle warps hold a ticket each and poll their own pool entry: with one shared
+// head that they advanced by compare-and-swap the 20,000 queries took 1,200 us.
 //
 // No wait in this engine is unbounded: every loop checks the launch's device
 // time budget (CertParams::budget_ns); on expiry the engine returns false and
@@ -40,12 +58,12 @@ struct TreeAgg {
   unsigned long long coll_key;     // min leaf_key over collision leaves (~0: none)
   unsigned long long margin_bits;  // min separation margin (bit pattern of a non-negative double)
   unsigned int undecided;          // any undecided leaf
-  unsigned int outstanding;        // live units: lanes working in it + pooled tasks
+  unsigned int outstanding;        // live units: warps holding part of it + pooled nodes
 };
 
 struct SubtreeTask {
-  unsigned long long path;
-  unsigned long long tag;  // 1 + (q << 24 | agg index (16 bits) << 8 | depth << 1 | family - 1); 0 = unpublished
+  unsigned long long path;  // the node's leaf key (path and depth)
+  unsigned long long tag;   // 1 + (q << 24 | agg index (16 bits) << 8 | family - 1); 0 = unpublished
 };
 
 // Launch-wide counters, one 128-byte line each: idle warps poll some of them
@@ -58,10 +76,9 @@ struct alignas(128) PaddedCounter {
 struct EngineState {
   PaddedCounter queue_head[2];  // next query of each family
   PaddedCounter finalized;      // queries finished (both families)
-  PaddedCounter task_reserve;   // pool slots reserved
-  PaddedCounter task_head;      // pool slots claimed
+  PaddedCounter task_reserve;   // pooled nodes published (or about to be)
+  PaddedCounter task_head;      // tickets of warps that took or wait for one
   PaddedCounter agg_next;       // TreeAgg records handed out
-  PaddedCounter hungry;         // fully idle warps waiting for subtrees
   PaddedCounter helpers;        // idle warps allowed to stay and wait
 };
 
@@ -75,38 +92,66 @@ struct EnginePools {
 
 constexpr int kMaxTreeDepth = 63;  // leaf keys need one bit below the deepest level
 
-// Work-sharing parameters of the loop below (compile-time):
-//   P2C_EXPORT_LANES   subtrees one warp may publish to the pool per iteration;
-//   P2C_EXPORT_FULL    1: only a warp whose lanes are all busy publishes;
-//   P2C_EXPORT_SLACK   a lane publishes when its shallowest pending level is
-//                      within this many levels of the warp's shallowest;
-//   P2C_POOL_POLL      a warp that still has busy lanes looks at the pool
-//                      every this many iterations (a fully idle warp every one);
-//   P2C_HUNGRY_PERIOD  iterations between reads of the idle-warp count (a
+// Shape of the loop below (compile-time):
+//   P2C_ENGINE_SLOTS   queries a warp keeps in flight (at most 32);
+//   P2C_ENGINE_STACK   pending nodes a warp can hold (a power of two);
+//   P2C_ROOT_BATCH     queries fetched together (three root samples each);
+//   P2C_EXPORT_LANES   nodes one warp may publish to the pool per iteration;
+//   P2C_OVERSUPPLY     unclaimed nodes the pool may hold before warps stop
+//                      publishing;
+//   P2C_BACKOFF        longest sleep between two polls of an idle warp (ns);
+//   P2C_EXPORT_ABOVE   a warp publishes nodes beyond this many;
+//   P2C_FINISH_BATCH   finished queries a warp collects before it writes their
+//                      results together (their writes are chains of dependent
+//                      loads, stores and atomics);
+//   P2C_GUIDED         a warp claims at most 1 / (P2C_GUIDED * warps) of the
+//                      queries left in a queue (and one more);
+//   P2C_HUNGRY_PERIOD  iterations between reads of the pool's counters (a
 //                      power of two).
+#ifndef P2C_ENGINE_SLOTS
+#define P2C_ENGINE_SLOTS 16
+#endif
+#ifndef P2C_ENGINE_STACK
+#define P2C_ENGINE_STACK 256
+#endif
+#ifndef P2C_ROOT_BATCH
+#define P2C_ROOT_BATCH 10
+#endif
 #ifndef P2C_EXPORT_LANES
-#define P2C_EXPORT_LANES 1
+#define P2C_EXPORT_LANES 6
 #endif
-#ifndef P2C_EXPORT_FULL
-#define P2C_EXPORT_FULL 1
+#ifndef P2C_OVERSUPPLY
+#define P2C_OVERSUPPLY 0
 #endif
-#ifndef P2C_EXPORT_SLACK
-#define P2C_EXPORT_SLACK 0
+#ifndef P2C_BACKOFF
+#define P2C_BACKOFF 256u
 #endif
-#ifndef P2C_POOL_POLL
-#define P2C_POOL_POLL 8
+#ifndef P2C_EXPORT_ABOVE
+#define P2C_EXPORT_ABOVE 32
+#endif
+#ifndef P2C_GUIDED
+#define P2C_GUIDED 1u
+#endif
+#ifndef P2C_FINISH_BATCH
+#define P2C_FINISH_BATCH 8
 #endif
 #ifndef P2C_HUNGRY_PERIOD
-#define P2C_HUNGRY_PERIOD 8
+#define P2C_HUNGRY_PERIOD 2
 #endif
+constexpr int kSlots = P2C_ENGINE_SLOTS;
+constexpr unsigned kStack = P2C_ENGINE_STACK;
+constexpr int kRootBatch = P2C_ROOT_BATCH;
+static_assert(kSlots <= 32, "slots are one warp mask");
+static_assert(kRootBatch <= 10, "three lanes per root");
+static_assert((kStack & (kStack - 1)) == 0 && kStack >= 160, "64 entries stay free for a depth-first descent");
 static_assert((P2C_HUNGRY_PERIOD & (P2C_HUNGRY_PERIOD - 1)) == 0, "P2C_HUNGRY_PERIOD must be a power of two");
 
 // Phase clock of one warp iteration, compiled only with -DP2C_ENGINE_PROFILE
 // (a measurement build; the library is built without it): lane 0 of every
 // warp adds the SM clock cycles spent in each phase of the loop below to
-// g_engine_prof (0 fetch, 1 donation, 2 pool take, 3 idle wait, 4 distance
-// sample, 5 classify, 6 record, 7 move to the next node, 8 export,
-// 9 finalise, 10 budget check, 11 iterations).
+// g_engine_prof (0 fetch, 1 pop, 2 pool take, 3 idle wait, 4 distance sample,
+// 5 classify, 6 record, 7 push, 8 export, 9 finalise, 10 budget check,
+// 11 iterations).
 #ifdef P2C_ENGINE_PROFILE
 static __device__ unsigned long long g_engine_prof[16];
 #define P2C_PROF_DECL              \
@@ -137,13 +182,9 @@ __device__ __forceinline__ unsigned long long leaf_key(unsigned long long path, 
   return path | (1ull << (63 - depth));
 }
 
-// Publication of pooled subtrees and the last decrement of a shared tree
-// (P2C_ACQ_REL): a release store of the task tag and an acquire load by its
-// taker, and an acquire-release decrement of the tree's outstanding units,
-// instead of full fences around relaxed accesses.
-#ifndef P2C_ACQ_REL
-#define P2C_ACQ_REL 1
-#endif
+// Publication of pooled nodes and the last decrement of a shared tree: a
+// release store of the task tag and an acquire load by its taker, and an
+// acquire-release decrement of the tree's outstanding units.
 __device__ __forceinline__ void store_release(unsigned long long* p, unsigned long long v) {
   asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
@@ -165,18 +206,72 @@ __device__ __forceinline__ unsigned volatile_load(const unsigned* p) {
   return *reinterpret_cast<const volatile unsigned*>(p);
 }
 
-// Shared per-slot reduction while a tree is private to its warp.
-struct SlotAgg {
-  double margin[32];     // min margin (as double; non-negative)
-  int undecided[32];
-  int outstanding[32];   // live lanes of this warp in the tree
-  int gidx[32];          // TreeAgg index once shared, else -1
+// A warp's shared state: its queries (struct-of-arrays [k][slot], so lanes
+// reading different slots hit different banks and lanes reading one slot
+// broadcast), their reductions, and the stack of pending nodes.
+struct EngineShared {
+  double p0[12][kSlots];
+  double p1[12][kSlots];
+  double nrm[4][kSlots];                 // motion norms (MotionRadius factors)
+  double T0[kSlots], T1[kSlots];
+  unsigned long long coll_key[kSlots];   // leftmost collision leaf known to this warp (~0: none)
+  unsigned long long margin[kSlots];     // min separation margin (bits); a colliding root's time of impact
+  long long qidx[kSlots];
+  int family[kSlots];
+  int undecided[kSlots];
+  int outstanding[kSlots];               // the query's nodes on this warp's stack
+  int gidx[kSlots];                      // TreeAgg index once shared, else -1
+  int batch[32];                         // slots of the roots fetched together
+  unsigned long long nkey[kStack];       // stack: leaf keys (path and depth), intervals, slots
+  double nt0[kStack], nt1[kStack];
+  unsigned char nslot[kStack];
 };
 
-struct EngineShared {
-  WarpSlots ws;
-  SlotAgg sa;
-};
+constexpr unsigned long long kRootKey = 1ull << 63;  // leaf_key of the root
+
+__device__ __forceinline__ void fill_slot(EngineShared& sh, int s, const Geo& g, double T0, double T1, int family,
+                                          long long q, unsigned long long coll_key, int gidx) {
+#pragma unroll
+  for (int i = 0; i < 12; ++i) {
+    sh.p0[i][s] = g.p0[i];
+    sh.p1[i][s] = g.p1[i];
+  }
+  double nrm[4];
+  NoCount nc;
+  motion_norms(SlotGeo<EngineShared>{sh, s}, nrm, nc);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) sh.nrm[i][s] = nrm[i];
+  sh.T0[s] = T0;
+  sh.T1[s] = T1;
+  sh.coll_key[s] = coll_key;
+  sh.margin[s] = 0x7ff0000000000000ull;  // +inf
+  sh.qidx[s] = q;
+  sh.family[s] = family;
+  sh.undecided[s] = 0;
+  sh.outstanding[s] = 1;
+  sh.gidx[s] = gidx;
+}
+
+// The tree's result from its reduction.
+__device__ __forceinline__ Outcome tree_outcome(unsigned long long coll_key, unsigned long long margin, bool undecided,
+                                                double T0, double T1) {
+  Outcome o{P2C_STATUS_SEPARATION, T0, T1, T1, __longlong_as_double((long long)margin)};
+  if (coll_key != ~0ull) {
+    o.status = P2C_STATUS_COLLISION;
+    o.margin = 0.0;
+    if (coll_key == kRootKey) {
+      o.toi = __longlong_as_double((long long)margin);
+    } else {  // the leaf is recovered from its key
+      const int d = 64 - __ffsll((long long)coll_key);
+      replay(T0, T1, coll_key & ~(1ull << (63 - d)), d, o.t0, o.t1);
+      o.toi = mul(0.5, add(o.t0, o.t1));
+    }
+  } else if (undecided) {
+    o.status = P2C_STATUS_UNDECIDED;
+    o.margin = 0.0;
+  }
+  return o;
+}
 
 // The problem a launch certifies: both families' queries.  P provides
 //   long long n(int family) const;
@@ -184,71 +279,30 @@ struct EngineShared {
 //   void load(int family, long long q, Geo&, double& T0, double& T1, int& bad) const;
 //   void finish(int family, long long q, const Outcome&) const;
 //   void invalid(int family, long long q, int bad, double T0, double T1) const;
-template <bool kDonate, bool kExport, bool kCount, class P>
+template <bool kExport, class P>
 __device__ bool run_engine(const P& prob, const CertParams& prm, int fetch1, int fetch2, bool ee_first,
                            EngineShared& sh, WarpStats& st, EngineState* es, const EnginePools& pools,
                            unsigned long long t_start) {
-  using Counter = typename std::conditional<kCount, OpCount, NoCount>::type;
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const unsigned lt_mask = (1u << lane) - 1u;
-  WarpSlots& ws = sh.ws;
-  SlotAgg& sa = sh.sa;
   const long long n1 = prob.n(1), n2 = prob.n(2);
   const unsigned long long n_total = (unsigned long long)(n1 + n2);
-  const double eps_space = prm.eps_space, eps_time = prm.eps_time;
-  const int max_depth = prm.max_depth;
 
-  int slot = -1, fam = 1, phase = 0, depth = 0, sub_depth = 0;
-  unsigned long long path = 0, donated = 0;
-  double t0 = 0.0, t1 = 0.0, T0 = 0.0, T1 = 0.0, d1root = 0.0;
-  double nrm[4];
-  Counter ops;
-  unsigned free_mask = FULL;
+  unsigned top = 0u, bottom = 0u;          // stack [bottom, top), indices modulo kStack
+  unsigned free_mask = kSlots == 32 ? FULL : (1u << kSlots) - 1u;
   int cur = ee_first ? 2 : 1;              // family whose queue this warp drains
   unsigned exhausted = (n1 == 0 ? 1u : 0u) | (n2 == 0 ? 2u : 0u);  // bit f-1: family f's queue is empty
-  bool hungry = false;                     // this warp is counted in es->hungry
   bool helper = false;                     // this warp is counted in es->helpers
-  unsigned backoff = 256;                  // ns slept per idle poll (doubles up to 512 ns)
-  unsigned long long pool_hungry = 0, pool_size = 0;
+  bool waiting = false;                    // this warp holds the ticket of a pool entry
+  unsigned long long ticket = 0;
+  unsigned backoff = 64;                   // ns slept per idle poll (doubles up to P2C_BACKOFF)
+  unsigned long long published = 0, tickets = 0;  // the pool's counters, as last read
+  unsigned done_mask = 0u;                 // slots whose query is finished here, result not yet written
+  long long claimed1 = 0, claimed2 = 0;    // queue positions known to be claimed
+  const unsigned warps = gridDim.x * (blockDim.x >> 5);
   bool ok = true;
-
-  auto queues_done = [&]() { return exhausted == 3u; };
   P2C_PROF_DECL
-
-  // Finish a tree: one result for query (f, q).
-  auto finalize = [&](int f, long long q, const Outcome& o) {
-    prob.finish(f, q, o);
-    atomicAdd(&es->finalized.v, 1ull);
-  };
-  auto outcome_from = [&](unsigned long long key, unsigned long long mbits, bool und, double RT0,
-                          double RT1) {
-    Outcome o;
-    if (key != ~0ull) {  // a non-root collision leaf: recover it from its key
-      const int d = 64 - __ffsll((long long)key);
-      const unsigned long long pth = key & ~(1ull << (63 - d));
-      double a, b;
-      replay(RT0, RT1, pth, d, a, b);
-      o.status = P2C_STATUS_COLLISION;
-      o.t0 = a;
-      o.t1 = b;
-      o.toi = mul(0.5, add(a, b));
-      o.margin = 0.0;
-    } else if (und) {
-      o.status = P2C_STATUS_UNDECIDED;
-      o.t0 = RT0;
-      o.t1 = RT1;
-      o.toi = RT1;
-      o.margin = 0.0;
-    } else {
-      o.status = P2C_STATUS_SEPARATION;
-      o.t0 = RT0;
-      o.t1 = RT1;
-      o.toi = RT1;
-      o.margin = __longlong_as_double((long long)mbits);
-    }
-    return o;
-  };
 
   P2C_PROF_START()
   for (unsigned iter = 0;; ++iter) {
@@ -261,444 +315,438 @@ __device__ bool run_engine(const P& prob, const CertParams& prm, int fetch1, int
       }
     }
     P2C_PROF_MARK(10)
+    const unsigned size = top - bottom;
+    // ---- results of finished queries, several at a time ------------------------
+    if (done_mask != 0u && (size == 0u || __popc(done_mask) >= P2C_FINISH_BATCH)) {
+      bool finish = (done_mask >> lane) & 1u;
+      if (finish) {
+        const int gi = sh.gidx[lane];
+        unsigned long long ck = sh.coll_key[lane], mb = sh.margin[lane];
+        bool und = sh.undecided[lane] != 0;
+        if (gi >= 0) {  // shared: add this warp's part; the last part writes the result
+          TreeAgg& A = pools.aggs[gi];
+          atomicMin(&A.margin_bits, mb);
+          if (und) atomicOr(&A.undecided, 1u);
+          finish = decrement_acq_rel(&A.outstanding) == 1u;
+          if (finish) {
+            ck = volatile_load(&A.coll_key);
+            mb = volatile_load(&A.margin_bits);
+            und = volatile_load(&A.undecided) != 0u;
+          }
+        }
+        if (finish)
+          prob.finish(sh.family[lane], sh.qidx[lane], tree_outcome(ck, mb, und, sh.T0[lane], sh.T1[lane]));
+      }
+      const unsigned finished = __ballot_sync(FULL, finish);
+      if (kExport && finished != 0u && lane == 0) atomicAdd(&es->finalized.v, (unsigned long long)__popc(finished));
+      free_mask |= done_mask;
+      done_mask = 0u;
+      __syncwarp();
+    }
+    P2C_PROF_MARK(9)
+    const bool read_pool = kExport && (iter & (P2C_HUNGRY_PERIOD - 1u)) == 0u;
+    if (read_pool) {  // read here, used at the end of the iteration
+      published = volatile_load(&es->task_reserve.v);
+      tickets = volatile_load(&es->task_head.v);
+    }
+    // This iteration's groups: `width` lanes per node (or root) hold it and
+    // its next levels in heap order (h = 1 the node, 2h and 2h + 1 its
+    // children); a root's group ends in two lanes for its endpoints (h = 0).
+    int levels = 1, width = 1, groups = 0;
+    bool roots = false;
     // ---- (A) new queries from the per-family queues -------------------------
-    unsigned idle = __ballot_sync(FULL, slot < 0);
-    if (idle != 0u && !queues_done()) {
+    if (size < 32u && exhausted != 3u) {
       if (exhausted & (1u << (cur - 1))) cur = 3 - cur;
-      const int fetch_limit = cur == 1 ? fetch1 : fetch2;
-      const int room = fetch_limit - (32 - __popc(free_mask));
-      if (room > 0) {
-        const long long nc = cur == 1 ? n1 : n2;
-        const int k = min(__popc(idle), room);
+      const int limit = min(cur == 1 ? fetch1 : fetch2, kSlots);
+      const long long nc = cur == 1 ? n1 : n2;
+      // smaller batches as the queue runs out, so that no warp is left with many queries at the end
+      const unsigned left = (unsigned)min(max(nc - (cur == 1 ? claimed1 : claimed2), 0ll), 1ll << 30);
+      const int share = (int)min((unsigned)kRootBatch, left / (P2C_GUIDED * warps) + 1u);
+      const int want = min(limit - (kSlots - __popc(free_mask)), share);
+      // wait for a full batch of free slots while there are nodes to work on
+      if (want > 0 && (size == 0u || 2 * want >= min(limit, share))) {
         unsigned long long base = 0;
-        if (lane == 0) base = atomicAdd(&es->queue_head[cur - 1].v, (unsigned long long)k);
+        if (lane == 0) base = atomicAdd(&es->queue_head[cur - 1].v, (unsigned long long)want);
         base = __shfl_sync(FULL, base, 0);
-        if ((long long)base + k >= nc) exhausted |= 1u << (cur - 1);
-        bool fresh = false;
-        const int r = __popc(idle & lt_mask);
-        if (slot < 0 && r < k) {
-          const long long q = (long long)base + r;
-          if (q < nc) {
-            const int s = nth_set_bit(free_mask, r);
-            int bad = 0;
+        (cur == 1 ? claimed1 : claimed2) = (long long)base + want;
+        if ((long long)base + want >= nc) exhausted |= 1u << (cur - 1);
+        const long long q = (long long)base + lane;
+        bool fresh = false, gone = false;
+        int s = 0;
+        if (lane < want && q < nc) {
+          if (prob.skip(cur, q)) {
+            gone = true;
+          } else {
             Geo g;
-            double RT0, RT1;
-            const bool dropped = prob.skip(cur, q);
-            if (!dropped) prob.load(cur, q, g, RT0, RT1, bad);
-            if (dropped) {
-              atomicAdd(&es->finalized.v, 1ull);
-            } else if (bad != 0) {
-              prob.invalid(cur, q, bad, RT0, RT1);
-              atomicAdd(&es->finalized.v, 1ull);
+            double T0, T1;
+            int bad = 0;
+            prob.load(cur, q, g, T0, T1, bad);
+            if (bad != 0) {
+              prob.invalid(cur, q, bad, T0, T1);
+              gone = true;
             } else {
-              slot = s;
+              s = nth_set_bit(free_mask, lane);
+              fill_slot(sh, s, g, T0, T1, cur, q, ~0ull, -1);
               fresh = true;
-              fam = cur;
-#pragma unroll
-              for (int i = 0; i < 12; ++i) {
-                ws.p0[i][s] = g.p0[i];
-                ws.p1[i][s] = g.p1[i];
-              }
-              ws.T0[s] = RT0;
-              ws.T1[s] = RT1;
-              ws.coll_key[s] = ~0ull;
-              ws.qidx[s] = q;
-              ws.family[s] = cur;
-              sa.margin[s] = INFINITY;
-              sa.undecided[s] = 0;
-              sa.outstanding[s] = 1;
-              sa.gidx[s] = -1;
-              T0 = RT0;
-              T1 = RT1;
-              motion_norms(SlotGeo<WarpSlots>{ws, s}, nrm, ops);
-#pragma unroll
-              for (int i = 0; i < 4; ++i) ws.nrm[i][s] = nrm[i];
-              phase = 0;
-              path = 0ull;
-              donated = 0ull;
-              depth = 0;
-              sub_depth = 0;
-              t0 = T0;
-              t1 = T1;
-              st.queries += 1;
             }
           }
         }
-        free_mask &= ~__reduce_or_sync(FULL, fresh ? (1u << slot) : 0u);
+        const unsigned dropped = __ballot_sync(FULL, gone), got = __ballot_sync(FULL, fresh);
+        if (kExport && dropped != 0u && lane == 0) atomicAdd(&es->finalized.v, (unsigned long long)__popc(dropped));
+        if (got == 0u) continue;
+        free_mask &= ~__reduce_or_sync(FULL, fresh ? (1u << s) : 0u);
+        if (fresh) sh.batch[__popc(got & lt_mask)] = s;
         __syncwarp();
+        groups = __popc(got);
+        st.queries += (unsigned)groups;
+        roots = true;
+        levels = groups == 1 ? 4 : (groups <= 3 ? 3 : (groups <= 6 ? 2 : 1));
+        width = (1 << levels) + 1;
       }
     }
     P2C_PROF_MARK(0)
-    // ---- (B) donation inside the warp ---------------------------------------
-    if (kDonate) {
-      idle = __ballot_sync(FULL, slot < 0);
-      if (idle != 0u) {
-        const unsigned long long pend =
-            (slot >= 0 && phase == 2) ? pending_levels(path, donated, depth, sub_depth) : 0ull;
-        const unsigned donors = __ballot_sync(FULL, pend != 0ull);
-        const int npair = min(__popc(idle), __popc(donors));
-        if (npair > 0) {
-          unsigned long long gpath = 0ull;
-          int gdepth = 0, gslot = -1;
-          if (((donors >> lane) & 1u) && __popc(donors & lt_mask) < npair) {
-            const int b = 63 - __clzll((long long)pend);
-            const int l = 64 - b;
-            donated |= (1ull << b);
-            gpath = (path & top_bits(l - 1)) | (1ull << b);
-            gdepth = l;
-            gslot = slot;
-            atomicAdd(&sa.outstanding[slot], 1);
-            const int gi = sa.gidx[slot];
-            if (gi >= 0) atomicAdd(&pools.aggs[gi].outstanding, 1u);
-            st.donations += 1;
-          }
-          const bool receiver = ((idle >> lane) & 1u) && __popc(idle & lt_mask) < npair;
-          const int src_lane = receiver ? nth_set_bit(donors, __popc(idle & lt_mask)) : lane;
-          const unsigned long long rpath = __shfl_sync(FULL, gpath, src_lane);
-          const int rdepth = __shfl_sync(FULL, gdepth, src_lane);
-          const int rslot = __shfl_sync(FULL, gslot, src_lane);
-          __syncwarp();
-          if (receiver) {
-            slot = rslot;
-            fam = ws.family[slot];
-            T0 = ws.T0[slot];
-            T1 = ws.T1[slot];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) nrm[i] = ws.nrm[i][slot];  // the owner's rounded values
-            path = rpath;
-            depth = rdepth;
-            sub_depth = rdepth;
-            donated = 0ull;
-            phase = 2;
-            double a, b;
-            replay(T0, T1, path, depth - 1, a, b);
-            t0 = mul(0.5, add(a, b));
-            t1 = b;
-          }
-          __syncwarp();
-        }
-      }
-    }
-    P2C_PROF_MARK(1)
-    // ---- (C) subtrees from the global pool ------------------------------------
-    if (kExport) {
-      idle = __ballot_sync(FULL, slot < 0);
-      if (idle != 0u && queues_done() && (idle == FULL || iter % P2C_POOL_POLL == 0u)) {
-        unsigned long long h = 0;
-        int take = 0;
-        if (lane == 0) {
-          h = volatile_load(&es->task_head.v);
-          const unsigned long long r = min(volatile_load(&es->task_reserve.v), pools.task_cap);
-          const unsigned long long avail = r > h ? r - h : 0ull;
-          take = (int)min((unsigned long long)__popc(idle), avail);
-          if (take > 0 && atomicCAS(&es->task_head.v, h, h + (unsigned long long)take) != h) take = 0;
-        }
-        take = __shfl_sync(FULL, take, 0);
-        h = __shfl_sync(FULL, h, 0);
-        const int r = __popc(idle & lt_mask);
-        bool fresh = false;
-        if (slot < 0 && r < take) {
-          // the slot was reserved by a producer that publishes it right after;
-          // wait for its tag, bounded by the time budget
-          const SubtreeTask* tk = pools.tasks + h + (unsigned long long)r;
-          unsigned long long tag = P2C_ACQ_REL ? load_acquire(&tk->tag) : volatile_load(&tk->tag);
-          for (unsigned spin = 0; tag == 0ull; ++spin) {
-            __nanosleep(64);
-            tag = P2C_ACQ_REL ? load_acquire(&tk->tag) : volatile_load(&tk->tag);
-            if ((spin & 255u) == 255u && prm.budget_ns != 0ull && (global_ns() - t_start) > prm.budget_ns) break;
-          }
-          if (tag != 0ull) {
-            if (!P2C_ACQ_REL) __threadfence();
-            tag -= 1ull;
-            const int f = (int)(tag & 1ull) + 1;
-            const int d = (int)((tag >> 1) & 127ull);
-            const int gi = (int)((tag >> 8) & 0xffffull);
-            const long long q = (long long)(tag >> 24);
-            const unsigned long long pth = volatile_load(&tk->path);
-            const int s = nth_set_bit(free_mask, r);
-            Geo g;
-            int bad = 0;
-            double RT0, RT1;
-            prob.load(f, q, g, RT0, RT1, bad);
-            slot = s;
-            fresh = true;
-            fam = f;
-#pragma unroll
-            for (int i = 0; i < 12; ++i) {
-              ws.p0[i][s] = g.p0[i];
-              ws.p1[i][s] = g.p1[i];
-            }
-            ws.T0[s] = RT0;
-            ws.T1[s] = RT1;
-            ws.coll_key[s] = volatile_load(&pools.aggs[gi].coll_key);
-            ws.qidx[s] = q;
-            ws.family[s] = f;
-            sa.margin[s] = INFINITY;
-            sa.undecided[s] = 0;
-            sa.outstanding[s] = 1;
-            sa.gidx[s] = gi;
-            T0 = RT0;
-            T1 = RT1;
-            NoCount nc;
-            motion_norms(SlotGeo<WarpSlots>{ws, s}, nrm, nc);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) ws.nrm[i][s] = nrm[i];
-            path = pth;
-            depth = d;
-            sub_depth = d;
-            donated = 0ull;
-            phase = 2;
-            double a, b;
-            replay(T0, T1, path, depth - 1, a, b);
-            t0 = mul(0.5, add(a, b));
-            t1 = b;
-          }
-        }
-        free_mask &= ~__reduce_or_sync(FULL, fresh ? (1u << slot) : 0u);
-        __syncwarp();
-      }
-      // a warp is hungry while all its lanes are idle and nothing is left to take
-      const bool want = queues_done() && __ballot_sync(FULL, slot < 0) == FULL;
-      if (want != hungry) {
-        if (lane == 0) {
-          if (want) atomicAdd(&es->hungry.v, 1ull);
-          else atomicAdd(&es->hungry.v, ~0ull);
-        }
-        hungry = want;
-      }
-    }
-    P2C_PROF_MARK(2)
-    const unsigned busy = __ballot_sync(FULL, slot >= 0);
-    if (busy == 0u) {
-      if (queues_done()) {
+    if (!roots) {
+      if (size == 0u) {
+        // ---- (B) no node and no query left: a node from the global pool ------
+        // A ticket names the pool entry this warp gets; it polls that entry
+        // alone, so waiting warps do not contend.
         if (!kExport) break;
-        if (volatile_load(&es->finalized.v) >= n_total) break;
-        // at most two idle warps per SM stay to take subtrees; the others leave
-        if (!helper) {
-          int stay = 0;
-          if (lane == 0) {
-            stay = atomicAdd(&es->helpers.v, 1ull) < pools.helper_cap;
-            if (!stay) atomicAdd(&es->helpers.v, ~0ull);
+        if (!waiting) {
+          if (!helper) {  // at most helper_cap idle warps stay to take nodes; the others leave
+            int stay = 0;
+            if (lane == 0) stay = atomicAdd(&es->helpers.v, 1ull) < pools.helper_cap;
+            helper = __shfl_sync(FULL, stay, 0) != 0;
+            if (!helper) break;
           }
-          helper = __shfl_sync(FULL, stay, 0) != 0;
-          if (!helper) break;
+          if (lane == 0) ticket = atomicAdd(&es->task_head.v, 1ull);
+          ticket = __shfl_sync(FULL, ticket, 0);
+          waiting = true;
+          backoff = 64u;
         }
-        __nanosleep(backoff);
-        backoff = min(backoff * 2u, 512u);
+        SubtreeTask* tk = pools.tasks + (ticket & (pools.task_cap - 1ull));
+        unsigned long long tag = 0;
+        if (lane == 0) tag = load_acquire(&tk->tag);
+        tag = __shfl_sync(FULL, tag, 0);
+        if (tag == 0ull) {
+          if (volatile_load(&es->finalized.v) >= n_total) break;
+          __nanosleep(backoff);
+          backoff = min(backoff * 2u, P2C_BACKOFF);
+          P2C_PROF_MARK(3)
+          continue;
+        }
+        waiting = false;
+        if (lane == 0) {  // into slot 0: every slot and the whole stack are free
+          tag -= 1ull;
+          const int f = (int)(tag & 1ull) + 1;
+          const int gi = (int)((tag >> 8) & 0xffffull);
+          const long long q = (long long)(tag >> 24);
+          const unsigned long long key = volatile_load(&tk->path);
+          store_release(&tk->tag, 0ull);  // the entry is free for the pool's next lap
+          Geo g;
+          int bad = 0;
+          double T0, T1, a, b;
+          prob.load(f, q, g, T0, T1, bad);
+          fill_slot(sh, 0, g, T0, T1, f, q, volatile_load(&pools.aggs[gi].coll_key), gi);
+          const int d = 64 - __ffsll((long long)key);
+          replay(T0, T1, key & ~(1ull << (63 - d)), d, a, b);
+          sh.nkey[0] = key;
+          sh.nt0[0] = a;
+          sh.nt1[0] = b;
+          sh.nslot[0] = 0;
+        }
+        free_mask &= ~1u;
+        bottom = 0u;
+        top = 1u;
+        __syncwarp();
+        P2C_PROF_MARK(2)
+        continue;
       }
-      P2C_PROF_MARK(3)
-      continue;
+      // ---- (C) pop nodes; with few of them, whole groups of descendants -----
+      groups = (int)min(size, 32u);
+      if (size <= 10u) levels = size == 1u ? 5 : (size == 2u ? 4 : (size <= 4u ? 3 : 2));
+      else groups = max(1, min(groups, (int)(kStack - 64u) - (int)size));  // room for a depth-first descent
+      width = (1 << levels) - 1;
+      top -= (unsigned)groups;
     }
     P2C_PROF_COUNT(11)
-    backoff = 256u;
-    st.iters += 1;
-    st.busy += (unsigned long long)__popc(busy);
-    // ---- (D) prune: a node right of a known collision is never needed --------
-    bool done_lane = false;
-    if (slot >= 0 && phase == 2 && depth > 0 && ws.coll_key[slot] < leaf_key(path, depth)) done_lane = true;
-    const bool active = slot >= 0 && !done_lane;
-    // ---- (E) one distance sample per active lane -----------------------------
-    double d = 0.0, mid = 0.0;
-    if (active) {
+    const int group = width == 1 ? lane : (int)((unsigned)(lane * (65536 / width + 1)) >> 16);
+    const int first = group * width;  // lane of the group's node
+    const bool in = group < groups;
+    int h = lane - first + 1, slot = 0;
+    if (roots && h >= width - 1) h = h == width ? -1 : 0;  // endpoints t1 (-1) and t0 (0)
+    unsigned long long key = kRootKey;
+    double t0 = 0.0, t1 = 0.0;
+    if (in) {
+      if (roots) {
+        slot = sh.batch[group];
+        t0 = sh.T0[slot];
+        t1 = sh.T1[slot];
+      } else {
+        const unsigned e = (top + (unsigned)(groups - 1 - group)) & (kStack - 1u);  // group 0 is the topmost
+        slot = sh.nslot[e];
+        key = sh.nkey[e];
+        t0 = sh.nt0[e];
+        t1 = sh.nt1[e];
+      }
+    }
+    // a node right of a known collision is never needed
+    const bool eval = in && !(sh.coll_key[slot] < key);
+    double mid = mul(0.5, add(t0, t1));
+    for (int b = 30 - __clz(max(h, 1)); b >= 0; --b) {  // down to this lane's descendant
+      const unsigned long long half = (key & (0ull - key)) >> 1;
+      if ((h >> b) & 1) {
+        t0 = mid;
+        key += half;
+      } else {
+        t1 = mid;
+        key -= half;
+      }
       mid = mul(0.5, add(t0, t1));
-      const double t = phase == 0 ? t0 : (phase == 1 ? t1 : mid);
-      d = fam == 1 ? distance_at<1>(SlotGeo<WarpSlots>{ws, slot}, t, ops)
-                   : distance_at<2>(SlotGeo<WarpSlots>{ws, slot}, t, ops);
-      st.evals += 1;
-      if (phase == 0 || (phase == 2 && depth > 0)) st.nodes += 1;
-      if (kCount) ops.add(phase == 2 ? 2 : 0);
+    }
+    const int fam = sh.family[slot];
+    P2C_PROF_MARK(1)
+    // ---- (D) one distance sample per lane ------------------------------------
+    double d = 0.0;
+    if (eval) {
+      NoCount ops;
+      const double t = h > 0 ? mid : (h == 0 ? t0 : t1);
+      const SlotGeo<EngineShared> g{sh, slot};
+      d = fam == 1 ? distance_at<1>(g, t, ops) : distance_at<2>(g, t, ops);
     }
     P2C_PROF_MARK(4)
-    // ---- (F) classify: 0 none, 1 collision, 2 separation, 3 undecided ---------
+    // ---- (E) classify: 0 none, 1 collision, 2 separation, 3 undecided ---------
+    const double eps_space = prm.eps_space;
+    const bool hit = eval && d <= eps_space;
     int leaf = 0;
-    double toi = 0.0, margin = 0.0;
-    if (active) {
-      if (phase == 0) {
-        if (d <= eps_space) {
-          leaf = 1;
-          toi = t0;
-        } else {
-          phase = 1;
-        }
-      } else if (phase == 1) {
-        d1root = d;
-        phase = 2;
-      } else {
-        if (d <= eps_space) {
-          leaf = 1;
-          toi = mid;
-        } else if (depth == 0 && d1root <= eps_space) {
-          leaf = 1;
-          toi = t1;
-        } else {
-          const double lb = sub(d, fam == 1 ? motion_radius<1>(nrm, t0, t1, ops) : motion_radius<2>(nrm, t0, t1, ops));
-          if (kCount) ops.add(1);
-          if (lb > eps_space) {
-            leaf = 2;
-            margin = max_std(0.0, sub(lb, eps_space));
-            if (kCount) ops.add(1);
-          } else if (depth >= max_depth || sub(t1, t0) <= eps_time) {
-            leaf = 3;
-          } else {
-            depth += 1;  // descend into the left child (its path bit stays 0)
-            t1 = mid;
-          }
+    double margin = 0.0;
+    bool split = false, root_hit = false;
+    if (roots) {
+      const unsigned hits = __ballot_sync(FULL, hit);
+      if (eval && h == 1) {
+        const bool hit0 = (hits >> (first + width - 2)) & 1u, hit1 = (hits >> (first + width - 1)) & 1u;
+        if (hit0 || hit || hit1) {  // the root is the only node; its time of impact is the first hit of t0, mid, t1
+          root_hit = true;
+          sh.coll_key[slot] = kRootKey;
+          sh.margin[slot] = (unsigned long long)__double_as_longlong(hit0 ? t0 : (hit ? mid : t1));
         }
       }
     }
+    if (eval && h > 0 && !root_hit) {
+      if (hit) {
+        leaf = 1;
+      } else {
+        NoCount ops;
+        const double nrm[4] = {sh.nrm[0][slot], sh.nrm[1][slot], sh.nrm[2][slot], sh.nrm[3][slot]};
+        const double lb = sub(d, fam == 1 ? motion_radius<1>(nrm, t0, t1, ops) : motion_radius<2>(nrm, t0, t1, ops));
+        if (lb > eps_space) {
+          leaf = 2;
+          margin = max_std(0.0, sub(lb, eps_space));
+        } else if (64 - __ffsll((long long)key) >= prm.max_depth || sub(t1, t0) <= prm.eps_time) {
+          leaf = 3;
+        } else {
+          split = true;
+        }
+      }
+    }
+    bool reached = eval && h > 0;
+    if (levels > 1) {
+      const unsigned splits = __ballot_sync(FULL, split);
+      for (int a = h >> 1; a > 0; a >>= 1) reached = reached && ((splits >> (first + a - 1)) & 1u);
+    }
+    const unsigned reached_mask = __ballot_sync(FULL, reached);
+    st.iters += 1u;
+    st.busy += (unsigned)__popc(reached_mask);
+    st.nodes += (unsigned)__popc(reached_mask);
+    st.evals += (unsigned)__popc(reached_mask) + (roots ? 2u * (unsigned)groups : 0u);
     P2C_PROF_MARK(5)
-    // ---- (G) record leaves ------------------------------------------------------
-    bool root_collision = false;
-    if (leaf != 0) {
-      if (leaf == 1 && depth == 0) {
-        root_collision = true;  // the root is the only node: finish below
-      } else {
-        const int gi = sa.gidx[slot];
-        if (leaf == 1) {
-          const unsigned long long key = leaf_key(path, depth);
-          atomicMin(&ws.coll_key[slot], key);
+    // ---- (F) record leaves ------------------------------------------------------
+    if (reached && leaf != 0) {
+      if (leaf == 1) {
+        if (key < sh.coll_key[slot]) {
+          atomicMin(&sh.coll_key[slot], key);
+          const int gi = sh.gidx[slot];
           if (gi >= 0) atomicMin(&pools.aggs[gi].coll_key, key);
-        } else if (leaf == 2) {
-          if (gi >= 0) atomicMin(&pools.aggs[gi].margin_bits, (unsigned long long)__double_as_longlong(margin));
-          else atomicMin((unsigned long long*)&sa.margin[slot], (unsigned long long)__double_as_longlong(margin));
-        } else {
-          if (gi >= 0) atomicOr(&pools.aggs[gi].undecided, 1u);
-          else sa.undecided[slot] = 1;
         }
-      }
-    }
-    __syncwarp();
-    P2C_PROF_MARK(6)
-    // ---- (H) after a leaf, move to the deepest pending right sibling ---------
-    if (leaf != 0 && !root_collision) {
-      const unsigned long long pend = pending_levels(path, donated, depth, sub_depth);
-      if (pend == 0ull) {
-        done_lane = true;
+      } else if (leaf == 2) {
+        const unsigned long long mb = (unsigned long long)__double_as_longlong(margin);
+        if (mb < sh.margin[slot]) atomicMin(&sh.margin[slot], mb);
       } else {
-        const int b = __ffsll((long long)pend) - 1;
-        const int l = 64 - b;
-        path = (path & top_bits(l - 1)) | (1ull << b);
-        donated &= top_bits(l - 1);
-        double a, bb;
-        replay(T0, T1, path, l - 1, a, bb);
-        t0 = mul(0.5, add(a, bb));
-        t1 = bb;
-        depth = l;
-        phase = 2;
+        sh.undecided[slot] = 1;
       }
     }
+    P2C_PROF_MARK(6)
+    // ---- (G) push the children of split nodes, the leftmost on top ----------------
+    const bool push = reached && split && h >= (1 << (levels - 1));
+    const unsigned pushers = __ballot_sync(FULL, push);
+    if (push) {
+      const unsigned e = top + 2u * (unsigned)__popc(pushers & ~lt_mask & ~(1u << lane));  // pairs of the lanes above
+      const unsigned r = e & (kStack - 1u), l = (e + 1u) & (kStack - 1u);
+      const unsigned long long half = (key & (0ull - key)) >> 1;
+      sh.nkey[r] = key + half;
+      sh.nt0[r] = mid;
+      sh.nt1[r] = t1;
+      sh.nslot[r] = (unsigned char)slot;
+      sh.nkey[l] = key - half;
+      sh.nt0[l] = t0;
+      sh.nt1[l] = mid;
+      sh.nslot[l] = (unsigned char)slot;
+    }
+    top += 2u * (unsigned)__popc(pushers);
     P2C_PROF_MARK(7)
-    // ---- (I) export pending subtrees to hungry warps ---------------------------
-    if (kExport) {
-      if ((iter & (P2C_HUNGRY_PERIOD - 1u)) == 0u) {
-        if (lane == 0) {
-          pool_hungry = (unsigned long long)volatile_load(&es->hungry.v);
-          const unsigned long long rsv = volatile_load(&es->task_reserve.v), hd = volatile_load(&es->task_head.v);
-          pool_size = rsv > hd ? rsv - hd : 0ull;
-          pool_size = rsv >= pools.task_cap ? ~0ull : pool_size;  // pool full: stop exporting
-        }
-        pool_hungry = __shfl_sync(FULL, pool_hungry, 0);
-        pool_size = __shfl_sync(FULL, pool_size, 0);
-      }
-      // a warp whose lanes are all busy (nothing left to donate inside it)
-      // gives work away: up to P2C_EXPORT_LANES subtrees per iteration, the
-      // shallowest ones
-      if ((!P2C_EXPORT_FULL || busy == FULL) && pool_hungry > 0ull && pool_size < pool_hungry * 4ull) {
-        const unsigned long long pend =
-            (slot >= 0 && !done_lane && phase == 2) ? pending_levels(path, donated, depth, sub_depth) : 0ull;
-        const int lvl = pend != 0ull ? __clzll((long long)pend) : 64;  // 64 - shallowest level's bit
-        const int best = __reduce_min_sync(FULL, (unsigned)lvl);
-        const unsigned exporters = __ballot_sync(FULL, pend != 0ull && lvl <= best + P2C_EXPORT_SLACK);
-        const bool me = ((exporters >> lane) & 1u) != 0u && __popc(exporters & lt_mask) < P2C_EXPORT_LANES;
-        if (me) {
-          int gi = sa.gidx[slot];
-          // a tree's first export moves its reduction from the slot to a pooled
-          // record; one lane of the warp claims the move (others skip this iteration)
-          if (gi == -1 && atomicCAS(&sa.gidx[slot], -1, -2) == -1) {
-            const unsigned long long idx = atomicAdd(&es->agg_next.v, 1ull);
-            if (idx < pools.agg_cap) {
-              TreeAgg& A = pools.aggs[idx];
-              A.coll_key = ws.coll_key[slot];
-              A.margin_bits = (unsigned long long)__double_as_longlong(sa.margin[slot]);
-              A.undecided = (unsigned)sa.undecided[slot];
-              A.outstanding = (unsigned)sa.outstanding[slot];
-              __threadfence();
-              atomicExch(&sa.gidx[slot], (int)idx);
-              gi = (int)idx;
-            } else {
-              atomicExch(&sa.gidx[slot], -1);  // pool exhausted: the tree stays in the warp
-            }
-          }
-          if (gi >= 0) {
-            const int b = 63 - __clzll((long long)pend);
-            const int l = 64 - b;
-            const unsigned long long task = atomicAdd(&es->task_reserve.v, 1ull);
-            if (task < pools.task_cap) {  // claims never pass task_cap, so no one waits past it
-              donated |= (1ull << b);
-              atomicAdd(&pools.aggs[gi].outstanding, 1u);
-              SubtreeTask* tk = pools.tasks + task;
-              tk->path = (path & top_bits(l - 1)) | (1ull << b);
-              const unsigned long long q = (unsigned long long)ws.qidx[slot];
-              const unsigned long long tag = ((q << 24) | ((unsigned long long)gi << 8) |
-                                              ((unsigned long long)l << 1) | (unsigned long long)(fam - 1)) + 1ull;
-              if (P2C_ACQ_REL) {
-                store_release(&tk->tag, tag);
-              } else {
-                __threadfence();
-                atomicExch(&tk->tag, tag);
-              }
-              st.donations += 1;
-            }
+    // ---- (H) a tree whose last node here is done is finished ----------------------
+    const unsigned same = __match_any_sync(FULL, in ? slot : -1);
+    const unsigned popped = __ballot_sync(FULL, in && lane == first);
+    unsigned done = 0u;
+    if (in && (same & lt_mask) == 0u) {  // one lane per query
+      const int left = sh.outstanding[slot] + 2 * __popc(pushers & same) - __popc(popped & same);
+      sh.outstanding[slot] = left;
+      if (left == 0) done = 1u << slot;
+    }
+    done_mask |= __reduce_or_sync(FULL, done);
+    __syncwarp();
+    // ---- (I) publish the shallowest nodes to hungry warps ---------------------------
+    // Waiting warps hold the tickets past the published count.  Only what one
+    // iteration cannot take is given away, at most P2C_EXPORT_LANES nodes per
+    // reading of the counters and none while P2C_OVERSUPPLY are unclaimed, so
+    // the unclaimed entries (at most P2C_OVERSUPPLY + P2C_EXPORT_LANES per
+    // warp) never reach the ring's size.
+    if (read_pool) {
+      const bool give = tickets + P2C_OVERSUPPLY > published && top - bottom > P2C_EXPORT_ABOVE;
+      if (__any_sync(FULL, give)) {  // the lanes' reads of the counters may differ
+        int count = min(max((int)(top - bottom) - P2C_EXPORT_ABOVE, 0), P2C_EXPORT_LANES);
+        const unsigned e = (bottom + (unsigned)lane) & (kStack - 1u);
+        const int es_slot = lane < count ? (int)sh.nslot[e] : -1;
+        unsigned mine = __match_any_sync(FULL, es_slot);
+        const bool lead = lane < count && (mine & lt_mask) == 0u;
+        // a tree's first published node moves its reduction to a pooled record
+        if (lead && sh.gidx[es_slot] < 0) {
+          const unsigned long long idx = atomicAdd(&es->agg_next.v, 1ull);
+          if (idx < pools.agg_cap) {
+            TreeAgg& A = pools.aggs[idx];
+            A.coll_key = sh.coll_key[es_slot];
+            A.margin_bits = 0x7ff0000000000000ull;
+            A.undecided = 0u;
+            A.outstanding = 1u;  // this warp's part
+            __threadfence();
+            sh.gidx[es_slot] = (int)idx;
           }
         }
+        __syncwarp();
+        const int gi = lane < count ? sh.gidx[es_slot] : -1;
+        const unsigned without = __ballot_sync(FULL, gi < 0);  // no record left, or beyond count
+        count = without != 0u ? __ffs((int)without) - 1 : count;
+        unsigned long long task = 0;
+        if (lane == 0 && count > 0) task = atomicAdd(&es->task_reserve.v, (unsigned long long)count);
+        task = __shfl_sync(FULL, task, 0);
+        mine &= count > 0 ? FULL >> (32 - count) : 0u;
+        unsigned gone = 0u;
+        if (lead && lane < count) {
+          const int given = __popc(mine), left = sh.outstanding[es_slot] - given;
+          sh.outstanding[es_slot] = left;
+          TreeAgg& A = pools.aggs[gi];
+          if (left == 0) {  // nothing of the tree stays: its part goes with one of the nodes
+            atomicMin(&A.margin_bits, sh.margin[es_slot]);
+            if (sh.undecided[es_slot] != 0) atomicOr(&A.undecided, 1u);
+            gone = 1u << es_slot;
+          }
+          const unsigned more = (unsigned)given - (left == 0 ? 1u : 0u);
+          if (more != 0u) atomicAdd(&A.outstanding, more);
+        }
+        __syncwarp();
+        if (lane < count) {
+          SubtreeTask* tk = pools.tasks + ((task + (unsigned long long)lane) & (pools.task_cap - 1ull));
+          // the taker of the ring's previous lap has long read the entry; wait for it all the same
+          for (unsigned spin = 0; volatile_load(&tk->tag) != 0ull; ++spin) {
+            __nanosleep(64);
+            if ((spin & 255u) == 255u && prm.budget_ns != 0ull && (global_ns() - t_start) > prm.budget_ns) break;
+          }
+          tk->path = sh.nkey[e];
+          const unsigned long long tag = (((unsigned long long)sh.qidx[es_slot] << 24) |
+                                          ((unsigned long long)gi << 8) |
+                                          (unsigned long long)(sh.family[es_slot] - 1)) + 1ull;
+          __threadfence();  // the leader's record updates come before the tag
+          store_release(&tk->tag, tag);
+        }
+        st.donations += (unsigned)count;
+        bottom += (unsigned)count;
+        free_mask |= __reduce_or_sync(FULL, gone);
         __syncwarp();
       }
     }
     P2C_PROF_MARK(8)
-    // ---- (J) a finished lane leaves its tree; the last unit finalises it ------
-    unsigned freed = 0u;
-    if (root_collision) {
-      Outcome o{P2C_STATUS_COLLISION, T0, T1, toi, 0.0};
-      finalize(fam, ws.qidx[slot], o);
-      freed = 1u << slot;
-      slot = -1;
-    } else if (done_lane) {
-      const int s = slot;
-      const long long q = ws.qidx[s];
-      const int f = fam;
-      const int gi = sa.gidx[s];
-      const bool last_here = atomicSub(&sa.outstanding[s], 1) == 1;
-      if (gi >= 0) {
-        bool last = false;
-        if (P2C_ACQ_REL) {
-          last = decrement_acq_rel(&pools.aggs[gi].outstanding) == 1u;
-        } else {
-          __threadfence();
-          last = atomicSub(&pools.aggs[gi].outstanding, 1u) == 1u;
-          if (last) __threadfence();
-        }
-        if (last) {
-          const TreeAgg& A = pools.aggs[gi];
-          const Outcome o = outcome_from(volatile_load(&A.coll_key), volatile_load(&A.margin_bits),
-                                         volatile_load(&A.undecided) != 0u, T0, T1);
-          finalize(f, q, o);
-        }
-      } else if (last_here) {
-        const unsigned long long mb = (unsigned long long)__double_as_longlong(sa.margin[s]);
-        const Outcome o = outcome_from(ws.coll_key[s], mb, sa.undecided[s] != 0, T0, T1);
-        finalize(f, q, o);
-      }
-      if (last_here) freed = 1u << s;
-      slot = -1;
-    }
-    free_mask |= __reduce_or_sync(FULL, freed);
-    __syncwarp();
-    P2C_PROF_MARK(9)
   }
   P2C_PROF_FLUSH()
-  if (kExport && hungry && lane == 0) atomicAdd(&es->hungry.v, ~0ull);
-  if (kCount) st.ops += ops.n;
   return ok;
+}
+
+// The recursion's own walk of one tree, depth-first on one lane, counting its
+// nodes, samples and FP64 operations (the census launch).  Returns false when
+// the time budget ends first.
+__device__ inline bool walk_tree(const Geo& g, int family, double T0, double T1, const CertParams& prm,
+                                 unsigned long long t_start, Outcome& out, CensusStats& st) {
+  struct Points {
+    const Geo& g;
+    __device__ __forceinline__ double p0(int k) const { return g.p0[k]; }
+    __device__ __forceinline__ double p1(int k) const { return g.p1[k]; }
+  };
+  const Points pts{g};
+  OpCount ops;
+  double nrm[4];
+  motion_norms(pts, nrm, ops);
+  auto sample = [&](double t) {
+    st.evals += 1;
+    return family == 1 ? distance_at<1>(pts, t, ops) : distance_at<2>(pts, t, ops);
+  };
+  double st0[kMaxTreeDepth + 1], st1[kMaxTreeDepth + 1];  // pending right siblings
+  int sdepth[kMaxTreeDepth + 1], pending = 0;
+  double t0 = T0, t1 = T1, margin = INFINITY;
+  int depth = 0;
+  bool undecided = false;
+  out = Outcome{P2C_STATUS_COLLISION, T0, T1, T0, 0.0};
+  st.nodes += 1;
+  const double d0 = sample(T0);
+  double d1 = 0.0;
+  bool done = d0 <= prm.eps_space;  // the root collides at t0
+  if (!done) d1 = sample(T1);
+  for (unsigned k = 0; !done; ++k) {
+    if ((k & 63u) == 63u && prm.budget_ns != 0ull && global_ns() - t_start > prm.budget_ns) return false;
+    const double mid = mul(0.5, add(t0, t1));
+    ops.add(2);
+    if (depth > 0) st.nodes += 1;
+    const double d = sample(mid);
+    if (d <= prm.eps_space || (depth == 0 && d1 <= prm.eps_space)) {
+      out.t0 = t0;
+      out.t1 = t1;
+      out.toi = d <= prm.eps_space ? mid : t1;
+      done = true;
+      break;
+    }
+    const double lb = sub(d, family == 1 ? motion_radius<1>(nrm, t0, t1, ops) : motion_radius<2>(nrm, t0, t1, ops));
+    ops.add(1);
+    if (lb > prm.eps_space) {
+      const double m = max_std(0.0, sub(lb, prm.eps_space));
+      ops.add(1);
+      if (m < margin) margin = m;
+    } else if (depth >= prm.max_depth || sub(t1, t0) <= prm.eps_time) {
+      undecided = true;
+    } else {
+      st0[pending] = mid;
+      st1[pending] = t1;
+      sdepth[pending++] = ++depth;
+      t1 = mid;
+      continue;
+    }
+    if (pending == 0) break;
+    --pending;
+    t0 = st0[pending];
+    t1 = st1[pending];
+    depth = sdepth[pending];
+  }
+  st.ops += ops.n;
+  if (!done)
+    out = undecided ? Outcome{P2C_STATUS_UNDECIDED, T0, T1, T1, 0.0}
+                    : Outcome{P2C_STATUS_SEPARATION, T0, T1, T1, margin};
+  return true;
 }
 
 }  // namespace p2c

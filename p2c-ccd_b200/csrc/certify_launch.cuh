@@ -11,9 +11,12 @@
 
 namespace p2c {
 
-constexpr int kCertifyThreads = 128;  // 4 warps per block, one WarpSlots each
+constexpr int kCertifyThreads = 128;  // 4 warps per block, one EngineShared each
 constexpr int kCertifyWarps = kCertifyThreads / 32;
-constexpr int kCertifyMinBlocks = 4;  // 16 warps per SM: caps registers at 128 per thread
+#ifndef P2C_CERTIFY_BLOCKS
+#define P2C_CERTIFY_BLOCKS 4
+#endif
+constexpr int kCertifyMinBlocks = P2C_CERTIFY_BLOCKS;  // 16 warps per SM: caps registers at 128 per thread
 
 // Device scratch of one certification launch (reset by the launcher).
 struct CertifyScratch {
@@ -23,15 +26,15 @@ struct CertifyScratch {
 };
 
 // Fixed-size pools of the cross-warp sharing (independent of the batch size):
-// reduction records of trees whose subtrees left their warp, and published
-// subtree tasks.  Task tags must read zero before each launch.
+// reduction records of trees whose nodes left their warp, and a ring of
+// published nodes, larger than what all warps together can have published and
+// not yet taken.  Task tags must read zero before each launch.
 constexpr unsigned long long kTreeAggCap = 8192;
 constexpr unsigned long long kTaskCap = 16384;
+static_assert((kTaskCap & (kTaskCap - 1ull)) == 0ull && kTaskCap >= P2C_OVERSUPPLY + 148ull * 16ull * P2C_EXPORT_LANES,
+              "the pool's ring holds every warp's unclaimed nodes");
 #ifndef P2C_HELPERS_PER_SM
-#define P2C_HELPERS_PER_SM 2
-#endif
-#ifndef P2C_FETCH_PCT
-#define P2C_FETCH_PCT 100
+#define P2C_HELPERS_PER_SM 8
 #endif
 constexpr unsigned long long kHelperWarps = 148ull * P2C_HELPERS_PER_SM;  // idle warps that stay for subtrees
 constexpr size_t kScratchHeaderBytes = (sizeof(CertifyScratch) + 255) & ~size_t(255);
@@ -85,7 +88,6 @@ inline CertParams make_params(const p2c_cert_config& cfg, const LaunchShape& sha
   p.max_depth = cfg.max_subdivision_depth;
   const long long warps = (long long)shape.grid * kCertifyWarps;
   long long per_warp = warps > 0 ? (n + warps - 1) / warps : 32;
-  per_warp = (per_warp * P2C_FETCH_PCT + 99) / 100;  // queries a warp takes at first, in percent of its share
   if (per_warp < 1) per_warp = 1;
   if (per_warp > 32) per_warp = 32;
   p.fetch_limit = (int)per_warp;
@@ -121,20 +123,32 @@ __device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
   return v;
 }
 
+__device__ __forceinline__ void add_stat(uint64_t* p, unsigned long long v) {
+  if (v) atomicAdd((unsigned long long*)p, v);
+}
+
+// The counters of a warp's loop are warp-uniform: one lane adds them.
 __device__ __forceinline__ void flush_stats(const WarpStats& st, bool ok, CertifyScratch* sc) {
-  const unsigned long long nodes = warp_sum(st.nodes), evals = warp_sum(st.evals),
-                           don = warp_sum(st.donations), q = warp_sum(st.queries), ops = warp_sum(st.ops);
+  if ((threadIdx.x & 31) != 0) return;
+  if (st.iters) atomicMax((unsigned long long*)&sc->stats.max_warp_iterations, (unsigned long long)st.iters);
+  add_stat(&sc->stats.busy_lane_iterations, st.busy);
+  add_stat(&sc->stats.nodes_evaluated, st.nodes);
+  add_stat(&sc->stats.distance_evals, st.evals);
+  add_stat(&sc->stats.donations, st.donations);
+  add_stat(&sc->stats.queries, st.queries);
+  if (!ok) atomicOr((unsigned long long*)&sc->stats.error_word, 1ull);
+}
+
+__device__ __forceinline__ void flush_census(const CensusStats& st, bool ok, CertifyScratch* sc) {
+  const unsigned long long nodes = warp_sum(st.nodes), evals = warp_sum(st.evals), q = warp_sum(st.queries),
+                           ops = warp_sum(st.ops);
   if ((threadIdx.x & 31) == 0) {
-    // iteration counters are warp-uniform: lane 0's copy is the warp's
-    if (st.iters) atomicMax((unsigned long long*)&sc->stats.max_warp_iterations, st.iters);
-    if (st.busy) atomicAdd((unsigned long long*)&sc->stats.busy_lane_iterations, st.busy);
-    if (nodes) atomicAdd((unsigned long long*)&sc->stats.nodes_evaluated, nodes);
-    if (evals) atomicAdd((unsigned long long*)&sc->stats.distance_evals, evals);
-    if (don) atomicAdd((unsigned long long*)&sc->stats.donations, don);
-    if (q) atomicAdd((unsigned long long*)&sc->stats.queries, q);
-    if (ops) atomicAdd((unsigned long long*)&sc->stats.fp64_ops, ops);
-    if (!ok) atomicOr((unsigned long long*)&sc->stats.error_word, 1ull);
+    add_stat(&sc->stats.nodes_evaluated, nodes);
+    add_stat(&sc->stats.distance_evals, evals);
+    add_stat(&sc->stats.queries, q);
+    add_stat(&sc->stats.fp64_ops, ops);
   }
+  if (!ok) atomicOr((unsigned long long*)&sc->stats.error_word, 1ull);
 }
 
 inline int export_stats(CertifyScratch* sc, p2c_certify_stats* stats_dev, cudaStream_t s) {

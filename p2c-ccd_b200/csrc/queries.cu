@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(kCertifyThreads, kCertifyMinBlocks)
   const bool ee_first = ((blockIdx.x * kCertifyWarps + (threadIdx.x >> 5)) & 1u) != 0u;
   // no cross-warp pools here: the scratch stays one record per work item
   const EnginePools no_pools{};
-  const bool ok = run_engine<true, false, false>(prob, prm, fetch_pt, fetch_ee, ee_first, sh, st, &sc->engine,
+  const bool ok = run_engine<false>(prob, prm, fetch_pt, fetch_ee, ee_first, sh, st, &sc->engine,
                                                  no_pools, t_start);
   flush_stats(st, ok, sc);
 }

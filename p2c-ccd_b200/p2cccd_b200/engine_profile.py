@@ -3,8 +3,8 @@
 Builds the library a second time with ``-DP2C_ENGINE_PROFILE`` into
 ``_build_profile/`` (beside the product build, which stays untouched): lane 0
 of every warp then adds the SM clock cycles of each phase of the engine's loop
-(fetch, donation, pool take, idle wait, distance sample, classify, record,
-move to the next node, export, finalise, budget check) to a per-file device
+(fetch, pop, pool take, idle wait, distance sample, classify, record, push,
+export, finalise, budget check) to a per-file device
 array that ``p2c_engine_profile_<file>`` reads back.  Each phase boundary
 synchronises the warp, so absolute cycles are inflated by a few hundred per
 phase; shares are what the breakdown is for.
@@ -19,8 +19,7 @@ import ctypes
 import json
 from pathlib import Path
 
-PHASES = ["fetch", "donate", "pool", "idle", "distance", "classify", "record", "move", "export", "finalise",
-          "budget"]
+PHASES = ["fetch", "pop", "pool", "idle", "distance", "classify", "record", "push", "export", "finalise", "budget"]
 PROFILE_LIB = Path(__file__).resolve().parent.parent / "_build_profile" / "libp2c_b200_profile.so"
 
 
