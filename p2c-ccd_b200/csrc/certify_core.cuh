@@ -114,15 +114,32 @@ P2C_HD double dist_point_segment(V3 p, V3 a, V3 b, C& c) {  // :82-90
   return dist_pp(p, vadd(a, vscale(ab, t)), c);
 }
 
+// A triangle of no area: the nearest of its three edges.  Out of line: rare,
+// and three inlined copies would push the common path out of the instruction
+// caches.
+template <class C>
+#ifdef __CUDA_ARCH__
+__noinline__
+#endif
+__host__ __device__ double dist_point_edges(V3 p, V3 a, V3 b, V3 cc, C& c) {
+  double m = dist_point_segment(p, a, b, c);
+  const double m1 = dist_point_segment(p, b, cc, c);
+  const double m2 = dist_point_segment(p, cc, a, c);
+  if (m1 < m) m = m1;  // std::min({...}) keeps the first smallest
+  if (m2 < m) m = m2;
+  return m;
+}
+
 // DistancePointTriangle, certificate_engine.cpp:133-184.  The Voronoi region
 // is found with the reference's tests, in its order, on the quantities it
 // computes; every region then ends in one of three forms: a vertex
 // (|p - v|), an edge (v = num / den, |p - (base + dir * v)|) or the face
-// (|dot(ap, n) / |n||).  Evaluating the tails after the region is known, one
-// form at a time, lets a warp whose lanes sit in different regions issue at
-// most one division and two square roots instead of one of each per region
-// present; every lane still performs exactly its region's operations, in the
-// reference's order, so the value is the same bit for bit.
+// (|dot(ap, n) / |n||).  All six projections and three minors are formed
+// without branches and the region is chosen by selects: a warp's lanes sit in
+// several regions anyway, so branches only add divergence (a warp runs one
+// division and two square roots per sample either way).  Every lane still
+// performs its region's operations in the reference's order, so the value is
+// the same bit for bit; the census counts only those.
 template <class C>
 P2C_HD double dist_point_triangle(V3 p, V3 a, V3 b, V3 cc, C& c) {
   const V3 ab = vsub(b, a);
@@ -130,85 +147,44 @@ P2C_HD double dist_point_triangle(V3 p, V3 a, V3 b, V3 cc, C& c) {
   const V3 n = vcross(ab, ac);
   c.add(20);
   const double nn2 = vdot(n, n);
-  if (nn2 <= kNumEps) {
-    double m = dist_point_segment(p, a, b, c);
-    const double m1 = dist_point_segment(p, b, cc, c);
-    const double m2 = dist_point_segment(p, cc, a, c);
-    if (m1 < m) m = m1;  // std::min({...}) keeps the first smallest
-    if (m2 < m) m = m2;
-    return m;
-  }
-  const V3 ap = vsub(p, a);
-  const double d1 = vdot(ab, ap);
-  const double d2 = vdot(ac, ap);
-  c.add(13);
-  int form;  // 0 vertex, 1 edge, 2 face
-  V3 base = a, dir = ab;
-  double num = 0.0, den = 1.0;
-  if (d1 <= 0.0 && d2 <= 0.0) {
-    form = 0;  // vertex a
-  } else {
-    const V3 bp = vsub(p, b);
-    const double d3 = vdot(ab, bp);
-    const double d4 = vdot(ac, bp);
-    c.add(13);
-    if (d3 >= 0.0 && d4 <= d3) {
-      form = 0;  // vertex b
-      base = b;
-    } else {
-      const double vc = sub(mul(d1, d4), mul(d3, d2));
-      c.add(3);
-      if (vc <= 0.0 && d1 >= 0.0 && d3 <= 0.0) {
-        form = 1;  // edge ab: v = d1 / (d1 - d3)
-        num = d1;
-        den = sub(d1, d3);
-        c.add(8);
-      } else {
-        const V3 cp = vsub(p, cc);
-        const double d5 = vdot(ab, cp);
-        const double d6 = vdot(ac, cp);
-        c.add(13);
-        if (d6 >= 0.0 && d5 <= d6) {
-          form = 0;  // vertex c
-          base = cc;
-        } else {
-          const double vb = sub(mul(d5, d2), mul(d1, d6));
-          c.add(3);
-          if (vb <= 0.0 && d2 >= 0.0 && d6 <= 0.0) {
-            form = 1;  // edge ac: w = d2 / (d2 - d6)
-            dir = ac;
-            num = d2;
-            den = sub(d2, d6);
-            c.add(8);
-          } else {
-            const double va = sub(mul(d3, d6), mul(d5, d4));
-            const double d43 = sub(d4, d3);
-            const double d56 = sub(d5, d6);
-            c.add(5);
-            if (va <= 0.0 && d43 >= 0.0 && d56 >= 0.0) {
-              form = 1;  // edge bc: w = d43 / (d43 + d56), from b along c - b
-              base = b;
-              dir = vsub(cc, b);
-              num = d43;
-              den = add(d43, d56);
-              c.add(11);
-            } else {
-              form = 2;  // face: dot(ap, n) / |n|
-              c.add(12);
-            }
-          }
-        }
-      }
-    }
-  }
-  if (form == 2) {
+  if (nn2 <= kNumEps) return dist_point_edges(p, a, b, cc, c);
+  const V3 ap = vsub(p, a), bp = vsub(p, b), cp = vsub(p, cc);
+  const double d1 = vdot(ab, ap), d2 = vdot(ac, ap);
+  const double d3 = vdot(ab, bp), d4 = vdot(ac, bp);
+  const double d5 = vdot(ab, cp), d6 = vdot(ac, cp);
+  const double vc = sub(mul(d1, d4), mul(d3, d2));
+  const double vb = sub(mul(d5, d2), mul(d1, d6));
+  const double va = sub(mul(d3, d6), mul(d5, d4));
+  const double d43 = sub(d4, d3), d56 = sub(d5, d6);
+  const bool at_a = d1 <= 0.0 && d2 <= 0.0;
+  const bool at_b = !at_a && d3 >= 0.0 && d4 <= d3;
+  const bool on_ab = !at_a && !at_b && vc <= 0.0 && d1 >= 0.0 && d3 <= 0.0;  // v = d1 / (d1 - d3)
+  const bool before_c = at_a || at_b || on_ab;
+  const bool at_c = !before_c && d6 >= 0.0 && d5 <= d6;
+  const bool on_ac = !before_c && !at_c && vb <= 0.0 && d2 >= 0.0 && d6 <= 0.0;  // w = d2 / (d2 - d6)
+  const bool before_bc = before_c || at_c || on_ac;
+  const bool on_bc = !before_bc && va <= 0.0 && d43 >= 0.0 && d56 >= 0.0;  // w = d43 / (d43 + d56), along c - b
+  const bool face = !before_bc && !on_bc;
+  const bool edge = on_ab || on_ac || on_bc;
+  // operations of the region, as the branches of the reference would run them
+  c.add(13 + (at_a ? 0 : 13 + (at_b ? 0 : 3 + (on_ab ? 8 : 13 + (at_c ? 0 : 3 + (on_ac ? 8 : 5 + (on_bc ? 11 : 12)))))));
+  double num = on_ab ? d1 : (on_ac ? d2 : d43);
+  double den = on_bc ? add(d43, d56) : sub(num, on_ab ? d3 : d6);
+  if (face) {
     num = vdot(ap, n);
     den = sqrt_rn(nn2);
   }
   double v = 0.0;
-  if (form != 0) v = dvd(num, den);
-  if (form == 2) return fabs(v);
-  const V3 q = form == 1 ? vadd(base, vscale(dir, v)) : base;
+  if (edge || face) v = dvd(num, den);
+  if (face) return fabs(v);
+  const bool from_b = at_b || on_bc;
+  const V3 base = {at_c ? cc.x : (from_b ? b.x : a.x), at_c ? cc.y : (from_b ? b.y : a.y),
+                   at_c ? cc.z : (from_b ? b.z : a.z)};
+  V3 q = base;
+  if (edge) {
+    const V3 head = {on_ab ? b.x : cc.x, on_ab ? b.y : cc.y, on_ab ? b.z : cc.z};
+    q = vadd(base, vscale(vsub(head, base), v));  // head - base is ab, ac or c - b
+  }
   c.add(9);
   const V3 d = vsub(p, q);
   return sqrt_rn(vdot(d, d));
@@ -225,35 +201,31 @@ P2C_HD double dist_segment_segment(V3 p1, V3 q1, V3 p2, V3 q2, C& c) {
   const double f = vdot(d2, r);
   c.add(24);
   double s = 0.0, t = 0.0;
-  if (a <= kNumEps && e <= kNumEps) return dist_pp(p1, p2, c);
-  if (a <= kNumEps) {
-    t = clamp_std(dvd(f, e), 0.0, 1.0);
-    c.add(1);
-  } else {
-    const double cd = vdot(d1, r);
-    c.add(5);
-    if (e <= kNumEps) {
-      s = clamp_std(dvd(-cd, a), 0.0, 1.0);
+  if (a <= kNumEps || e <= kNumEps) {  // a point, or two
+    if (a <= kNumEps && e <= kNumEps) return dist_pp(p1, p2, c);
+    if (a <= kNumEps) {
+      t = clamp_std(dvd(f, e), 0.0, 1.0);
       c.add(1);
     } else {
-      const double b = vdot(d1, d2);
-      const double denom = sub(mul(a, e), mul(b, b));
-      c.add(8);
-      if (denom != 0.0) {
-        s = clamp_std(dvd(sub(mul(b, f), mul(cd, e)), denom), 0.0, 1.0);
-        c.add(4);
-      }
-      t = dvd(add(mul(b, s), f), e);
-      c.add(3);
-      if (t < 0.0) {
-        t = 0.0;
-        s = clamp_std(dvd(-cd, a), 0.0, 1.0);
-        c.add(1);
-      } else if (t > 1.0) {
-        t = 1.0;
-        s = clamp_std(dvd(sub(b, cd), a), 0.0, 1.0);
-        c.add(2);
-      }
+      s = clamp_std(dvd(-vdot(d1, r), a), 0.0, 1.0);
+      c.add(6);
+    }
+  } else {
+    const double cd = vdot(d1, r);
+    const double b = vdot(d1, d2);
+    const double denom = sub(mul(a, e), mul(b, b));
+    c.add(13);
+    if (denom != 0.0) {
+      s = clamp_std(dvd(sub(mul(b, f), mul(cd, e)), denom), 0.0, 1.0);
+      c.add(4);
+    }
+    t = dvd(add(mul(b, s), f), e);
+    c.add(3);
+    const bool below = t < 0.0;
+    if (below || t > 1.0) {  // one division for both ends
+      t = below ? 0.0 : 1.0;
+      s = clamp_std(dvd(below ? -cd : sub(b, cd), a), 0.0, 1.0);
+      c.add(below ? 1 : 2);
     }
   }
   c.add(12);
@@ -346,6 +318,7 @@ __device__ __forceinline__ void replay(double T0, double T1, unsigned long long 
   }
   a = T0;
   b = T1;
+#pragma unroll 1
   for (int l = 1; l <= depth; ++l) {
     const double m = mul(0.5, add(a, b));
     if ((path >> (64 - l)) & 1ull) a = m;
@@ -406,7 +379,7 @@ struct CertParams {
 
 // Counters of one warp's loop (warp-uniform).
 struct WarpStats {
-  unsigned nodes = 0, evals = 0, donations = 0, queries = 0, iters = 0, busy = 0;
+  unsigned nodes = 0, donations = 0, queries = 0, iters = 0;
 };
 
 // Counters of the census launch (per thread).
@@ -423,6 +396,7 @@ __device__ __forceinline__ T pick(const T (&a)[2], int f) {
 }
 
 __device__ __forceinline__ int nth_set_bit(unsigned m, int r) {
+#pragma unroll 1
   for (int i = 0; i < r; ++i) m &= m - 1u;
   return __ffs((int)m) - 1;
 }

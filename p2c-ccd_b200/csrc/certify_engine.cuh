@@ -34,15 +34,22 @@
 // record, and the last one writes the result.  Nodes right of a known
 // collision are pruned: the recursion never reaches them.
 //
-// Bound by issue and by dependent FP64 chains, not by memory (128 x 128 cloth
-// certification: 750 instructions per 32 nodes, DRAM idle, 4 warps per
-// scheduler).  Against the engine that tied a lane to a subtree and handed
-// subtrees between lanes (one sample, then donation, per iteration), on a
-// B200: two 40,960-triangle spheres 75 -> 33 us (12 iterations on the longest
-// warp instead of 27), 20,000 plain queries 365 -> 190 us, a 60,000-triangle
-// cloth's 295,000 self candidates 780 -> 470 us, 64 uneven scenes 283 -> 200 us.
-// Idle warps hold a ticket each and poll their own pool entry: with one shared
-// head that they advanced by compare-and-swap the 20,000 queries took 1,200 us.
+// Bound by instruction issue and the latency of dependent FP64 chains, not by
+// memory: on a 624k-triangle cloth's edge-edge trees 600 instructions per 32
+// nodes, 57 % of the issue slots and 37 % of the FP64 pipe busy, DRAM idle, four
+// warps per scheduler (128 registers).  So a full iteration has a path of its
+// own without the groups' bookkeeping, the sample is one out-of-line function
+// for both paths, and all warps work on one family at a time: the code is 67 KB,
+// and instruction fetch stalls cost up to 20 % otherwise.  Against the engine
+// that tied a lane to a subtree and handed subtrees between lanes, on a B200:
+// two 40,960-triangle spheres 75 -> 33 us (12 iterations on the longest warp
+// instead of 27), 20,000 plain queries 365 -> 180 us, a 60,000-triangle cloth's
+// 295,000 self candidates 780 -> 420 us, a 624k-triangle cloth's 1.9 M any-hit
+// certificates 10.3 -> 8.5 ms, 64 uneven scenes 283 -> 190 us.  Idle warps hold a
+// ticket each and poll their own pool entry: with one shared head that they
+// advanced by compare-and-swap the 20,000 queries took 1,200 us.  A bracket of
+// the distance in single precision that spared 95 % of the FP64 samples made
+// the loop longer, not shorter (cloth 445 -> 690 us), and was dropped.
 //
 // No wait in this engine is unbounded: every loop checks the launch's device
 // time budget (CertParams::budget_ns); on expiry the engine returns false and
@@ -213,6 +220,7 @@ struct EngineShared {
   double p0[12][kSlots];
   double p1[12][kSlots];
   double nrm[4][kSlots];                 // motion norms (MotionRadius factors)
+  double rate[2][kSlots];                // the two that the radius takes, once the largest are chosen
   double T0[kSlots], T1[kSlots];
   unsigned long long coll_key[kSlots];   // leftmost collision leaf known to this warp (~0: none)
   unsigned long long margin[kSlots];     // min separation margin (bits); a colliding root's time of impact
@@ -224,7 +232,7 @@ struct EngineShared {
   int batch[32];                         // slots of the roots fetched together
   unsigned long long nkey[kStack];       // stack: leaf keys (path and depth), intervals, slots
   double nt0[kStack], nt1[kStack];
-  unsigned char nslot[kStack];
+  unsigned short nmeta[kStack];          // slot | depth << 8
 };
 
 constexpr unsigned long long kRootKey = 1ull << 63;  // leaf_key of the root
@@ -241,6 +249,8 @@ __device__ __forceinline__ void fill_slot(EngineShared& sh, int s, const Geo& g,
   motion_norms(SlotGeo<EngineShared>{sh, s}, nrm, nc);
 #pragma unroll
   for (int i = 0; i < 4; ++i) sh.nrm[i][s] = nrm[i];
+  sh.rate[0][s] = family == 1 ? nrm[0] : max_std(nrm[0], nrm[1]);
+  sh.rate[1][s] = family == 1 ? max_std(max_std(nrm[1], nrm[2]), nrm[3]) : max_std(nrm[2], nrm[3]);
   sh.T0[s] = T0;
   sh.T1[s] = T1;
   sh.coll_key[s] = coll_key;
@@ -250,6 +260,58 @@ __device__ __forceinline__ void fill_slot(EngineShared& sh, int s, const Geo& g,
   sh.undecided[s] = 0;
   sh.outstanding[s] = 1;
   sh.gidx[s] = gidx;
+}
+
+// Motion radius of slot s over [t0, t1].  A product with a positive half width
+// rounds monotonically, so the largest of the reference's products is the
+// product with the largest norm, bit for bit; a zero half width (a zero-width
+// root) takes the reference's own order, which an infinite norm can tell apart.
+__device__ __forceinline__ double slot_radius(const EngineShared& sh, int s, double t0, double t1) {
+  const double h = mul(0.5, max_std(0.0, sub(t1, t0)));
+  if (h > 0.0) return add(mul(h, sh.rate[0][s]), mul(h, sh.rate[1][s]));
+  NoCount ops;
+  const double nrm[4] = {sh.nrm[0][s], sh.nrm[1][s], sh.nrm[2][s], sh.nrm[3][s]};
+  return sh.family[s] == 1 ? motion_radius<1>(nrm, t0, t1, ops) : motion_radius<2>(nrm, t0, t1, ops);
+}
+
+// One FP64 sample.  Out of line: inlined into both paths of the loop it cost
+// 15 % where both families are certified.
+static __device__ __noinline__ double slot_distance(const EngineShared& sh, int s, int family, double t) {
+  NoCount ops;
+  const SlotGeo<EngineShared> g{sh, s};
+  return family == 1 ? distance_at<1>(g, t, ops) : distance_at<2>(g, t, ops);
+}
+
+// A node goes to stack entry e.
+__device__ __forceinline__ void put_node(EngineShared& sh, unsigned e, unsigned long long key, double t0, double t1,
+                                         int slot, int depth) {
+  e &= kStack - 1u;
+  sh.nkey[e] = key;
+  sh.nt0[e] = t0;
+  sh.nt1[e] = t1;
+  sh.nmeta[e] = (unsigned short)(slot | (depth << 8));
+}
+
+// Both children of a split node, the left one on top.
+__device__ __forceinline__ void push_children(EngineShared& sh, unsigned e, unsigned long long key, double t0,
+                                              double mid, double t1, int slot, int depth) {
+  const unsigned long long half = (1ull << 62) >> depth;  // the sentinel bit of the children
+  put_node(sh, e, key + half, mid, t1, slot, depth + 1);
+  put_node(sh, e + 1u, key - half, t0, mid, slot, depth + 1);
+}
+
+// A leaf joins its tree's reduction here: a collision, a separation's margin.
+__device__ __forceinline__ void record_collision(EngineShared& sh, int slot, unsigned long long key,
+                                                 const EnginePools& pools) {
+  if (key < sh.coll_key[slot]) {
+    atomicMin(&sh.coll_key[slot], key);
+    const int gi = sh.gidx[slot];
+    if (gi >= 0) atomicMin(&pools.aggs[gi].coll_key, key);
+  }
+}
+__device__ __forceinline__ void record_margin(EngineShared& sh, int slot, double margin) {
+  const unsigned long long mb = (unsigned long long)__double_as_longlong(margin);
+  if (mb < sh.margin[slot]) atomicMin(&sh.margin[slot], mb);
 }
 
 // The tree's result from its reduction.
@@ -280,7 +342,7 @@ __device__ __forceinline__ Outcome tree_outcome(unsigned long long coll_key, uns
 //   void finish(int family, long long q, const Outcome&) const;
 //   void invalid(int family, long long q, int bad, double T0, double T1) const;
 template <bool kExport, class P>
-__device__ bool run_engine(const P& prob, const CertParams& prm, int fetch1, int fetch2, bool ee_first,
+__device__ bool run_engine(const P& prob, const CertParams& prm, int fetch1, int fetch2,
                            EngineShared& sh, WarpStats& st, EngineState* es, const EnginePools& pools,
                            unsigned long long t_start) {
   const unsigned FULL = 0xffffffffu;
@@ -291,7 +353,10 @@ __device__ bool run_engine(const P& prob, const CertParams& prm, int fetch1, int
 
   unsigned top = 0u, bottom = 0u;          // stack [bottom, top), indices modulo kStack
   unsigned free_mask = kSlots == 32 ? FULL : (1u << kSlots) - 1u;
-  int cur = ee_first ? 2 : 1;              // family whose queue this warp drains
+  // Family whose queue this warp drains: edge-edge, then vertex-face, the same
+  // on every warp, so that the instruction caches hold one family's sample at a
+  // time (odd warps starting with the other family cost 6 % on a cloth's two queues).
+  int cur = 2;
   unsigned exhausted = (n1 == 0 ? 1u : 0u) | (n2 == 0 ? 2u : 0u);  // bit f-1: family f's queue is empty
   bool helper = false;                     // this warp is counted in es->helpers
   bool waiting = false;                    // this warp holds the ticket of a pool entry
@@ -349,11 +414,8 @@ __device__ bool run_engine(const P& prob, const CertParams& prm, int fetch1, int
       published = volatile_load(&es->task_reserve.v);
       tickets = volatile_load(&es->task_head.v);
     }
-    // This iteration's groups: `width` lanes per node (or root) hold it and
-    // its next levels in heap order (h = 1 the node, 2h and 2h + 1 its
-    // children); a root's group ends in two lanes for its endpoints (h = 0).
-    int levels = 1, width = 1, groups = 0;
     bool roots = false;
+    int fetched = 0;
     // ---- (A) new queries from the per-family queues -------------------------
     if (size < 32u && exhausted != 3u) {
       if (exhausted & (1u << (cur - 1))) cur = 3 - cur;
@@ -397,11 +459,9 @@ __device__ bool run_engine(const P& prob, const CertParams& prm, int fetch1, int
         free_mask &= ~__reduce_or_sync(FULL, fresh ? (1u << s) : 0u);
         if (fresh) sh.batch[__popc(got & lt_mask)] = s;
         __syncwarp();
-        groups = __popc(got);
-        st.queries += (unsigned)groups;
+        fetched = __popc(got);
+        st.queries += (unsigned)fetched;
         roots = true;
-        levels = groups == 1 ? 4 : (groups <= 3 ? 3 : (groups <= 6 ? 2 : 1));
-        width = (1 << levels) + 1;
       }
     }
     P2C_PROF_MARK(0)
@@ -449,10 +509,7 @@ __device__ bool run_engine(const P& prob, const CertParams& prm, int fetch1, int
           fill_slot(sh, 0, g, T0, T1, f, q, volatile_load(&pools.aggs[gi].coll_key), gi);
           const int d = 64 - __ffsll((long long)key);
           replay(T0, T1, key & ~(1ull << (63 - d)), d, a, b);
-          sh.nkey[0] = key;
-          sh.nt0[0] = a;
-          sh.nt1[0] = b;
-          sh.nslot[0] = 0;
+          put_node(sh, 0u, key, a, b, 0, d);
         }
         free_mask &= ~1u;
         bottom = 0u;
@@ -461,149 +518,173 @@ __device__ bool run_engine(const P& prob, const CertParams& prm, int fetch1, int
         P2C_PROF_MARK(2)
         continue;
       }
-      // ---- (C) pop nodes; with few of them, whole groups of descendants -----
-      groups = (int)min(size, 32u);
-      if (size <= 10u) levels = size == 1u ? 5 : (size == 2u ? 4 : (size <= 4u ? 3 : 2));
-      else groups = max(1, min(groups, (int)(kStack - 64u) - (int)size));  // room for a depth-first descent
-      width = (1 << levels) - 1;
-      top -= (unsigned)groups;
     }
     P2C_PROF_COUNT(11)
-    const int group = width == 1 ? lane : (int)((unsigned)(lane * (65536 / width + 1)) >> 16);
-    const int first = group * width;  // lane of the group's node
-    const bool in = group < groups;
-    int h = lane - first + 1, slot = 0;
-    if (roots && h >= width - 1) h = h == width ? -1 : 0;  // endpoints t1 (-1) and t0 (0)
-    unsigned long long key = kRootKey;
-    double t0 = 0.0, t1 = 0.0;
-    if (in) {
-      if (roots) {
-        slot = sh.batch[group];
-        t0 = sh.T0[slot];
-        t1 = sh.T1[slot];
-      } else {
-        const unsigned e = (top + (unsigned)(groups - 1 - group)) & (kStack - 1u);  // group 0 is the topmost
-        slot = sh.nslot[e];
+    st.iters += 1u;
+    const double eps_space = prm.eps_space;
+    if (!roots && size > 10u) {
+      // ---- (C) up to 32 nodes, one per lane -----------------------------------------
+      const int count = max(1, min((int)min(size, 32u), (int)(kStack - 64u) - (int)size));  // room for a descent
+      top -= (unsigned)count;
+      const bool in = lane < count;
+      int slot = 0, depth = 0;
+      unsigned long long key = 0;
+      double t0 = 0.0, t1 = 0.0;
+      if (in) {
+        const unsigned e = (top + (unsigned)(count - 1 - lane)) & (kStack - 1u);  // lane 0 takes the topmost
+        const unsigned meta = sh.nmeta[e];
+        slot = (int)(meta & 0xffu);
+        depth = (int)(meta >> 8);
         key = sh.nkey[e];
         t0 = sh.nt0[e];
         t1 = sh.nt1[e];
       }
-    }
-    // a node right of a known collision is never needed
-    const bool eval = in && !(sh.coll_key[slot] < key);
-    double mid = mul(0.5, add(t0, t1));
-    for (int b = 30 - __clz(max(h, 1)); b >= 0; --b) {  // down to this lane's descendant
-      const unsigned long long half = (key & (0ull - key)) >> 1;
-      if ((h >> b) & 1) {
-        t0 = mid;
-        key += half;
-      } else {
-        t1 = mid;
-        key -= half;
-      }
-      mid = mul(0.5, add(t0, t1));
-    }
-    const int fam = sh.family[slot];
-    P2C_PROF_MARK(1)
-    // ---- (D) one distance sample per lane ------------------------------------
-    double d = 0.0;
-    if (eval) {
-      NoCount ops;
-      const double t = h > 0 ? mid : (h == 0 ? t0 : t1);
-      const SlotGeo<EngineShared> g{sh, slot};
-      d = fam == 1 ? distance_at<1>(g, t, ops) : distance_at<2>(g, t, ops);
-    }
-    P2C_PROF_MARK(4)
-    // ---- (E) classify: 0 none, 1 collision, 2 separation, 3 undecided ---------
-    const double eps_space = prm.eps_space;
-    const bool hit = eval && d <= eps_space;
-    int leaf = 0;
-    double margin = 0.0;
-    bool split = false, root_hit = false;
-    if (roots) {
-      const unsigned hits = __ballot_sync(FULL, hit);
-      if (eval && h == 1) {
-        const bool hit0 = (hits >> (first + width - 2)) & 1u, hit1 = (hits >> (first + width - 1)) & 1u;
-        if (hit0 || hit || hit1) {  // the root is the only node; its time of impact is the first hit of t0, mid, t1
-          root_hit = true;
-          sh.coll_key[slot] = kRootKey;
-          sh.margin[slot] = (unsigned long long)__double_as_longlong(hit0 ? t0 : (hit ? mid : t1));
-        }
-      }
-    }
-    if (eval && h > 0 && !root_hit) {
-      if (hit) {
-        leaf = 1;
-      } else {
-        NoCount ops;
-        const double nrm[4] = {sh.nrm[0][slot], sh.nrm[1][slot], sh.nrm[2][slot], sh.nrm[3][slot]};
-        const double lb = sub(d, fam == 1 ? motion_radius<1>(nrm, t0, t1, ops) : motion_radius<2>(nrm, t0, t1, ops));
-        if (lb > eps_space) {
-          leaf = 2;
-          margin = max_std(0.0, sub(lb, eps_space));
-        } else if (64 - __ffsll((long long)key) >= prm.max_depth || sub(t1, t0) <= prm.eps_time) {
-          leaf = 3;
+      const double mid = mul(0.5, add(t0, t1));
+      P2C_PROF_MARK(1)
+      bool split = false;
+      const bool eval = in && !(sh.coll_key[slot] < key);  // a node right of a known collision is never needed
+      if (eval) {
+        const double d = slot_distance(sh, slot, sh.family[slot], mid);
+        if (d <= eps_space) {
+          record_collision(sh, slot, key, pools);
         } else {
-          split = true;
+          const double lb = sub(d, slot_radius(sh, slot, t0, t1));
+          if (lb > eps_space) record_margin(sh, slot, max_std(0.0, sub(lb, eps_space)));
+          else if (depth >= prm.max_depth || sub(t1, t0) <= prm.eps_time) sh.undecided[slot] = 1;
+          else split = true;
         }
       }
-    }
-    bool reached = eval && h > 0;
-    if (levels > 1) {
-      const unsigned splits = __ballot_sync(FULL, split);
-      for (int a = h >> 1; a > 0; a >>= 1) reached = reached && ((splits >> (first + a - 1)) & 1u);
-    }
-    const unsigned reached_mask = __ballot_sync(FULL, reached);
-    st.iters += 1u;
-    st.busy += (unsigned)__popc(reached_mask);
-    st.nodes += (unsigned)__popc(reached_mask);
-    st.evals += (unsigned)__popc(reached_mask) + (roots ? 2u * (unsigned)groups : 0u);
-    P2C_PROF_MARK(5)
-    // ---- (F) record leaves ------------------------------------------------------
-    if (reached && leaf != 0) {
-      if (leaf == 1) {
-        if (key < sh.coll_key[slot]) {
-          atomicMin(&sh.coll_key[slot], key);
-          const int gi = sh.gidx[slot];
-          if (gi >= 0) atomicMin(&pools.aggs[gi].coll_key, key);
-        }
-      } else if (leaf == 2) {
-        const unsigned long long mb = (unsigned long long)__double_as_longlong(margin);
-        if (mb < sh.margin[slot]) atomicMin(&sh.margin[slot], mb);
+      P2C_PROF_MARK(4)
+      const unsigned pushers = __ballot_sync(FULL, split);
+      st.nodes += (unsigned)__popc(__ballot_sync(FULL, eval));
+      if (split)
+        push_children(sh, top + 2u * (unsigned)__popc(pushers & (0xfffffffeu << lane)), key, t0, mid, t1, slot, depth);
+      top += 2u * (unsigned)__popc(pushers);
+      P2C_PROF_MARK(7)
+      const unsigned same = __match_any_sync(FULL, in ? slot : -1);
+      bool done = false;
+      if (in && (same & lt_mask) == 0u) {  // one lane per query
+        const int left = sh.outstanding[slot] + 2 * __popc(pushers & same) - __popc(same);
+        sh.outstanding[slot] = left;
+        done = left == 0;
+      }
+      if (__any_sync(FULL, done)) done_mask |= __reduce_or_sync(FULL, done ? 1u << slot : 0u);
+      __syncwarp();
+    } else {
+      // ---- (D) roots, or a few nodes with their descendants: groups of lanes --------
+      int levels, groups;
+      if (roots) {
+        groups = fetched;
+        levels = groups == 1 ? 4 : (groups <= 3 ? 3 : (groups <= 6 ? 2 : 1));
       } else {
-        sh.undecided[slot] = 1;
+        groups = (int)size;
+        levels = size == 1u ? 5 : (size == 2u ? 4 : (size <= 4u ? 3 : 2));
+        top -= size;
       }
+      const int width = (1 << levels) + (roots ? 1 : -1);
+      const int group = (int)((unsigned)(lane * (65536 / width + 1)) >> 16);
+      const int first = group * width;  // lane of the group's node
+      const bool in = group < groups;
+      int h = lane - first + 1, slot = 0, depth = 0;
+      if (roots && h >= width - 1) h = h == width ? -1 : 0;  // endpoints t1 (-1) and t0 (0)
+      unsigned long long key = kRootKey;
+      double t0 = 0.0, t1 = 0.0;
+      if (in) {
+        if (roots) {
+          slot = sh.batch[group];
+          t0 = sh.T0[slot];
+          t1 = sh.T1[slot];
+        } else {
+          const unsigned e = (top + (unsigned)(groups - 1 - group)) & (kStack - 1u);  // group 0 is the topmost
+          const unsigned meta = sh.nmeta[e];
+          slot = (int)(meta & 0xffu);
+          depth = (int)(meta >> 8);
+          key = sh.nkey[e];
+          t0 = sh.nt0[e];
+          t1 = sh.nt1[e];
+        }
+      }
+      const bool eval = in && !(sh.coll_key[slot] < key);
+      double mid = mul(0.5, add(t0, t1));
+#pragma unroll 1
+      for (int b = 30 - __clz(max(h, 1)); b >= 0; --b) {  // down to this lane's descendant
+        const unsigned long long half = depth < 63 ? (1ull << 62) >> depth : 0ull;
+        depth += 1;
+        if ((h >> b) & 1) {
+          t0 = mid;
+          key += half;
+        } else {
+          t1 = mid;
+          key -= half;
+        }
+        mid = mul(0.5, add(t0, t1));
+      }
+      P2C_PROF_MARK(1)
+      double d = 0.0;
+      if (eval) d = slot_distance(sh, slot, sh.family[slot], h > 0 ? mid : (h == 0 ? t0 : t1));
+      P2C_PROF_MARK(4)
+      // classify: 0 none, 1 collision, 2 separation, 3 undecided
+      const bool hit = eval && d <= eps_space;
+      int leaf = 0;
+      double margin = 0.0;
+      bool split = false, root_hit = false;
+      if (roots) {
+        const unsigned hits = __ballot_sync(FULL, hit);
+        if (eval && h == 1) {
+          const bool hit0 = (hits >> (first + width - 2)) & 1u, hit1 = (hits >> (first + width - 1)) & 1u;
+          if (hit0 || hit || hit1) {  // the root is the only node; its time of impact is the first hit of t0, mid, t1
+            root_hit = true;
+            sh.coll_key[slot] = kRootKey;
+            sh.margin[slot] = (unsigned long long)__double_as_longlong(hit0 ? t0 : (hit ? mid : t1));
+          }
+        }
+      }
+      if (eval && h > 0 && !root_hit) {
+        if (hit) {
+          leaf = 1;
+        } else {
+          const double lb = sub(d, slot_radius(sh, slot, t0, t1));
+          if (lb > eps_space) {
+            leaf = 2;
+            margin = max_std(0.0, sub(lb, eps_space));
+          } else if (depth >= prm.max_depth || sub(t1, t0) <= prm.eps_time) {
+            leaf = 3;
+          } else {
+            split = true;
+          }
+        }
+      }
+      bool reached = eval && h > 0;
+      if (levels > 1) {
+        const unsigned splits = __ballot_sync(FULL, split);
+#pragma unroll 1
+        for (int a = h >> 1; a > 0; a >>= 1) reached = reached && ((splits >> (first + a - 1)) & 1u);
+      }
+      st.nodes += (unsigned)__popc(__ballot_sync(FULL, reached));
+      P2C_PROF_MARK(5)
+      if (reached) {
+        if (leaf == 1) record_collision(sh, slot, key, pools);
+        else if (leaf == 2) record_margin(sh, slot, margin);
+        else if (leaf == 3) sh.undecided[slot] = 1;
+      }
+      P2C_PROF_MARK(6)
+      const bool push = reached && split && h >= (1 << (levels - 1));
+      const unsigned pushers = __ballot_sync(FULL, push);
+      if (push)
+        push_children(sh, top + 2u * (unsigned)__popc(pushers & (0xfffffffeu << lane)), key, t0, mid, t1, slot, depth);
+      top += 2u * (unsigned)__popc(pushers);
+      P2C_PROF_MARK(7)
+      const unsigned same = __match_any_sync(FULL, in ? slot : -1);
+      const unsigned popped = __ballot_sync(FULL, in && lane == first);
+      unsigned done = 0u;
+      if (in && (same & lt_mask) == 0u) {  // one lane per query
+        const int left = sh.outstanding[slot] + 2 * __popc(pushers & same) - __popc(popped & same);
+        sh.outstanding[slot] = left;
+        if (left == 0) done = 1u << slot;
+      }
+      done_mask |= __reduce_or_sync(FULL, done);
+      __syncwarp();
     }
-    P2C_PROF_MARK(6)
-    // ---- (G) push the children of split nodes, the leftmost on top ----------------
-    const bool push = reached && split && h >= (1 << (levels - 1));
-    const unsigned pushers = __ballot_sync(FULL, push);
-    if (push) {
-      const unsigned e = top + 2u * (unsigned)__popc(pushers & ~lt_mask & ~(1u << lane));  // pairs of the lanes above
-      const unsigned r = e & (kStack - 1u), l = (e + 1u) & (kStack - 1u);
-      const unsigned long long half = (key & (0ull - key)) >> 1;
-      sh.nkey[r] = key + half;
-      sh.nt0[r] = mid;
-      sh.nt1[r] = t1;
-      sh.nslot[r] = (unsigned char)slot;
-      sh.nkey[l] = key - half;
-      sh.nt0[l] = t0;
-      sh.nt1[l] = mid;
-      sh.nslot[l] = (unsigned char)slot;
-    }
-    top += 2u * (unsigned)__popc(pushers);
-    P2C_PROF_MARK(7)
-    // ---- (H) a tree whose last node here is done is finished ----------------------
-    const unsigned same = __match_any_sync(FULL, in ? slot : -1);
-    const unsigned popped = __ballot_sync(FULL, in && lane == first);
-    unsigned done = 0u;
-    if (in && (same & lt_mask) == 0u) {  // one lane per query
-      const int left = sh.outstanding[slot] + 2 * __popc(pushers & same) - __popc(popped & same);
-      sh.outstanding[slot] = left;
-      if (left == 0) done = 1u << slot;
-    }
-    done_mask |= __reduce_or_sync(FULL, done);
-    __syncwarp();
     // ---- (I) publish the shallowest nodes to hungry warps ---------------------------
     // Waiting warps hold the tickets past the published count.  Only what one
     // iteration cannot take is given away, at most P2C_EXPORT_LANES nodes per
@@ -615,7 +696,7 @@ __device__ bool run_engine(const P& prob, const CertParams& prm, int fetch1, int
       if (__any_sync(FULL, give)) {  // the lanes' reads of the counters may differ
         int count = min(max((int)(top - bottom) - P2C_EXPORT_ABOVE, 0), P2C_EXPORT_LANES);
         const unsigned e = (bottom + (unsigned)lane) & (kStack - 1u);
-        const int es_slot = lane < count ? (int)sh.nslot[e] : -1;
+        const int es_slot = lane < count ? (int)(sh.nmeta[e] & 0xffu) : -1;
         unsigned mine = __match_any_sync(FULL, es_slot);
         const bool lead = lane < count && (mine & lt_mask) == 0u;
         // a tree's first published node moves its reduction to a pooled record
@@ -656,6 +737,7 @@ __device__ bool run_engine(const P& prob, const CertParams& prm, int fetch1, int
         if (lane < count) {
           SubtreeTask* tk = pools.tasks + ((task + (unsigned long long)lane) & (pools.task_cap - 1ull));
           // the taker of the ring's previous lap has long read the entry; wait for it all the same
+#pragma unroll 1
           for (unsigned spin = 0; volatile_load(&tk->tag) != 0ull; ++spin) {
             __nanosleep(64);
             if ((spin & 255u) == 255u && prm.budget_ns != 0ull && (global_ns() - t_start) > prm.budget_ns) break;

@@ -131,9 +131,9 @@ __device__ __forceinline__ void add_stat(uint64_t* p, unsigned long long v) {
 __device__ __forceinline__ void flush_stats(const WarpStats& st, bool ok, CertifyScratch* sc) {
   if ((threadIdx.x & 31) != 0) return;
   if (st.iters) atomicMax((unsigned long long*)&sc->stats.max_warp_iterations, (unsigned long long)st.iters);
-  add_stat(&sc->stats.busy_lane_iterations, st.busy);
+  add_stat(&sc->stats.busy_lane_iterations, st.nodes);
   add_stat(&sc->stats.nodes_evaluated, st.nodes);
-  add_stat(&sc->stats.distance_evals, st.evals);
+  add_stat(&sc->stats.distance_evals, (unsigned long long)st.nodes + 2ull * st.queries);  // a root takes three
   add_stat(&sc->stats.donations, st.donations);
   add_stat(&sc->stats.queries, st.queries);
   if (!ok) atomicOr((unsigned long long*)&sc->stats.error_word, 1ull);

@@ -93,10 +93,9 @@ __global__ void __launch_bounds__(kCertifyThreads, kCertifyMinBlocks)
   EngineShared& sh = reinterpret_cast<EngineShared*>(smem_raw)[threadIdx.x >> 5];
   WarpStats st;
   const unsigned long long t_start = global_ns();
-  const bool ee_first = ((blockIdx.x * kCertifyWarps + (threadIdx.x >> 5)) & 1u) != 0u;
   // no cross-warp pools here: the scratch stays one record per work item
   const EnginePools no_pools{};
-  const bool ok = run_engine<false>(prob, prm, fetch_pt, fetch_ee, ee_first, sh, st, &sc->engine,
+  const bool ok = run_engine<false>(prob, prm, fetch_pt, fetch_ee, sh, st, &sc->engine,
                                                  no_pools, t_start);
   flush_stats(st, ok, sc);
 }
