@@ -9,10 +9,11 @@
 // until the first hit.  Here both phases run on the persistent certifier:
 //
 //   1. prep: group id and a descending score key per candidate, group sizes;
-//   2. two stable radix sorts order the candidates by (group, score desc,
-//      index) and a scan of the group sizes gives every candidate its rank;
-//   3. a third stable sort by min(rank, K) lays the proposals out rank-major
-//      (all groups' first proposals, then all second ones, ...);
+//   2. the K best candidates of each group by (score desc, index) get their
+//      ranks (anyhit_order.cuh); nothing reads a rank past K;
+//   3. the proposals are laid out rank-major (all groups' first proposals,
+//      then all second ones, ...).  K above kPickRanks: three stable radix
+//      sorts of all candidates give ranks and layout instead;
 //   4. the engine certifies the proposals in that order; a hit lowers its
 //      group's minimum hit rank, and a proposal behind a known hit is dropped
 //      before it is evaluated (ones already running finish as speculation);
@@ -29,9 +30,11 @@
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 #include <cub/device/device_select.cuh>
+#include <thrust/iterator/counting_iterator.h>
 
 #include <algorithm>
 
+#include "anyhit_order.cuh"
 #include "certify_core.cuh"
 #include "certify_launch.cuh"
 #include "scene_pairs.cuh"
@@ -63,11 +66,11 @@ struct AnyhitLayout {
   unsigned* grp = nullptr;
   unsigned* rank = nullptr;
   unsigned char* state = nullptr;
-  unsigned char* flags = nullptr;
   unsigned long long* skey[2] = {nullptr, nullptr};
   unsigned* val[2] = {nullptr, nullptr};
   unsigned* key32[2] = {nullptr, nullptr};
   unsigned* fb_list = nullptr;
+  OrderSpace order;
   unsigned* g_size = nullptr;
   unsigned* g_start = nullptr;
   unsigned* g_min_hit = nullptr;
@@ -76,6 +79,18 @@ struct AnyhitLayout {
   void* tmp = nullptr;
   size_t tmp_bytes = 0;
   size_t total = 0;
+};
+
+// Fallback candidates: not a proposal, in a group without a proposal hit.
+struct IsFallback {
+  const unsigned long long* count;
+  const unsigned *grp, *rank, *min_hit;
+  unsigned groups, K;
+  __device__ __forceinline__ bool operator()(unsigned c) const {
+    if ((unsigned long long)c >= *count) return false;
+    const unsigned g = grp[c];
+    return g < groups && rank[c] >= K && min_hit[g] == kNone;
+  }
 };
 
 size_t cub_temp_bytes(long long cap, long long groups) {
@@ -87,8 +102,8 @@ size_t cub_temp_bytes(long long cap, long long groups) {
                                   (unsigned*)nullptr, n);
   cub::DeviceScan::ExclusiveSum(nullptr, c, (const unsigned*)nullptr, (unsigned*)nullptr,
                                 (int)std::max(groups, 1ll));
-  cub::DeviceSelect::Flagged(nullptr, d, (const unsigned*)nullptr, (const unsigned char*)nullptr,
-                             (unsigned*)nullptr, (int*)nullptr, n);
+  cub::DeviceSelect::If(nullptr, d, thrust::counting_iterator<unsigned>(0u), (unsigned*)nullptr, (int*)nullptr, n,
+                        IsFallback{});
   return std::max(std::max(a, b), std::max(c, d));
 }
 
@@ -107,7 +122,6 @@ AnyhitLayout carve(void* base, long long cap, long long groups) {
   L.grp = static_cast<unsigned*>(take(n * 4));
   L.rank = static_cast<unsigned*>(take(n * 4));
   L.state = static_cast<unsigned char*>(take(n));
-  L.flags = static_cast<unsigned char*>(take(n));
   L.skey[0] = static_cast<unsigned long long*>(take(n * 8));
   L.skey[1] = static_cast<unsigned long long*>(take(n * 8));
   L.val[0] = static_cast<unsigned*>(take(n * 4));
@@ -120,9 +134,21 @@ AnyhitLayout carve(void* base, long long cap, long long groups) {
   L.g_min_hit = static_cast<unsigned*>(take(g * 4));
   L.g_min_fb = static_cast<unsigned*>(take(g * 4));
   L.g_fcalls = static_cast<unsigned long long*>(take(g * 8));
+  carve_order(L.order, cap, groups, 1, take);
   L.tmp_bytes = cub_temp_bytes(cap, groups);
   L.tmp = take(L.tmp_bytes);
   L.total = off;
+  // the full sorts and the selection never run in one call: they share their buffers
+  L.order.grp = L.grp;
+  L.order.key = L.skey[0];
+  L.order.rank = L.rank;
+  L.order.g_size = L.g_size;
+  L.order.hist = L.key32[0];
+  L.order.hist_words = (unsigned)n;
+  L.order.ent_key = L.skey[1];
+  L.order.ent_idx = L.val[0];
+  L.order.list = L.val[1];
+  L.order.n_top = &L.ctr->n_top;
   return L;
 }
 
@@ -151,13 +177,6 @@ __device__ __forceinline__ unsigned long long score_key_desc(double s, bool& nan
   return ~asc;
 }
 
-// Adds 1 to table[key] for every active lane, one atomic per distinct key.
-__device__ __forceinline__ void warp_count(unsigned* table, unsigned key, bool active) {
-  const unsigned act = __activemask();
-  const unsigned m = __match_any_sync(act, active ? key : kNone);
-  if (active && (threadIdx.x & 31) == __ffs((int)m) - 1) atomicAdd(table + key, (unsigned)__popc(m));
-}
-
 __global__ void init_kernel(AnyhitLayout L, long long groups, p2c_anyhit_summary* summary) {
   const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (g < groups) {
@@ -170,36 +189,61 @@ __global__ void init_kernel(AnyhitLayout L, long long groups, p2c_anyhit_summary
     *L.ctr = AnyhitCounters{};
     if (summary != nullptr) *summary = p2c_anyhit_summary{};
   }
+  order_reset(L.order, g, (long long)gridDim.x * blockDim.x);
 }
 
-__global__ void prep_kernel(ScenePairs sp, long long n_a, long long n_b, const int32_t* obj_a, const int32_t* obj_b,
-                            int n_obj, const double* scores, const unsigned long long* count, long long cap,
-                            AnyhitLayout L) {
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= cap) return;
+// Group and key of every candidate, group sizes.  A block takes a span of
+// consecutive candidates: pairs are sorted, so most of a span is one group
+// and its count is one atomic (per-warp atomics on one group's counter were
+// most of this kernel's time: 222 -> 66 us for 7.6 M candidates of 54 groups).
+// fill (the full sorts): slots past the count get the last key.
+__global__ void __launch_bounds__(kOrderThreads)
+    prep_kernel(ScenePairs sp, long long n_a, long long n_b, const int32_t* obj_a, const int32_t* obj_b, int n_obj,
+                const double* scores, const unsigned long long* count, long long cap, bool fill, AnyhitLayout L) {
+  constexpr int kEach = kOrderSpan / kOrderThreads;
+  __shared__ unsigned main_group, sum;
   const long long n = candidate_count(count, cap);
+  const long long end = fill ? cap : n;
   const unsigned groups = (unsigned)n_obj * (unsigned)n_obj;
-  unsigned g = groups;
-  unsigned long long key = ~0ull;
-  if (c < n) {
-    const unsigned long long pair = sp.pairs[c];
-    const long long a = (long long)(pair >> 32), b = (long long)(pair & 0xffffffffull);
-    const int oa = a < n_a ? __ldg(obj_a + a) : -1, ob = b < n_b ? __ldg(obj_b + b) : -1;
-    if (oa >= 0 && ob >= 0 && oa < n_obj && ob < n_obj) {
-      const unsigned lo = (unsigned)min(oa, ob), hi = (unsigned)max(oa, ob);
-      g = lo * (unsigned)n_obj + hi;
-      bool nan = false;
-      key = score_key_desc(scores[c], nan);
-      if (nan) atomicOr(&L.ctr->error_word, 16ull);
-    } else {
-      atomicOr(&L.ctr->error_word, 8ull);
+  for (long long base = (long long)blockIdx.x * kOrderSpan; base < end; base += (long long)gridDim.x * kOrderSpan) {
+    unsigned g[kEach];
+#pragma unroll
+    for (int i = 0; i < kEach; ++i) {
+      const long long c = base + i * kOrderThreads + threadIdx.x;
+      g[i] = groups;
+      if (c >= end) continue;
+      unsigned long long key = ~0ull;
+      if (c < n) {
+        const unsigned long long pair = sp.pairs[c];
+        const long long a = (long long)(pair >> 32), b = (long long)(pair & 0xffffffffull);
+        const int oa = a < n_a ? __ldg(obj_a + a) : -1, ob = b < n_b ? __ldg(obj_b + b) : -1;
+        if (oa >= 0 && ob >= 0 && oa < n_obj && ob < n_obj) {
+          const unsigned lo = (unsigned)min(oa, ob), hi = (unsigned)max(oa, ob);
+          g[i] = lo * (unsigned)n_obj + hi;
+          bool nan = false;
+          key = score_key_desc(scores[c], nan);
+          if (nan) atomicOr(&L.ctr->error_word, 16ull);
+        } else {
+          atomicOr(&L.ctr->error_word, 8ull);
+        }
+      }
+      L.grp[c] = g[i];
+      L.rank[c] = kNone;
+      L.state[c] = 0;
+      L.skey[0][c] = key;
+      if (fill) L.val[0][c] = (unsigned)c;
     }
+    if (threadIdx.x == 0) {
+      main_group = g[0];
+      sum = 0u;
+    }
+    __syncthreads();
+    SpanCount counter(main_group);
+#pragma unroll
+    for (int i = 0; i < kEach; ++i) counter.add(L.order, g[i]);
+    counter.finish(L.order, &sum);
+    __syncthreads();
   }
-  L.grp[c] = g;
-  L.state[c] = 0;
-  L.skey[0][c] = key;
-  L.val[0][c] = (unsigned)c;
-  warp_count(L.g_size, g, g < groups);
 }
 
 __global__ void group_key_kernel(long long cap, AnyhitLayout L) {
@@ -225,21 +269,6 @@ __global__ void rank_kernel(long long cap, unsigned groups, unsigned K, AnyhitLa
   const unsigned top = __ballot_sync(act, g < groups && r < K);
   if ((threadIdx.x & 31) == __ffs((int)act) - 1 && top != 0u)
     atomicAdd(&L.ctr->n_top, (unsigned long long)__popc(top));
-}
-
-// Fallback candidates: not a proposal, in a group without a proposal hit.
-__global__ void fallback_flags_kernel(const unsigned long long* count, long long cap, unsigned groups, unsigned K,
-                                      AnyhitLayout L) {
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= cap) return;
-  const long long n = candidate_count(count, cap);
-  bool f = false;
-  if (c < n) {
-    const unsigned g = L.grp[c];
-    f = g < groups && L.rank[c] >= K && L.g_min_hit[g] == kNone;
-  }
-  L.flags[c] = f ? 1 : 0;
-  L.key32[0][c] = (unsigned)c;
 }
 
 // One phase of the any-hit as an engine problem over a work list of
@@ -390,14 +419,26 @@ int launch_group_anyhit(const p2c_scene& scene, int family, const unsigned long 
   const int* obj_b = family == 1 ? scene.f_obj : scene.e_obj;
   ScenePairs sp{scene.v_t0, scene.v_t1, scene.faces, scene.edges, pairs, T0, T1};
 
+  int rc = P2C_OK;
   P2C_CUDA(reset_scratch(L.sc, s, true));
   init_kernel<<<grid_for(groups, kThreads), kThreads, 0, s>>>(L, groups, summary);
   P2C_CUDA(cudaGetLastError());
+  // K up to kPickRanks: selection (2.5 M edge-edge candidates of a 624k-triangle cloth,
+  // K = 4096: 270 us against 632 for the sorts); above, a group's proposals may not fit
+  // one block.
+  const bool sorts = K > kPickRanks;
   if (cap > 0) {
     const long long n_a = family == 1 ? scene.nv : scene.ne, n_b = family == 1 ? scene.nf : scene.ne;
-    prep_kernel<<<grid_for(cap, kThreads), kThreads, 0, s>>>(sp, n_a, n_b, obj_a, obj_b, scene.n_obj, scores, count,
-                                                             cap, L);
+    const unsigned spans = (unsigned)((cap + kOrderSpan - 1) / kOrderSpan);
+    prep_kernel<<<spans, kOrderThreads, 0, s>>>(sp, n_a, n_b, obj_a, obj_b, scene.n_obj, scores, count, cap, sorts, L);
     P2C_CUDA(cudaGetLastError());
+  }
+  if (cap > 0 && K > 0 && !sorts) {
+    L.order.K = K;
+    rc = launch_order(L.order, count, nullptr, s);
+    if (rc != P2C_OK) return rc;
+  }
+  if (cap > 0 && sorts) {
     size_t tb = L.tmp_bytes;
     // (score desc, index): stable over the index order of the input
     P2C_CUDA(cub::DeviceRadixSort::SortPairs(L.tmp, tb, L.skey[0], L.skey[1], L.val[0], L.val[1], (int)cap, 0, 64,
@@ -412,26 +453,26 @@ int launch_group_anyhit(const p2c_scene& scene, int family, const unsigned long 
     P2C_CUDA(cub::DeviceScan::ExclusiveSum(L.tmp, tb, L.g_size, L.g_start, (int)groups, s));
     rank_kernel<<<grid_for(cap, kThreads), kThreads, 0, s>>>(cap, G, K, L);
     P2C_CUDA(cudaGetLastError());
+    // proposals rank-major: (rank, group, score desc, index)
+    tb = L.tmp_bytes;
+    P2C_CUDA(cub::DeviceRadixSort::SortPairs(L.tmp, tb, L.key32[0], L.key32[1], L.val[0], L.val[1], (int)cap, 0,
+                                             bit_width(K), s));
   }
   LaunchShape shape;
-  int rc = certify_shape(anyhit_certify_kernel, &shape);
+  rc = certify_shape(anyhit_certify_kernel, &shape);
   if (rc != P2C_OK) return rc;
   const CertParams prm = make_params(cfg, shape, 32ll * shape.grid * kCertifyWarps);
   if (cap > 0 && K > 0) {
-    // proposals rank-major: (rank, group, score desc, index)
-    size_t tb = L.tmp_bytes;
-    P2C_CUDA(cub::DeviceRadixSort::SortPairs(L.tmp, tb, L.key32[0], L.key32[1], L.val[0], L.val[1], (int)cap, 0,
-                                             bit_width(K), s));
     const AnyhitProblem prop{sp, family, L.val[1], &L.ctr->n_top, nullptr, L.grp, L.rank, L.g_min_hit, L.state,
                              &L.ctr->error_word};
     anyhit_certify_kernel<<<shape.grid, kCertifyThreads, shape.smem, s>>>(prop, prm, pools_at(L.sc), L.sc);
     P2C_CUDA(cudaGetLastError());
   }
   if (cap > 0) {
-    fallback_flags_kernel<<<grid_for(cap, kThreads), kThreads, 0, s>>>(count, cap, G, K, L);
-    P2C_CUDA(cudaGetLastError());
     size_t tb = L.tmp_bytes;
-    P2C_CUDA(cub::DeviceSelect::Flagged(L.tmp, tb, L.key32[0], L.flags, L.fb_list, &L.ctr->fb_count, (int)cap, s));
+    const IsFallback is_fallback{count, L.grp, L.rank, L.g_min_hit, G, K};
+    P2C_CUDA(cub::DeviceSelect::If(L.tmp, tb, thrust::counting_iterator<unsigned>(0u), L.fb_list, &L.ctr->fb_count,
+                                   (int)cap, is_fallback, s));
     P2C_CUDA(reset_engine(L.sc, s));
     const AnyhitProblem fb{sp, family, L.fb_list, nullptr, &L.ctr->fb_count, L.grp, nullptr, L.g_min_fb, L.state,
                            &L.ctr->error_word};

@@ -8,22 +8,25 @@
 // the scene and family added to the key), so groups of different scenes
 // never mix and every scene gets exactly the calls, hits and groups it gets
 // alone.  The candidates of all scenes form one index space, segment
-// k = family_index * n_scenes + scene; the group and score sorts, the ranks,
-// the two certification phases and the call recovery run once over it (about
-// twenty launches whatever the number of scenes), and each segment gets its
-// own p2c_anyhit_summary.
+// k = family_index * n_scenes + scene; the choice of proposals and their
+// ranks (anyhit_order.cuh; three full sorts above kPickRanks proposals a
+// group), the two certification phases and the call recovery run once over it
+// (about twenty launches whatever the number of scenes), and each segment
+// gets its own p2c_anyhit_summary.
 //
-// Proposals are sorted rank-major with the family as the top key bit, so the
-// point-triangle proposals precede the edge-edge ones and the engine reads
-// them as its two queues (it picks the distance function by queue family).
+// Proposals lie rank-major, point-triangle ones before edge-edge ones, and
+// the engine reads them as its two queues (it picks the distance function by
+// queue family).
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 #include <cub/device/device_select.cuh>
 #include <cub/block/block_scan.cuh>
+#include <thrust/iterator/counting_iterator.h>
 
 #include <algorithm>
 #include <vector>
 
+#include "anyhit_order.cuh"
 #include "certify_core.cuh"
 #include "certify_launch.cuh"
 #include "scene_pairs.cuh"
@@ -60,11 +63,11 @@ struct Layout {
   unsigned* grp = nullptr;
   unsigned* rank = nullptr;
   unsigned char* state = nullptr;
-  unsigned char* flags = nullptr;
   unsigned long long* skey[2] = {nullptr, nullptr};
   unsigned* val[2] = {nullptr, nullptr};
   unsigned* key32[2] = {nullptr, nullptr};
   unsigned* fb_list = nullptr;
+  OrderSpace order;
   unsigned* g_size = nullptr;
   unsigned* g_start = nullptr;
   unsigned* g_min_hit = nullptr;
@@ -73,6 +76,16 @@ struct Layout {
   void* tmp = nullptr;
   size_t tmp_bytes = 0;
   size_t total = 0;
+};
+
+// Fallback candidates: not a proposal, in a group without a proposal hit.
+struct IsFallback {
+  const unsigned *grp, *rank, *min_hit;
+  unsigned groups, K;
+  __device__ __forceinline__ bool operator()(unsigned c) const {
+    const unsigned g = grp[c];
+    return g < groups && rank[c] >= K && min_hit[g] == kNone;
+  }
 };
 
 size_t cub_temp_bytes(long long cap, long long groups) {
@@ -84,12 +97,12 @@ size_t cub_temp_bytes(long long cap, long long groups) {
                                   (unsigned*)nullptr, n);
   cub::DeviceScan::ExclusiveSum(nullptr, c, (const unsigned*)nullptr, (unsigned*)nullptr,
                                 (int)std::max(groups, 1ll));
-  cub::DeviceSelect::Flagged(nullptr, d, (const unsigned*)nullptr, (const unsigned char*)nullptr,
-                             (unsigned*)nullptr, (int*)nullptr, n);
+  cub::DeviceSelect::If(nullptr, d, thrust::counting_iterator<unsigned>(0u), (unsigned*)nullptr, (int*)nullptr, n,
+                        IsFallback{});
   return std::max(std::max(a, b), std::max(c, d));
 }
 
-Layout carve(void* base, int n_scenes, long long cap, long long groups) {
+Layout carve(void* base, int n_scenes, long long cap, long long cap_vf, long long groups) {
   Layout L;
   size_t off = 0;
   char* b = static_cast<char*>(base);
@@ -109,7 +122,6 @@ Layout carve(void* base, int n_scenes, long long cap, long long groups) {
   L.grp = static_cast<unsigned*>(take(n * 4));
   L.rank = static_cast<unsigned*>(take(n * 4));
   L.state = static_cast<unsigned char*>(take(n));
-  L.flags = static_cast<unsigned char*>(take(n));
   L.skey[0] = static_cast<unsigned long long*>(take(n * 8));
   L.skey[1] = static_cast<unsigned long long*>(take(n * 8));
   L.val[0] = static_cast<unsigned*>(take(n * 4));
@@ -122,9 +134,22 @@ Layout carve(void* base, int n_scenes, long long cap, long long groups) {
   L.g_min_hit = static_cast<unsigned*>(take(g * 4));
   L.g_min_fb = static_cast<unsigned*>(take(g * 4));
   L.g_fcalls = static_cast<unsigned long long*>(take(g * 8));
+  carve_order(L.order, cap, groups, 2, take);
   L.tmp_bytes = cub_temp_bytes(cap, groups);
   L.tmp = take(L.tmp_bytes);
   L.total = off;
+  // the full sorts and the selection never run in one call: they share their buffers
+  L.order.grp = L.grp;
+  L.order.key = L.skey[0];
+  L.order.rank = L.rank;
+  L.order.g_size = L.g_size;
+  L.order.hist = L.key32[0];
+  L.order.hist_words = (unsigned)n;
+  L.order.ent_key = L.skey[1];
+  L.order.ent_idx = L.val[0];
+  L.order.list = L.val[1];
+  L.order.n_top = L.ctr->n_top;
+  L.order.cap_first = cap_vf;
   return L;
 }
 
@@ -228,6 +253,7 @@ __global__ void init_groups_kernel(Layout L, long long groups, p2c_anyhit_summar
   }
   if (summaries != nullptr)
     for (long long i = g; i < 2ll * n; i += (long long)gridDim.x * blockDim.x) summaries[i] = p2c_anyhit_summary{};
+  order_reset(L.order, g, (long long)gridDim.x * blockDim.x);
 }
 
 // Last segment k with off[k] <= v (segments may be empty).
@@ -250,49 +276,64 @@ __device__ __forceinline__ unsigned long long score_key_desc(double s, bool& nan
   return ~asc;
 }
 
-__device__ __forceinline__ void warp_count(unsigned* table, unsigned key, bool active) {
-  const unsigned act = __activemask();
-  const unsigned m = __match_any_sync(act, active ? key : kNone);
-  if (active && (threadIdx.x & 31) == __ffs((int)m) - 1) atomicAdd(table + key, (unsigned)__popc(m));
-}
-
-// Per candidate: segment, group, descending score key; group sizes.
-__global__ void prep_kernel(const p2c_batch_scene* scenes, int n, unsigned mask, const double* const* scores,
-                            const unsigned long long* seeds, long long cap, unsigned long long groups, Layout L) {
+// Per candidate: segment, group, descending score key; group sizes.  A block
+// takes a span of consecutive candidates: pairs are sorted, so most of a span
+// is one group and its count is one atomic.
+__global__ void __launch_bounds__(kOrderThreads)
+    prep_kernel(const p2c_batch_scene* scenes, int n, unsigned mask, const double* const* scores,
+                const unsigned long long* seeds, long long cap, unsigned groups, bool fill, Layout L) {
+  constexpr int kEach = kOrderSpan / kOrderThreads;
+  __shared__ unsigned main_group, sum;
   const int k_total = 2 * n;
-  for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < cap;
-       c += (long long)gridDim.x * blockDim.x) {
-    const int k = find_seg(L.cand_off, k_total, (unsigned long long)c);
-    const int f = k < n ? 0 : 1, s = k < n ? k : k - n;
-    const p2c_batch_scene& d = scenes[s];
-    const long long local = c - (long long)__ldg(L.cand_off + k);
-    unsigned g = (unsigned)groups;
-    unsigned long long key = ~0ull;
-    if (local < seg_count(d, f, mask)) {
-      const unsigned long long pair = (f == 0 ? d.vf_pairs : d.ee_pairs)[local];
-      const long long a = (long long)(pair >> 32), b = (long long)(pair & 0xffffffffull);
-      const long long n_a = f == 0 ? d.nv : d.ne, n_b = f == 0 ? d.nf : d.ne;
-      const int* obj_a = f == 0 ? d.v_obj : d.e_obj;
-      const int* obj_b = f == 0 ? d.f_obj : d.e_obj;
-      const int oa = a < n_a ? __ldg(obj_a + a) : -1, ob = b < n_b ? __ldg(obj_b + b) : -1;
-      if (oa >= 0 && ob >= 0 && oa < d.n_obj && ob < d.n_obj) {
-        const unsigned lo = (unsigned)min(oa, ob), hi = (unsigned)max(oa, ob);
-        g = (unsigned)__ldg(L.group_off + k) + lo * (unsigned)d.n_obj + hi;
-        const double sc = scores != nullptr ? scores[2 * s + f][local]
-                                            : stub_score(seeds != nullptr ? seeds[s] : 0ull, f + 1, pair);
-        bool nan = false;
-        key = score_key_desc(sc, nan);
-        if (nan) atomicOr(L.seg_err + k, 16ull);
-      } else {
-        atomicOr(L.seg_err + k, 8ull);
+  for (long long base = (long long)blockIdx.x * kOrderSpan; base < cap; base += (long long)gridDim.x * kOrderSpan) {
+    unsigned g[kEach];
+    int k = find_seg(L.cand_off, k_total, (unsigned long long)base);
+#pragma unroll
+    for (int i = 0; i < kEach; ++i) {
+      const long long c = base + i * kOrderThreads + threadIdx.x;
+      g[i] = groups;
+      if (c >= cap) continue;
+      while (k + 1 < k_total && __ldg(L.cand_off + k + 1) <= (unsigned long long)c) ++k;  // last segment at or before c
+      const int f = k < n ? 0 : 1, s = k < n ? k : k - n;
+      const p2c_batch_scene& d = scenes[s];
+      const long long local = c - (long long)__ldg(L.cand_off + k);
+      unsigned long long key = ~0ull;
+      if (local < seg_count(d, f, mask)) {
+        const unsigned long long pair = (f == 0 ? d.vf_pairs : d.ee_pairs)[local];
+        const long long a = (long long)(pair >> 32), b = (long long)(pair & 0xffffffffull);
+        const long long n_a = f == 0 ? d.nv : d.ne, n_b = f == 0 ? d.nf : d.ne;
+        const int* obj_a = f == 0 ? d.v_obj : d.e_obj;
+        const int* obj_b = f == 0 ? d.f_obj : d.e_obj;
+        const int oa = a < n_a ? __ldg(obj_a + a) : -1, ob = b < n_b ? __ldg(obj_b + b) : -1;
+        if (oa >= 0 && ob >= 0 && oa < d.n_obj && ob < d.n_obj) {
+          const unsigned lo = (unsigned)min(oa, ob), hi = (unsigned)max(oa, ob);
+          g[i] = (unsigned)__ldg(L.group_off + k) + lo * (unsigned)d.n_obj + hi;
+          const double sc = scores != nullptr ? scores[2 * s + f][local]
+                                              : stub_score(seeds != nullptr ? seeds[s] : 0ull, f + 1, pair);
+          bool nan = false;
+          key = score_key_desc(sc, nan);
+          if (nan) atomicOr(L.seg_err + k, 16ull);
+        } else {
+          atomicOr(L.seg_err + k, 8ull);
+        }
       }
+      L.seg[c] = (unsigned)k;
+      L.grp[c] = g[i];
+      L.rank[c] = kNone;
+      L.state[c] = 0;
+      L.skey[0][c] = key;
+      if (fill) L.val[0][c] = (unsigned)c;
     }
-    L.seg[c] = (unsigned)k;
-    L.grp[c] = g;
-    L.state[c] = 0;
-    L.skey[0][c] = key;
-    L.val[0][c] = (unsigned)c;
-    warp_count(L.g_size, g, g < (unsigned)groups);
+    if (threadIdx.x == 0) {
+      main_group = g[0];
+      sum = 0u;
+    }
+    __syncthreads();
+    SpanCount counter(main_group);
+#pragma unroll
+    for (int i = 0; i < kEach; ++i) counter.add(L.order, g[i]);
+    counter.finish(L.order, &sum);
+    __syncthreads();
   }
 }
 
@@ -326,18 +367,21 @@ __global__ void rank_kernel(long long cap, long long cap_vf, unsigned groups, un
   }
 }
 
-// Fallback candidates: not a proposal, in a group without a proposal hit.
-__global__ void fallback_flags_kernel(long long cap, long long cap_vf, unsigned groups, unsigned K, Layout L) {
-  for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < cap;
-       c += (long long)gridDim.x * blockDim.x) {
-    const unsigned g = L.grp[c];
-    const bool f = g < groups && L.rank[c] >= K && L.g_min_hit[g] == kNone;
-    L.flags[c] = f ? 1 : 0;
-    L.key32[0][c] = (unsigned)c;
-    const unsigned act = __activemask();
-    const unsigned m = __ballot_sync(act, f && c < cap_vf);
-    if ((threadIdx.x & 31) == __ffs((int)act) - 1 && m) atomicAdd(&L.ctr->n_fb_vf, (unsigned long long)__popc(m));
+// Fallback candidates of family 1: the list is in index order, one warp
+// searches it 32 ways at a time.
+__global__ void fallback_split_kernel(long long cap_vf, Layout L) {
+  const int n = L.ctr->fb_count, lane = threadIdx.x;
+  int lo = 0, len = n;  // the first entry at or past cap_vf lies in [lo, lo + len]
+  while (len > 0) {
+    const int step = (len + 31) / 32, at = lo + lane * step;
+    const bool before = at < lo + len && (long long)L.fb_list[at] < cap_vf;
+    const int m = __popc(__ballot_sync(0xffffffffu, before));  // a prefix of the lanes
+    if (m == 0) break;
+    const int next = lo + (m - 1) * step + 1;  // past the last entry known to lie before cap_vf
+    len = min(step - 1, lo + len - next);
+    lo = next;
   }
+  if (lane == 0) L.ctr->n_fb_vf = (unsigned long long)lo;
 }
 
 // One phase over a work list of candidate indices: family 1 entries first.
@@ -504,10 +548,10 @@ int launch_batch_anyhit(const p2c_batch_scene* h, const p2c_batch_scene* scenes,
   const Sizes z = sizes_of(h, n, mask);
   int rc = check_sizes(z);
   if (rc != P2C_OK) return rc;
-  const Layout need = carve(nullptr, n, z.cap, z.groups);
+  const Layout need = carve(nullptr, n, z.cap, z.cap_vf, z.groups);
   if (ws == nullptr || ws_bytes < need.total)
     return fail(P2C_ERR_INVALID, "batch any-hit workspace too small: %zu < %zu bytes", ws_bytes, need.total);
-  Layout L = carve(ws, n, z.cap, z.groups);
+  Layout L = carve(ws, n, z.cap, z.cap_vf, z.groups);
   const long long C = z.cap;
   const unsigned G = (unsigned)z.groups;
   const unsigned K = (unsigned)std::min<long long>(top_k, std::max(z.max_seg_cap, 0ll));
@@ -523,37 +567,50 @@ int launch_batch_anyhit(const p2c_batch_scene* h, const p2c_batch_scene* scenes,
   if (rc != P2C_OK) return rc;
   const CertParams prm = make_params(cfg, shape, 32ll * shape.grid * kCertifyWarps);
   if (C > 0) {
-    prep_kernel<<<grid_for(C, kThreads), kThreads, 0, s>>>(scenes, n, mask, scores, seeds, C, G, L);
+    // K up to kPickRanks: selection; above, a group's proposals may not fit one
+    // block (the line and both sides' times: groups.cu, one family of one scene)
+    const bool sorts = K > kPickRanks;
+    const unsigned spans = (unsigned)((C + kOrderSpan - 1) / kOrderSpan);
+    prep_kernel<<<spans, kOrderThreads, 0, s>>>(scenes, n, mask, scores, seeds, C, G, sorts, L);
     P2C_CUDA(cudaGetLastError());
     size_t tb = L.tmp_bytes;
-    // (score desc, index)
-    P2C_CUDA(cub::DeviceRadixSort::SortPairs(L.tmp, tb, L.skey[0], L.skey[1], L.val[0], L.val[1], (int)C, 0, 64, s));
-    group_key_kernel<<<grid_for(C, kThreads), kThreads, 0, s>>>(C, L);
-    P2C_CUDA(cudaGetLastError());
-    // (group, score desc, index)
-    tb = L.tmp_bytes;
-    P2C_CUDA(cub::DeviceRadixSort::SortPairs(L.tmp, tb, L.key32[0], L.key32[1], L.val[1], L.val[0], (int)C, 0,
-                                             std::max(1, bit_width(G)), s));
-    if (G > 0) {
+    if (sorts) {
+      // (score desc, index)
+      P2C_CUDA(cub::DeviceRadixSort::SortPairs(L.tmp, tb, L.skey[0], L.skey[1], L.val[0], L.val[1], (int)C, 0, 64,
+                                               s));
+      group_key_kernel<<<grid_for(C, kThreads), kThreads, 0, s>>>(C, L);
+      P2C_CUDA(cudaGetLastError());
+      // (group, score desc, index)
       tb = L.tmp_bytes;
-      P2C_CUDA(cub::DeviceScan::ExclusiveSum(L.tmp, tb, L.g_size, L.g_start, (int)G, s));
-    }
-    rank_kernel<<<grid_for(C, kThreads), kThreads, 0, s>>>(C, z.cap_vf, G, K, kbits, L);
-    P2C_CUDA(cudaGetLastError());
-    if (K > 0) {
+      P2C_CUDA(cub::DeviceRadixSort::SortPairs(L.tmp, tb, L.key32[0], L.key32[1], L.val[1], L.val[0], (int)C, 0,
+                                               std::max(1, bit_width(G)), s));
+      if (G > 0) {
+        tb = L.tmp_bytes;
+        P2C_CUDA(cub::DeviceScan::ExclusiveSum(L.tmp, tb, L.g_size, L.g_start, (int)G, s));
+      }
+      rank_kernel<<<grid_for(C, kThreads), kThreads, 0, s>>>(C, z.cap_vf, G, K, kbits, L);
+      P2C_CUDA(cudaGetLastError());
       // proposals: family-major, then rank-major: (family, rank, group, score desc, index)
       tb = L.tmp_bytes;
       P2C_CUDA(cub::DeviceRadixSort::SortPairs(L.tmp, tb, L.key32[0], L.key32[1], L.val[0], L.val[1], (int)C, 0,
                                                kbits + 1, s));
+    } else if (K > 0) {
+      L.order.K = K;
+      // the low word of the family-2 segments' first group
+      rc = launch_order(L.order, nullptr, reinterpret_cast<const unsigned*>(L.group_off + n), s);
+      if (rc != P2C_OK) return rc;
+    }
+    if (K > 0) {
       BatchAnyhitProblem prop{scenes, n, L.val[1], L.ctr->n_top, (unsigned long long)z.cap_vf, nullptr, nullptr,
                               L.seg, L.cand_off, L.grp, L.rank, L.g_min_hit, L.state, L.seg_err, T0, T1};
       batch_anyhit_certify_kernel<<<shape.grid, kCertifyThreads, shape.smem, s>>>(prop, prm, pools_at(L.sc), L.sc);
       P2C_CUDA(cudaGetLastError());
     }
-    fallback_flags_kernel<<<grid_for(C, kThreads), kThreads, 0, s>>>(C, z.cap_vf, G, K, L);
-    P2C_CUDA(cudaGetLastError());
     tb = L.tmp_bytes;
-    P2C_CUDA(cub::DeviceSelect::Flagged(L.tmp, tb, L.key32[0], L.flags, L.fb_list, &L.ctr->fb_count, (int)C, s));
+    P2C_CUDA(cub::DeviceSelect::If(L.tmp, tb, thrust::counting_iterator<unsigned>(0u), L.fb_list, &L.ctr->fb_count,
+                                   (int)C, IsFallback{L.grp, L.rank, L.g_min_hit, G, K}, s));
+    fallback_split_kernel<<<1, 32, 0, s>>>(z.cap_vf, L);
+    P2C_CUDA(cudaGetLastError());
     P2C_CUDA(reset_engine(L.sc, s));
     BatchAnyhitProblem fb{scenes, n, L.fb_list, nullptr, 0ull, &L.ctr->fb_count, &L.ctr->n_fb_vf,
                           L.seg, L.cand_off, L.grp, nullptr, L.g_min_fb, L.state, L.seg_err, T0, T1};
@@ -590,7 +647,7 @@ extern "C" {
 size_t p2c_batch_anyhit_workspace_bytes(const p2c_batch_scene* scenes_host, int32_t n_scenes, uint32_t family_mask) {
   if (scenes_host == nullptr || n_scenes < 1 || family_mask == 0u || family_mask > 3u) return 0;
   const p2c::Sizes z = p2c::sizes_of(scenes_host, n_scenes, family_mask);
-  return p2c::carve(nullptr, n_scenes, z.cap, z.groups).total;
+  return p2c::carve(nullptr, n_scenes, z.cap, z.cap_vf, z.groups).total;
 }
 
 int p2c_batch_anyhit(const p2c_batch_scene* scenes_host, const p2c_batch_scene* scenes_dev, int32_t n_scenes,
