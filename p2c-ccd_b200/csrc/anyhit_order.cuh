@@ -299,10 +299,7 @@ __global__ void __launch_bounds__(kOrderThreads) order_plan_kernel(OrderSpace o,
       const unsigned* bins = o.hist + ((size_t)d << o.bin_bits);
       unsigned sum = 0u;
 #pragma unroll 8
-      for (int b = 0; b < each; b += 4) {
-        const uint4 v = *reinterpret_cast<const uint4*>(bins + lane * each + b);
-        sum += v.x + v.y + v.z + v.w;
-      }
+      for (int b = 0; b < each; ++b) sum += bins[lane * each + b];
       const unsigned incl = warp_inclusive_sum(sum, lane);
       const int who = __ffs((int)__ballot_sync(0xffffffffu, incl >= o.K)) - 1;  // the group is larger than K
       unsigned below = __shfl_sync(0xffffffffu, incl - sum, who);

@@ -20,20 +20,23 @@
 // 1e-12) when cost_target is finite and positive, the contact interval
 // oracle_trace[:, 6:8] and the label oracle_trace[:, 0] > 0.5.
 //
-// Device layout: one thread per row parses and validates; two stable radix
-// sorts give the order; a gather writes the sorted costs and flags and the
-// group heads; one warp per group finds the stopping position with ballots
-// and folds the group's sums lane by lane in order.  The reference adds its
-// work totals one term at a time into double accumulators, so the totals
-// depend on the order of the additions: every term goes to a slot whose
-// position is its place in the reference's sequence (positive terms only;
-// empty slots are +0.0, which adds exactly nothing to a sum that starts at
-// +0.0 and only grows), the non-zero slots are compacted in order, and one
-// warp per total adds them in sequence from shared-memory tiles that the
-// rest of its block streams in.  Every total is therefore the reference's
-// to the bit.
+// Device layout: one thread per row parses, validates and writes the row's
+// 32-byte walk record; one stable radix sort by query id makes the groups
+// contiguous; each group orders its own rows by (priority desc, cost asc,
+// index) in shared memory (larger ones in tiles that are merged); one warp per
+// group finds the stopping position with ballots and folds the group's sums
+// row by row in order.  The reference adds its work totals one term at a time
+// into double accumulators, so the totals depend on the order of the
+// additions: every term goes to a slot whose position is its place in the
+// reference's sequence (empty slots are +0.0, which adds exactly nothing to a
+// sum that starts at +0.0 and only grows), the non-zero slots are compacted
+// in order, and each total is the exact left-to-right sum formed from
+// composable pieces (the ordered fold below).  Every total is therefore the
+// reference's to the bit.
+#include <cooperative_groups.h>
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_select.cuh>
+#include <thrust/iterator/counting_iterator.h>
 
 #include <cmath>
 
@@ -43,6 +46,13 @@ namespace p2c {
 namespace {
 
 constexpr int kThreads = 256;
+constexpr int kWarpRows = 256;    // rows a warp orders
+constexpr int kTileThreads = 512;
+constexpr unsigned kTileRows = 4096;  // rows a block orders
+constexpr int kFoldThreads = 512;
+constexpr int kFoldPerThread = 8;  // consecutive terms per thread
+constexpr int kFoldChunk = kFoldThreads * kFoldPerThread;
+constexpr int kFoldWarps = kFoldThreads / 32;
 constexpr unsigned char kColl = 1, kOverlap = 2, kHighUnc = 4;
 
 // Integer totals, in p2c_dense_group_stats order of the counters below.
@@ -68,6 +78,30 @@ struct DenseAcc {
   unsigned long long first_error;  // (row << 2) | kind; ~0 none
   int n_groups;                    // DeviceSelect's count of group heads
   int n_terms;                     // DeviceSelect's count of non-zero work terms
+  unsigned long long big;          // groups ordered in tiles (<< 32) and their rows
+  unsigned next[2];                // the next group to order, to walk
+  unsigned n_tiles;
+  unsigned longest;                // rows of the largest group ordered in tiles
+  unsigned fold_blocks[3];         // finished blocks of each total's chunk sums
+};
+
+// What the walk reads of one row: one 32-byte sector at a random place.
+struct __align__(16) WalkRow {
+  double full, narrow;  // PositiveCost(full, 1), PositiveCost(narrow, full)
+  unsigned long long flags, pad;
+};
+
+struct Tile {
+  unsigned start, len;
+};
+
+// One piece of kFoldChunk terms of a total: its sum (any order, to predict the
+// binade it is added in), that binade's last place, and the increments of the
+// running sum for an even and an odd one.
+struct FoldPieces {
+  double* sum[3];
+  int* ulp[3];
+  ulonglong2* inc[3];
 };
 
 struct DenseLayout {
@@ -75,15 +109,12 @@ struct DenseLayout {
   unsigned long long* key[2] = {nullptr, nullptr};   // sort A: priority desc | cost asc
   unsigned long long* qkey[2] = {nullptr, nullptr};  // sort B: query id
   unsigned* idx[3] = {nullptr, nullptr, nullptr};
-  double* full = nullptr;  // PositiveCost(full, 1), input order
-  double* narrow = nullptr;
-  unsigned char* flags = nullptr;
-  double* s_full = nullptr;  // sorted order
-  double* s_narrow = nullptr;
-  unsigned char* s_flags = nullptr;
-  unsigned char* head = nullptr;
-  unsigned* iota = nullptr;
+  WalkRow* rows = nullptr;  // input order
   unsigned* g_start = nullptr;
+  unsigned* big_at = nullptr;   // groups ordered in tiles: first row in the sequence of their rows
+  unsigned* big_start = nullptr;
+  Tile* tiles = nullptr;
+  FoldPieces pieces = {};
   double* terms = nullptr;    // 2n + n slots (2 per candidate + 1 per group at most)
   double* compact = nullptr;  // the non-zero terms, in order
   double* g_full = nullptr;   // per group: the summed full costs
@@ -93,17 +124,25 @@ struct DenseLayout {
   size_t total = 0;
 };
 
+// A row whose query id differs from the one before it.
+struct IsHead {
+  const unsigned long long* qid;
+  __device__ bool operator()(unsigned i) const { return i == 0u || qid[i] != qid[i - 1]; }
+};
+
 struct NonZeroTerm {
   __host__ __device__ bool operator()(double x) const { return x != 0.0; }
 };
+
+size_t fold_chunks(long long terms) { return (size_t)((terms + kFoldChunk - 1) / kFoldChunk); }
 
 size_t cub_bytes(long long n) {
   const int m = (int)(n > 0 ? n : 1);
   size_t a = 0, b = 0, c = 0;
   cub::DeviceRadixSort::SortPairs(nullptr, a, (const unsigned long long*)nullptr, (unsigned long long*)nullptr,
                                   (const unsigned*)nullptr, (unsigned*)nullptr, m);
-  cub::DeviceSelect::Flagged(nullptr, b, (const unsigned*)nullptr, (const unsigned char*)nullptr,
-                             (unsigned*)nullptr, (int*)nullptr, m);
+  cub::DeviceSelect::If(nullptr, b, thrust::counting_iterator<unsigned>(0u), (unsigned*)nullptr, (int*)nullptr, m,
+                        IsHead{});
   cub::DeviceSelect::If(nullptr, c, (const double*)nullptr, (double*)nullptr, (int*)nullptr, 3 * m, NonZeroTerm{});
   return std::max(a, std::max(b, c));
 }
@@ -123,15 +162,17 @@ DenseLayout carve(void* base, long long n) {
   for (auto& k : L.key) k = (unsigned long long*)take(8 * m);
   for (auto& k : L.qkey) k = (unsigned long long*)take(8 * m);
   for (auto& v : L.idx) v = (unsigned*)take(4 * m);
-  L.full = (double*)take(8 * m);
-  L.narrow = (double*)take(8 * m);
-  L.flags = (unsigned char*)take(m);
-  L.s_full = (double*)take(8 * m);
-  L.s_narrow = (double*)take(8 * m);
-  L.s_flags = (unsigned char*)take(m);
-  L.head = (unsigned char*)take(m);
-  L.iota = (unsigned*)take(4 * m);
+  L.rows = (WalkRow*)take(sizeof(WalkRow) * m);
   L.g_start = (unsigned*)take(4 * m);
+  L.big_at = (unsigned*)take(4 * (m / kWarpRows + 1));
+  L.big_start = (unsigned*)take(4 * (m / kWarpRows + 1));
+  L.tiles = (Tile*)take(sizeof(Tile) * (m / kWarpRows + 1));
+  for (int k = 0; k < 3; ++k) {
+    const size_t c = fold_chunks(k == 0 ? 3 * (long long)m : (long long)m);
+    L.pieces.sum[k] = (double*)take(8 * c);
+    L.pieces.ulp[k] = (int*)take(4 * c);
+    L.pieces.inc[k] = (ulonglong2*)take(16 * c);
+  }
   L.terms = (double*)take(8 * 3 * m);
   L.compact = (double*)take(8 * 3 * m);
   L.g_full = (double*)take(8 * m);
@@ -164,10 +205,15 @@ struct ParseIn {
 
 __global__ void init_kernel(DenseLayout L) {
   if (threadIdx.x < kNumCounters) L.acc->ctr[threadIdx.x] = 0;
+  if (threadIdx.x < 3) L.acc->fold_blocks[threadIdx.x] = 0;
   if (threadIdx.x == 0) {
     L.acc->first_error = ~0ull;
     L.acc->n_groups = 0;
     L.acc->n_terms = 0;
+    L.acc->big = 0;
+    L.acc->next[0] = L.acc->next[1] = 0;
+    L.acc->n_tiles = 0;
+    L.acc->longest = 0;
   }
 }
 
@@ -212,120 +258,353 @@ __global__ void __launch_bounds__(kThreads) parse_kernel(ParseIn in, long long n
     kind = 2;
   if (kind) atomicMin(&L.acc->first_error, ((unsigned long long)i << 2) | kind);
   const double fc = positive_cost(full, 1.0);
-  L.full[i] = fc;
-  L.narrow[i] = positive_cost(narrow, fc);
   const double lo = it0 < c0 ? c0 : it0;  // std::max(interval_t0, contact_t0)
   const double hi = c1 < it1 ? c1 : it1;  // std::min(interval_t1, contact_t1)
-  L.flags[i] = (unsigned char)((tr[0] > 0.5 ? kColl : 0) | (lo <= hi ? kOverlap : 0) |
-                               (unc >= threshold ? kHighUnc : 0));
+  WalkRow row;
+  row.full = fc;
+  row.narrow = positive_cost(narrow, fc);
+  row.flags = (tr[0] > 0.5 ? kColl : 0) | (lo <= hi ? kOverlap : 0) | (unc >= threshold ? kHighUnc : 0);
+  row.pad = 0;
+  L.rows[i] = row;
   L.idx[0][i] = (unsigned)i;
-  if (keep_order)
-    L.qkey[0][i] = qid;
-  else
-    L.key[0][i] = ((unsigned long long)(~float_key_asc(prio)) << 32) | float_key_asc(cost);
+  L.qkey[0][i] = qid;
+  if (!keep_order) L.key[0][i] = ((unsigned long long)(~float_key_asc(prio)) << 32) | float_key_asc(cost);
 }
 
-__global__ void __launch_bounds__(kThreads) gather_qid_kernel(const unsigned long long* qid, const unsigned* order,
-                                                              long long n, unsigned long long* out) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = qid[order[i]];
+// ---- the order inside a group ----------------------------------------------
+//
+// Rows of a group lie together in index order; they are ordered by (key,
+// index).  Groups of up to 256 rows are sorted by one warp each in registers,
+// larger ones in tiles of 4096 by one block each, and the tiles are
+// merged pairwise by one cooperative launch (which returns at once when no
+// group is larger than a tile).  Each row's key is read once; the sort over
+// all rows by the 64-bit key that this stands in for was 8 radix passes:
+// 168 us for 1 M rows, the ordering kernels 52.
+
+__device__ __forceinline__ bool entry_less(unsigned long long ka, unsigned ia, unsigned long long kb, unsigned ib) {
+  return ka < kb || (ka == kb && ia < ib);
 }
 
-// Sorted costs and flags, group heads, and the count of moved rows.
-__global__ void __launch_bounds__(kThreads) gather_kernel(const unsigned* order, const unsigned long long* sorted_qid,
-                                                          long long n, DenseLayout L) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  bool moved = false;
-  if (i < n) {
-    const unsigned j = order[i];
-    L.s_full[i] = L.full[j];
-    L.s_narrow[i] = L.narrow[j];
-    L.s_flags[i] = L.flags[j];
-    L.head[i] = (i == 0 || sorted_qid[i] != sorted_qid[i - 1]) ? 1 : 0;
-    L.iota[i] = (unsigned)i;
-    moved = j != (unsigned)i;
+// Bitonic sort of a warp's 32 * E entries in registers; entry e of a lane has
+// place lane * E + e, so the steps below E stay inside a lane, the others go
+// between lanes.  The stages are loops, not unrolled: five sizes of straight
+// code missed the instruction cache (65 us a million rows, as loops 46).
+template <int E>
+__device__ __forceinline__ void warp_sort(unsigned long long (&key)[E], unsigned (&idx)[E], int lane) {
+#pragma unroll 1
+  for (int k = 2; k <= 32 * E; k <<= 1) {
+#pragma unroll 1
+    for (int j = k >> 1; j >= E; j >>= 1) {
+      const bool low = (lane & (j / E)) == 0;
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const unsigned long long ok = __shfl_xor_sync(0xffffffffu, key[e], j / E);
+        const unsigned oi = __shfl_xor_sync(0xffffffffu, idx[e], j / E);
+        const bool up = ((lane * E + e) & k) == 0;
+        if (entry_less(ok, oi, key[e], idx[e]) == (low == up)) {
+          key[e] = ok;
+          idx[e] = oi;
+        }
+      }
+    }
+#pragma unroll
+    for (int j = E >> 1; j > 0; j >>= 1) {
+      if (j >= k) continue;
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        if ((e & j) != 0) continue;
+        const int b = e | j;
+        const bool up = ((lane * E + e) & k) == 0;
+        if (entry_less(key[b], idx[b], key[e], idx[e]) == up) {
+          const unsigned long long tk = key[e];
+          const unsigned ti = idx[e];
+          key[e] = key[b];
+          idx[e] = idx[b];
+          key[b] = tk;
+          idx[b] = ti;
+        }
+      }
+    }
   }
-  const unsigned m = __ballot_sync(0xffffffffu, moved);
-  if ((threadIdx.x & 31) == 0 && m) atomicAdd(&L.acc->ctr[kReordered], (unsigned long long)__popc(m));
 }
 
-// Adds v of lanes [lo, hi) to s in lane order (every lane returns the same s).
-__device__ __forceinline__ double fold_lanes(double s, double v, int lo, int hi) {
-  for (int j = lo; j < hi; ++j) s += __shfl_sync(0xffffffffu, v, j);
-  return s;
+// Orders the len <= 32 * E rows at order.
+template <int E>
+__device__ __forceinline__ void warp_order(unsigned* order, unsigned len, const unsigned long long* key, int lane) {
+  unsigned long long k[E];
+  unsigned idx[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) idx[e] = (unsigned)(e * 32 + lane) < len ? order[e * 32 + lane] : 0xffffffffu;
+#pragma unroll
+  for (int e = 0; e < E; ++e) k[e] = idx[e] != 0xffffffffu ? key[idx[e]] : ~0ull;
+  warp_sort<E>(k, idx, lane);
+#pragma unroll
+  for (int e = 0; e < E; ++e)
+    if ((unsigned)(lane * E + e) < len) order[lane * E + e] = idx[e];
 }
 
-// One warp per group: the walk of group_scheduler.cpp:116-232.
-__global__ void __launch_bounds__(kThreads) group_kernel(long long n, unsigned limit, double penalty, DenseLayout L) {
+// Bitonic sort of size (a power of two) entries by a block; 32 consecutive
+// compare pairs span 64 entries, so steps of at most 32 stay within one warp's
+// entries.
+__device__ __forceinline__ void block_sort(unsigned long long* key, unsigned* idx, unsigned size) {
+  for (unsigned k = 2; k <= size; k <<= 1) {
+    for (unsigned j = k >> 1; j > 0; j >>= 1) {
+      for (unsigned p = threadIdx.x; p < size / 2; p += kTileThreads) {
+        const unsigned a = 2u * p - (p & (j - 1u)), b = a + j;
+        const unsigned long long ka = key[a], kb = key[b];
+        const unsigned ia = idx[a], ib = idx[b];
+        if (entry_less(kb, ib, ka, ia) == ((a & k) == 0u)) {
+          key[a] = kb;
+          key[b] = ka;
+          idx[a] = ib;
+          idx[b] = ia;
+        }
+      }
+      if (j > 32u) __syncthreads();
+      else __syncwarp();
+    }
+    __syncthreads();
+  }
+}
+
+// The next group of a warp: groups differ by a factor of hundreds in size, so
+// warps draw them (the draw for the next one travels while one is worked on).
+struct GroupDraw {
+  unsigned* next;
+  unsigned drawn;
+  __device__ __forceinline__ GroupDraw(unsigned* n, int lane) : next(n), drawn(0u) { draw(lane); }
+  __device__ __forceinline__ void draw(int lane) {
+    if (lane == 0) drawn = atomicAdd(next, 1u);
+  }
+  __device__ __forceinline__ unsigned take(int lane) {
+    const unsigned g = __shfl_sync(0xffffffffu, drawn, 0);
+    draw(lane);
+    return g;
+  }
+};
+
+// order: rows by (query id, index) in, by (query id, key, index) out.
+__global__ void __launch_bounds__(kThreads) order_small_kernel(long long n, unsigned* order, DenseLayout L) {
+  const int lane = threadIdx.x & 31;
+  const unsigned G = (unsigned)L.acc->n_groups;
+  GroupDraw draw(&L.acc->next[0], lane);
+  for (unsigned g = draw.take(lane); g < G; g = draw.take(lane)) {
+    const unsigned begin = L.g_start[g];
+    const unsigned len = (g + 1 < G ? L.g_start[g + 1] : (unsigned)n) - begin;
+    if (len < 2u) continue;
+    if (len > (unsigned)kWarpRows) {
+      if (lane == 0) {
+        const unsigned tiles = (len + kTileRows - 1) / kTileRows;
+        const unsigned at = atomicAdd(&L.acc->n_tiles, tiles);
+        for (unsigned k = 0; k < tiles; ++k) L.tiles[at + k] = Tile{begin + k * kTileRows, min(kTileRows, len - k * kTileRows)};
+        if (len > kTileRows) {
+          const unsigned long long b = atomicAdd(&L.acc->big, (1ull << 32) | len);
+          L.big_start[b >> 32] = begin;
+          L.big_at[b >> 32] = (unsigned)b;
+          atomicMax(&L.acc->longest, len);
+        }
+      }
+      continue;
+    }
+    if (len <= 32u) warp_order<1>(order + begin, len, L.key[0], lane);
+    else if (len <= 64u) warp_order<2>(order + begin, len, L.key[0], lane);
+    else if (len <= 128u) warp_order<4>(order + begin, len, L.key[0], lane);
+    else warp_order<8>(order + begin, len, L.key[0], lane);
+  }
+}
+
+// One block per tile; keys of tiles to be merged go along.
+__global__ void __launch_bounds__(kTileThreads) order_tile_kernel(unsigned* order, DenseLayout L) {
+  extern __shared__ __align__(16) unsigned char tile_raw[];
+  unsigned long long* key = reinterpret_cast<unsigned long long*>(tile_raw);
+  unsigned* idx = reinterpret_cast<unsigned*>(tile_raw + kTileRows * 8);
+  const unsigned n = L.acc->n_tiles;
+  for (unsigned t = blockIdx.x; t < n; t += gridDim.x) {
+    const Tile tile = L.tiles[t];
+    unsigned size = 2u;
+    while (size < tile.len) size <<= 1;
+    for (unsigned e = threadIdx.x; e < size; e += kTileThreads) {
+      const unsigned j = e < tile.len ? order[tile.start + e] : 0xffffffffu;
+      idx[e] = j;
+      key[e] = e < tile.len ? L.key[0][j] : ~0ull;
+    }
+    __syncthreads();
+    block_sort(key, idx, size);
+    for (unsigned e = threadIdx.x; e < tile.len; e += kTileThreads) {
+      order[tile.start + e] = idx[e];
+      L.key[1][tile.start + e] = key[e];
+    }
+    __syncthreads();
+  }
+}
+
+// Pairwise merges of the tiles of groups larger than one: every thread writes
+// kMergeOut consecutive places, from where the merge path crosses their first.
+constexpr int kMergeOut = 8;
+
+__global__ void __launch_bounds__(kThreads) order_merge_kernel(unsigned* order, DenseLayout L) {
+  const unsigned long long big = L.acc->big;
+  const unsigned n_big = (unsigned)(big >> 32), rows = (unsigned)big, longest = L.acc->longest;
+  if (n_big == 0u) return;  // the same in every block
+  cooperative_groups::grid_group grid = cooperative_groups::this_grid();
+  unsigned long long* key[2] = {L.key[1], L.qkey[0]};
+  unsigned* idx[2] = {order, L.idx[1]};
+  int src = 0;
+  const unsigned stride = gridDim.x * kThreads, t = blockIdx.x * kThreads + threadIdx.x;
+  for (unsigned long long width = kTileRows; width < longest; width *= 2ull) {
+    for (unsigned long long v0 = (unsigned long long)t * kMergeOut; v0 < rows;
+         v0 += (unsigned long long)stride * kMergeOut) {
+      const unsigned vend = (unsigned)min((unsigned long long)rows, v0 + kMergeOut);
+      unsigned v = (unsigned)v0;
+      while (v < vend) {  // pieces of one pair of runs of one group
+        unsigned lo = 0u, hi = n_big - 1u;
+        while (lo < hi) {
+          const unsigned mid = (lo + hi + 1u) >> 1;
+          if (L.big_at[mid] <= v) lo = mid;
+          else hi = mid - 1u;
+        }
+        const unsigned at = L.big_at[lo], len = (lo + 1u < n_big ? L.big_at[lo + 1u] : rows) - at;
+        const unsigned a = v - at;  // place in the group
+        const unsigned long long pair = (unsigned long long)a / (2ull * width) * (2ull * width);
+        const unsigned base = L.big_start[lo] + (unsigned)pair;
+        const unsigned left = (unsigned)min(width, (unsigned long long)len - pair);
+        const unsigned both = (unsigned)min(2ull * width, (unsigned long long)len - pair);
+        const unsigned right = both - left;
+        const unsigned d = a - (unsigned)pair, dend = min(both, d + (vend - v));
+        const unsigned long long *ka = key[src] + base, *kb = ka + left;
+        const unsigned *ia = idx[src] + base, *ib = ia + left;
+        unsigned x0 = d > right ? d - right : 0u, x1 = min(d, left);  // entries of the left run before place d
+        while (x0 < x1) {
+          const unsigned m = (x0 + x1) >> 1, o = d - 1u - m;
+          const bool left_first = ka[m] < kb[o] || (ka[m] == kb[o] && ia[m] < ib[o]);
+          if (left_first) x0 = m + 1u;
+          else x1 = m;
+        }
+        unsigned x = x0, y = d - x0;
+        for (unsigned p = d; p < dend; ++p) {
+          const bool take_left = y >= right || (x < left && (ka[x] < kb[y] || (ka[x] == kb[y] && ia[x] < ib[y])));
+          key[1 - src][base + p] = take_left ? ka[x] : kb[y];
+          idx[1 - src][base + p] = take_left ? ia[x] : ib[y];
+          if (take_left) ++x;
+          else ++y;
+        }
+        v += dend - d;
+      }
+    }
+    grid.sync();
+    src = 1 - src;
+  }
+  if (src == 0) return;
+  for (unsigned v = t; v < rows; v += stride) {
+    unsigned lo = 0u, hi = n_big - 1u;
+    while (lo < hi) {
+      const unsigned mid = (lo + hi + 1u) >> 1;
+      if (L.big_at[mid] <= v) lo = mid;
+      else hi = mid - 1u;
+    }
+    const unsigned p = L.big_start[lo] + (v - L.big_at[lo]);
+    order[p] = L.idx[1][p];
+  }
+}
+
+// One warp per group: the walk of group_scheduler.cpp:116-232.  Rows are read
+// through the order; every slot of the group's terms is written.  Bound by the
+// chain of dependent additions of the two sums, so both run side by side over
+// all 32 lanes (rows that add nothing add +0.0): walk and the gather of sorted
+// costs before it took 99 us for 1 M rows, now 43.
+__global__ void __launch_bounds__(kThreads, 4) group_kernel(const unsigned* order, long long n, unsigned limit,
+                                                         double penalty, DenseLayout L) {
   __shared__ unsigned long long s_ctr[kNumCounters];
+  __shared__ double2 s_add[kThreads / 32][32];
   if (threadIdx.x < kNumCounters) s_ctr[threadIdx.x] = 0;
   __syncthreads();
   const int lane = threadIdx.x & 31;
-  const long long G = L.acc->n_groups;
-  const long long warps = (long long)gridDim.x * (kThreads / 32);
-  unsigned long long c[kNumCounters] = {};
-  for (long long g = (long long)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5); g < G; g += warps) {
-    const long long begin = L.g_start[g];
-    const long long end = g + 1 < G ? (long long)L.g_start[g + 1] : n;
-    const long long slot0 = 2 * begin + g;  // this group's 2 * size + 1 term slots
-    double gfull = 0.0, wbfp = 0.0, gcost = 0.0;
+  const unsigned G = (unsigned)L.acc->n_groups;
+  double2* add = s_add[threadIdx.x >> 5];
+  unsigned c[kNumCounters] = {};  // none exceeds 2 n < 2^30
+  // slots past the last group's: the compaction runs over 3 n
+  for (long long i = 2 * n + G + (long long)blockIdx.x * kThreads + threadIdx.x; i < 3 * n;
+       i += (long long)gridDim.x * kThreads)
+    L.terms[i] = 0.0;
+  GroupDraw draw(&L.acc->next[1], lane);
+  for (unsigned g = draw.take(lane); g < G; g = draw.take(lane)) {
+    const unsigned begin = L.g_start[g];
+    const unsigned end = g + 1 < G ? L.g_start[g + 1] : (unsigned)n;
+    const unsigned slot0 = 2 * begin + g;  // this group's 2 * size + 1 term slots
+    double gfull = 0.0, wbfp = 0.0, gcost = 0.0, last_term = 0.0;
     bool truth = false, predicted = false;
     int state = 0;  // 0 proposals, 1 full fallback, 2 resolved
-    long long rank = 0;
-    unsigned long long calls = 0, fallback = 0, hits = 0, misses = 0;
+    unsigned rank = 0;
+    unsigned calls = 0, fallback = 0, hits = 0, misses = 0;
     bool high_group = false;
-    for (long long base = begin; base < end; base += 32) {
-      const long long pos = base + lane;
-      const int nvalid = (int)min(32ll, end - base);
+    for (unsigned base = begin; base < end; base += 32) {
+      const unsigned pos = base + lane;
+      const int nvalid = (int)min(32u, end - base);
       const bool in = lane < nvalid;
-      const double f = in ? L.s_full[pos] : 0.0;
-      const double nr = in ? L.s_narrow[pos] : 0.0;
-      const unsigned char fl = in ? L.s_flags[pos] : 0;
-      const long long my_slot = slot0 + 2 * (pos - begin);
-      gfull = fold_lanes(gfull, f, 0, nvalid);
+      double f = 0.0, nr = 0.0;
+      unsigned fl = 0;
+      bool moved = false;
+      if (in) {
+        const unsigned j = order[pos];
+        const WalkRow r = L.rows[j];
+        f = r.full;
+        nr = r.narrow;
+        fl = (unsigned)r.flags;
+        moved = j != pos;
+      }
+      const unsigned m_moved = __ballot_sync(0xffffffffu, moved);
+      c[kReordered] += __popc(m_moved);
+      const unsigned my_slot = slot0 + 2 * (pos - begin);
       truth = truth || __any_sync(0xffffffffu, fl & kColl);
       int from = 0;
+      double term0 = 0.0, term1 = 0.0, w = 0.0;  // this row's terms; what it adds to the cost before a hit
+      bool cost_here = false;                     // the group's cost is the sum so far plus `extra`s
+      double extra0 = 0.0, extra1 = 0.0;
       if (state == 0) {
-        const unsigned attempts = (unsigned)(pos - begin + 1);
+        const unsigned attempts = pos - begin + 1;
         const bool stop = in && ((fl & kHighUnc) || ((fl & kColl) && ((fl & kOverlap) || attempts >= limit)));
         const unsigned m = __ballot_sync(0xffffffffu, stop);
         const int t = m ? __ffs(m) - 1 : nvalid;
         const bool pre = lane < t;
         if (pre) {  // narrow call; a colliding miss adds its penalty
-          L.terms[my_slot] = nr;
-          if (fl & kColl) L.terms[my_slot + 1] = f * penalty;
+          term0 = nr;
+          w = nr;
+          if (fl & kColl) {
+            term1 = f * penalty;
+            w = nr + term1;
+          }
         }
-        const double wv = (fl & kColl) ? nr + f * penalty : nr;
-        wbfp = fold_lanes(wbfp, wv, 0, t);
-        calls += (unsigned long long)t;
-        misses += (unsigned long long)__popc(__ballot_sync(0xffffffffu, pre && (fl & kColl)));
+        calls += (unsigned)t;
+        misses += __popc(__ballot_sync(0xffffffffu, pre && (fl & kColl)));
         if (m) {
-          const unsigned char sfl = (unsigned char)__shfl_sync(0xffffffffu, (int)fl, t);
+          const unsigned sfl = __shfl_sync(0xffffffffu, fl, t);
           const double snr = __shfl_sync(0xffffffffu, nr, t);
           const double sf = __shfl_sync(0xffffffffu, f, t);
-          const long long sslot = slot0 + 2 * (base + t - begin);
           rank = base + t - begin + 1;
           if (sfl & kHighUnc) {
             state = 1;
             from = t;
             high_group = true;
           } else if (sfl & kOverlap) {  // a hit inside the predicted interval
-            if (lane == 0) L.terms[sslot] = snr;
+            if (lane == t) term0 = snr;
             calls += 1;
             hits += 1;
-            gcost = wbfp + snr;
+            cost_here = true;
+            extra0 = snr;
             predicted = true;
             state = 2;
           } else {  // a miss at the attempt limit: penalty, then one full fallback call
-            if (lane == 0) {
-              L.terms[sslot] = snr;
-              L.terms[sslot + 1] = sf * penalty;
-              L.terms[slot0 + 2 * (end - begin)] = sf;
+            if (lane == t) {
+              term0 = snr;
+              term1 = sf * penalty;
             }
+            last_term = sf;
             calls += 2;
             fallback += 1;
             misses += 1;
-            gcost = (wbfp + snr) + sf;
+            cost_here = true;
+            extra0 = snr;
+            extra1 = sf;
             predicted = true;
             state = 2;
           }
@@ -336,20 +615,38 @@ __global__ void __launch_bounds__(kThreads) group_kernel(long long n, unsigned l
         const unsigned m = __ballot_sync(0xffffffffu, fb && (fl & kColl));
         const int q = m ? __ffs(m) - 1 : nvalid;
         const int last = m ? q + 1 : nvalid;
-        if (fb && lane < last) L.terms[my_slot] = f;
-        calls += (unsigned long long)(last - from);
-        fallback += (unsigned long long)(last - from);
-        wbfp = fold_lanes(wbfp, f, from, q);
+        if (fb && lane < last) term0 = f;
+        if (fb && lane < q) w = f;
+        calls += (last - from);
+        fallback += (last - from);
         if (m) {
           const double qf = __shfl_sync(0xffffffffu, f, q);
           rank = base + q - begin + 1;
-          gcost = wbfp + qf;
+          cost_here = true;
+          extra0 = qf;
           predicted = true;
           state = 2;
         }
       }
+      if (in) {
+        L.terms[my_slot] = term0;
+        L.terms[my_slot + 1] = term1;
+      }
+      add[lane] = make_double2(f, w);
+      __syncwarp();
+      for (int j0 = 0; j0 < nvalid; j0 += 8) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const double2 a = add[j0 + j];
+          gfull += a.x;
+          wbfp += a.y;
+        }
+      }
+      __syncwarp();
+      if (cost_here) gcost = (wbfp + extra0) + extra1;
     }
     if (lane == 0) {
+      L.terms[slot0 + 2 * (end - begin)] = last_term;
       L.g_full[g] = gfull;
       L.g_cost[g] = predicted ? gcost : 0.0;
       c[kGroups] += 1;
@@ -363,21 +660,19 @@ __global__ void __launch_bounds__(kThreads) group_kernel(long long n, unsigned l
       c[kFP] += (!truth && predicted) ? 1 : 0;
       c[kFN] += (truth && !predicted) ? 1 : 0;
       c[kHighUncGroups] += high_group ? 1 : 0;
-      c[kRankSum] += predicted ? (unsigned long long)rank : 0;
+      c[kRankSum] += predicted ? rank : 0;
     }
   }
   if (lane == 0)
     for (int k = 0; k < kNumCounters; ++k)
-      if (k != kReordered && c[k]) atomicAdd(&s_ctr[k], c[k]);
+      if (c[k]) atomicAdd(&s_ctr[k], (unsigned long long)c[k]);
   __syncthreads();
-  if (threadIdx.x < kNumCounters && threadIdx.x != kReordered && s_ctr[threadIdx.x])
-    atomicAdd(&L.acc->ctr[threadIdx.x], s_ctr[threadIdx.x]);
+  if (threadIdx.x < kNumCounters && s_ctr[threadIdx.x]) atomicAdd(&L.acc->ctr[threadIdx.x], s_ctr[threadIdx.x]);
 }
 
 struct FoldJob {
   const double* src[3];
-  const int* count[3];   // device counts, or null: the fixed counts
-  long long fixed[3];
+  const int* count[3];  // device counts
   double* out[3];
 };
 
@@ -394,16 +689,10 @@ struct FoldJob {
 // ((a then b)[p] = a[p] + b[(p + a[p]) mod 2]), and a block scan gives every
 // term the S in front of it.  The first term whose exact sum could reach the
 // top of the binade (or an infinite term) is added with the hardware DADD;
-// the fold then continues from it in the new binade, with a chunk as long as
-// the terms taken so far (steps come every few terms while s is small).
+// the fold then continues from it in the new binade.
 // Each such step at least doubles s, so there are at most a few dozen of
 // them.  A zero-start sum takes its first non-zero term exactly.
 
-constexpr int kFoldThreads = 512;
-constexpr int kFoldPerThread = 8;  // consecutive terms per thread
-constexpr int kFoldChunk = kFoldThreads * kFoldPerThread;
-constexpr int kFoldWarps = kFoldThreads / 32;
-constexpr int kFoldSmall = 64;  // shortest chunk after a binade step
 constexpr unsigned long long kTwo53 = 1ull << 53;
 
 struct IncPair {
@@ -433,161 +722,334 @@ __device__ __forceinline__ IncPair warp_inclusive(IncPair v, int lane) {
   return v;
 }
 
+// The exponent of the last place of a positive double.
+__device__ __forceinline__ int ulp_of(double s) { return max(ilogb(s), -1022) - 52; }
+
+// What a term of q units adds to an even and to an odd S.
+__device__ __forceinline__ IncPair term_increments(double q) {
+  const double mf = floor(q);
+  const double f = q - mf;
+  const unsigned long long m = (unsigned long long)mf;
+  const bool above = f > 0.5, tie = f == 0.5;
+  IncPair c;
+  c.e = m + (above ? 1ull : (tie ? (m & 1ull) : 0ull));
+  c.o = m + (above ? 1ull : (tie ? ((m + 1ull) & 1ull) : 0ull));
+  return c;
+}
+
 struct FoldShared {
   unsigned long long we[32], wo[32];
   double s;
-  long long pos;
   int first;
-  int len;  // terms the next iteration takes
 };
 
-// One block per total.
-__global__ void __launch_bounds__(kFoldThreads) fold_kernel(FoldJob job) {
-  __shared__ FoldShared sh;
-  const int b = blockIdx.x;  // selects without indexing the parameter arrays dynamically
-  const double* src = b == 0 ? job.src[0] : (b == 1 ? job.src[1] : job.src[2]);
-  const int* cp = b == 0 ? job.count[0] : (b == 1 ? job.count[1] : job.count[2]);
-  const long long cnt = cp ? (long long)*cp : (b == 0 ? job.fixed[0] : (b == 1 ? job.fixed[1] : job.fixed[2]));
+// x * 2^-ue as two exact factors (2^1074 alone is not a double).  A product
+// that underflows is far below one half of a unit, one that overflows far above
+// the binade.
+struct UnitScale {
+  double a, b;
+  __device__ __forceinline__ explicit UnitScale(int ue) : a(ldexp(1.0, -ue / 2)), b(ldexp(1.0, -ue - -ue / 2)) {}
+  __device__ __forceinline__ double operator()(double x) const { return x * a * b; }
+};
+
+// Adds the terms [begin, end) to sh.s; every thread of the block takes part.
+// The terms of a chunk stay in registers over its binade steps, those already
+// added count as zero.  Returns early when the sum is infinite.
+__device__ __forceinline__ void fold_range(FoldShared& sh, const double* src, long long begin, long long end) {
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
   const IncPair zero{0ull, 0ull};
+  double x[kFoldPerThread], nx[kFoldPerThread];
+#pragma unroll
+  for (int k = 0; k < kFoldPerThread; ++k) {
+    const long long i = begin + t * kFoldPerThread + k;
+    nx[k] = i < end ? src[i] : 0.0;
+  }
+  for (long long base = begin; base < end; base += kFoldChunk) {
+    const int chunk = (int)min((long long)kFoldChunk, end - base);
+#pragma unroll
+    for (int k = 0; k < kFoldPerThread; ++k) {
+      x[k] = nx[k];
+      const long long i = base + kFoldChunk + t * kFoldPerThread + k;
+      nx[k] = i < end ? src[i] : 0.0;
+    }
+    int start = 0;  // terms of the chunk already added
+    while (start < chunk) {
+      const double s = sh.s;
+      if (isinf(s)) return;
+      // the sum grows about linearly, so the next binade step is about as many
+      // terms away as have been added: do not look much further
+      const int len = (int)min((long long)chunk, start + max(256ll, base + start));
+      if (t == 0) sh.first = len;
+      __syncthreads();  // everyone read s; first is reset
+      if (s == 0.0) {   // 0 + x == x: the first non-zero term starts the sum
+        int mine = len;
+#pragma unroll
+        for (int k = kFoldPerThread - 1; k >= 0; --k) {
+          const int i = t * kFoldPerThread + k;
+          if (i >= start && i < len && x[k] != 0.0) mine = i;
+        }
+        if (mine < len) atomicMin(&sh.first, mine);
+        __syncthreads();
+        const int f = sh.first;
+#pragma unroll
+        for (int k = 0; k < kFoldPerThread; ++k)
+          if (f < len && t * kFoldPerThread + k == f) sh.s = x[k];
+        start = min(f + 1, len);
+        __syncthreads();
+        continue;
+      }
+      const int ue = ulp_of(s);
+      const UnitScale units(ue);
+      const unsigned long long S = (unsigned long long)units(s);
+      IncPair inc[kFoldPerThread];
+      unsigned long long m[kFoldPerThread];
+      bool big[kFoldPerThread];
+      IncPair incl = zero;
+      const bool idle = (w + 1) * 32 * kFoldPerThread <= start || w * 32 * kFoldPerThread >= len;  // a whole warp
+      if (!idle) {
+        IncPair local = zero;
+#pragma unroll
+        for (int k = 0; k < kFoldPerThread; ++k) {
+          const int i = t * kFoldPerThread + k;
+          const double q = i >= start && i < len ? units(x[k]) : 0.0;
+          big[k] = !(q < 9007199254740992.0);
+          m[k] = 0;
+          if (big[k]) {
+            inc[k] = IncPair{kTwo53, kTwo53};  // never applied: the binade step comes first
+          } else {
+            m[k] = (unsigned long long)floor(q);
+            inc[k] = term_increments(q);
+          }
+          local = compose(local, inc[k]);
+        }
+        incl = warp_inclusive(local, lane);
+      }
+      if (lane == 31) {
+        sh.we[w] = incl.e;
+        sh.wo[w] = incl.o;
+      }
+      __syncthreads();
+      if (w == 0) {
+        const IncPair v = warp_inclusive(lane < kFoldWarps ? IncPair{sh.we[lane], sh.wo[lane]} : zero, lane);
+        IncPair ex = shfl_up_pair(v, 1);
+        if (lane == 0) ex = zero;
+        __syncwarp();
+        sh.we[lane] = ex.e;
+        sh.wo[lane] = ex.o;
+      }
+      __syncthreads();
+      IncPair ein = shfl_up_pair(incl, 1);
+      if (lane == 0) ein = zero;
+      const IncPair wp{sh.we[w], sh.wo[w]};
+      const IncPair ex = compose(wp, ein);
+      unsigned long long P = S + ((S & 1ull) ? ex.o : ex.e);
+      int mine = len;
+      unsigned long long P_at = 0;
+      if (!idle) {
+#pragma unroll
+        for (int k = 0; k < kFoldPerThread; ++k) {
+          const bool in = t * kFoldPerThread + k < len;
+          if (in && mine == len) {
+            if (big[k] || P >= kTwo53 || P + m[k] >= kTwo53) {
+              mine = t * kFoldPerThread + k;
+              P_at = P;
+            } else {
+              P += (P & 1ull) ? inc[k].o : inc[k].e;
+            }
+          }
+        }
+      }
+      if (mine < len) atomicMin(&sh.first, mine);
+      __syncthreads();
+      const int c = sh.first;
+      if (c == len) {  // no binade step: the last thread holds the end of the chunk
+        if (t == (len - 1) / kFoldPerThread) sh.s = ldexp((double)P, ue);
+      } else if (mine == c) {
+#pragma unroll
+        for (int k = 0; k < kFoldPerThread; ++k)
+          if (t * kFoldPerThread + k == c) sh.s = ldexp((double)P_at, ue) + x[k];
+      }
+      start = min(c + 1, len);
+      __syncthreads();
+    }
+  }
+}
+
+// One block per total, its terms straight through.
+__global__ void __launch_bounds__(kFoldThreads) fold_kernel(const double* src, long long cnt, double* out) {
+  __shared__ FoldShared sh;
+  if (threadIdx.x == 0) sh.s = 0.0;
+  __syncthreads();
+  fold_range(sh, src, 0, cnt);
+  if (threadIdx.x == 0) *out = sh.s;
+}
+
+// The three totals of a replay, pieces of kFoldChunk terms on all SMs.  What a
+// piece adds to the sum is a pair of increments once the sum's binade is
+// known, and the sum of all terms before the piece, added in any order,
+// predicts it.  One block per total then strings the pieces together: 512 at a
+// time by a scan of their pairs, up to the first one whose prediction was
+// wrong or in which the sum leaves its binade; that one is folded term by
+// term.  Exact whatever the prediction.  The straight fold is a chain of one
+// 4,096-term chunk after the other: 221 us for the three totals of 1 M rows,
+// now 106.
+__device__ __forceinline__ long long job_count(const FoldJob& job, int b) {
+  const int* cp = b == 0 ? job.count[0] : (b == 1 ? job.count[1] : job.count[2]);
+  return (long long)*cp;
+}
+
+// Sums of the pieces; the last block of a total turns them into the binade in
+// front of each piece.
+__global__ void __launch_bounds__(kFoldThreads) piece_sum_kernel(FoldJob job, FoldPieces pc, DenseAcc* acc) {
+  __shared__ double warp_sum[kFoldWarps], carry;
+  __shared__ bool last;
+  const int b = blockIdx.y, t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const double* src = b == 0 ? job.src[0] : (b == 1 ? job.src[1] : job.src[2]);
+  double* sum = b == 0 ? pc.sum[0] : (b == 1 ? pc.sum[1] : pc.sum[2]);
+  int* ulp = b == 0 ? pc.ulp[0] : (b == 1 ? pc.ulp[1] : pc.ulp[2]);
+  const long long cnt = job_count(job, b), pieces = (cnt + kFoldChunk - 1) / kFoldChunk;
+  for (long long c = blockIdx.x; c < pieces; c += gridDim.x) {
+    const long long base = c * kFoldChunk;
+    double s = 0.0;
+#pragma unroll
+    for (int k = 0; k < kFoldPerThread; ++k) {
+      const long long i = base + k * kFoldThreads + t;
+      s += i < cnt ? src[i] : 0.0;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) warp_sum[w] = s;
+    __syncthreads();
+    if (t == 0) {
+      double v = 0.0;
+      for (int k = 0; k < kFoldWarps; ++k) v += warp_sum[k];
+      sum[c] = v;
+    }
+    __syncthreads();
+  }
+  __threadfence();
+  __syncthreads();
   if (t == 0) {
-    sh.s = 0.0;
-    sh.pos = 0;
-    sh.len = kFoldSmall;
+    last = atomicAdd(&acc->fold_blocks[b], 1u) == gridDim.x - 1;
+    carry = 0.0;
   }
   __syncthreads();
-  double x[kFoldPerThread];
-  long long loaded = -1;  // chunk start the registers hold
-  while (true) {
-    const double s = sh.s;
-    const long long pos = sh.pos;
-    if (pos >= cnt || isinf(s)) break;
-    const int want = sh.len;
-    const int len = (int)min((long long)want, cnt - pos);
-    const int next_len = min(kFoldChunk, 2 * want);
-    if (loaded != pos) {
+  if (!last) return;
+  __threadfence();
+  for (long long c0 = 0; c0 < pieces; c0 += kFoldThreads) {
+    const double v = c0 + t < pieces ? __ldcg(sum + c0 + t) : 0.0;
+    double incl = v;
 #pragma unroll
-      for (int k = 0; k < kFoldPerThread; ++k) {
-        const int i = t * kFoldPerThread + k;
-        x[k] = i < len ? src[pos + i] : 0.0;
-      }
+    for (int o = 1; o < 32; o <<= 1) {
+      const double up = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += up;
     }
-    double nx[kFoldPerThread];  // the next chunk, in case this one has no binade step
+    if (lane == 31) warp_sum[w] = incl;
+    __syncthreads();
+    double before = carry;
+    for (int k = 0; k < w; ++k) before += warp_sum[k];
+    double ex = __shfl_up_sync(0xffffffffu, incl, 1);
+    if (lane == 0) ex = 0.0;
+    if (c0 + t < pieces) ulp[c0 + t] = ulp_of(before + ex);
+    __syncthreads();
+    if (t == kFoldThreads - 1) carry = before + incl;
+    __syncthreads();
+  }
+}
+
+// The increments of each piece in its predicted binade; ~0 for both when a
+// term is too large for their 64-bit counts (then the sum soon leaves the
+// binade anyway).
+__global__ void __launch_bounds__(kFoldThreads) piece_inc_kernel(FoldJob job, FoldPieces pc) {
+  __shared__ IncPair warp_inc[kFoldWarps];
+  const int b = blockIdx.y, t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const double* src = b == 0 ? job.src[0] : (b == 1 ? job.src[1] : job.src[2]);
+  const int* ulp = b == 0 ? pc.ulp[0] : (b == 1 ? pc.ulp[1] : pc.ulp[2]);
+  ulonglong2* out = b == 0 ? pc.inc[0] : (b == 1 ? pc.inc[1] : pc.inc[2]);
+  const long long cnt = job_count(job, b), pieces = (cnt + kFoldChunk - 1) / kFoldChunk;
+  for (long long c = blockIdx.x; c < pieces; c += gridDim.x) {
+    const long long base = c * kFoldChunk + t * kFoldPerThread;
+    const UnitScale units(ulp[c]);
+    IncPair local{0ull, 0ull};
+    bool big = false;
 #pragma unroll
     for (int k = 0; k < kFoldPerThread; ++k) {
-      const int i = t * kFoldPerThread + k;
-      nx[k] = (i < next_len && pos + len + i < cnt) ? src[pos + len + i] : 0.0;
-    }
-    if (t == 0) sh.first = len;
-    __syncthreads();  // everyone read s and pos; first is reset
-    if (s == 0.0) {  // 0 + x == x: the first non-zero term starts the sum
-#pragma unroll
-      for (int k = 0; k < kFoldPerThread; ++k) {
-        const int i = t * kFoldPerThread + k;
-        if (i < len && x[k] != 0.0) {
-          atomicMin(&sh.first, i);
-          break;
-        }
-      }
-      __syncthreads();
-      const int f = sh.first;
-#pragma unroll
-      for (int k = 0; k < kFoldPerThread; ++k)
-        if (t * kFoldPerThread + k == f) sh.s = x[k];
-      if (t == 0) {
-        sh.pos = pos + (f < len ? f + 1 : len);
-        sh.len = f < len ? kFoldSmall : next_len;
-      }
-      loaded = -1;
-      __syncthreads();
-      continue;
-    }
-    const int ue = max(ilogb(s), -1022) - 52;
-    const unsigned long long S = (unsigned long long)ldexp(s, -ue);
-    IncPair inc[kFoldPerThread];
-    unsigned long long m[kFoldPerThread];
-    bool big[kFoldPerThread];
-    IncPair local = zero;
-#pragma unroll
-    for (int k = 0; k < kFoldPerThread; ++k) {
-      inc[k] = zero;
-      m[k] = 0;
-      big[k] = false;
-      if (t * kFoldPerThread + k < len) {
-        const double q = ldexp(x[k], -ue);
-        big[k] = !(q < 9007199254740992.0);
-        if (big[k]) {
-          inc[k] = IncPair{kTwo53, kTwo53};  // never applied: the binade step comes first
-        } else {
-          const double mf = floor(q);
-          const double f = q - mf;
-          m[k] = (unsigned long long)mf;
-          const bool above = f > 0.5, tie = f == 0.5;
-          inc[k].e = m[k] + (above ? 1ull : (tie ? (m[k] & 1ull) : 0ull));
-          inc[k].o = m[k] + (above ? 1ull : (tie ? ((m[k] + 1ull) & 1ull) : 0ull));
-        }
-      }
-      local = compose(local, inc[k]);
+      const double q = units(base + k < cnt ? src[base + k] : 0.0);
+      if (!(q < 2251799813685248.0)) big = true;  // 2^51: 4096 of them stay below 2^64
+      else local = compose(local, term_increments(q));
     }
     const IncPair incl = warp_inclusive(local, lane);
-    if (lane == 31) {
-      sh.we[w] = incl.e;
-      sh.wo[w] = incl.o;
-    }
-    __syncthreads();
+    if (lane == 31) warp_inc[w] = incl;
+    big = __syncthreads_or(big);
     if (w == 0) {
-      const IncPair v = warp_inclusive(lane < kFoldWarps ? IncPair{sh.we[lane], sh.wo[lane]} : zero, lane);
-      IncPair ex = shfl_up_pair(v, 1);
-      if (lane == 0) ex = zero;
-      __syncwarp();
-      sh.we[lane] = ex.e;
-      sh.wo[lane] = ex.o;
+      const IncPair v = warp_inclusive(lane < kFoldWarps ? warp_inc[lane] : IncPair{0ull, 0ull}, lane);
+      if (lane == 31) out[c] = big ? make_ulonglong2(~0ull, ~0ull) : make_ulonglong2(v.e, v.o);
     }
     __syncthreads();
-    IncPair ein = shfl_up_pair(incl, 1);
-    if (lane == 0) ein = zero;
-    const IncPair wp{sh.we[w], sh.wo[w]};
-    const IncPair ex = compose(wp, ein);
-    unsigned long long P = S + ((S & 1ull) ? ex.o : ex.e);
-    int mine = len;
-    unsigned long long P_at = 0;
-#pragma unroll
-    for (int k = 0; k < kFoldPerThread; ++k) {
-      const bool in = t * kFoldPerThread + k < len;
-      if (in && mine == len) {
-        if (big[k] || P >= kTwo53 || P + m[k] >= kTwo53) {
-          mine = t * kFoldPerThread + k;
-          P_at = P;
-        } else {
-          P += (P & 1ull) ? inc[k].o : inc[k].e;
-        }
+  }
+}
+
+// One block per total.
+__global__ void __launch_bounds__(kFoldThreads) piece_fold_kernel(FoldJob job, FoldPieces pc) {
+  __shared__ FoldShared sh;
+  const int b = blockIdx.x, t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const double* src = b == 0 ? job.src[0] : (b == 1 ? job.src[1] : job.src[2]);
+  const int* ulp = b == 0 ? pc.ulp[0] : (b == 1 ? pc.ulp[1] : pc.ulp[2]);
+  const ulonglong2* inc = b == 0 ? pc.inc[0] : (b == 1 ? pc.inc[1] : pc.inc[2]);
+  const long long cnt = job_count(job, b), pieces = (cnt + kFoldChunk - 1) / kFoldChunk;
+  const IncPair zero{0ull, 0ull};
+  if (t == 0) sh.s = 0.0;
+  __syncthreads();
+  long long c = 0;  // pieces added
+  while (c < pieces && !isinf(sh.s)) {
+    const double s = sh.s;
+    const int avail = (int)min((long long)kFoldThreads, pieces - c);
+    int done = 0;
+    if (s > 0.0) {
+      const int ue = ulp_of(s);
+      const unsigned long long S = (unsigned long long)UnitScale(ue)(s);
+      bool fits = false;
+      IncPair mine = zero;
+      if (t < avail && ulp[c + t] == ue) {
+        const ulonglong2 v = inc[c + t];
+        fits = v.x < kTwo53 && v.y < kTwo53;
+        if (fits) mine = IncPair{v.x, v.y};
       }
-    }
-    if (mine < len) atomicMin(&sh.first, mine);
-    __syncthreads();
-    const int c = sh.first;
-    if (c == len) {  // no binade step: the last thread holds the end of the chunk
-      if (t == (len - 1) / kFoldPerThread) {
-        sh.s = ldexp((double)P, ue);
-        sh.pos = pos + len;
-        sh.len = next_len;
+      if (t == 0) sh.first = avail;
+      const IncPair incl = warp_inclusive(mine, lane);
+      if (lane == 31) {
+        sh.we[w] = incl.e;
+        sh.wo[w] = incl.o;
       }
-    } else if (mine == c) {
-#pragma unroll
-      for (int k = 0; k < kFoldPerThread; ++k)
-        if (t * kFoldPerThread + k == c) sh.s = ldexp((double)P_at, ue) + x[k];
-      sh.pos = pos + c + 1;
-      // s grows about linearly in the terms taken, so the next step is about
-      // as many terms away as have been taken so far
-      sh.len = (int)max((long long)kFoldSmall, min((long long)kFoldChunk, pos + c + 1));
+      __syncthreads();
+      if (w == 0) {
+        const IncPair v = warp_inclusive(lane < kFoldWarps ? IncPair{sh.we[lane], sh.wo[lane]} : zero, lane);
+        IncPair ex = shfl_up_pair(v, 1);
+        if (lane == 0) ex = zero;
+        __syncwarp();
+        sh.we[lane] = ex.e;
+        sh.wo[lane] = ex.o;
+      }
+      __syncthreads();
+      IncPair ein = shfl_up_pair(incl, 1);
+      if (lane == 0) ein = zero;
+      const IncPair ex = compose(IncPair{sh.we[w], sh.wo[w]}, ein);
+      const unsigned long long P = S + ((S & 1ull) ? ex.o : ex.e);  // right up to the first piece that fails
+      // the sum never falls, so a piece stays in the binade iff it ends in it
+      const bool ok = fits && P < kTwo53 && P + ((P & 1ull) ? mine.o : mine.e) < kTwo53;
+      if (t < avail && !ok) atomicMin(&sh.first, t);
+      __syncthreads();
+      done = sh.first;
+      if (done > 0 && t == done - 1) {
+        const unsigned long long end = P + ((P & 1ull) ? mine.o : mine.e);
+        sh.s = ldexp((double)end, ue);
+      }
+      __syncthreads();
     }
-    __syncthreads();
-    if (sh.pos == pos + len) {
-#pragma unroll
-      for (int k = 0; k < kFoldPerThread; ++k) x[k] = nx[k];
-      loaded = pos + len;
-    } else {
-      loaded = -1;
+    c += done;
+    if (done < avail) {
+      fold_range(sh, src, c * kFoldChunk, min(cnt, (c + 1) * kFoldChunk));
+      ++c;
     }
   }
   if (t == 0) *(b == 0 ? job.out[0] : (b == 1 ? job.out[1] : job.out[2])) = sh.s;
@@ -654,7 +1116,11 @@ int p2c_dense_group_early_stop(int64_t n, const uint64_t* query_id_dev, const ui
   const size_t need = carve(nullptr, n).total;
   if (workspace_dev == nullptr || workspace_bytes < need)
     return fail(P2C_ERR_INVALID, "dense group workspace too small: %zu < %zu bytes", workspace_bytes, need);
-  DenseLayout L = carve(workspace_dev, n);
+  // 16-byte records: the size that callers are told has room for this
+  char* base = reinterpret_cast<char*>(((uintptr_t)workspace_dev + 15) & ~(uintptr_t)15);
+  if ((size_t)(base - static_cast<char*>(workspace_dev)) + need > workspace_bytes)
+    return fail(P2C_ERR_INVALID, "dense group workspace too small: %zu < %zu bytes", workspace_bytes, need + 16);
+  DenseLayout L = carve(base, n);
   cudaStream_t s = as_stream(stream);
   init_kernel<<<1, 32, 0, s>>>(L);
   P2C_CUDA(cudaMemsetAsync(stats_dev, 0, sizeof(p2c_dense_group_stats), s));
@@ -669,33 +1135,43 @@ int p2c_dense_group_early_stop(int64_t n, const uint64_t* query_id_dev, const ui
                      uncertainty_score_dev};
     const int keep = config->preserve_input_order ? 1 : 0;
     parse_kernel<<<grid_for(n), kThreads, 0, s>>>(in, n, config->uncertainty_fallback_threshold, keep, L);
-    size_t tb = L.tmp_bytes;
-    const unsigned* order = L.idx[0];
-    if (!keep) {  // stable: priority desc, then cost asc, then index
-      P2C_CUDA(cub::DeviceRadixSort::SortPairs(L.tmp, tb, L.key[0], L.key[1], L.idx[0], L.idx[1], (int)n, 0, 64, s));
-      gather_qid_kernel<<<grid_for(n), kThreads, 0, s>>>(in.query_id, L.idx[1], n, L.qkey[0]);
-      order = L.idx[1];
-    }
-    tb = L.tmp_bytes;  // stable by query id: the final order
-    P2C_CUDA(cub::DeviceRadixSort::SortPairs(L.tmp, tb, L.qkey[0], L.qkey[1], order, L.idx[2], (int)n, 0, qbits, s));
-    gather_kernel<<<grid_for(n), kThreads, 0, s>>>(L.idx[2], L.qkey[1], n, L);
+    size_t tb = L.tmp_bytes;  // stable by query id
+    unsigned* order = L.idx[2];
+    P2C_CUDA(cub::DeviceRadixSort::SortPairs(L.tmp, tb, L.qkey[0], L.qkey[1], L.idx[0], order, (int)n, 0, qbits, s));
     tb = L.tmp_bytes;
-    P2C_CUDA(cub::DeviceSelect::Flagged(L.tmp, tb, L.iota, L.head, L.g_start, &L.acc->n_groups, (int)n, s));
-    P2C_CUDA(cudaMemsetAsync(L.terms, 0, sizeof(double) * 3 * (size_t)n, s));
+    P2C_CUDA(cub::DeviceSelect::If(L.tmp, tb, thrust::counting_iterator<unsigned>(0u), L.g_start, &L.acc->n_groups,
+                                   (int)n, IsHead{L.qkey[1]}, s));
     DeviceInfo info;
     if (int rc = current_device_info(&info)) return rc;
     const long long want = (n + (kThreads / 32) - 1) / (kThreads / 32);
     const int grid = (int)std::max(1ll, std::min(want, (long long)info.sm_count * 8));
-    group_kernel<<<grid, kThreads, 0, s>>>(n, config->representative_attempt_limit,
+    if (!keep) {  // priority desc, then cost asc, then index inside each group
+      order_small_kernel<<<grid, kThreads, 0, s>>>(n, order, L);
+      if (n > kWarpRows) {
+        const size_t smem = kTileRows * 12;
+        const int tiles = (int)std::min<long long>(n / kWarpRows + 1, info.sm_count * 4);
+        order_tile_kernel<<<tiles, kTileThreads, smem, s>>>(order, L);
+      }
+      if (n > (long long)kTileRows) {
+        void* args[] = {&order, &L};
+        P2C_CUDA(cudaLaunchCooperativeKernel((const void*)order_merge_kernel, dim3(info.sm_count), dim3(kThreads), args,
+                                             0, s));
+      }
+    }
+    group_kernel<<<grid, kThreads, 0, s>>>(order, n, config->representative_attempt_limit,
                                            config->interval_miss_penalty_scale, L);
-    tb = L.tmp_bytes;
-    P2C_CUDA(cub::DeviceSelect::If(L.tmp, tb, L.terms, L.compact, &L.acc->n_terms, (int)(3 * n), NonZeroTerm{}, s));
     FoldJob job{{L.compact, L.g_full, L.g_cost},
                 {&L.acc->n_terms, &L.acc->n_groups, &L.acc->n_groups},
-                {0, 0, 0},
                 {&stats_dev->learned_exact_work, &stats_dev->no_proposal_exact_work,
                  &stats_dev->cost_before_first_positive_sum}};
-    fold_kernel<<<3, kFoldThreads, 0, s>>>(job);
+    tb = L.tmp_bytes;
+    P2C_CUDA(cub::DeviceSelect::If(L.tmp, tb, L.terms, L.compact, &L.acc->n_terms, (int)(3 * n), NonZeroTerm{}, s));
+    const dim3 pieces((unsigned)std::min<long long>((3 * n + kFoldChunk - 1) / kFoldChunk, info.sm_count * 4), 3);
+    if (3 * n > kFoldChunk) {  // a first piece is folded term by term whatever its prediction
+      piece_sum_kernel<<<pieces, kFoldThreads, 0, s>>>(job, L.pieces, L.acc);
+      piece_inc_kernel<<<pieces, kFoldThreads, 0, s>>>(job, L.pieces);
+    }
+    piece_fold_kernel<<<3, kFoldThreads, 0, s>>>(job, L.pieces);
   }
   finish_kernel<<<1, 32, 0, s>>>(n, L, stats_dev);
   P2C_CUDA(cudaGetLastError());
@@ -706,8 +1182,7 @@ int p2c_ordered_sum(const double* terms_dev, int64_t n, double* out_dev, void* s
   using namespace p2c;
   if (n < 0) return fail(P2C_ERR_INVALID, "term count must be non-negative");
   if (out_dev == nullptr || (n > 0 && terms_dev == nullptr)) return fail(P2C_ERR_INVALID, "term or output pointer is null");
-  FoldJob job{{terms_dev, terms_dev, terms_dev}, {nullptr, nullptr, nullptr}, {n, 0, 0}, {out_dev, out_dev, out_dev}};
-  fold_kernel<<<1, kFoldThreads, 0, as_stream(stream)>>>(job);
+  fold_kernel<<<1, kFoldThreads, 0, as_stream(stream)>>>(terms_dev, n, out_dev);
   P2C_CUDA(cudaGetLastError());
   return P2C_OK;
 }
