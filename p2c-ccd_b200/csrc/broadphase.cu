@@ -654,39 +654,6 @@ __global__ void __launch_bounds__(kThreads) scatter_kernel(Lists L, const double
   }
 }
 
-// Pairs a warp has found, written 64 at a time: one atomic and two coalesced
-// stores instead of an atomic per step that finds any.
-struct PairBuffer {
-  unsigned long long* slots;  // shared, 96
-  unsigned n;                 // warp-uniform
-
-  __device__ __forceinline__ void flush(unsigned count, unsigned long long* out, unsigned long long cap,
-                                        unsigned long long* total) {
-    const int lane = threadIdx.x & 31;
-    __syncwarp();
-    unsigned long long base = 0;
-    if (lane == 0) base = atomicAdd(total, (unsigned long long)count);
-    base = __shfl_sync(kFull, base, 0);
-    for (unsigned k = (unsigned)lane; k < count; k += 32u)
-      if (base + k < cap) out[base + k] = slots[k];
-    __syncwarp();
-    if (count + (unsigned)lane < n) {  // at most 31 stay
-      const unsigned long long rest = slots[count + (unsigned)lane];
-      slots[lane] = rest;
-    }
-    n -= count;
-    __syncwarp();
-  }
-  __device__ __forceinline__ void append(bool found, unsigned long long key, unsigned long long* out,
-                                         unsigned long long cap, unsigned long long* total) {
-    const unsigned mask = __ballot_sync(kFull, found);
-    if (mask == 0u) return;
-    if (found) slots[n + (unsigned)__popc(mask & ((1u << (threadIdx.x & 31)) - 1u))] = key;
-    n += (unsigned)__popc(mask);
-    if (n >= 64u) flush(64u, out, cap, total);
-  }
-};
-
 // Lanes that share one scanning box: they look its columns' runs up side by
 // side and walk all runs as one list, eight entries at a time.  A 624k-triangle
 // cloth's candidates with 4 / 8 / 16 / 32 lanes per box: 1.89 / 1.81 / 1.96 /

@@ -290,4 +290,38 @@ __device__ __forceinline__ unsigned long long pair_key(unsigned a, unsigned b, i
   return pack_shift > 0 ? (((unsigned long long)a << pack_shift) | b) : (((unsigned long long)a << 32) | b);
 }
 
+
+// Pairs a warp has found, written 64 at a time: one atomic and two coalesced
+// stores instead of an atomic per step that finds any.
+struct PairBuffer {
+  unsigned long long* slots;  // shared, 96
+  unsigned n;                 // warp-uniform
+
+  __device__ __forceinline__ void flush(unsigned count, unsigned long long* out, unsigned long long cap,
+                                        unsigned long long* total) {
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+    unsigned long long base = 0;
+    if (lane == 0) base = atomicAdd(total, (unsigned long long)count);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    for (unsigned k = (unsigned)lane; k < count; k += 32u)
+      if (base + k < cap) out[base + k] = slots[k];
+    __syncwarp();
+    if (count + (unsigned)lane < n) {  // at most 31 stay
+      const unsigned long long rest = slots[count + (unsigned)lane];
+      slots[lane] = rest;
+    }
+    n -= count;
+    __syncwarp();
+  }
+  __device__ __forceinline__ void append(bool found, unsigned long long key, unsigned long long* out,
+                                         unsigned long long cap, unsigned long long* total) {
+    const unsigned mask = __ballot_sync(0xffffffffu, found);
+    if (mask == 0u) return;
+    if (found) slots[n + (unsigned)__popc(mask & ((1u << (threadIdx.x & 31)) - 1u))] = key;
+    n += (unsigned)__popc(mask);
+    if (n >= 64u) flush(64u, out, cap, total);
+  }
+};
+
 }  // namespace p2c

@@ -4,13 +4,14 @@
 // (proposal/proposal_features.cpp:122-205, 236-259), the 32-feature rows the
 // learned scheduler reads, kept on the device after p2c_proxy_candidates.
 //
-//   1. density: a sort of the slab ids and one of (object, slab) give the
-//      distinct slab and object counts and the cross-object same-slab pair
-//      count (pairs in one slab minus pairs in one (slab, object)); each
-//      element adds the number of earlier elements of its run;
-//   2. the first proxy (in scene order) of each (slab, type, object, patch):
-//      two stable sorts order the proxies by that tuple and then by index,
-//      and every candidate side finds its proxy by binary search;
+//   1. density: the distinct slab and object counts and the cross-object
+//      same-slab pair count (pairs in one slab minus pairs in one
+//      (slab, object));
+//   2. the first proxy (in scene order) of each (slab, type, object, patch),
+//      which every candidate side looks up;
+//      With width hints, counters indexed by (object, slab) and a hash table
+//      of the tuples; otherwise a sort of the slab ids, one of (object, slab)
+//      and one or two stable ones by the tuple give runs and an order to search;
 //   3. one thread per candidate forms the row with the reference's double
 //      arithmetic (bit-identical with --fmad=false) and float clamps.
 // p2c_runtime_feature_rows is the runtime form without a scene
@@ -18,6 +19,7 @@
 #include <cub/device/device_radix_sort.cuh>
 
 #include <algorithm>
+#include <cstring>
 
 #include "p2c_internal.cuh"
 
@@ -40,10 +42,19 @@ struct FeatureLayout {
   unsigned long long* k2;        // n: (slab << 8 | type) of the lookup order
   unsigned long long* ko;        // n: (object << patch_bits | patch) of the lookup order
   unsigned* idx;                 // n: proxy index of the lookup order
+  // tables
+  unsigned long long* hash_key;  // packed tuples, ~0 empty
+  unsigned* hash_first;          // their smallest proxy indices
+  unsigned hash_size;            // a power of two, at least 2 n
+  unsigned* group_count;         // 2^kGroupBits: proxies of (object, slab)
+  unsigned* slab_count;          // 2^kGroupBits
+  unsigned* object_seen;         // 2^kGroupBits
   void* tmp;
   size_t tmp_bytes;
   size_t total;
 };
+
+constexpr int kGroupBits = 14;
 
 FeatureLayout carve(void* base, long long n) {
   FeatureLayout L{};
@@ -63,6 +74,13 @@ FeatureLayout carve(void* base, long long n) {
   L.k2 = static_cast<unsigned long long*>(take(8 * N));
   L.ko = static_cast<unsigned long long*>(take(8 * N));
   L.idx = static_cast<unsigned*>(take(4 * N));
+  L.hash_size = 64;
+  while (L.hash_size < 2 * N) L.hash_size <<= 1;
+  L.hash_key = static_cast<unsigned long long*>(take(12 * (size_t)L.hash_size));
+  L.hash_first = reinterpret_cast<unsigned*>(L.hash_key == nullptr ? nullptr : L.hash_key + L.hash_size);
+  L.group_count = static_cast<unsigned*>(take((size_t)12 << kGroupBits));
+  L.slab_count = L.group_count == nullptr ? nullptr : L.group_count + (1 << kGroupBits);
+  L.object_seen = L.group_count == nullptr ? nullptr : L.group_count + (2 << kGroupBits);
   size_t t = 0;
   cub::DeviceRadixSort::SortPairs(nullptr, t, (const unsigned long long*)nullptr, (unsigned long long*)nullptr,
                                   (const unsigned*)nullptr, (unsigned*)nullptr, (int)N);
@@ -187,6 +205,81 @@ __global__ void packed_keys_kernel(p2c_proxy_scene sc, FeatureLayout L, PackedKe
   L.val[0][i] = (unsigned)i;
 }
 
+// Finaliser of splitmix64 (Steele, Lea and Flood 2014).
+__device__ __forceinline__ unsigned hash_of(unsigned long long x) {
+  x = (x ^ (x >> 30)) * 0xbf58476d1ce4e5b9ull;
+  x = (x ^ (x >> 27)) * 0x94d049bb133111ebull;
+  return (unsigned)(x ^ (x >> 31));
+}
+
+// The tables: one pass over the proxies instead of three sorts and two passes
+// over their runs.
+__global__ void tables_kernel(p2c_proxy_scene sc, FeatureLayout L, PackedKey pk, int sb, unsigned long long* err) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  unsigned slab = 0, obj = 0, patch = 0;
+  bool fits = false;
+  if (i < sc.n) {
+    slab = sc.slab_id[i], obj = sc.object_id[i], patch = sc.patch_id[i];
+    fits = pk.fits(slab, obj, patch, sb);
+    if (!fits) atomicOr(err, 4ull);
+  }
+  // proxies of one (object, slab) lie together: one atomic a warp and group
+  const unsigned group = fits ? (obj << sb) | slab : 0xffffffffu;
+  const unsigned m = __match_any_sync(0xffffffffu, group);
+  if (!fits) return;
+  if ((threadIdx.x & 31) == __ffs((int)m) - 1) {
+    atomicAdd(L.group_count + group, (unsigned)__popc(m));
+    atomicAdd(L.slab_count + slab, (unsigned)__popc(m));
+    L.object_seen[obj] = 1u;
+  }
+  const unsigned long long k = pk.make(slab, sc.proxy_type[i], obj, patch);
+  for (unsigned at = hash_of(k);; ++at) {  // at most half full: an end is always found
+    at &= L.hash_size - 1u;
+    const unsigned long long old = atomicCAS(L.hash_key + at, ~0ull, k);
+    if (old == ~0ull || old == k) {
+      atomicMin(L.hash_first + at, (unsigned)i);
+      return;
+    }
+  }
+}
+
+constexpr int kDensityThreads = 1024;
+
+// The sums runs_kernel forms, from the tables, into acc.
+__global__ void __launch_bounds__(kDensityThreads) table_sums_kernel(FeatureLayout L, int sb, int ob) {
+  unsigned long long same_slab = 0, same_group = 0, slabs = 0, objects = 0;
+  auto pairs = [](unsigned c) { return (unsigned long long)c * (c ? c - 1u : 0u) / 2ull; };
+  for (int k = threadIdx.x; k < 1 << (sb + ob); k += kDensityThreads) same_group += pairs(L.group_count[k]);
+  for (int k = threadIdx.x; k < 1 << sb; k += kDensityThreads) {
+    const unsigned c = L.slab_count[k];
+    same_slab += pairs(c);
+    slabs += c ? 1 : 0;
+  }
+  for (int k = threadIdx.x; k < 1 << ob; k += kDensityThreads) objects += L.object_seen[k] ? 1 : 0;
+  for (int o = 16; o > 0; o >>= 1) {
+    same_slab += __shfl_xor_sync(0xffffffffu, same_slab, o);
+    same_group += __shfl_xor_sync(0xffffffffu, same_group, o);
+    slabs += __shfl_xor_sync(0xffffffffu, slabs, o);
+    objects += __shfl_xor_sync(0xffffffffu, objects, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    if (same_slab) atomicAdd(L.acc + 0, same_slab);
+    if (same_group) atomicAdd(L.acc + 1, same_group);
+    if (slabs) atomicAdd(L.acc + 2, slabs);
+    if (objects) atomicAdd(L.acc + 3, objects);
+  }
+}
+
+// FindCandidatePrimitive from the hash table.
+__device__ __forceinline__ long long find_proxy_hashed(const FeatureLayout& L, unsigned long long k) {
+  for (unsigned at = hash_of(k);; ++at) {
+    at &= L.hash_size - 1u;
+    const unsigned long long e = L.hash_key[at];
+    if (e == k) return (long long)L.hash_first[at];
+    if (e == ~0ull) return -1;
+  }
+}
+
 __device__ __forceinline__ long long find_proxy_packed(const FeatureLayout& L, long long n, unsigned long long k) {
   const long long lo = lower_bound(L.k2, n, k);
   return (lo < n && L.k2[lo] == k) ? (long long)L.val[1][lo] : -1;
@@ -227,15 +320,13 @@ __device__ __forceinline__ double overlap(const double* l, const double* r, int 
   return dmax0(dmin_(l[3 + k], r[3 + k]) - dmax_(l[k], r[k]));
 }
 
-__global__ void rows_kernel(p2c_proxy_scene sc, FeatureLayout L, const p2c_candidate_record* cand, long long cap,
-                            const uint64_t* counts, const p2c_candidate_density* density,
-                            p2c_proposal_feature_row* rows, unsigned long long* err, bool packed, PackedKey pk,
-                            int sb) {
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long m = (long long)min((unsigned long long)counts[1], (unsigned long long)cap);
-  if (c >= m) return;
-  const p2c_candidate_record r = cand[c];
-  p2c_proposal_feature_row row{};
+// How the candidate sides find their proxies.
+enum class Lookup { kTuples, kPacked, kHashed };
+
+__device__ __forceinline__ void feature_row(const p2c_proxy_scene& sc, const FeatureLayout& L,
+                                            const p2c_candidate_record& r, const p2c_candidate_density* density,
+                                            p2c_proposal_feature_row& row, unsigned long long* err, Lookup how,
+                                            const PackedKey& pk, int sb) {
   // ValidateCandidateRecord (common/validators.cpp:160-181)
   bool ok = r.schema_version == 1u && r.candidate_id != 0 && r.query_id != 0 &&
             (r.proxy_type_a == 1 || r.proxy_type_a == 2) && (r.proxy_type_b == 1 || r.proxy_type_b == 2) &&
@@ -244,13 +335,18 @@ __global__ void rows_kernel(p2c_proxy_scene sc, FeatureLayout L, const p2c_candi
   const long long n = sc.n;
   const int pb = id_bits(sc.patch_bits);
   long long ia, ib;
-  if (packed) {  // a side with ids past the hints matches no proxy (all proxies fit them)
-    ia = pk.fits(r.slab_id, r.object_a_id, r.patch_a_id, sb)
-             ? find_proxy_packed(L, n, pk.make(r.slab_id, r.proxy_type_a, r.object_a_id, r.patch_a_id))
-             : -1;
-    ib = pk.fits(r.slab_id, r.object_b_id, r.patch_b_id, sb)
-             ? find_proxy_packed(L, n, pk.make(r.slab_id, r.proxy_type_b, r.object_b_id, r.patch_b_id))
-             : -1;
+  if (how != Lookup::kTuples) {  // a side with ids past the hints matches no proxy (all proxies fit them)
+    const bool fa = pk.fits(r.slab_id, r.object_a_id, r.patch_a_id, sb),
+               fb = pk.fits(r.slab_id, r.object_b_id, r.patch_b_id, sb);
+    const unsigned long long ka = pk.make(r.slab_id, r.proxy_type_a, r.object_a_id, r.patch_a_id),
+                             kb = pk.make(r.slab_id, r.proxy_type_b, r.object_b_id, r.patch_b_id);
+    if (how == Lookup::kHashed) {
+      ia = fa ? find_proxy_hashed(L, ka) : -1;
+      ib = fb ? find_proxy_hashed(L, kb) : -1;
+    } else {
+      ia = fa ? find_proxy_packed(L, n, ka) : -1;
+      ib = fb ? find_proxy_packed(L, n, kb) : -1;
+    }
   } else {
     ia = find_proxy(L, n, ((unsigned long long)r.slab_id << 8) | r.proxy_type_a,
                     ((unsigned long long)r.object_a_id << pb) | r.patch_a_id);
@@ -259,7 +355,6 @@ __global__ void rows_kernel(p2c_proxy_scene sc, FeatureLayout L, const p2c_candi
   }
   if (!ok || ia < 0 || ib < 0) {
     atomicOr(err, (!ok ? 1ull : 0ull) | (ia < 0 || ib < 0 ? 2ull : 0ull));
-    rows[c] = row;
     return;
   }
   const double* A = sc.bounds + 6 * ia;
@@ -313,7 +408,9 @@ __global__ void rows_kernel(p2c_proxy_scene sc, FeatureLayout L, const p2c_candi
   double centre = 0.5 * (t0 + t1);
   const double below_one = 0x1.fffffffffffffp-1;
   centre = centre < 0.0 ? 0.0 : (below_one < centre ? below_one : centre);
-  row.interval_targets[(unsigned)(centre * 8.0)] = 1.0f;
+  const unsigned bin = (unsigned)(centre * 8.0);
+#pragma unroll
+  for (unsigned k = 0; k < 8; ++k) row.interval_targets[k] = k == bin ? 1.0f : 0.0f;  // no dynamic index: registers
   row.family_targets[0] = 1.0f;
   row.family_targets[1] = 1.0f;
   row.priority_target = clamp_feature(0.5 * (double)r.rt_hit_count + 0.5 * d.candidates_per_proxy);
@@ -321,7 +418,41 @@ __global__ void rows_kernel(p2c_proxy_scene sc, FeatureLayout L, const p2c_candi
   const double f19 = (double)f[19];
   row.uncertainty_target = clamp_feature(1.0 - (f19 < 1.0 ? f19 : 1.0));
   row.target_mask = 31u;
-  rows[c] = row;
+}
+
+// One thread per candidate forms its row in registers; the warp turns its 32
+// rows over in shared memory and writes them as whole lines.  Written by each
+// thread for itself (256 bytes apart) and with two binary searches in turn,
+// the rows of 280,000 candidates took 88 us.
+constexpr int kRowThreads = 128;
+constexpr int kRowWords = (int)sizeof(p2c_proposal_feature_row) / 4;
+static_assert(sizeof(p2c_proposal_feature_row) == 256, "ProposalFeatureRow layout");
+
+__global__ void __launch_bounds__(kRowThreads) rows_kernel(p2c_proxy_scene sc, FeatureLayout L,
+                                                           const p2c_candidate_record* cand, long long cap,
+                                                           const uint64_t* counts,
+                                                           const p2c_candidate_density* density,
+                                                           p2c_proposal_feature_row* rows, unsigned long long* err,
+                                                           Lookup how, PackedKey pk, int sb) {
+  __shared__ unsigned turn[kRowThreads / 32][32 * (kRowWords + 1)];
+  const int lane = threadIdx.x & 31;
+  const long long first = ((long long)blockIdx.x * kRowThreads + threadIdx.x) - lane;
+  const long long m = (long long)min((unsigned long long)counts[1], (unsigned long long)cap);
+  if (first >= m) return;
+  unsigned* words = turn[threadIdx.x >> 5];
+  if (first + lane < m) {
+    const p2c_candidate_record r = cand[first + lane];
+    p2c_proposal_feature_row row{};
+    feature_row(sc, L, r, density, row, err, how, pk, sb);
+    unsigned w[kRowWords];
+    memcpy(w, &row, sizeof(row));
+#pragma unroll
+    for (int k = 0; k < kRowWords; ++k) words[lane * (kRowWords + 1) + k] = w[k];
+  }
+  __syncwarp();
+  const int live = (int)min(32ll, m - first);
+  unsigned* out = reinterpret_cast<unsigned*>(rows + first);
+  for (int k = lane; k < live * kRowWords; k += 32) out[k] = words[k / kRowWords * (kRowWords + 1) + k % kRowWords];
 }
 
 // BuildRuntimeFeatureRowFromDerived (proposal/proposal_policy.cpp:184-226):
@@ -452,7 +583,19 @@ int p2c_proposal_feature_rows(const p2c_proxy_scene* scene, const p2c_candidate_
   const int sb = id_bits(sc.slab_bits), ob = id_bits(sc.object_bits), pb = id_bits(sc.patch_bits);
   P2C_CUDA(cudaMemsetAsync(L.acc, 0, 32, s));
   P2C_CUDA(cudaMemsetAsync(error_word_dev, 0, sizeof(uint64_t), s));
-  if (n > 0) {
+  const bool packed = sc.slab_bits > 0 && sc.object_bits > 0 && sc.patch_bits > 0 && sb + 8 + ob + pb <= 64;
+  PackedKey pk{ob, pb};
+  // Tables: two passes where the sorts are 22 launches (51,200 proxies: 15 us
+  // against 128).  A word of 64 bits could equal the empty key; more (object,
+  // slab) groups than 2^14 would take longer to sum on one block than to sort.
+  const bool hashed = packed && sb + 8 + ob + pb < 64 && sb + ob <= kGroupBits;
+  if (n > 0 && hashed) {
+    P2C_CUDA(cudaMemsetAsync(L.hash_key, 0xff, 12 * (size_t)L.hash_size, s));
+    P2C_CUDA(cudaMemsetAsync(L.group_count, 0, (size_t)12 << kGroupBits, s));
+    tables_kernel<<<grid_for(n), kThreads, 0, s>>>(sc, L, pk, sb, reinterpret_cast<unsigned long long*>(error_word_dev));
+    table_sums_kernel<<<1, kDensityThreads, 0, s>>>(L, sb, ob);
+  }
+  if (n > 0 && !hashed) {
     size_t tb;
     // density: runs of slab ids, then of (object, slab)
     density_keys_kernel<<<grid_for(n), kThreads, 0, s>>>(sc, L, 0, sb);
@@ -465,16 +608,14 @@ int p2c_proposal_feature_rows(const p2c_proxy_scene* scene, const p2c_candidate_
                                              s));
     runs_kernel<<<grid_for(n), kThreads, 0, s>>>(L, n, 1, 3, sb);
   }
-  const bool packed = sc.slab_bits > 0 && sc.object_bits > 0 && sc.patch_bits > 0 && sb + 8 + ob + pb <= 64;
-  PackedKey pk{ob, pb};
-  if (n > 0 && packed) {
+  if (n > 0 && packed && !hashed) {
     // lookup order in one sort of (slab, type, object, patch) words, ties by proxy index (stable)
     size_t tb = L.tmp_bytes;
     packed_keys_kernel<<<grid_for(n), kThreads, 0, s>>>(sc, L, pk, sb,
                                                          reinterpret_cast<unsigned long long*>(error_word_dev));
     P2C_CUDA(cub::DeviceRadixSort::SortPairs(L.tmp, tb, L.key[0], L.k2, L.val[0], L.val[1], (int)n, 0,
                                              sb + 8 + ob + pb, s));
-  } else if (n > 0) {
+  } else if (n > 0 && !hashed) {
     size_t tb;
     // lookup order: (slab, type, object, patch), ties by proxy index (stable passes)
     lookup_keys_kernel<<<grid_for(n), kThreads, 0, s>>>(sc, L, pb);
@@ -488,9 +629,10 @@ int p2c_proposal_feature_rows(const p2c_proxy_scene* scene, const p2c_candidate_
   }
   density_kernel<<<1, 32, 0, s>>>(sc, L, counts_dev, density_dev);
   if (cap > 0)
-    rows_kernel<<<grid_for(cap), kThreads, 0, s>>>(sc, L, candidates_dev, cap, counts_dev, density_dev, rows_dev,
-                                                  reinterpret_cast<unsigned long long*>(error_word_dev), packed, pk,
-                                                  sb);
+    rows_kernel<<<(unsigned)((cap + kRowThreads - 1) / kRowThreads), kRowThreads, 0, s>>>(
+        sc, L, candidates_dev, cap, counts_dev, density_dev, rows_dev,
+        reinterpret_cast<unsigned long long*>(error_word_dev),
+        hashed ? Lookup::kHashed : (packed ? Lookup::kPacked : Lookup::kTuples), pk, sb);
   P2C_CUDA(cudaGetLastError());
   return P2C_OK;
 }

@@ -6,20 +6,20 @@
 //   1. one radix sort orders the proxies by (slab, column of the min corner
 //      over the two narrower axes, quantised min along the widest axis), and
 //      they are gathered into that order as struct-of-arrays;
-//   2. a column-subdivided sweep: each proxy scans the columns and the
-//      sweep-axis window its partners' min corners can lie in, and emits the
+//   2. a column-subdivided sweep: eight lanes look up the columns and the
+//      sweep-axis windows a proxy's partners can lie in, walk them together and emit the
 //      pairs of different objects whose time intervals and inclusive AABBs
 //      overlap, as (lo << 32 | hi) keys, each pair once;
 //   3. one radix sort of the keys gives the reference's (i, j) hit order and
 //      the 64-byte RawCandidateHit records are written from the keys;
-//   4. dense ranks of the slab ids and of the (object, patch) pairs keep the
-//      order of the reference's compaction key (slab, first object, first
-//      patch, second object, second patch, first type, second type), so two
-//      stable radix sorts of exact bit widths order the hits by it; the
+//   4. the hits are sorted by the reference's compaction key (slab, first
+//      object, first patch, second object, second patch, first type, second
+//      type), packed into one word by the ids' width hints, or, without hints
+//      that fit, by dense ranks of the slab ids and of the (object, patch)
+//      pairs in one or two stable radix sorts of exact bit widths; the
 //      head of every run writes one CandidateRecord (ids 1, 2, ... in key
 //      order) with the run's hit count, the float maximum of its motion
 //      bounds and its flags.
-#include <cooperative_groups.h>
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 
@@ -31,8 +31,6 @@
 
 namespace p2c {
 namespace {
-
-namespace cg = cooperative_groups;
 
 static_assert(sizeof(p2c_raw_candidate_hit) == 64, "RawCandidateHit layout");
 static_assert(sizeof(p2c_candidate_record) == 80, "CandidateRecord layout");
@@ -63,9 +61,10 @@ struct ProxyStats {
 };
 
 // Columns over the two non-sweep axes (each box stored in the column of its
-// min corner) and a 16-bit quantiser of the sweep-axis min.
+// min corner) and a 16-bit quantiser of the sweep-axis min, of which the low
+// drop_bits are zero.
 struct ProxyGrid {
-  int axis, a1, a2, g1, g2;
+  int axis, a1, a2, g1, g2, drop_bits;
   double base0, scale0, base1, inv1, base2, inv2, reach1, reach2;
 };
 
@@ -252,7 +251,7 @@ __device__ __forceinline__ int clamp_index(double c, int hi) {
 // Sweep axis = the widest spread of min corners; columns over the other two
 // axes one (direct table: a column costs one 16-byte load) or two (binary
 // search) mean extents wide, at most kMaxColumns each.
-__global__ void grid_kernel(ProxyLayout L, long long n) {
+__global__ void grid_kernel(ProxyLayout L, long long n, int drop_bits) {
   const double width_mult = L.table_bits > 0 ? 1.0 : 2.0;
   if (threadIdx.x != 0) return;
   const ProxyStats& S = *L.stats;
@@ -284,6 +283,7 @@ __global__ void grid_kernel(ProxyLayout L, long long n) {
   }
   g.g1 = gg[0];
   g.g2 = gg[1];
+  g.drop_bits = drop_bits;
   g.base1 = base[g.a1];
   g.inv1 = inv[0];
   g.base2 = base[g.a2];
@@ -301,7 +301,7 @@ __device__ __forceinline__ int proxy_column(double x, double base, double inv, i
 
 // Monotone (non-decreasing) in x.
 __device__ __forceinline__ unsigned proxy_quantise(double x, const ProxyGrid& g) {
-  return (unsigned)clamp_index(floor((x - g.base0) * g.scale0), 65535);
+  return (unsigned)clamp_index(floor((x - g.base0) * g.scale0), 65535) >> g.drop_bits << g.drop_bits;
 }
 
 __global__ void cell_keys_kernel(p2c_proxy_scene sc, ProxyLayout L) {
@@ -379,24 +379,22 @@ __device__ __forceinline__ long long lower_bound(const unsigned long long* __res
 // GenerateRawCandidatesCpu's (candidate_buffer.cpp:158-173: different
 // objects, same slab, TimeOverlap, inclusive AabbOverlap).
 //
-// kSweepLanes lanes share one box and take its columns in turn: the work of
-// a box is a chain of dependent loads (a column lookup, a search for the
-// window's start, then the window's walk), and splitting it shortens the
-// chain and fills the SMs.  With narrow slab ids a direct (slab, column)
-// table gives each column's run and lets columns whose boxes cannot reach
-// the scanning box be skipped; otherwise a binary search over all keys
-// finds each window.
+// kSweepLanes lanes share one box: they look its columns up side by side (a
+// direct (slab, column) table when slab ids are narrow, which also skips
+// columns that cannot reach the box; else a binary search over all keys),
+// lay the windows end to end and walk them together, and a warp stages its
+// pairs.  One lane walking each window, with an atomic for every step that
+// found a pair, took 209 us for 51,200 proxies with 280,000 hits; now 108.
 constexpr int kSweepLanes = 8;
+constexpr unsigned kWholeRun = 8;  // a column of at most this many entries is walked without a search
 
-// 6 blocks of 256 threads per SM (40 registers, a few spilled values): more
-// warps to hide the walk's load latency than the 4 blocks the unbounded
-// 54-register build allows (1.64 M proxies: 7.6 -> 7.1 ms per step).
-__global__ void __launch_bounds__(kThreads, 6) sweep_kernel(ProxyLayout L, long long n, unsigned long long cap,
+__global__ void __launch_bounds__(kThreads, 4) sweep_kernel(ProxyLayout L, long long n, unsigned long long cap,
                                                          int rank_bits) {
+  __shared__ unsigned long long slots[kThreads / 32][96];
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long p = t / kSweepLanes;
-  const int lane = (int)(t % kSweepLanes);
-  if (p >= n) return;
+  const long long p = min(t / kSweepLanes, n - 1);
+  const int member = (int)(t % kSweepLanes);
+  PairBuffer found_pairs{slots[threadIdx.x >> 5], 0u};
   const ProxyGrid g = *L.grid;
   const double* __restrict__ B = L.s_box;
   const unsigned long long* __restrict__ K = L.key[1];
@@ -411,53 +409,84 @@ __global__ void __launch_bounds__(kThreads, 6) sweep_kernel(ProxyLayout L, long 
   const int c1b = proxy_column(ahi, g.base1, g.inv1, g.g1);
   const int c2a = proxy_column(blo - g.reach2 - (fabs(blo) + g.reach2) * 0x1p-40, g.base2, g.inv2, g.g2);
   const int c2b = proxy_column(bhi, g.base2, g.inv2, g.g2);
-  const int n2 = c2b - c2a + 1, n_cells = (c1b - c1a + 1) * n2;
+  const int n2 = c2b - c2a + 1;
+  int n_cells = (c1b - c1a + 1) * n2;
+  // past the end, or past the slab width hint (error word bit 8)
+  if (t / kSweepLanes >= n || (L.table_bits > 0 && (slab >> L.table_bits))) n_cells = 0;
   const unsigned q_lo = proxy_quantise(lo, g), q_hi = proxy_quantise(hi, g);
   // column-axis bounds rounded outward: a pair that overlaps in doubles
   // overlaps in these floats, so they reject most entries with one load
   const float f_alo = __double2float_rd(alo), f_ahi = __double2float_ru(ahi), f_blo = __double2float_rd(blo),
               f_bhi = __double2float_ru(bhi);
-  // one partner entry j: prefilter, ownership, exact overlap, object and time tests, then append
-  auto visit = [&](long long j) {
-    const float4 f = L.s_f[j];
-    if (f.y < f_alo || f_ahi < f.x || f.w < f_blo || f_bhi < f.z) return;
-    const double lj = B[j];
-    const unsigned idj = L.order[1][j];
-    if (lj < lo || (lj == lo && idj <= id) || lj > hi) return;  // owned by the other box / no overlap
-    if (B[3 * n + j] < alo || ahi < B[2 * n + j] || B[5 * n + j] < blo || bhi < B[4 * n + j]) return;
-    if (L.s_obj[j] == obj || !(t0 < L.s_t1[j] && L.s_t0[j] < t1)) return;
-    const cg::coalesced_group grp = cg::coalesced_threads();
-    unsigned long long base = 0;
-    if (grp.thread_rank() == 0) base = atomicAdd(L.counter, (unsigned long long)grp.size());
-    base = grp.shfl(base, 0);
-    const unsigned long long slot = base + grp.thread_rank();
-    if (slot < cap)
-      L.pairs[0][slot] = ((unsigned long long)min(id, idj) << rank_bits) | (unsigned long long)max(id, idj);
-  };
-  if (L.table_bits > 0) {
-    if (slab >> L.table_bits) return;  // past the slab width hint (error word bit 8)
-    const unsigned k_alo = fkey_down(alo), k_blo = fkey_down(blo);
-    for (int k = lane; k < n_cells; k += kSweepLanes) {
-      const int c1 = c1a + k / n2, c2 = c2a + k % n2;
-      const uint4 c = L.cells[(slab << kCellBits) | (unsigned long long)(c1 * g.g2 + c2)];
-      // empty, or no box of this column reaches the scanning box on a column axis
-      if (c.x >= c.y || c.z < k_alo || c.w < k_blo) continue;
-      unsigned b = c.x, r = c.y;
-      while (b < r) {  // first entry of the column with q >= q_lo
-        const unsigned m = (b + r) >> 1;
-        if ((unsigned)(K[m] & 0xffffull) < q_lo) b = m + 1;
-        else r = m;
+  const unsigned k_alo = fkey_down(alo), k_blo = fkey_down(blo);
+  for (int k = member; __any_sync(kFull, k - member < n_cells); k += kSweepLanes) {
+    unsigned begin = 0u, len = 0u;  // this lane's window
+    if (k < n_cells) {
+      const unsigned cell = (unsigned)((c1a + k / n2) * g.g2 + c2a + k % n2);
+      if (L.table_bits > 0) {
+        const uint4 c = L.cells[(slab << kCellBits) | cell];
+        // not empty, and some box of this column reaches the scanning box on both column axes
+        if (c.x < c.y && c.z >= k_alo && c.w >= k_blo) {
+          begin = c.x;
+          len = c.y - c.x;
+          if (len > kWholeRun) {
+            unsigned b = c.x, r = c.y;
+            while (b < r) {  // first entry of the column with q >= q_lo
+              const unsigned m = (b + r) >> 1;
+              if ((unsigned)(K[m] & 0xffffull) < q_lo) b = m + 1;
+              else r = m;
+            }
+            begin = b;
+            r = c.y;
+            while (b < r) {  // first one with q > q_hi
+              const unsigned m = (b + r) >> 1;
+              if ((unsigned)(K[m] & 0xffffull) <= q_hi) b = m + 1;
+              else r = m;
+            }
+            len = b - begin;
+          }
+        }
+      } else {
+        const unsigned long long key = (slab << 30) | ((unsigned long long)cell << 16);
+        begin = (unsigned)lower_bound(K, n, key | q_lo);
+        len = (unsigned)lower_bound(K, n, (key | q_hi) + 1ull) - begin;
       }
-      for (unsigned j = b; j < c.y && (unsigned)(K[j] & 0xffffull) <= q_hi; ++j) visit(j);
     }
-    return;
+    unsigned before = len;  // inclusive, then exclusive sum of the windows over the box's lanes
+#pragma unroll
+    for (int d = 1; d < kSweepLanes; d <<= 1) {
+      const unsigned up = __shfl_up_sync(kFull, before, d, kSweepLanes);
+      if (member >= d) before += up;
+    }
+    const unsigned entries = __shfl_sync(kFull, before, kSweepLanes - 1, kSweepLanes);
+    before -= len;
+    begin -= before;
+    for (unsigned e = (unsigned)member; __any_sync(kFull, e - (unsigned)member < entries); e += kSweepLanes) {
+      int run = 0;  // the last window that starts at or before entry e
+#pragma unroll
+      for (int d = kSweepLanes / 2; d > 0; d >>= 1) {
+        const unsigned at = __shfl_sync(kFull, before, run + d, kSweepLanes);
+        if (at <= e) run += d;
+      }
+      const unsigned j = __shfl_sync(kFull, begin, run, kSweepLanes) + e;
+      bool found = false;
+      unsigned long long key = 0ull;
+      if (e < entries) {
+        const float4 f = L.s_f[j];
+        const double lj = B[j];
+        if (!(f.y < f_alo || f_ahi < f.x || f.w < f_blo || f_bhi < f.z) && !(lj < lo || lj > hi)) {
+          const unsigned idj = L.order[1][j];
+          // the box with the smaller (min, index) owns the pair
+          found = !(lj == lo && idj <= id) && !(B[3 * n + j] < alo || ahi < B[2 * n + j] || B[5 * n + j] < blo ||
+                                                bhi < B[4 * n + j]) &&
+                  L.s_obj[j] != obj && t0 < L.s_t1[j] && L.s_t0[j] < t1;
+          key = ((unsigned long long)min(id, idj) << rank_bits) | (unsigned long long)max(id, idj);
+        }
+      }
+      found_pairs.append(found, key, L.pairs[0], cap, L.counter);
+    }
   }
-  for (int k = lane; k < n_cells; k += kSweepLanes) {
-    const int c1 = c1a + k / n2, c2 = c2a + k % n2;
-    const unsigned long long cell = (slab << 30) | ((unsigned long long)(c1 * g.g2 + c2) << 16);
-    const unsigned long long k_end = cell | q_hi;
-    for (long long j = lower_bound(K, n, cell | q_lo); j < n && K[j] <= k_end; ++j) visit(j);
-  }
+  if (found_pairs.n != 0u) found_pairs.flush(found_pairs.n, L.pairs[0], cap, L.counter);
 }
 
 // Dense ranks that preserve the compaction key's order
@@ -518,9 +547,19 @@ __device__ __forceinline__ bool bound_valid(float v) {
 // two proxy types 1 / 2 as one bit each): one key (D, first, second, types)
 // when it fits 64 bits, else two chunks (second, types) and (D, first).
 struct CompactionKey {
-  int rank_bits;  // bits of a proxy index and of an (object, patch) rank
-  int d_bits;     // bits of a slab rank
+  int rank_bits;  // bits of a proxy index
+  int d_bits;     // bits of a slab rank (or id)
+  int op_bits;    // bits of an (object, patch) rank (or pair of ids)
   bool single;    // the whole key fits one 64-bit chunk
+  int id_patch;   // >= 0: ids instead of ranks, with that many patch bits
+  __device__ __forceinline__ unsigned long long slab(const p2c_proxy_scene& sc, const ProxyLayout& L,
+                                                     unsigned i) const {
+    return id_patch >= 0 ? sc.slab_id[i] : L.rank_slab[i];
+  }
+  __device__ __forceinline__ unsigned long long op(const p2c_proxy_scene& sc, const ProxyLayout& L,
+                                                   unsigned i) const {
+    return id_patch >= 0 ? ((unsigned long long)sc.object_id[i] << id_patch) | sc.patch_id[i] : L.rank_op[i];
+  }
 };
 
 __global__ void raw_hits_kernel(p2c_proxy_scene sc, ProxyLayout L, const unsigned long long* sorted,
@@ -557,10 +596,10 @@ __global__ void raw_hits_kernel(p2c_proxy_scene sc, ProxyLayout L, const unsigne
   const unsigned f = sw ? j : i, t = sw ? i : j;
   const unsigned long long types = ((unsigned long long)((sc.proxy_type[f] - 1u) & 1u) << 1) |
                                    ((sc.proxy_type[t] - 1u) & 1u);
-  const unsigned long long lo = ((unsigned long long)L.rank_op[t] << 2) | types;  // rank_bits + 2 bits
-  const unsigned long long hi = ((unsigned long long)L.rank_slab[i] << ck.rank_bits) | L.rank_op[f];
+  const unsigned long long lo = (ck.op(sc, L, t) << 2) | types;  // op_bits + 2 bits
+  const unsigned long long hi = (ck.slab(sc, L, i) << ck.op_bits) | ck.op(sc, L, f);
   if (ck.single) {
-    L.ck[0][h] = (hi << (ck.rank_bits + 2)) | lo;
+    L.ck[0][h] = (hi << (ck.op_bits + 2)) | lo;
   } else {
     L.ck[0][h] = lo;
     L.ck[1][h] = hi;
@@ -629,10 +668,10 @@ __global__ void external_hits_kernel(p2c_proxy_scene sc, ProxyLayout L, const p2
   const unsigned f = sw ? j : i, t = sw ? i : j;
   const unsigned long long types = ((unsigned long long)((sc.proxy_type[f] - 1u) & 1u) << 1) |
                                    ((sc.proxy_type[t] - 1u) & 1u);
-  const unsigned long long lo = ((unsigned long long)L.rank_op[t] << 2) | types;
-  const unsigned long long hi = ((unsigned long long)L.rank_slab[i] << ck.rank_bits) | L.rank_op[f];
+  const unsigned long long lo = (ck.op(sc, L, t) << 2) | types;
+  const unsigned long long hi = (ck.slab(sc, L, i) << ck.op_bits) | ck.op(sc, L, f);
   if (ck.single) {
-    L.ck[0][h] = (hi << (ck.rank_bits + 2)) | lo;
+    L.ck[0][h] = (hi << (ck.op_bits + 2)) | lo;
   } else {
     L.ck[0][h] = lo;
     L.ck[1][h] = hi;
@@ -736,9 +775,28 @@ int proxy_checks(const p2c_proxy_scene* scene) {
   return P2C_OK;
 }
 
-// Validation, the sorted proxy layout of the sweep and the dense slab and
-// (object, patch) ranks the compaction keys are built from.
-int prepare(ProxyRun& R, cudaStream_t s) {
+// Keys from the ids themselves when the hinted widths fit one word and cost at
+// most one radix pass more than the ranks would: that saves two scans, a sort
+// and eight small launches (51,200 proxies: 69 us).
+CompactionKey compaction_key(const ProxyRun& R) {
+  CompactionKey ckey;
+  ckey.rank_bits = R.rank_bits;
+  ckey.d_bits = std::min(R.rank_bits, R.slab_bits);  // slab ranks < min(n, 2^slab_bits)
+  ckey.op_bits = R.rank_bits;
+  ckey.id_patch = -1;
+  const int by_rank = ckey.d_bits + 2 * ckey.op_bits + 2, by_id = R.slab_bits + 2 * (R.object_bits + R.patch_bits) + 2;
+  if (by_id <= 64 && (by_id + 7) / 8 <= (by_rank + 7) / 8 + 1) {
+    ckey.d_bits = R.slab_bits;
+    ckey.op_bits = R.object_bits + R.patch_bits;
+    ckey.id_patch = R.patch_bits;
+  }
+  ckey.single = ckey.d_bits + 2 * ckey.op_bits + 2 <= 64;
+  return ckey;
+}
+
+// Validation, the sorted proxy layout of the sweep and, for compaction keys
+// by rank, the dense slab and (object, patch) ranks.
+int prepare(ProxyRun& R, const CompactionKey& ckey, cudaStream_t s) {
   const p2c_proxy_scene& sc = R.sc;
   ProxyLayout& L = R.L;
   const long long n = R.n;
@@ -746,17 +804,21 @@ int prepare(ProxyRun& R, cudaStream_t s) {
   if (n > 0) {
     stats_init_kernel<<<1, 32, 0, s>>>(L);
     keys_kernel<<<grid_for(n), kThreads, 0, s>>>(sc, L);
-    grid_kernel<<<1, 32, 0, s>>>(L, n);
+    // 30 + slab_bits key bits: up to six slab bits cost no fifth radix pass when
+    // the quantiser gives up as many as exceed 32 (a column holds a few boxes)
+    const int drop_bits = L.table_bits > 2 ? L.table_bits - 2 : 0;
+    grid_kernel<<<1, 32, 0, s>>>(L, n, drop_bits);
     cell_keys_kernel<<<grid_for(n), kThreads, 0, s>>>(sc, L);
     size_t tb = L.tmp_bytes;
     // (slab, column, quantised min) order, ties in proxy order
-    P2C_CUDA(cub::DeviceRadixSort::SortPairs(L.tmp, tb, L.key[0], L.key[1], L.order[0], L.order[1], (int)n, 0,
-                                             30 + R.slab_bits, s));
+    P2C_CUDA(cub::DeviceRadixSort::SortPairs(L.tmp, tb, L.key[0], L.key[1], L.order[0], L.order[1], (int)n,
+                                             drop_bits, 30 + R.slab_bits, s));
     gather_kernel<<<grid_for(n), kThreads, 0, s>>>(sc, L);
     if (L.table_bits > 0) {
       P2C_CUDA(cudaMemsetAsync(L.cells, 0, L.table_bytes, s));
       table_kernel<<<grid_for(n), kThreads, 0, s>>>(L, n);
     }
+    if (ckey.id_patch >= 0) return P2C_OK;
     // dense slab ranks from the sorted keys; dense (object, patch) ranks from one more sort
     slab_flags_kernel<<<grid_for(n), kThreads, 0, s>>>(L, n);
     tb = L.tmp_bytes;
@@ -779,17 +841,21 @@ int prepare(ProxyRun& R, cudaStream_t s) {
 int compact(ProxyRun& R, const CompactionKey& ckey, const p2c_raw_candidate_hit* raw, long long cap,
             p2c_candidate_record* candidates_dev, uint64_t* counts_dev, cudaStream_t s) {
   ProxyLayout& L = R.L;
-  const int rank_bits = ckey.rank_bits;
   const int n_chunks = ckey.single ? 1 : 2;
   const unsigned long long* chunk[2] = {L.ck[0], L.ck[1]};
-  const int chunk_bits[2] = {ckey.single ? ckey.d_bits + 2 * rank_bits + 2 : rank_bits + 2, ckey.d_bits + rank_bits};
+  const int chunk_bits[2] = {ckey.single ? ckey.d_bits + 2 * ckey.op_bits + 2 : ckey.op_bits + 2,
+                             ckey.d_bits + ckey.op_bits};
   unsigned* perm_in = L.perm[0];
   unsigned* perm_out = L.perm[1];
   size_t tb;
   for (int c = 0; c < n_chunks; ++c) {
-    gather_chunk_kernel<<<grid_for(cap), kThreads, 0, s>>>(chunk[c], perm_in, L.gk[0], cap);
+    const unsigned long long* keys = chunk[0];  // the first chunk is in hit order, as perm_in is
+    if (c > 0) {
+      gather_chunk_kernel<<<grid_for(cap), kThreads, 0, s>>>(chunk[c], perm_in, L.gk[0], cap);
+      keys = L.gk[0];
+    }
     tb = L.tmp_bytes;
-    P2C_CUDA(cub::DeviceRadixSort::SortPairs(L.tmp, tb, L.gk[0], L.gk[1], perm_in, perm_out, (int)cap, 0,
+    P2C_CUDA(cub::DeviceRadixSort::SortPairs(L.tmp, tb, keys, L.gk[1], perm_in, perm_out, (int)cap, 0,
                                              chunk_bits[c], s));
     std::swap(perm_in, perm_out);
   }
@@ -800,14 +866,6 @@ int compact(ProxyRun& R, const CompactionKey& ckey, const p2c_raw_candidate_hit*
                                                     reinterpret_cast<unsigned long long*>(counts_dev));
   P2C_CUDA(cudaGetLastError());
   return P2C_OK;
-}
-
-CompactionKey compaction_key(const ProxyRun& R) {
-  CompactionKey ckey;
-  ckey.rank_bits = R.rank_bits;
-  ckey.d_bits = std::min(R.rank_bits, R.slab_bits);  // slab ranks < min(n, 2^slab_bits)
-  ckey.single = ckey.d_bits + 2 * R.rank_bits + 2 <= 64;
-  return ckey;
 }
 
 int setup(const p2c_proxy_scene* scene, long long raw_cap, void* workspace_dev, size_t workspace_bytes,
@@ -843,7 +901,8 @@ int p2c_proxy_candidates(const p2c_proxy_scene* scene, p2c_raw_candidate_hit* ra
   ProxyRun R;
   if (int rc = setup(scene, raw_cap, workspace_dev, workspace_bytes, R)) return rc;
   cudaStream_t s = as_stream(stream);
-  if (int rc = prepare(R, s)) return rc;
+  const CompactionKey ckey = compaction_key(R);
+  if (int rc = prepare(R, ckey, s)) return rc;
   ProxyLayout& L = R.L;
   const long long n = R.n, cap = raw_cap;
   if (cap > 0) fill_kernel<<<grid_for(cap), kThreads, 0, s>>>(L.pairs[0], cap);
@@ -851,7 +910,6 @@ int p2c_proxy_candidates(const p2c_proxy_scene* scene, p2c_raw_candidate_hit* ra
   if (n > 0) sweep_kernel<<<grid_for(n * kSweepLanes), kThreads, 0, s>>>(L, n, (unsigned long long)cap, R.rank_bits);
   if (cap > 0) {
     size_t tb = L.tmp_bytes;
-    const CompactionKey ckey = compaction_key(R);
     // the hits in (i, j) order
     P2C_CUDA(cub::DeviceRadixSort::SortKeys(L.tmp, tb, L.pairs[0], L.pairs[1], (int)cap, 0, 2 * R.rank_bits, s));
     raw_hits_kernel<<<grid_for(cap), kThreads, 0, s>>>(R.sc, L, L.pairs[1], (unsigned long long)cap, ckey, raw_dev);
@@ -880,13 +938,13 @@ int p2c_compact_raw_candidates(const p2c_proxy_scene* scene, const p2c_raw_candi
   ProxyRun R;
   if (int rc = setup(scene, n_raw, workspace_dev, workspace_bytes, R)) return rc;
   cudaStream_t s = as_stream(stream);
-  if (int rc = prepare(R, s)) return rc;
+  const CompactionKey ckey = compaction_key(R);
+  if (int rc = prepare(R, ckey, s)) return rc;
   set_hits_kernel<<<1, 32, 0, s>>>(R.L, n_raw);
   if (n_raw == 0) {
     records_kernel<<<1, kThreads, 0, s>>>(R.sc, R.L, R.L.perm[0], raw_dev, 0, candidates_dev,
                                           reinterpret_cast<unsigned long long*>(counts_dev));
   } else {
-    const CompactionKey ckey = compaction_key(R);
     external_hits_kernel<<<grid_for(n_raw), kThreads, 0, s>>>(R.sc, R.L, raw_dev, n_raw, ckey);
     if (int rc = compact(R, ckey, raw_dev, n_raw, candidates_dev, counts_dev, s)) return rc;
   }
