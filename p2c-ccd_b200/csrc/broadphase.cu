@@ -31,16 +31,16 @@
 //   4. one sweep launch for both families: 16 lanes share a box, look up its
 //      columns' runs side by side and walk the runs' entries together;
 //   5. pair lists that fit are ranked by counting smaller keys (all SMs at
-//      once); longer ones are radix sorted.
+//      once); longer ones are put into rows by their first primitive, and
+//      each row orders itself (pair_rows.cuh).
 // Overlapping boxes of different objects imply overlapping object envelopes
 // (each box lies inside its object's envelope), so beyond culling only the
 // same-object rule remains.
-#include <cub/device/device_radix_sort.cuh>
-
 #include <algorithm>
 #include <cmath>
 
 #include "broadphase.cuh"
+#include "pair_rows.cuh"
 
 namespace p2c {
 namespace {
@@ -797,22 +797,8 @@ __global__ void __launch_bounds__(kThreads, P2C_SWEEP_BLOCKS)
   if (eeb.n != 0u) eeb.flush(eeb.n, ee.out, ee.cap, &sc->ee_count);
 }
 
-__global__ void fill_u64_kernel(unsigned long long* p, long long n, unsigned long long v) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) p[i] = v;
-}
-
 __device__ __forceinline__ unsigned long long unpack_pair(unsigned long long k, int shift) {
   return ((k >> shift) << 32) | (k & ((1ull << shift) - 1ull));
-}
-
-// Packed (a << shift | b) keys back to (a << 32 | b); padding stays ~0.
-__global__ void unpack_pairs_kernel(unsigned long long* p, long long n, int shift) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const unsigned long long k = p[i];
-  if (k == ~0ull) return;
-  p[i] = unpack_pair(k, shift);
 }
 
 __device__ __forceinline__ void export_counts(const SceneScratch* sc, unsigned long long* counts) {
@@ -898,13 +884,6 @@ struct Carver {
   }
 };
 
-size_t sort_keys_temp_bytes(long long n) {
-  size_t bytes = 0;
-  cub::DoubleBuffer<unsigned long long> k(nullptr, nullptr);
-  cub::DeviceRadixSort::SortKeys(nullptr, bytes, k, (int)(n > 0 ? n : 1));
-  return bytes;
-}
-
 struct Layout {
   SceneScratch* sc;
   size_t zero_bytes;  // the scratch and the bin counts behind it start at zero
@@ -914,9 +893,7 @@ struct Layout {
   unsigned* cprim;    // their primitive indices
   uint2* spot;        // their bins and ranks
   unsigned long long* unsorted[2];  // pair lists before the rank sort
-  void* sort_tmp;
-  size_t sort_tmp_bytes;
-  unsigned long long* pair_alt;
+  RowScratch rows;                  // for longer lists
   size_t total;
 };
 
@@ -938,9 +915,7 @@ Layout carve(void* base, long long nv, long long nf, long long ne, long long pai
   L.spot = c.take<uint2>(n);
   L.unsorted[0] = c.take<unsigned long long>(std::min(pair_cap, kRankSortCap));
   L.unsorted[1] = c.take<unsigned long long>(std::min(pair_cap, kRankSortCap));
-  L.sort_tmp_bytes = pair_cap > kRankSortCap ? sort_keys_temp_bytes(pair_cap) : 0;
-  L.sort_tmp = c.take<char>((long long)L.sort_tmp_bytes);
-  L.pair_alt = c.take<unsigned long long>(pair_cap > kRankSortCap ? pair_cap : 1);
+  if (pair_cap > kRankSortCap) L.rows = carve_rows(nv + ne, pair_cap, [&](size_t b) { return (void*)c.take<char>((long long)b); });
   L.total = c.off + 256;
   return L;
 }
@@ -952,16 +927,6 @@ int bit_length(long long x) {
     x >>= 1;
   }
   return b;
-}
-
-int sort_pairs(unsigned long long* pairs, long long cap, int key_bits, const Layout& lay, cudaStream_t s) {
-  if (cap <= 1) return P2C_OK;
-  cub::DoubleBuffer<unsigned long long> k(pairs, lay.pair_alt);
-  size_t tb = lay.sort_tmp_bytes;
-  P2C_CUDA(cub::DeviceRadixSort::SortKeys(lay.sort_tmp, tb, k, (int)cap, 0, key_bits, s));
-  if (k.Current() != pairs)
-    P2C_CUDA(cudaMemcpyAsync(pairs, k.Current(), sizeof(unsigned long long) * cap, cudaMemcpyDeviceToDevice, s));
-  return P2C_OK;
 }
 
 }  // namespace
@@ -1034,10 +999,6 @@ int launch_broadphase(const p2c_scene& scene, unsigned long long* vf_out, long l
   const int vf_shift = sort_out ? std::max(1, bit_length(scene.nf)) : 0;
   const int ee_shift = sort_out ? std::max(1, bit_length(scene.ne)) : 0;
   const bool rank_sort = sort_out && pair_cap <= kRankSortCap;
-  if (sort_out && !rank_sort && vf_cap > 0)
-    fill_u64_kernel<<<grid_for(vf_cap, 256), 256, 0, s>>>(vf_out, vf_cap, ~0ull);
-  if (sort_out && !rank_sort && ee_cap > 0)
-    fill_u64_kernel<<<grid_for(ee_cap, 256), 256, 0, s>>>(ee_out, ee_cap, ~0ull);
   if (n > 0) {
     P2C_CUDA(launch_pdl(cull_kernel, dim3(grid_for(n, kThreads)), dim3(kThreads), 0, s, scene.v_t0, scene.v_t1,
                         lists, scene.thickness, cull, ordered ? 1 : 0, L.cbox, L.cprim, L.sc, (int)L.budget,
@@ -1068,12 +1029,12 @@ int launch_broadphase(const p2c_scene& scene, unsigned long long* vf_out, long l
                         RankList{L.unsorted[1], ee_out, ee_cap, ee_shift}, vf_blocks, (const SceneScratch*)L.sc,
                         counts_dev));
   } else if (sort_out) {
-    rc = sort_pairs(vf_out, vf_cap, bit_length(scene.nv) + vf_shift, L, s);
+    unsigned long long* const pairs[2] = {vf_out, ee_out};
+    const long long cap[2] = {vf_cap, ee_cap}, rows[2] = {scene.nv, scene.ne};
+    const unsigned long long* const count[2] = {&L.sc->vf_count, &L.sc->ee_count};
+    const int shift[2] = {vf_shift, ee_shift};
+    rc = launch_pair_rows(L.rows, pairs, cap, count, shift, rows, s);
     if (rc != P2C_OK) return rc;
-    rc = sort_pairs(ee_out, ee_cap, bit_length(scene.ne) + ee_shift, L, s);
-    if (rc != P2C_OK) return rc;
-    if (vf_cap > 0) unpack_pairs_kernel<<<grid_for(vf_cap, 256), 256, 0, s>>>(vf_out, vf_cap, vf_shift);
-    if (ee_cap > 0) unpack_pairs_kernel<<<grid_for(ee_cap, 256), 256, 0, s>>>(ee_out, ee_cap, ee_shift);
   }
   if (!rank_sort)  // the rank sort writes the counts itself
     P2C_CUDA(launch_pdl(export_counts_kernel, dim3(1), dim3(1), 0, s, (const SceneScratch*)L.sc, counts_dev));
