@@ -97,13 +97,6 @@ struct BroadScratch {
   unsigned blocks_done;              // single scene: cull blocks finished (the last sizes the grid)
 };
 
-// The next 32 sweep slots for the calling warp (one atomic per warp).
-__device__ __forceinline__ long long next_warp_slots(unsigned long long* next) {
-  unsigned long long base = 0;
-  if ((threadIdx.x & 31) == 0) base = atomicAdd(next, 32ull);
-  return (long long)__shfl_sync(0xffffffffu, base, 0);
-}
-
 // Prefix of the partner object's run in a split low field (0 unsplit): a
 // box of object o (0 or 1) walks the entries of object 1 - o.
 __device__ __forceinline__ unsigned split_prefix(const Grid& g, int32_t obj) {
@@ -163,32 +156,11 @@ __device__ __forceinline__ unsigned quantise(double x, const Grid& g) {
   return c < 0.0 ? 0u : (c >= (double)g.qmax ? g.qmax : (unsigned)c);
 }
 
-// Walk over the candidate entries of one scanning box: the columns its
-// partners' min corners can lie in, and in each the quantised window
-// [q(lo), q(hi)] of the partner list.
+// Where the partners of a scanning box can lie: the columns of their min
+// corners, and in each the quantised window [q(lo), q(hi)] of the partner list.
 struct Walker {
-  int c1, c1_end, c2_begin, c2, c2_end;
-  unsigned j, j_end, q_lo, q_hi;
-
-  __device__ __forceinline__ bool next_cell(const SortedBoxes& Q, const Grid& g) {
-    for (;;) {
-      if (++c2 > c2_end) {
-        c2 = c2_begin;
-        if (++c1 > c1_end) return false;
-      }
-      const int cell = c1 * g.g2 + c2;
-      unsigned b = Q.cell_begin[cell], e = Q.cell_end[cell];
-      const unsigned end = e;
-      while (b < e) {  // first entry with q >= q_lo
-        const unsigned m = (b + e) >> 1;
-        if (Q.q[m] < q_lo) b = m + 1;
-        else e = m;
-      }
-      j = b;
-      j_end = end;
-      if (j < j_end && Q.q[j] <= q_hi) return true;
-    }
-  }
+  int c1, c1_end, c2_begin, c2_end;
+  unsigned q_lo, q_hi;
 };
 
 __device__ __forceinline__ void walker_init(Walker& w, const Grid& g, double lo, double hi, double alo, double ahi,
@@ -201,52 +173,8 @@ __device__ __forceinline__ void walker_init(Walker& w, const Grid& g, double lo,
   w.c1_end = column(ahi, g.base1, g.inv1, g.g1);
   w.c2_begin = column(l2, g.base2, g.inv2, g.g2);
   w.c2_end = column(bhi, g.base2, g.inv2, g.g2);
-  w.c2 = w.c2_begin - 1;
-  w.j = w.j_end = 0;
   w.q_lo = quantise(lo, g);
   w.q_hi = quantise(hi, g);
-}
-
-// The same walk with the columns of one box shared by several lanes: lane l
-// of a group of `step` takes columns l, l + step, ... of the box's
-// rectangle (row-major over [c1, c1_end] x [c2_begin, c2_end]).
-struct StridedWalker {
-  int c1a, c2a, n2, n_cells, k, step;
-  unsigned j, j_end, q_lo, q_hi;
-
-  __device__ __forceinline__ bool next_cell(const SortedBoxes& Q, const Grid& g) {
-    for (;;) {
-      k += step;
-      if (k >= n_cells) return false;
-      const int cell = (c1a + k / n2) * g.g2 + (c2a + k % n2);
-      unsigned b = Q.cell_begin[cell], e = Q.cell_end[cell];
-      const unsigned end = e;
-      while (b < e) {  // first entry with q >= q_lo
-        const unsigned m = (b + e) >> 1;
-        if (Q.q[m] < q_lo) b = m + 1;
-        else e = m;
-      }
-      j = b;
-      j_end = end;
-      if (j < j_end && Q.q[j] <= q_hi) return true;
-    }
-  }
-};
-
-__device__ __forceinline__ void strided_walker_init(StridedWalker& w, const Grid& g, double lo, double hi, double alo,
-                                                    double ahi, double blo, double bhi, double reach1, double reach2,
-                                                    int lane, int step, unsigned prefix) {
-  Walker v;
-  walker_init(v, g, lo, hi, alo, ahi, blo, bhi, reach1, reach2);
-  w.c1a = v.c1;
-  w.c2a = v.c2_begin;
-  w.n2 = v.c2_end - v.c2_begin + 1;
-  w.n_cells = (v.c1_end - v.c1 + 1) * w.n2;
-  w.step = step;
-  w.k = lane - step;
-  w.j = w.j_end = 0;
-  w.q_lo = v.q_lo + prefix;
-  w.q_hi = v.q_hi + prefix;
 }
 
 // A scanning box held in registers for the length of its walk.

@@ -24,7 +24,7 @@
 //      passes for up to 256 scenes, 64-bit keys beyond), a gather into one
 //      struct-of-arrays in sorted order and per-scene column tables holding
 //      sorted positions;
-//   6. sweeps that walk only their own scene's columns, appending pairs as
+//   6. one sweep of both families over each scene's own columns, appending pairs as
 //      (scene << w | packed pair), w the widest scene's packed pair, into a buffer of the scenes' summed
 //      capacities (scene s owns its capacity's slice, pre-filled with its
 //      padding key);
@@ -109,10 +109,7 @@ struct BatchBroad {
   unsigned* cell_begin;      // 3 x total cells
   unsigned* cell_end;
   unsigned long long* pack[2][2];  // vf / ee pair buffers and their sort alternates
-  uint4* chunks[2];                // queued pieces of long windows (box, first, end), per family
-  unsigned long long* chunk_count; // 2 counters
-  unsigned long long chunk_cap;    // chunks each queue holds
-  unsigned long long* sweep_next;  // 2 counters: next slot of the vertex-face / edge-edge sweep
+  unsigned long long* sweep_next;  // next boxes of the sweep
   int pair_bits[2];                // packed pair bits of the widest scene, per family
 };
 
@@ -544,324 +541,190 @@ __global__ void fill_pack_kernel(unsigned long long* pack, const unsigned long l
   pack[i] = ((unsigned long long)s << bits) | pair_mask(bits);
 }
 
-// Warp append of found pairs, one atomic per scene present in the warp.
-__device__ __forceinline__ void append_scene_pair(bool found, int s, unsigned long long key, unsigned long long* pack,
-                                                  const unsigned long long* cap_off, BroadScratch* sc, bool vf,
-                                                  int bits) {
-  unsigned todo = __ballot_sync(kFull, found);
-  const int lane = threadIdx.x & 31;
-  while (todo) {
-    const int leader = __ffs((int)todo) - 1;
-    const int ls = __shfl_sync(kFull, s, leader);
-    const bool mine = found && s == ls;
-    const unsigned mask = __ballot_sync(kFull, mine);
-    todo &= ~mask;
-    unsigned long long base = 0;
-    if (lane == leader) base = atomicAdd(vf ? &sc[ls].vf_count : &sc[ls].ee_count, (unsigned long long)__popc(mask));
-    base = __shfl_sync(kFull, base, leader);
-    if (mine) {
-      const unsigned long long slot = base + (unsigned long long)__popc(mask & ((1u << lane) - 1u));
-      const unsigned long long cap = cap_off[s + 1] - cap_off[s];
-      if (slot < cap) pack[cap_off[s] + slot] = ((unsigned long long)s << bits) | key;
+// Pairs a warp has found, packed with their scenes, written 64 at a time with
+// one atomic for each scene among 32 of them.
+struct ScenePairBuffer {
+  unsigned long long* slots;  // shared, 96
+  unsigned n;                 // warp-uniform
+
+  __device__ __forceinline__ void flush(unsigned count, const BatchBroad& B, int family) {
+    const int lane = threadIdx.x & 31, bits = B.pair_bits[family];
+    const unsigned long long* cap_off = family == 0 ? B.off.vf_cap : B.off.ee_cap;
+    __syncwarp();
+    for (unsigned k0 = 0; k0 < count; k0 += 32u) {
+      const bool live = k0 + (unsigned)lane < count;
+      const unsigned long long key = live ? slots[k0 + (unsigned)lane] : 0ull;
+      const int s = live ? (int)(key >> bits) : -1;
+      const unsigned same = __match_any_sync(kFull, s);
+      const int leader = __ffs((int)same) - 1;
+      unsigned long long base = 0;
+      if (live && lane == leader)
+        base = atomicAdd(family == 0 ? &B.sc[s].vf_count : &B.sc[s].ee_count, (unsigned long long)__popc(same));
+      base = __shfl_sync(kFull, base, leader);
+      if (live) {
+        const unsigned long long slot = base + (unsigned long long)__popc(same & ((1u << lane) - 1u));
+        if (slot < cap_off[s + 1] - cap_off[s]) B.pack[family][0][cap_off[s] + slot] = key;
+      }
     }
+    __syncwarp();
+    if (count + (unsigned)lane < n) {  // at most 31 stay
+      const unsigned long long rest = slots[count + (unsigned)lane];
+      slots[lane] = rest;
+    }
+    n -= count;
+    __syncwarp();
   }
-}
-
-__device__ __forceinline__ SortedBoxes scene_view(const BatchBroad& B, int s, int l) {
-  SortedBoxes Q = B.S;
-  Q.cell_begin = cell_table(B, B.cell_begin, s, l);
-  Q.cell_end = cell_table(B, B.cell_end, s, l);
-  return Q;
-}
-
-// Lanes that share one scanning box's columns in the batched sweeps: 2
-// (the batch fills the GPU many times over, so splitting further only adds
-// work; 256 uneven scenes: 11.4 ms with 1 lane, 11.1 with 2, 12.2 with 4).
-#ifndef P2C_BATCH_SWEEP_LANES
-#define P2C_BATCH_SWEEP_LANES 2
-#endif
-constexpr int kBatchSweepLanes = P2C_BATCH_SWEEP_LANES;
-#ifndef P2C_BATCH_SWEEP_BLOCKS
-#define P2C_BATCH_SWEEP_BLOCKS 4
-#endif
-constexpr int kBatchSweepBlocks = P2C_BATCH_SWEEP_BLOCKS;  // resident blocks the sweeps are compiled for
-
-// Long windows: a lane that has tested kChunk entries of one column's window
-// and is not through it hands the rest to the chunk queue in pieces of
-// kChunk entries, which a second launch spreads over the whole GPU.  A few
-// boxes long along the sweep axis (swept far during the step) have windows
-// of hundreds of partners; walked by one lane they set the length of the
-// whole launch.  When the queue is full the lane walks on by itself.
-constexpr unsigned kChunk = 32;
-// Queue capacity per family: one chunk per 8 primitives of the batch, within
-// [4096, 2^20] (a small batch keeps a small workspace).
-__host__ __device__ inline unsigned long long chunk_cap_for(unsigned long long prims) {
-  const unsigned long long c = prims / 8;
-  return c < 4096ull ? 4096ull : (c > (1ull << 20) ? (1ull << 20) : c);
-}
-
-// A scanning box of the vertex-face sweep and the partner list it walks.
-struct VfScan {
-  Box6 pb;
-  FBox pf;
-  double lo;
-  int32_t pid, pobj;
-  bool from_vertex;
-  int exclude_self, shift;
-  const int32_t* faces;
-  SortedBoxes Q;
+  __device__ __forceinline__ void append(bool found, unsigned long long key, const BatchBroad& B, int family) {
+    const unsigned mask = __ballot_sync(kFull, found);
+    if (mask == 0u) return;
+    if (found) slots[n + (unsigned)__popc(mask & ((1u << (threadIdx.x & 31)) - 1u))] = key;
+    n += (unsigned)__popc(mask);
+    if (n >= 64u) flush(64u, B, family);
+  }
 };
 
-__device__ __forceinline__ void vf_scan_at(const BatchBroad& B, unsigned long long i, int s, bool from_vertex,
-                                           VfScan& c) {
-  const p2c_batch_scene& d = B.scenes[s];
-  c.Q = scene_view(B, s, from_vertex ? 1 : 0);
-  c.from_vertex = from_vertex;
-  c.faces = d.faces;
-  c.exclude_self = d.exclude_self;
-  c.shift = max(1, bit_length_dev(d.nf));
-  c.lo = B.S.lo[i];
-  c.pid = B.S.id[i];
-  c.pobj = B.S.obj[i];
-  c.pb = box_at(B.S, (long long)i);
-  c.pf = fbox_of(c.pb);
-}
+// Lanes that share one scanning box: they look its columns' windows up side by
+// side and walk all of them as one list, as the single-scene sweep does.
+constexpr int kSweepLanes = 8;
+constexpr unsigned kWholeRun = 8;  // a column of at most this many entries is walked without a search
 
-// Partner entry j: a pair this box owns, overlapping on all axes and allowed
-// by the object rules (the reference's BuildVFCandidates conditions).
-__device__ __forceinline__ bool vf_test(const VfScan& c, unsigned j, unsigned long long& key) {
-  const float4 qf = c.Q.fb[j];
-  const double qlo = c.Q.lo[j];
-  const bool own = c.from_vertex ? (qlo >= c.lo) : (qlo > c.lo);
-  if (!(own && fmay_overlap(c.pf, qf) && overlap3(c.pb, qlo, c.Q, j))) return false;
-  const int32_t qobj = c.Q.obj[j];
-  const int32_t vtx = c.from_vertex ? c.pid : c.Q.id[j];
-  const int32_t fc = c.from_vertex ? c.Q.id[j] : c.pid;
-  if (c.pobj == qobj) {
-    if (c.exclude_self) return false;
-    const int32_t* fv = c.faces + 3 * (long long)fc;
-    if (__ldg(fv) == vtx || __ldg(fv + 1) == vtx || __ldg(fv + 2) == vtx) return false;
-  }
-  key = pair_key((unsigned)vtx, (unsigned)fc, c.shift);
-  return true;
-}
-
-// A scanning edge of the edge-edge sweep.
-struct EeScan {
-  Box6 pb;
-  FBox pf;
-  double lo;
-  int32_t eid, eobj, a0, a1;
-  int exclude_self, shift;
-  const int32_t* edges;
-  SortedBoxes E;
-};
-
-__device__ __forceinline__ void ee_scan_at(const BatchBroad& B, unsigned long long i, int s, EeScan& c) {
-  const p2c_batch_scene& d = B.scenes[s];
-  c.E = scene_view(B, s, 2);
-  c.edges = d.edges;
-  c.exclude_self = d.exclude_self;
-  c.shift = max(1, bit_length_dev(d.ne));
-  c.lo = B.S.lo[i];
-  c.eid = B.S.id[i];
-  c.eobj = B.S.obj[i];
-  c.a0 = __ldg(c.edges + 2 * (long long)c.eid);
-  c.a1 = __ldg(c.edges + 2 * (long long)c.eid + 1);
-  c.pb = box_at(B.S, (long long)i);
-  c.pf = fbox_of(c.pb);
-}
-
-__device__ __forceinline__ bool ee_test(const EeScan& c, unsigned j, unsigned long long& key) {
-  const float4 qf = c.E.fb[j];
-  const double qlo = c.E.lo[j];
-  const int32_t oid = c.E.id[j];
-  const bool own = qlo > c.lo || (qlo == c.lo && oid > c.eid);
-  if (!(own && fmay_overlap(c.pf, qf) && overlap3(c.pb, qlo, c.E, j))) return false;
-  if (c.E.obj[j] == c.eobj) {
-    if (c.exclude_self) return false;
-    const int32_t b0 = __ldg(c.edges + 2 * (long long)oid), b1 = __ldg(c.edges + 2 * (long long)oid + 1);
-    if (c.a0 == b0 || c.a0 == b1 || c.a1 == b0 || c.a1 == b1) return false;
-  }
-  key = pair_key((unsigned)min(c.eid, oid), (unsigned)max(c.eid, oid), c.shift);
-  return true;
-}
-
-// Hand the rest of the current window, from w.j on, to the chunk queue.
-// Returns false (the lane walks on by itself) when the queue is full.
-__device__ __forceinline__ bool offload_window(StridedWalker& w, const SortedBoxes& Q, unsigned long long box,
-                                               uint4* queue, unsigned long long* queue_count,
-                                               unsigned long long cap) {
-  unsigned b = w.j, e = w.j_end;
-  while (b < e) {  // first entry past the window
-    const unsigned m = (b + e) >> 1;
-    if (Q.q[m] <= w.q_hi) b = m + 1;
-    else e = m;
-  }
-  const unsigned je = b;
-  const unsigned long long pieces = (je - w.j + kChunk - 1) / kChunk;
-  const unsigned long long base = atomicAdd(queue_count, pieces);
-  if (base + pieces > cap) {
-    for (unsigned long long k = base; k < cap; ++k) queue[k] = make_uint4(0u, 0u, 0u, 0u);  // empty
-    return false;
-  }
-  for (unsigned long long k = 0; k < pieces; ++k) {
-    const unsigned jb = w.j + (unsigned)k * kChunk;
-    queue[base + k] = make_uint4((unsigned)box, jb, min(jb + kChunk, je), 0u);
-  }
-  return true;
-}
-
-// Vertex-face pairs, ownership as in the single-scene sweep: a vertex owns
-// the pairs whose face minimum is >= its minimum, a face the others.
-__device__ __forceinline__ void sweep_vf_slot(const BatchBroad& B, unsigned long long tt, unsigned long long P) {
-  const unsigned long long i = tt / kBatchSweepLanes;
-  const int lane = (int)(tt % kBatchSweepLanes);
-  bool live = false;
-  int s = 0;
-  bool from_vertex = false;
-  if (i < P) {
-    const unsigned long long key = sorted_key(B, i);
-    const int l = (int)((key >> kBatchListShift) & 3ull);
-    live = l <= 1;
-    s = (int)(key >> kBatchSceneShift);
-    from_vertex = l == 0;
-  }
-  if (!__any_sync(kFull, live)) return;
-  StridedWalker w;
-  VfScan c;
-  unsigned run = 0;  // entries of the current window tested here
-  if (live) {
-    vf_scan_at(B, i, s, from_vertex, c);
-    const Grid& g = B.sc[s].grid;
-    strided_walker_init(w, g, c.lo, c.pb.hi, c.pb.alo, c.pb.ahi, c.pb.blo, c.pb.bhi,
-                        from_vertex ? g.reach1[1] : g.reach1[0], from_vertex ? g.reach2[1] : g.reach2[0], lane,
-                        kBatchSweepLanes, split_prefix(g, c.pobj));
-    live = w.next_cell(c.Q, g);
-  }
+// Both families in one launch.  Vertex-face pairs: a vertex owns the pairs
+// whose face minimum is >= its minimum, a face the others.  Edge-edge pairs:
+// an edge owns the pairs whose partner minimum is larger (ties: larger index).
+// Bound by dependent loads.  Two lanes per box with a queue for long windows,
+// an atomic for every step that found a pair and four launches: 379 us for a
+// served group of eight scenes, 83 for 64 uneven scenes; now 178 and 63.
+__global__ void __launch_bounds__(kThreads, 4) sweep_kernel(BatchBroad B, int vf_on, int ee_on) {
+  __shared__ unsigned long long slots[2][kThreads / 32][96];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int member = lane & (kSweepLanes - 1), sub = lane / kSweepLanes;
+  constexpr unsigned kBoxes = 32 / kSweepLanes;
+  ScenePairBuffer vfb{slots[0][warp], 0u}, eeb{slots[1][warp], 0u};
+  const unsigned n = (unsigned)*B.n_keyed, steps = (n + kBoxes - 1u) / kBoxes;
+  const unsigned take = max(1u, min(32u, steps / (gridDim.x * (kThreads / 32) * 8u)));
   for (;;) {
-    if (!__any_sync(kFull, live)) break;
-    bool found = false;
-    unsigned long long key = 0;
-    if (live) {
-      found = vf_test(c, w.j, key);
-      ++w.j;
-      if (w.j >= w.j_end || c.Q.q[w.j] > w.q_hi) {
-        live = w.next_cell(c.Q, B.sc[s].grid);
-        run = 0;
-      } else if (++run == kChunk) {
-        if (offload_window(w, c.Q, i, B.chunks[0], B.chunk_count + 0, B.chunk_cap)) {
-          live = w.next_cell(c.Q, B.sc[s].grid);
-          run = 0;
+    unsigned first = 0;
+    if (lane == 0) first = (unsigned)atomicAdd(B.sweep_next, (unsigned long long)take);
+    first = __shfl_sync(kFull, first, 0);
+    if (first >= steps) break;
+    for (unsigned t = first; t < min(first + take, steps); ++t) {
+      const unsigned i = t * kBoxes + (unsigned)sub;
+      bool live = i < n;
+      int l = 0, s = 0;
+      if (live) {
+        const unsigned long long key = sorted_key(B, i);
+        l = (int)((key >> kBatchListShift) & 3ull);
+        s = (int)(key >> kBatchSceneShift);
+        live = l == 2 ? ee_on != 0 : (l <= 1 && vf_on != 0);
+      }
+      const int partner = l == 2 ? 2 : 1 - l;
+      int c1a = 0, c2a = 0, n2 = 1, columns = 0, id = 0, obj = 0;
+      unsigned q_lo = 0, q_hi = 0;
+      double lo = 0.0, hi = 0.0;
+      FBox pf{0.f, 0.f, 0.f, 0.f};
+      if (live) {
+        const Grid& g = B.sc[s].grid;
+        const Box6 pb = box_at(B.S, (long long)i);
+        Walker w;
+        walker_init(w, g, pb.lo, pb.hi, pb.alo, pb.ahi, pb.blo, pb.bhi, g.reach1[partner], g.reach2[partner]);
+        id = B.S.id[i];
+        obj = B.S.obj[i];
+        lo = pb.lo;
+        hi = pb.hi;
+        pf = fbox_of(pb);
+        c1a = w.c1;
+        c2a = w.c2_begin;
+        n2 = w.c2_end - w.c2_begin + 1;
+        columns = (w.c1_end - w.c1 + 1) * n2;
+        q_lo = w.q_lo + split_prefix(g, obj);
+        q_hi = w.q_hi + split_prefix(g, obj);
+      }
+      const unsigned* begins = cell_table(B, B.cell_begin, s, partner);
+      const unsigned* ends = cell_table(B, B.cell_end, s, partner);
+      for (int c = member; __any_sync(kFull, c - member < columns); c += kSweepLanes) {
+        unsigned offset = 0, len = 0;
+        if (c < columns) {
+          const int cell = (c1a + c / n2) * B.sc[s].grid.g2 + c2a + c % n2;
+          unsigned b = begins[cell], e = ends[cell];
+          if (e - b > kWholeRun) {
+            const unsigned end = e;
+            while (b < e) {  // first entry with q >= q_lo
+              const unsigned m = (b + e) >> 1;
+              if (B.S.q[m] < q_lo) b = m + 1;
+              else e = m;
+            }
+            offset = b;
+            e = end;
+            while (b < e) {  // first one with q > q_hi
+              const unsigned m = (b + e) >> 1;
+              if (B.S.q[m] <= q_hi) b = m + 1;
+              else e = m;
+            }
+            len = b - offset;
+          } else if (e > b) {
+            offset = b;
+            len = e - b;
+          }
+        }
+        unsigned before = len;  // inclusive, then exclusive sum of the windows over the box's lanes
+#pragma unroll
+        for (int d = 1; d < kSweepLanes; d <<= 1) {
+          const unsigned up = __shfl_up_sync(kFull, before, d, kSweepLanes);
+          if (member >= d) before += up;
+        }
+        const unsigned entries = __shfl_sync(kFull, before, kSweepLanes - 1, kSweepLanes);
+        before -= len;
+        offset -= before;
+        for (unsigned k = (unsigned)member; __any_sync(kFull, k - (unsigned)member < entries); k += kSweepLanes) {
+          int run = 0;  // the last window that starts at or before entry k
+#pragma unroll
+          for (int d = kSweepLanes / 2; d > 0; d >>= 1) {
+            const unsigned at = __shfl_sync(kFull, before, run + d, kSweepLanes);
+            if (at <= k) run += d;
+          }
+          const unsigned j = __shfl_sync(kFull, offset, run, kSweepLanes) + k;
+          bool found = false;
+          unsigned long long key = 0;
+          if (k < entries) {
+            const float4 qf = B.S.fb[j];
+            const double qlo = B.S.lo[j];
+            if (qlo >= lo && qlo <= hi && fmay_overlap(pf, qf)) {
+              const int qid = B.S.id[j];
+              const bool own = l == 0 || qlo > lo || (l == 2 && qid > id);
+              if (own && overlap3(box_at(B.S, (long long)i), qlo, B.S, j)) {
+                const p2c_batch_scene& d = B.scenes[s];
+                found = true;
+                if (B.S.obj[j] == obj) {  // the reference's object rules
+                  if (d.exclude_self) {
+                    found = false;
+                  } else if (l == 2) {
+                    const int32_t* ea = d.edges + 2 * (long long)id;
+                    const int32_t* eb = d.edges + 2 * (long long)qid;
+                    const int a0 = __ldg(ea), a1 = __ldg(ea + 1), b0 = __ldg(eb), b1 = __ldg(eb + 1);
+                    found = !(a0 == b0 || a0 == b1 || a1 == b0 || a1 == b1);
+                  } else {
+                    const int vtx = l == 0 ? id : qid;
+                    const int32_t* fv = d.faces + 3 * (long long)(l == 0 ? qid : id);
+                    found = !(__ldg(fv) == vtx || __ldg(fv + 1) == vtx || __ldg(fv + 2) == vtx);
+                  }
+                }
+                if (found) {
+                  const int shift = max(1, bit_length_dev(l == 2 ? d.ne : d.nf));
+                  const unsigned a = l == 2 ? (unsigned)min(id, qid) : (unsigned)(l == 0 ? id : qid);
+                  const unsigned b = l == 2 ? (unsigned)max(id, qid) : (unsigned)(l == 0 ? qid : id);
+                  key = ((unsigned long long)s << B.pair_bits[l == 2 ? 1 : 0]) | pair_key(a, b, shift);
+                }
+              }
+            }
+          }
+          vfb.append(found && l != 2, key, B, 0);
+          eeb.append(found && l == 2, key, B, 1);
         }
       }
     }
-    append_scene_pair(found, s, key, B.pack[0][0], B.off.vf_cap, B.sc, true, B.pair_bits[0]);
   }
-}
-
-// Every (kept box, lane) slot, taken 32 at a time by whichever warp is free
-// (the number of kept boxes is known only on the device).
-__global__ void __launch_bounds__(kThreads, kBatchSweepBlocks) sweep_vf_kernel(BatchBroad B, int dynamic) {
-  const unsigned long long n = *B.n_keyed, work = n * kBatchSweepLanes;
-  if (!dynamic) {  // one slot per thread, the grid sized for every primitive
-    const unsigned long long base = (unsigned long long)blockIdx.x * blockDim.x;
-    if (base < work) sweep_vf_slot(B, base + threadIdx.x, n);
-    return;
-  }
-  for (;;) {
-    const unsigned long long base = (unsigned long long)next_warp_slots(B.sweep_next + 0);
-    if (base >= work) break;
-    sweep_vf_slot(B, base + (threadIdx.x & 31), n);
-  }
-}
-
-// Edge-edge pairs: an edge owns the pairs whose partner minimum is larger
-// (ties: larger edge index).
-__device__ __forceinline__ void sweep_ee_slot(const BatchBroad& B, unsigned long long tt, unsigned long long P) {
-  const unsigned long long i = tt / kBatchSweepLanes;
-  const int lane = (int)(tt % kBatchSweepLanes);
-  bool live = false;
-  int s = 0;
-  if (i < P) {
-    const unsigned long long key = sorted_key(B, i);
-    live = ((key >> kBatchListShift) & 3ull) == 2ull;
-    s = (int)(key >> kBatchSceneShift);
-  }
-  if (!__any_sync(kFull, live)) return;
-  StridedWalker w;
-  EeScan c;
-  unsigned run = 0;
-  if (live) {
-    ee_scan_at(B, i, s, c);
-    const Grid& g = B.sc[s].grid;
-    strided_walker_init(w, g, c.lo, c.pb.hi, c.pb.alo, c.pb.ahi, c.pb.blo, c.pb.bhi, g.reach1[2], g.reach2[2], lane,
-                        kBatchSweepLanes, split_prefix(g, c.eobj));
-    live = w.next_cell(c.E, g);
-  }
-  for (;;) {
-    if (!__any_sync(kFull, live)) break;
-    bool found = false;
-    unsigned long long key = 0;
-    if (live) {
-      found = ee_test(c, w.j, key);
-      ++w.j;
-      if (w.j >= w.j_end || c.E.q[w.j] > w.q_hi) {
-        live = w.next_cell(c.E, B.sc[s].grid);
-        run = 0;
-      } else if (++run == kChunk) {
-        if (offload_window(w, c.E, i, B.chunks[1], B.chunk_count + 1, B.chunk_cap)) {
-          live = w.next_cell(c.E, B.sc[s].grid);
-          run = 0;
-        }
-      }
-    }
-    append_scene_pair(found, s, key, B.pack[1][0], B.off.ee_cap, B.sc, false, B.pair_bits[1]);
-  }
-}
-
-__global__ void __launch_bounds__(kThreads, kBatchSweepBlocks) sweep_ee_kernel(BatchBroad B, int dynamic) {
-  const unsigned long long n = *B.n_keyed, work = n * kBatchSweepLanes;
-  if (!dynamic) {  // one slot per thread, the grid sized for every primitive
-    const unsigned long long base = (unsigned long long)blockIdx.x * blockDim.x;
-    if (base < work) sweep_ee_slot(B, base + threadIdx.x, n);
-    return;
-  }
-  for (;;) {
-    const unsigned long long base = (unsigned long long)next_warp_slots(B.sweep_next + 1);
-    if (base >= work) break;
-    sweep_ee_slot(B, base + (threadIdx.x & 31), n);
-  }
-}
-
-// The queued pieces of long windows, one lane each (at most kChunk entries).
-template <int kFamily>
-__global__ void __launch_bounds__(kThreads) chunk_kernel(BatchBroad B) {
-  const unsigned long long n = min(B.chunk_count[kFamily - 1], B.chunk_cap);
-  for (unsigned long long base = (unsigned long long)blockIdx.x * blockDim.x; base < n;
-       base += (unsigned long long)gridDim.x * blockDim.x) {
-    const unsigned long long k = base + threadIdx.x;
-    uint4 item = make_uint4(0u, 0u, 0u, 0u);
-    if (k < n) item = B.chunks[kFamily - 1][k];
-    const bool live = item.z > item.y;
-    int s = 0;
-    VfScan cv;
-    EeScan ce;
-    if (live) {
-      const unsigned long long key = sorted_key(B, item.x);
-      s = (int)(key >> kBatchSceneShift);
-      if (kFamily == 1) vf_scan_at(B, item.x, s, ((key >> kBatchListShift) & 3ull) == 0ull, cv);
-      else ee_scan_at(B, item.x, s, ce);
-    }
-    for (unsigned t = 0; t < kChunk; ++t) {
-      const unsigned j = item.y + t;
-      bool found = false;
-      unsigned long long key = 0;
-      if (live && j < item.z) found = kFamily == 1 ? vf_test(cv, j, key) : ee_test(ce, j, key);
-      if (kFamily == 1) append_scene_pair(found, s, key, B.pack[0][0], B.off.vf_cap, B.sc, true, B.pair_bits[0]);
-      else append_scene_pair(found, s, key, B.pack[1][0], B.off.ee_cap, B.sc, false, B.pair_bits[1]);
-    }
-  }
+  if (vfb.n != 0u) vfb.flush(vfb.n, B, 0);
+  if (eeb.n != 0u) eeb.flush(eeb.n, B, 1);
 }
 
 // ---- 7. scatter sorted pairs into the scenes' buffers --------------------------------
@@ -969,11 +832,7 @@ Carve carve(void* base, const p2c_batch_scene* scenes_dev, int n, const Totals& 
   B.key32 = 0;
   B.sorted_buf = 0;
   B.n_keyed = static_cast<unsigned long long*>(take(8));
-  B.chunk_count = static_cast<unsigned long long*>(take(16));
-  B.sweep_next = static_cast<unsigned long long*>(take(16));
-  B.chunk_cap = chunk_cap_for(t.P);
-  B.chunks[0] = static_cast<uint4*>(take(16 * B.chunk_cap));
-  B.chunks[1] = static_cast<uint4*>(take(16 * B.chunk_cap));
+  B.sweep_next = static_cast<unsigned long long*>(take(8));
   B.vals[0] = static_cast<unsigned*>(take(4 * P));
   B.vals[1] = static_cast<unsigned*>(take(4 * P));
   B.S.lo = static_cast<double*>(take(8 * P));
@@ -1050,8 +909,7 @@ int launch_batch_candidates(const p2c_batch_scene* h, const p2c_batch_scene* dev
   P2C_CUDA(cudaMemsetAsync(B.cell_begin, 0, 4 * 3 * (size_t)t.cells, s));
   P2C_CUDA(cudaMemsetAsync(B.cell_end, 0, 4 * 3 * (size_t)t.cells, s));
   P2C_CUDA(cudaMemsetAsync(B.n_keyed, 0, sizeof(unsigned long long), s));
-  P2C_CUDA(cudaMemsetAsync(B.chunk_count, 0, 2 * sizeof(unsigned long long), s));
-  P2C_CUDA(cudaMemsetAsync(B.sweep_next, 0, 2 * sizeof(unsigned long long), s));
+  P2C_CUDA(cudaMemsetAsync(B.sweep_next, 0, sizeof(unsigned long long), s));
   prep_kernel<<<1, kPrepThreads, 0, s>>>(B);
   P2C_CUDA(cudaGetLastError());
   const unsigned long long P = t.P;
@@ -1105,21 +963,9 @@ int launch_batch_candidates(const p2c_batch_scene* h, const p2c_batch_scene* dev
   }
   P2C_CUDA(cudaGetLastError());
   if (P > 0) {
-    // with culling (often a few per cent kept) warps take sweep slots from a
-    // counter over a resident grid; without, one slot per thread over a grid
-    // for every primitive (faster on dense sheets: no slot fetches)
-#ifdef P2C_BATCH_SWEEP_DYNAMIC
-    const int dynamic = P2C_BATCH_SWEEP_DYNAMIC;
-#else
-    const int dynamic = any_cull ? 1 : 0;
-#endif
-    const unsigned slots = grid_for((long long)P * kBatchSweepLanes, kThreads);
-    const unsigned vf_grid = dynamic ? std::min(slots, resident_grid(sweep_vf_kernel, info)) : slots;
-    const unsigned ee_grid = dynamic ? std::min(slots, resident_grid(sweep_ee_kernel, info)) : slots;
-    if (t.vf > 0) sweep_vf_kernel<<<vf_grid, kThreads, 0, s>>>(B, dynamic);
-    if (t.ee > 0) sweep_ee_kernel<<<ee_grid, kThreads, 0, s>>>(B, dynamic);
-    if (t.vf > 0) chunk_kernel<1><<<resident_grid(chunk_kernel<1>, info), kThreads, 0, s>>>(B);
-    if (t.ee > 0) chunk_kernel<2><<<resident_grid(chunk_kernel<2>, info), kThreads, 0, s>>>(B);
+    if (t.vf > 0 || t.ee > 0)
+      sweep_kernel<<<std::min(grid_for((long long)P * kSweepLanes, kThreads), resident_grid(sweep_kernel, info)), kThreads,
+                     0, s>>>(B, t.vf > 0 ? 1 : 0, t.ee > 0 ? 1 : 0);
     P2C_CUDA(cudaGetLastError());
   }
   for (int f = 0; f < 2; ++f) {
