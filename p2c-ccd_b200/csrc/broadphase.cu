@@ -28,7 +28,7 @@
 //   3. counting sort into the bins: each box's rank in its bin (one atomic per
 //      warp and bin), each column's place, then the boxes to their places.  The
 //      order inside a bin does not matter, so no radix passes are needed;
-//   4. one sweep launch for both families: 16 lanes share a box, look up its
+//   4. one sweep launch for both families: 8 lanes share a box, look up its
 //      columns' runs side by side and walk the runs' entries together;
 //   5. pair lists that fit are ranked by counting smaller keys (all SMs at
 //      once); longer ones are put into rows by their first primitive, and
@@ -915,7 +915,8 @@ Layout carve(void* base, long long nv, long long nf, long long ne, long long pai
   L.spot = c.take<uint2>(n);
   L.unsorted[0] = c.take<unsigned long long>(std::min(pair_cap, kRankSortCap));
   L.unsorted[1] = c.take<unsigned long long>(std::min(pair_cap, kRankSortCap));
-  if (pair_cap > kRankSortCap) L.rows = carve_rows(nv + ne, pair_cap, [&](size_t b) { return (void*)c.take<char>((long long)b); });
+  const long long caps[2] = {pair_cap, pair_cap};
+  if (pair_cap > kRankSortCap) L.rows = carve_rows(nv + ne, caps, [&](size_t b) { return (void*)c.take<char>((long long)b); });
   L.total = c.off + 256;
   return L;
 }
@@ -1029,11 +1030,9 @@ int launch_broadphase(const p2c_scene& scene, unsigned long long* vf_out, long l
                         RankList{L.unsorted[1], ee_out, ee_cap, ee_shift}, vf_blocks, (const SceneScratch*)L.sc,
                         counts_dev));
   } else if (sort_out) {
-    unsigned long long* const pairs[2] = {vf_out, ee_out};
-    const long long cap[2] = {vf_cap, ee_cap}, rows[2] = {scene.nv, scene.ne};
-    const unsigned long long* const count[2] = {&L.sc->vf_count, &L.sc->ee_count};
-    const int shift[2] = {vf_shift, ee_shift};
-    rc = launch_pair_rows(L.rows, pairs, cap, count, shift, rows, s);
+    const long long rows[2] = {scene.nv, scene.ne};
+    rc = launch_pair_rows(L.rows, SceneRows{vf_out, &L.sc->vf_count, vf_cap, vf_shift},
+                          SceneRows{ee_out, &L.sc->ee_count, ee_cap, ee_shift}, rows, s);
     if (rc != P2C_OK) return rc;
   }
   if (!rank_sort)  // the rank sort writes the counts itself

@@ -25,12 +25,11 @@
 //      struct-of-arrays in sorted order and per-scene column tables holding
 //      sorted positions;
 //   6. one sweep of both families over each scene's own columns, appending pairs as
-//      (scene << w | packed pair), w the widest scene's packed pair, into a buffer of the scenes' summed
-//      capacities (scene s owns its capacity's slice, pre-filled with its
-//      padding key);
-//   7. ONE sort of all pairs and a scatter into each scene's own buffer,
-//      unpacked to (a << 32 | b) and padded with ~0: every scene's list comes
-//      out exactly as p2c_scene_candidates with sorted pairs writes it.
+//      (scene << w | packed pair), w the widest scene's packed pair, into a buffer of
+//      the scenes' summed capacities (scene s owns its capacity's slice);
+//   7. ONE ordering of all pairs by rows (pair_rows.cuh), straight into each scene's
+//      own buffer as (a << 32 | b), padded with ~0: every scene's list comes out
+//      exactly as p2c_scene_candidates with sorted pairs writes it.
 #include <cub/block/block_scan.cuh>
 #include <cub/device/device_radix_sort.cuh>
 
@@ -40,6 +39,7 @@
 
 #include "broadphase.cuh"
 #include "count_sort.cuh"
+#include "pair_rows.cuh"
 
 namespace p2c {
 
@@ -90,6 +90,7 @@ struct Offsets {
   unsigned long long* ee_cap;  // n + 1
   unsigned long long* cell;    // n + 1 (cells per list; a scene's tables are 3 x its budget)
   unsigned long long* vert;    // n + 1 (vertices)
+  unsigned long long* edge;    // n + 1 (edges)
 };
 
 struct BatchBroad {
@@ -108,7 +109,7 @@ struct BatchBroad {
   SortedBoxes S;             // P entries in sorted order (cell tables unused here)
   unsigned* cell_begin;      // 3 x total cells
   unsigned* cell_end;
-  unsigned long long* pack[2][2];  // vf / ee pair buffers and their sort alternates
+  unsigned long long* pack[2];     // vf / ee pairs as found, each scene's in its capacity's slice
   unsigned long long* sweep_next;  // next boxes of the sweep
   int pair_bits[2];                // packed pair bits of the widest scene, per family
 };
@@ -146,13 +147,13 @@ __device__ __forceinline__ int cull_count(const p2c_batch_scene& d) {
 __global__ void __launch_bounds__(kPrepThreads) prep_kernel(BatchBroad B) {
   using Scan = cub::BlockScan<unsigned long long, kPrepThreads>;
   __shared__ typename Scan::TempStorage tmp;
-  __shared__ unsigned long long carry[5];
-  if (threadIdx.x < 5) carry[threadIdx.x] = 0ull;
+  __shared__ unsigned long long carry[6];
+  if (threadIdx.x < 6) carry[threadIdx.x] = 0ull;
   __syncthreads();
-  unsigned long long* outs[5] = {B.off.prim, B.off.vf_cap, B.off.ee_cap, B.off.cell, B.off.vert};
+  unsigned long long* outs[6] = {B.off.prim, B.off.vf_cap, B.off.ee_cap, B.off.cell, B.off.vert, B.off.edge};
   for (int base = 0; base < B.n; base += kPrepThreads) {
     const int s = base + (int)threadIdx.x;
-    unsigned long long v[5] = {0ull, 0ull, 0ull, 0ull, 0ull};
+    unsigned long long v[6] = {0ull, 0ull, 0ull, 0ull, 0ull, 0ull};
     if (s < B.n) {
       const p2c_batch_scene& d = B.scenes[s];
       const long long np = d.nv + d.nf + d.ne;
@@ -161,8 +162,9 @@ __global__ void __launch_bounds__(kPrepThreads) prep_kernel(BatchBroad B) {
       v[2] = (unsigned long long)d.ee_cap;
       v[3] = (unsigned long long)cell_budget(np);
       v[4] = (unsigned long long)d.nv;
+      v[5] = (unsigned long long)d.ne;
     }
-    for (int k = 0; k < 5; ++k) {
+    for (int k = 0; k < 6; ++k) {
       unsigned long long excl = 0ull, total = 0ull;
       Scan(tmp).ExclusiveSum(v[k], excl, total);
       if (s < B.n) outs[k][s] = carry[k] + excl;
@@ -171,7 +173,7 @@ __global__ void __launch_bounds__(kPrepThreads) prep_kernel(BatchBroad B) {
       __syncthreads();
     }
   }
-  if (threadIdx.x < 5) outs[threadIdx.x][B.n] = carry[threadIdx.x];
+  if (threadIdx.x < 6) outs[threadIdx.x][B.n] = carry[threadIdx.x];
 }
 
 // ---- 2. vertex envelopes and axis statistics ----------------------------------
@@ -532,15 +534,6 @@ __global__ void __launch_bounds__(kThreads) gather_kernel(BatchBroad B) {
 }
 
 // ---- 6. sweeps -------------------------------------------------------------------
-// Scene s's padding key: sorts after all of its pairs, before scene s + 1's.
-__global__ void fill_pack_kernel(unsigned long long* pack, const unsigned long long* cap_off, int n,
-                                 unsigned long long total, int bits) {
-  const unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= total) return;
-  const int s = find_segment(cap_off, n, i);
-  pack[i] = ((unsigned long long)s << bits) | pair_mask(bits);
-}
-
 // Pairs a warp has found, packed with their scenes, written 64 at a time with
 // one atomic for each scene among 32 of them.
 struct ScenePairBuffer {
@@ -563,7 +556,7 @@ struct ScenePairBuffer {
       base = __shfl_sync(kFull, base, leader);
       if (live) {
         const unsigned long long slot = base + (unsigned long long)__popc(same & ((1u << lane) - 1u));
-        if (slot < cap_off[s + 1] - cap_off[s]) B.pack[family][0][cap_off[s] + slot] = key;
+        if (slot < cap_off[s + 1] - cap_off[s]) B.pack[family][cap_off[s] + slot] = key;
       }
     }
     __syncwarp();
@@ -727,26 +720,51 @@ __global__ void __launch_bounds__(kThreads, 4) sweep_kernel(BatchBroad B, int vf
   if (eeb.n != 0u) eeb.flush(eeb.n, B, 1);
 }
 
-// ---- 7. scatter sorted pairs into the scenes' buffers --------------------------------
-__global__ void scatter_pairs_kernel(BatchBroad B, const unsigned long long* __restrict__ sorted, int family,
-                                     unsigned long long total) {
-  const unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= total) return;
-  const unsigned long long k = sorted[i];
-  const int bits = B.pair_bits[family];
-  const int s = (int)(k >> bits);
-  const unsigned long long* cap_off = family == 0 ? B.off.vf_cap : B.off.ee_cap;
-  const unsigned long long local = i - cap_off[s];
-  const p2c_batch_scene& d = B.scenes[s];
-  unsigned long long* out = reinterpret_cast<unsigned long long*>(family == 0 ? d.vf_pairs : d.ee_pairs);
-  const unsigned long long p = k & pair_mask(bits);
-  if (p == pair_mask(bits)) {
-    out[local] = ~0ull;
-  } else {
-    const int shift = max(1, bit_length_dev(family == 0 ? d.nf : d.ne));
-    out[local] = ((p >> shift) << 32) | (p & ((1ull << shift) - 1ull));
+// ---- 7. pairs into the scenes' buffers, in order ------------------------------
+// All scenes' pairs of one family as rows of all their vertices or edges
+// (pair_rows.cuh).
+struct BatchRows {
+  const p2c_batch_scene* scenes;
+  const BroadScratch* sc;
+  unsigned long long* pack;
+  const unsigned long long* cap_off;
+  const unsigned long long* row_base;  // off.vert or off.edge
+  int n, bits, family;
+  long long cap;
+  __device__ __forceinline__ int shift(int s) const {
+    return max(1, bit_length_dev(family == 0 ? scenes[s].nf : scenes[s].ne));
   }
-}
+  __device__ __forceinline__ bool live(long long i) const {
+    const int s = find_segment(cap_off, n, (unsigned long long)i);
+    return (unsigned long long)i - cap_off[s] < (family == 0 ? sc[s].vf_count : sc[s].ee_count);
+  }
+  __device__ __forceinline__ bool load(long long i, unsigned long long& key) const {
+    if (!live(i)) return false;
+    key = pack[i];
+    return true;
+  }
+  __device__ __forceinline__ unsigned long long row(unsigned long long key) const {
+    const int s = (int)(key >> bits);
+    return row_base[s] + ((key & pair_mask(bits)) >> shift(s));
+  }
+  __device__ __forceinline__ unsigned long long b_mask(unsigned long long key) const {
+    return (1ull << shift((int)(key >> bits))) - 1ull;
+  }
+  __device__ __forceinline__ unsigned long long* out(int s) const {
+    return reinterpret_cast<unsigned long long*>(family == 0 ? scenes[s].vf_pairs : scenes[s].ee_pairs);
+  }
+  __device__ __forceinline__ void pad(long long i) const {
+    const int s = find_segment(cap_off, n, (unsigned long long)i);
+    out(s)[(unsigned long long)i - cap_off[s]] = ~0ull;
+  }
+  __device__ __forceinline__ void store(unsigned place, unsigned long long key, const unsigned* rows) const {
+    const int s = (int)(key >> bits), sh = shift(s);
+    const unsigned base = family == 0 ? 0u : rows[-1];
+    const unsigned first = row_base[s] == 0ull ? 0u : rows[(long long)row_base[s] - 1] - base;  // the scene's first place
+    out(s)[place - first] = ((key & pair_mask(bits)) >> sh << 32) | (key & ((1ull << sh) - 1ull));
+  }
+  __device__ __forceinline__ unsigned long long* input() const { return pack; }
+};
 
 __global__ void export_counts_kernel(BatchBroad B) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -762,7 +780,7 @@ __global__ void export_counts_kernel(BatchBroad B) {
 
 // ---- workspace ---------------------------------------------------------------------
 struct Totals {
-  unsigned long long P = 0, V = 0, vf = 0, ee = 0, cells = 0;
+  unsigned long long P = 0, V = 0, E = 0, vf = 0, ee = 0, cells = 0;
   int pair_bits[2] = {2, 2};  // widest packed pair of any scene: vf, ee
 };
 
@@ -772,6 +790,7 @@ Totals totals_of(const p2c_batch_scene* h, int n) {
     const long long np = h[s].nv + h[s].nf + h[s].ne;
     t.P += (unsigned long long)np;
     t.V += (unsigned long long)h[s].nv;
+    t.E += (unsigned long long)h[s].ne;
     t.vf += (unsigned long long)h[s].vf_cap;
     t.ee += (unsigned long long)h[s].ee_cap;
     t.cells += (unsigned long long)cell_budget(np);
@@ -782,23 +801,18 @@ Totals totals_of(const p2c_batch_scene* h, int n) {
 }
 
 size_t sort_temp_bytes(const Totals& t) {
-  size_t b = 0, c = 0;
   size_t a32 = 0, a64 = 0;
   const int np = (int)std::max<unsigned long long>(t.P, 1ull);
   cub::DeviceRadixSort::SortPairs(nullptr, a32, (const unsigned*)nullptr, (unsigned*)nullptr, (const unsigned*)nullptr,
                                   (unsigned*)nullptr, np);
   cub::DeviceRadixSort::SortPairs(nullptr, a64, (const unsigned long long*)nullptr, (unsigned long long*)nullptr,
                                   (const unsigned*)nullptr, (unsigned*)nullptr, np);
-  const size_t a = std::max(count_sort_scratch_bytes((long long)np), std::max(a32, a64));
-  cub::DeviceRadixSort::SortKeys(nullptr, b, (const unsigned long long*)nullptr, (unsigned long long*)nullptr,
-                                 (int)std::max<unsigned long long>(t.vf, 1ull));
-  cub::DeviceRadixSort::SortKeys(nullptr, c, (const unsigned long long*)nullptr, (unsigned long long*)nullptr,
-                                 (int)std::max<unsigned long long>(t.ee, 1ull));
-  return std::max(a, std::max(b, c));
+  return std::max(count_sort_scratch_bytes((long long)np), std::max(a32, a64));
 }
 
 struct Carve {
   BatchBroad B;
+  RowScratch rows = {};
   void* tmp = nullptr;
   size_t tmp_bytes = 0;
   size_t total = 0;
@@ -823,6 +837,7 @@ Carve carve(void* base, const p2c_batch_scene* scenes_dev, int n, const Totals& 
   B.off.cell = static_cast<unsigned long long*>(take(8 * (size_t)(n + 1)));
   B.sc = static_cast<BroadScratch*>(take(sizeof(BroadScratch) * (size_t)n));
   B.off.vert = static_cast<unsigned long long*>(take(8 * (size_t)(n + 1)));
+  B.off.edge = static_cast<unsigned long long*>(take(8 * (size_t)(n + 1)));
   B.cbox = static_cast<double*>(take(48 * P));
   B.cprim = static_cast<unsigned*>(take(4 * P));
   B.keys[0] = static_cast<unsigned long long*>(take(8 * P));
@@ -847,11 +862,10 @@ Carve carve(void* base, const p2c_batch_scene* scenes_dev, int n, const Totals& 
   B.S.obj = static_cast<int32_t*>(take(4 * P));
   B.cell_begin = static_cast<unsigned*>(take(4 * 3 * (size_t)t.cells));
   B.cell_end = static_cast<unsigned*>(take(4 * 3 * (size_t)t.cells));
-  for (int f = 0; f < 2; ++f) {
-    const size_t cap = (size_t)std::max<unsigned long long>(f == 0 ? t.vf : t.ee, 1ull);
-    B.pack[f][0] = static_cast<unsigned long long*>(take(8 * cap));
-    B.pack[f][1] = static_cast<unsigned long long*>(take(8 * cap));
-  }
+  B.pack[0] = static_cast<unsigned long long*>(take(8 * (size_t)std::max<unsigned long long>(t.vf, 1ull)));
+  B.pack[1] = static_cast<unsigned long long*>(take(8 * (size_t)std::max<unsigned long long>(t.ee, 1ull)));
+  const long long caps[2] = {(long long)t.vf, (long long)t.ee};
+  C.rows = carve_rows((long long)(t.V + t.E), caps, take);
   C.tmp_bytes = sort_temp_bytes(t);
   C.tmp = take(C.tmp_bytes);
   C.total = off;
@@ -955,28 +969,17 @@ int launch_batch_candidates(const p2c_batch_scene* h, const p2c_batch_scene* dev
                     s>>>(B);
     P2C_CUDA(cudaGetLastError());
   }
-  for (int f = 0; f < 2; ++f) {
-    const unsigned long long tot = f == 0 ? t.vf : t.ee;
-    if (tot > 0)
-      fill_pack_kernel<<<grid_for((long long)tot, 256), 256, 0, s>>>(B.pack[f][0], f == 0 ? B.off.vf_cap : B.off.ee_cap,
-                                                                       n, tot, B.pair_bits[f]);
-  }
-  P2C_CUDA(cudaGetLastError());
   if (P > 0) {
     if (t.vf > 0 || t.ee > 0)
       sweep_kernel<<<std::min(grid_for((long long)P * kSweepLanes, kThreads), resident_grid(sweep_kernel, info)), kThreads,
                      0, s>>>(B, t.vf > 0 ? 1 : 0, t.ee > 0 ? 1 : 0);
     P2C_CUDA(cudaGetLastError());
   }
-  for (int f = 0; f < 2; ++f) {
-    const unsigned long long tot = f == 0 ? t.vf : t.ee;
-    if (tot == 0) continue;
-    size_t tb = C.tmp_bytes;
-    P2C_CUDA(cub::DeviceRadixSort::SortKeys(C.tmp, tb, B.pack[f][0], B.pack[f][1], (int)tot, 0,
-                                            B.pair_bits[f] + scene_bits, s));
-    scatter_pairs_kernel<<<grid_for((long long)tot, 256), 256, 0, s>>>(B, B.pack[f][1], f, tot);
-    P2C_CUDA(cudaGetLastError());
-  }
+  const BatchRows vf{B.scenes, B.sc, B.pack[0], B.off.vf_cap, B.off.vert, n, B.pair_bits[0], 0, (long long)t.vf};
+  const BatchRows ee{B.scenes, B.sc, B.pack[1], B.off.ee_cap, B.off.edge, n, B.pair_bits[1], 1, (long long)t.ee};
+  const long long rows[2] = {(long long)t.V, (long long)t.E};
+  rc = launch_pair_rows(C.rows, vf, ee, rows, s);
+  if (rc != P2C_OK) return rc;
   export_counts_kernel<<<grid_for(n, 128), 128, 0, s>>>(B);
   P2C_CUDA(cudaGetLastError());
   return P2C_OK;

@@ -5,9 +5,10 @@
 // cent of a scene), and their number is known only on the device: a library
 // sort sized on the host would rank every culled entry as well.  Each 8-bit
 // pass is three launches over tiles of kCsTile items:
-//   upsweep    per-tile digit histograms, stored digit-major;
+//   upsweep    digit histograms of the live tiles, stored digit-major;
 //   scan       exclusive sum over all (digit, tile) counts: the first output
-//              position of each tile's run of each digit;
+//              position of each tile's run of each digit (what lies behind the
+//              live tiles' counts is scanned too, and never read);
 //   downsweep  a stable block radix sort of the tile on the digit, then each
 //              item goes to its run's position plus its rank in the run.
 // Tiles at or beyond the count exit at once, so a pass costs in proportion
@@ -30,21 +31,25 @@ constexpr int kCsBins = 256;  // 8-bit digits
 
 inline unsigned cs_tiles(long long cap) { return (unsigned)std::max<long long>(1, (cap + kCsTile - 1) / kCsTile); }
 
+__device__ __forceinline__ unsigned cs_live_tiles(unsigned long long n) {
+  return (unsigned)((n + kCsTile - 1) / kCsTile);
+}
+
 template <class K>
 __global__ void __launch_bounds__(kCsThreads) cs_upsweep_kernel(const K* __restrict__ keys,
                                                                 const unsigned long long* __restrict__ count,
-                                                                int shift, unsigned* __restrict__ hist, unsigned tiles) {
+                                                                int shift, unsigned* __restrict__ hist) {
   __shared__ unsigned h[kCsBins];
-  for (int b = threadIdx.x; b < kCsBins; b += kCsThreads) h[b] = 0u;
-  __syncthreads();
   const unsigned long long n = *count;
   const unsigned long long base = (unsigned long long)blockIdx.x * kCsTile;
-  if (base < n) {
+  if (base >= n) return;  // uniform per block
+  const unsigned tiles = cs_live_tiles(n);
+  for (int b = threadIdx.x; b < kCsBins; b += kCsThreads) h[b] = 0u;
+  __syncthreads();
 #pragma unroll
-    for (int k = 0; k < kCsItems; ++k) {
-      const unsigned long long i = base + (unsigned long long)(k * kCsThreads + threadIdx.x);
-      if (i < n) atomicAdd(&h[(unsigned)(keys[i] >> shift) & (kCsBins - 1)], 1u);
-    }
+  for (int k = 0; k < kCsItems; ++k) {
+    const unsigned long long i = base + (unsigned long long)(k * kCsThreads + threadIdx.x);
+    if (i < n) atomicAdd(&h[(unsigned)(keys[i] >> shift) & (kCsBins - 1)], 1u);
   }
   __syncthreads();
   for (int b = threadIdx.x; b < kCsBins; b += kCsThreads) hist[(size_t)b * tiles + blockIdx.x] = h[b];
@@ -58,6 +63,7 @@ struct CsDown {
     struct {
       unsigned start[kCsBins];  // first tile position of each digit's run
       unsigned long long out[kCsBins];
+      unsigned warp_sum[kCsThreads / 32];
     } runs;
   };
 };
@@ -67,14 +73,14 @@ __global__ void __launch_bounds__(kCsThreads) cs_downsweep_kernel(const K* __res
                                                                   const V* __restrict__ vals_in,
                                                                   K* __restrict__ keys_out, V* __restrict__ vals_out,
                                                                   const unsigned long long* __restrict__ count,
-                                                                  int shift, const unsigned* __restrict__ offsets,
-                                                                  unsigned tiles) {
+                                                                  int shift, const unsigned* __restrict__ offsets) {
   using D = CsDown<K, V>;
   __shared__ typename D::Storage sm;
   __shared__ unsigned hist[kCsBins];
   const unsigned long long n = *count;
   const unsigned long long base = (unsigned long long)blockIdx.x * kCsTile;
   if (base >= n) return;  // uniform per block
+  const unsigned tiles = cs_live_tiles(n);
   const unsigned live = (unsigned)min((unsigned long long)kCsTile, n - base);
   // blocked arrangement: thread t holds items t * kCsItems + k of the tile
   K k[kCsItems];
@@ -98,15 +104,21 @@ __global__ void __launch_bounds__(kCsThreads) cs_downsweep_kernel(const K* __res
   __syncthreads();
   typename D::Sort(sm.sort).Sort(k, v, shift, shift + 8);
   __syncthreads();  // the union's sort storage is reused below
-  if (threadIdx.x == 0) {
-    unsigned run = 0;
-    for (int b = 0; b < kCsBins; ++b) {
-      sm.runs.start[b] = run;
-      run += hist[b];
-    }
+  static_assert(kCsThreads == kCsBins, "one thread per digit below");
+  sm.runs.out[threadIdx.x] = (unsigned long long)offsets[(size_t)threadIdx.x * tiles + blockIdx.x];
+  // exclusive sum of the digit counts
+  const unsigned mine = hist[threadIdx.x];
+  unsigned incl = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned up = __shfl_up_sync(0xffffffffu, incl, o);
+    if ((threadIdx.x & 31) >= o) incl += up;
   }
-  for (int b = threadIdx.x; b < kCsBins; b += kCsThreads)
-    sm.runs.out[b] = (unsigned long long)offsets[(size_t)b * tiles + blockIdx.x];
+  if ((threadIdx.x & 31) == 31) sm.runs.warp_sum[threadIdx.x >> 5] = incl;
+  __syncthreads();
+  unsigned before = incl - mine;
+  for (unsigned w = 0; w < threadIdx.x >> 5; ++w) before += sm.runs.warp_sum[w];
+  sm.runs.start[threadIdx.x] = before;
   __syncthreads();
 #pragma unroll
   for (int j = 0; j < kCsItems; ++j) {
@@ -146,10 +158,10 @@ int count_sort_pairs(K* k0, V* v0, K* k1, V* v1, const unsigned long long* count
   V* va[2] = {v0, v1};
   int cur = 0;
   for (int shift = 0; shift < end_bit; shift += 8) {
-    cs_upsweep_kernel<K><<<tiles, kCsThreads, 0, s>>>(ka[cur], count_dev, shift, hist, tiles);
+    cs_upsweep_kernel<K><<<tiles, kCsThreads, 0, s>>>(ka[cur], count_dev, shift, hist);
     P2C_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, hist, offs, (int)entries, s));
     cs_downsweep_kernel<K, V><<<tiles, kCsThreads, 0, s>>>(ka[cur], va[cur], ka[1 - cur], va[1 - cur], count_dev,
-                                                           shift, offs, tiles);
+                                                           shift, offs);
     P2C_CUDA(cudaGetLastError());
     cur = 1 - cur;
   }

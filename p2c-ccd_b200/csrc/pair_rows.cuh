@@ -37,71 +37,97 @@ struct RowCounters {
   unsigned n_mid, next_mid, n_tiles, longest;
 };
 
-// One list: packed keys a << shift | b in, a << 32 | b out, ~0 past the count.
-struct RowList {
+// One list of pairs of one scene: packed keys a << shift | b in, a << 32 | b
+// out in place, ~0 past the count.  A source tells a list's live entries, the
+// row of a key, the bits of b in it, and where the key of a place goes.
+struct SceneRows {
   unsigned long long* pairs;
-  unsigned long long* placed;  // cap
   const unsigned long long* count;
   long long cap;
   int shift;
-  unsigned* row;  // counts, then starts, then ends of the rows, from row_base on
-  long long rows;
+  __device__ __forceinline__ bool live(long long i) const { return (unsigned long long)i < *count; }
+  __device__ __forceinline__ bool load(long long i, unsigned long long& key) const {
+    if (!live(i)) return false;
+    key = pairs[i];
+    return true;
+  }
+  __device__ __forceinline__ unsigned long long row(unsigned long long key) const { return key >> shift; }
+  __device__ __forceinline__ unsigned long long b_mask(unsigned long long) const { return (1ull << shift) - 1ull; }
+  __device__ __forceinline__ void pad(long long i) const { pairs[i] = ~0ull; }
+  __device__ __forceinline__ void store(unsigned place, unsigned long long key, const unsigned*) const {
+    pairs[place] = ((key >> shift) << 32) | (key & b_mask(key));
+  }
+  __device__ __forceinline__ unsigned long long* input() const { return pairs; }
+};
+
+template <class Source>
+struct RowList {
+  Source src;
+  unsigned long long* placed;  // cap
+  unsigned* row;               // counts, then starts, then ends of the rows; row[-1] is where the list starts
+  long long rows;              // row[rows], of no pair, is where it ends
   RowCounters* ctr;
   RowSpan* mid;
   RowSpan* tiles;
   unsigned* big_at;
   unsigned* big_start;
-  __device__ __forceinline__ unsigned n() const { return (unsigned)min(*count, (unsigned long long)cap); }
+  int list;
+  __device__ __forceinline__ unsigned base() const { return list == 0 ? 0u : row[-1]; }
+  __device__ __forceinline__ unsigned n() const { return row[rows] - base(); }
+  __device__ __forceinline__ unsigned start(unsigned long long r) const {
+    return r == 0ull ? 0u : row[(long long)r - 1] - base();
+  }
 };
 
+template <class Source>
 struct RowLists {
-  RowList l[2];
+  RowList<Source> l[2];
 };
 
 namespace {
 
-__global__ void __launch_bounds__(kRowThreads) row_count_kernel(RowLists L) {
-  const RowList& R = L.l[blockIdx.y];
-  const unsigned n = R.n();
-  for (unsigned i = blockIdx.x * kRowThreads + threadIdx.x; i < n; i += gridDim.x * kRowThreads)
-    atomicAdd(R.row + (R.pairs[i] >> R.shift), 1u);
-}
-
-// The rows of the second list follow the first's in one scan.
-__device__ __forceinline__ unsigned row_base(const RowLists& L, int list) { return list == 0 ? 0u : L.l[0].n(); }
-
-__global__ void __launch_bounds__(kRowThreads) row_place_kernel(RowLists L) {
-  const RowList& R = L.l[blockIdx.y];
-  const unsigned n = R.n(), base = row_base(L, blockIdx.y);
-  for (unsigned i = blockIdx.x * kRowThreads + threadIdx.x; i < n; i += gridDim.x * kRowThreads) {
-    const unsigned long long k = R.pairs[i];
-    R.placed[atomicAdd(R.row + (k >> R.shift), 1u) - base] = k;
+template <class Source>
+__global__ void __launch_bounds__(kRowThreads) row_count_kernel(RowLists<Source> L) {
+  const RowList<Source>& R = L.l[blockIdx.y];
+  for (long long i = (long long)blockIdx.x * kRowThreads + threadIdx.x; i < R.src.cap;
+       i += (long long)gridDim.x * kRowThreads) {
+    unsigned long long k;
+    if (R.src.load(i, k)) atomicAdd(R.row + R.src.row(k), 1u);
   }
 }
 
-__device__ __forceinline__ unsigned long long row_pair(unsigned long long a, unsigned long long b) {
-  return (a << 32) | b;
+template <class Source>
+__global__ void __launch_bounds__(kRowThreads) row_place_kernel(RowLists<Source> L) {
+  const RowList<Source>& R = L.l[blockIdx.y];
+  const unsigned base = R.base();
+  for (long long i = (long long)blockIdx.x * kRowThreads + threadIdx.x; i < R.src.cap;
+       i += (long long)gridDim.x * kRowThreads) {
+    unsigned long long k;
+    if (R.src.load(i, k)) R.placed[atomicAdd(R.row + R.src.row(k), 1u) - base] = k;
+  }
 }
 
-// Short rows in place; longer ones are listed by their first pair.
-__global__ void __launch_bounds__(kRowThreads) row_short_kernel(RowLists L) {
-  const RowList& R = L.l[blockIdx.y];
-  const unsigned n = R.n(), base = row_base(L, blockIdx.y);
+// Short rows; longer ones are listed by their first pair.  Entries past a
+// list's count are padded.
+template <class Source>
+__global__ void __launch_bounds__(kRowThreads) row_short_kernel(RowLists<Source> L) {
+  const RowList<Source>& R = L.l[blockIdx.y];
+  const unsigned n = R.n(), base = R.base();
   const int lane = threadIdx.x & 31;
-  for (long long p0 = (long long)blockIdx.x * kRowThreads; p0 < R.cap; p0 += (long long)gridDim.x * kRowThreads) {
+  for (long long p0 = (long long)blockIdx.x * kRowThreads; p0 < R.src.cap; p0 += (long long)gridDim.x * kRowThreads) {
     const long long pl = p0 + threadIdx.x;
     const unsigned p = (unsigned)pl;
     bool is_mid = false;
     unsigned start = 0u, len = 0u;
     if (pl < n) {
-      const unsigned long long k = R.placed[p], a = k >> R.shift;
-      const unsigned end = R.row[a] - base;
-      start = a == 0ull ? 0u : R.row[a - 1] - base;
+      const unsigned long long k = R.placed[p], r = R.src.row(k);
+      const unsigned end = R.row[r] - base;
+      start = R.start(r);
       len = end - start;
       if (len <= kRowCountMax) {
         unsigned smaller = 0u;
         for (unsigned j = start; j < end; ++j) smaller += R.placed[j] < k ? 1u : 0u;
-        R.pairs[start + smaller] = row_pair(a, k & ((1ull << R.shift) - 1ull));
+        R.src.store(start + smaller, k, R.row);
       } else if (p == start) {
         if (len <= kRowWarpMax) {
           is_mid = true;
@@ -118,9 +144,8 @@ __global__ void __launch_bounds__(kRowThreads) row_short_kernel(RowLists L) {
           }
         }
       }
-    } else if (pl < R.cap) {
-      R.pairs[pl] = ~0ull;
     }
+    if (pl < R.src.cap && !R.src.live(pl)) R.src.pad(pl);
     const unsigned m = __ballot_sync(0xffffffffu, is_mid);
     if (m) {
       unsigned at = 0u;
@@ -176,39 +201,38 @@ __device__ __forceinline__ void row_warp_sort(unsigned (&v)[E], int lane) {
   }
 }
 
-template <int E>
-__device__ __forceinline__ void row_warp_order(const RowList& R, RowSpan s, int lane) {
-  const unsigned long long mask = (1ull << R.shift) - 1ull;  // b < 2^31: the padding sorts last
+template <int E, class Source>
+__device__ __forceinline__ void row_warp_order(const RowList<Source>& R, RowSpan s, int lane) {
+  const unsigned long long first = R.placed[s.start], mask = R.src.b_mask(first);  // b < 2^31: padding sorts last
   unsigned v[E];
 #pragma unroll
   for (int e = 0; e < E; ++e) {
     const unsigned i = (unsigned)(e * 32 + lane);
     v[e] = i < s.len ? (unsigned)(R.placed[s.start + i] & mask) : 0xffffffffu;
   }
-  const unsigned long long a = R.placed[s.start] >> R.shift;
   row_warp_sort<E>(v, lane);
 #pragma unroll
   for (int e = 0; e < E; ++e) {
     const unsigned i = (unsigned)(lane * E + e);
-    if (i < s.len) R.pairs[s.start + i] = row_pair(a, v[e]);
+    if (i < s.len) R.src.store(s.start + i, (first & ~mask) | v[e], R.row);
   }
 }
 
-// Tiles of long rows, a block each; then rows of 17 to 1,024 pairs, a warp each.  Tiles of one-tile rows go out, those to be merged back to placed.
-__global__ void __launch_bounds__(kRowThreads, 4) row_long_kernel(RowLists L) {
+// Tiles of long rows, a block each; then rows of 17 to 1,024 pairs, a warp each.
+// Tiles of one-tile rows go out, those to be merged back to placed.
+template <class Source>
+__global__ void __launch_bounds__(kRowThreads, 4) row_long_kernel(RowLists<Source> L) {
   __shared__ unsigned word[kRowTile];
-  const RowList& R = L.l[blockIdx.y];
+  const RowList<Source>& R = L.l[blockIdx.y];
   const unsigned n_tiles = R.ctr->n_tiles;
-  const unsigned long long mask = (1ull << R.shift) - 1ull;
-  const unsigned base = row_base(L, blockIdx.y);
   for (unsigned t = blockIdx.x; t < n_tiles; t += gridDim.x) {
     const RowSpan s = R.tiles[t];
     unsigned size = 2u;
     while (size < s.len) size <<= 1;
+    const unsigned long long first = R.placed[s.start], mask = R.src.b_mask(first), r = R.src.row(first);
     for (unsigned e = threadIdx.x; e < size; e += kRowThreads)
       word[e] = e < s.len ? (unsigned)(R.placed[s.start + e] & mask) : 0xffffffffu;
-    const unsigned long long a = R.placed[s.start] >> R.shift;
-    const unsigned row_len = R.row[a] - (a == 0ull ? base : R.row[a - 1]);
+    const unsigned row_len = R.row[r] - R.base() - R.start(r);
     __syncthreads();
     // 32 consecutive compare pairs span 64 words: steps of at most 32 stay within one warp's words
     for (unsigned k = 2; k <= size; k <<= 1) {
@@ -226,10 +250,11 @@ __global__ void __launch_bounds__(kRowThreads, 4) row_long_kernel(RowLists L) {
       }
       __syncthreads();
     }
-    if (row_len <= kRowTile)
-      for (unsigned e = threadIdx.x; e < s.len; e += kRowThreads) R.pairs[s.start + e] = row_pair(a, word[e]);
-    else
-      for (unsigned e = threadIdx.x; e < s.len; e += kRowThreads) R.placed[s.start + e] = row_pair(a, word[e]);
+    for (unsigned e = threadIdx.x; e < s.len; e += kRowThreads) {
+      const unsigned long long key = (first & ~mask) | word[e];
+      if (row_len <= kRowTile) R.src.store(s.start + e, key, R.row);
+      else R.placed[s.start + e] = key;
+    }
     __syncthreads();
   }
   const unsigned n_mid = R.ctr->n_mid;
@@ -253,7 +278,8 @@ __global__ void __launch_bounds__(kRowThreads, 4) row_long_kernel(RowLists L) {
 }
 
 // Which big row place v of their sequence belongs to.
-__device__ __forceinline__ unsigned row_big(const RowList& R, unsigned n_big, unsigned v) {
+template <class Source>
+__device__ __forceinline__ unsigned row_big(const RowList<Source>& R, unsigned n_big, unsigned v) {
   unsigned lo = 0u, hi = n_big - 1u;
   while (lo < hi) {
     const unsigned mid = (lo + hi + 1u) >> 1;
@@ -263,9 +289,11 @@ __device__ __forceinline__ unsigned row_big(const RowList& R, unsigned n_big, un
   return lo;
 }
 
-// Pairwise merges of the tiles of rows longer than one: every thread writes
-// kRowMergeOut consecutive places, from where the merge path crosses the first.
-__global__ void __launch_bounds__(kRowThreads) row_merge_kernel(RowLists L) {
+// Pairwise merges of the tiles of rows longer than one, between placed and the
+// places of the same numbers in the input: every thread writes kRowMergeOut
+// consecutive places, from where the merge path crosses the first.
+template <class Source>
+__global__ void __launch_bounds__(kRowThreads) row_merge_kernel(RowLists<Source> L) {
   const unsigned longest = max(L.l[0].ctr->longest, L.l[1].ctr->longest);
   if (longest == 0u) return;  // the same in every block
   cooperative_groups::grid_group grid = cooperative_groups::this_grid();
@@ -273,11 +301,11 @@ __global__ void __launch_bounds__(kRowThreads) row_merge_kernel(RowLists L) {
   int src = 0;
   for (unsigned long long width = kRowTile; width < longest; width *= 2ull) {
     for (int list = 0; list < 2; ++list) {
-      const RowList& R = L.l[list];
+      const RowList<Source>& R = L.l[list];
       const unsigned long long big = R.ctr->big;
       const unsigned n_big = (unsigned)(big >> 32), total = (unsigned)big;
-      const unsigned long long* from = src == 0 ? R.placed : R.pairs;
-      unsigned long long* to = src == 0 ? R.pairs : R.placed;
+      const unsigned long long* from = src == 0 ? R.placed : R.src.input();
+      unsigned long long* to = src == 0 ? R.src.input() : R.placed;
       for (unsigned long long v0 = (unsigned long long)t * kRowMergeOut; v0 < total;
            v0 += (unsigned long long)stride * kRowMergeOut) {
         const unsigned vend = (unsigned)min((unsigned long long)total, v0 + kRowMergeOut);
@@ -309,14 +337,14 @@ __global__ void __launch_bounds__(kRowThreads) row_merge_kernel(RowLists L) {
     grid.sync();
     src = 1 - src;
   }
-  if (src != 0) return;  // the last merge wrote to pairs
   for (int list = 0; list < 2; ++list) {
-    const RowList& R = L.l[list];
+    const RowList<Source>& R = L.l[list];
     const unsigned long long big = R.ctr->big;
     const unsigned n_big = (unsigned)(big >> 32), total = (unsigned)big;
+    const unsigned long long* from = src == 0 ? R.placed : R.src.input();
     for (unsigned v = t; v < total; v += stride) {
       const unsigned r = row_big(R, n_big, v), p = R.big_start[r] + (v - R.big_at[r]);
-      R.pairs[p] = R.placed[p];
+      R.src.store(p, from[p], R.row);
     }
   }
 }
@@ -343,14 +371,15 @@ struct RowScratch {
 };
 
 template <class Take>
-RowScratch carve_rows(long long rows, long long pair_cap, Take take) {
+RowScratch carve_rows(long long rows, const long long pair_cap[2], Take take) {
   RowScratch s;
-  const size_t cap = (size_t)(pair_cap > 0 ? pair_cap : 1);
-  s.zero_bytes = 256 + (size_t)(rows > 0 ? rows : 1) * 4;
+  rows += 2;  // the two ends
+  s.zero_bytes = 256 + (size_t)rows * 4;
   char* zero = static_cast<char*>(take(s.zero_bytes));
   s.ctr = reinterpret_cast<RowCounters*>(zero);
   s.row = reinterpret_cast<unsigned*>(zero == nullptr ? nullptr : zero + 256);
   for (int k = 0; k < 2; ++k) {
+    const size_t cap = (size_t)(pair_cap[k] > 0 ? pair_cap[k] : 1);
     s.placed[k] = static_cast<unsigned long long*>(take(cap * 8));
     s.mid[k] = static_cast<RowSpan*>(take((cap / (kRowCountMax + 1) + 1) * sizeof(RowSpan)));
     s.tiles[k] = static_cast<RowSpan*>(take((cap / kRowWarpMax + 1) * sizeof(RowSpan)));
@@ -362,32 +391,31 @@ RowScratch carve_rows(long long rows, long long pair_cap, Take take) {
   return s;
 }
 
-// Sorts both lists in place (a list of capacity 0 takes no part).
-inline int launch_pair_rows(const RowScratch& w, unsigned long long* const pairs[2], const long long cap[2],
-                            const unsigned long long* const count[2], const int shift[2], const long long rows[2],
-                            cudaStream_t s) {
-  RowLists L;
-  long long most = 0;
-  for (int k = 0; k < 2; ++k) {
-    L.l[k] = RowList{pairs[k], w.placed[k], count[k], cap[k],   shift[k],    w.row + (k == 0 ? 0 : rows[0]),
-                     rows[k],  w.ctr + k,   w.mid[k], w.tiles[k], w.big_at[k], w.big_start[k]};
-    most = std::max(most, cap[k]);
-  }
+// Sorts both lists (one of capacity 0 takes no part).
+template <class Source>
+int launch_pair_rows(const RowScratch& w, const Source& first, const Source& second, const long long rows[2],
+                     cudaStream_t s) {
+  RowLists<Source> L;
+  const Source* src[2] = {&first, &second};
+  for (int k = 0; k < 2; ++k)
+    L.l[k] = RowList<Source>{*src[k],  w.placed[k], w.row + (k == 0 ? 0 : rows[0] + 1), rows[k], w.ctr + k, w.mid[k],
+                             w.tiles[k], w.big_at[k], w.big_start[k], k};
+  const long long most = std::max(first.cap, second.cap);
   if (most == 0) return P2C_OK;
   DeviceInfo info;
   if (int rc = current_device_info(&info)) return rc;
-  const unsigned blocks = (unsigned)std::min<long long>((most + kRowThreads - 1) / kRowThreads, 8ll * info.sm_count);
+  const dim3 blocks((unsigned)std::min<long long>((most + kRowThreads - 1) / kRowThreads, 8ll * info.sm_count), 2);
   P2C_CUDA(cudaMemsetAsync(w.ctr, 0, w.zero_bytes, s));
-  row_count_kernel<<<dim3(blocks, 2), kRowThreads, 0, s>>>(L);
+  row_count_kernel<<<blocks, kRowThreads, 0, s>>>(L);
   size_t bytes = w.scan_bytes;
-  P2C_CUDA(cub::DeviceScan::ExclusiveSum(w.scan, bytes, w.row, w.row, (int)std::max(1ll, rows[0] + rows[1]), s));
-  row_place_kernel<<<dim3(blocks, 2), kRowThreads, 0, s>>>(L);
-  row_short_kernel<<<dim3(blocks, 2), kRowThreads, 0, s>>>(L);
+  P2C_CUDA(cub::DeviceScan::ExclusiveSum(w.scan, bytes, w.row, w.row, (int)(rows[0] + rows[1] + 2), s));
+  row_place_kernel<<<blocks, kRowThreads, 0, s>>>(L);
+  row_short_kernel<<<blocks, kRowThreads, 0, s>>>(L);
   row_long_kernel<<<dim3((unsigned)info.sm_count * 4u, 2), kRowThreads, 0, s>>>(L);
   if (most > (long long)kRowTile) {
     void* args[] = {&L};
-    P2C_CUDA(cudaLaunchCooperativeKernel((const void*)row_merge_kernel, dim3((unsigned)info.sm_count), dim3(kRowThreads),
-                                         args, 0, s));
+    P2C_CUDA(cudaLaunchCooperativeKernel((const void*)row_merge_kernel<Source>, dim3((unsigned)info.sm_count),
+                                         dim3(kRowThreads), args, 0, s));
   }
   P2C_CUDA(cudaGetLastError());
   return P2C_OK;
