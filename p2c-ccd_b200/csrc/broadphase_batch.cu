@@ -293,87 +293,96 @@ __device__ __forceinline__ void max_if_larger(unsigned long long* p, unsigned lo
 // envelope.  Kept boxes are appended (one atomic per warp) to a compact list
 // of (box, primitive) entries that everything after works on, and their
 // extents per (scene, list) size the column grids.
+// A block takes kCullSpan consecutive primitives: its start (the search for its
+// scene, then the scene's table entry) is a chain of dependent loads that 256
+// primitives alone do not cover (64 uneven scenes, 7.2 M primitives: 130 us with
+// 256 a block, 118 with 1024).
+constexpr unsigned kCullSpan = 4 * kThreads;
+
 __global__ void __launch_bounds__(kThreads) cull_kernel(BatchBroad B, unsigned long long P) {
-  const unsigned long long g = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
-  bool keep = false, other = false;
-  int s = -1, l = 3;
-  double b[6] = {0, 0, 0, 0, 0, 0};
   __shared__ int block_scene;
-  if (threadIdx.x == 0) block_scene = find_segment(B.off.prim, B.n, (unsigned long long)blockIdx.x * blockDim.x);
+  const unsigned long long block_first = (unsigned long long)blockIdx.x * kCullSpan;
+  if (threadIdx.x == 0) block_scene = find_segment(B.off.prim, B.n, block_first);
   __syncthreads();
-  if (g < P) {
-    s = scene_from(B.off.prim, B.n, block_scene, g);
-    const p2c_batch_scene& d = B.scenes[s];
-    const long long loc = (long long)(g - B.off.prim[s]);
-    l = loc < d.nv ? 0 : (loc < d.nv + d.nf ? 1 : 2);
-    const long long i = l == 0 ? loc : (l == 1 ? loc - d.nv : loc - d.nv - d.nf);
-    const int o = (l == 0 ? d.v_obj : (l == 1 ? d.f_obj : d.e_obj))[i];
-    keep = !(l == 0 && o < 0);
-    if (l == 0) swept_box<1>(d.v_t0, d.v_t1, nullptr, i, d.thickness, b);
-    else if (l == 1) swept_box<3>(d.v_t0, d.v_t1, d.faces, i, d.thickness, b);
-    else swept_box<2>(d.v_t0, d.v_t1, d.edges, i, d.thickness, b);
-    const int cull = cull_count(d);
-    if (keep && cull > 0) {
-      const BroadScratch& sc = B.sc[s];
-      bool near_other = false;
-      for (int q = 0; q < cull && !near_other; ++q) {
-        if (q == o || sc.obj_hi[q][0] == 0ull) continue;
-        bool ov = true;
+  for (unsigned long long g = block_first + threadIdx.x; g - threadIdx.x < min(P, block_first + kCullSpan);
+       g += kThreads) {
+    bool keep = false, other = false;
+    int s = -1, l = 3;
+    double b[6] = {0, 0, 0, 0, 0, 0};
+    if (g < P) {
+      s = scene_from(B.off.prim, B.n, block_scene, g);
+      const p2c_batch_scene& d = B.scenes[s];
+      const long long loc = (long long)(g - B.off.prim[s]);
+      l = loc < d.nv ? 0 : (loc < d.nv + d.nf ? 1 : 2);
+      const long long i = l == 0 ? loc : (l == 1 ? loc - d.nv : loc - d.nv - d.nf);
+      const int o = (l == 0 ? d.v_obj : (l == 1 ? d.f_obj : d.e_obj))[i];
+      keep = !(l == 0 && o < 0);
+      if (l == 0) swept_box<1>(d.v_t0, d.v_t1, nullptr, i, d.thickness, b);
+      else if (l == 1) swept_box<3>(d.v_t0, d.v_t1, d.faces, i, d.thickness, b);
+      else swept_box<2>(d.v_t0, d.v_t1, d.edges, i, d.thickness, b);
+      const int cull = cull_count(d);
+      if (keep && cull > 0) {
+        const BroadScratch& sc = B.sc[s];
+        bool near_other = false;
+        for (int q = 0; q < cull && !near_other; ++q) {
+          if (q == o || sc.obj_hi[q][0] == 0ull) continue;
+          bool ov = true;
 #pragma unroll
-        for (int a = 0; a < 3; ++a) {
-          const double olo = unorder_key(~sc.obj_nlo[q][a]), ohi = unorder_key(sc.obj_hi[q][a]);
-          ov = ov && b[a] <= ohi && olo <= b[3 + a];
+          for (int a = 0; a < 3; ++a) {
+            const double olo = unorder_key(~sc.obj_nlo[q][a]), ohi = unorder_key(sc.obj_hi[q][a]);
+            ov = ov && b[a] <= ohi && olo <= b[3 + a];
+          }
+          near_other = ov;
         }
-        near_other = ov;
+        keep = near_other;
       }
-      keep = near_other;
+      other = keep && o != 0 && o != 1 && d.exclude_self && d.n_obj == 2;
     }
-    other = keep && o != 0 && o != 1 && d.exclude_self && d.n_obj == 2;
-  }
-  if (__any_sync(kFull, other) && other) atomicOr(&B.sc[s].obj_other, 1ull);  // only malformed two-object scenes
-  // compaction of the kept boxes
-  {
-    const unsigned m = __ballot_sync(kFull, keep);
-    if (m != 0u) {
-      const int lane = threadIdx.x & 31;
-      const int leader = __ffs((int)m) - 1;
-      unsigned long long base = 0;
-      if (lane == leader) base = atomicAdd(B.n_keyed, (unsigned long long)__popc(m));
-      base = __shfl_sync(kFull, base, leader);
-      if (keep) {
-        const unsigned long long c = base + (unsigned long long)__popc(m & ((1u << lane) - 1u));
-        double* dst = B.cbox + 6 * c;
+    if (__any_sync(kFull, other) && other) atomicOr(&B.sc[s].obj_other, 1ull);  // only malformed two-object scenes
+    // compaction of the kept boxes
+    {
+      const unsigned m = __ballot_sync(kFull, keep);
+      if (m != 0u) {
+        const int lane = threadIdx.x & 31;
+        const int leader = __ffs((int)m) - 1;
+        unsigned long long base = 0;
+        if (lane == leader) base = atomicAdd(B.n_keyed, (unsigned long long)__popc(m));
+        base = __shfl_sync(kFull, base, leader);
+        if (keep) {
+          const unsigned long long c = base + (unsigned long long)__popc(m & ((1u << lane) - 1u));
+          double* dst = B.cbox + 6 * c;
 #pragma unroll
-        for (int k = 0; k < 6; ++k) dst[k] = b[k];
-        B.cprim[c] = (unsigned)g;
+          for (int k = 0; k < 6; ++k) dst[k] = b[k];
+          B.cprim[c] = (unsigned)g;
+        }
       }
     }
-  }
-  // per (scene, list) extents; most warps hold one scene and one list
-  unsigned todo = __ballot_sync(kFull, keep);
-  while (todo) {
-    const int leader = __ffs((int)todo) - 1;
-    const int ls = __shfl_sync(kFull, s, leader), ll = __shfl_sync(kFull, l, leader);
-    const bool mine = keep && s == ls && l == ll;
-    const unsigned mask = __ballot_sync(kFull, mine);
-    todo &= ~mask;
-    ListStats& S = B.sc[ls].list[ll];
-    if ((threadIdx.x & 31) == leader) atomicAdd(&S.active, (unsigned long long)__popc(mask));
+    // per (scene, list) extents; most warps hold one scene and one list
+    unsigned todo = __ballot_sync(kFull, keep);
+    while (todo) {
+      const int leader = __ffs((int)todo) - 1;
+      const int ls = __shfl_sync(kFull, s, leader), ll = __shfl_sync(kFull, l, leader);
+      const bool mine = keep && s == ls && l == ll;
+      const unsigned mask = __ballot_sync(kFull, mine);
+      todo &= ~mask;
+      ListStats& S = B.sc[ls].list[ll];
+      if ((threadIdx.x & 31) == leader) atomicAdd(&S.active, (unsigned long long)__popc(mask));
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      unsigned long long ext = mine ? (unsigned long long)__double_as_longlong(b[3 + a] - b[a]) : 0ull;
-      unsigned long long lo = mine ? order_key(b[a]) : ~0ull;
-      unsigned long long hi = mine ? order_key(b[3 + a]) : 0ull;
+      for (int a = 0; a < 3; ++a) {
+        unsigned long long ext = mine ? (unsigned long long)__double_as_longlong(b[3 + a] - b[a]) : 0ull;
+        unsigned long long lo = mine ? order_key(b[a]) : ~0ull;
+        unsigned long long hi = mine ? order_key(b[3 + a]) : 0ull;
 #pragma unroll
-      for (int sh = 16; sh > 0; sh >>= 1) {
-        ext = max(ext, __shfl_xor_sync(kFull, ext, sh));
-        lo = min(lo, __shfl_xor_sync(kFull, lo, sh));
-        hi = max(hi, __shfl_xor_sync(kFull, hi, sh));
-      }
-      if ((threadIdx.x & 31) == leader) {
-        max_if_larger(&S.ext_max[a], ext);
-        max_if_larger(&S.nlo_min[a], ~lo);
-        max_if_larger(&S.hi_max[a], hi);
+        for (int sh = 16; sh > 0; sh >>= 1) {
+          ext = max(ext, __shfl_xor_sync(kFull, ext, sh));
+          lo = min(lo, __shfl_xor_sync(kFull, lo, sh));
+          hi = max(hi, __shfl_xor_sync(kFull, hi, sh));
+        }
+        if ((threadIdx.x & 31) == leader) {
+          max_if_larger(&S.ext_max[a], ext);
+          max_if_larger(&S.nlo_min[a], ~lo);
+          max_if_larger(&S.hi_max[a], hi);
+        }
       }
     }
   }
@@ -928,7 +937,7 @@ int launch_batch_candidates(const p2c_batch_scene* h, const p2c_batch_scene* dev
   P2C_CUDA(cudaGetLastError());
   const unsigned long long P = t.P;
   if (t.V > 0) envelope_kernel<<<grid_for((long long)t.V, kThreads), kThreads, 0, s>>>(B, t.V);
-  if (P > 0) cull_kernel<<<grid_for((long long)P, kThreads), kThreads, 0, s>>>(B, P);
+  if (P > 0) cull_kernel<<<grid_for((long long)P, kCullSpan), kThreads, 0, s>>>(B, P);
   grid_kernel<<<grid_for(n, 128), 128, 0, s>>>(B);
   P2C_CUDA(cudaGetLastError());
   DeviceInfo info;
