@@ -1953,6 +1953,12 @@ def main():
     GROUP_ROWS = max(1, args.group_rows)
     BATCH_SCENES, AUTOTUNE_REPS = max(1, args.scenes), max(0, args.autotune_reps)
     CLOTH_N = max(9, args.cloth_n)
+    if args.impl == "b200" and not args.no_cpu_baseline:
+        import oracle
+
+        if not (oracle.ref_available() and oracle.REF_TOOL_SO.exists()):
+            args.no_cpu_baseline = True
+            print("no CPU baseline: the reference libraries are not built here", file=sys.stderr)
     if args.impl == "reference":
         line = run_reference(args)
     elif args.workload == "serve":
