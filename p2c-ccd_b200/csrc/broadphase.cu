@@ -136,8 +136,7 @@ struct Binned {
 };
 
 __device__ __forceinline__ int bin_z(double x, const BinGrid& g) {
-  const double c = floor((x - g.base0) * g.inv0);  // monotone in x: the runs rely on it
-  return c < 0.0 ? 0 : (c >= (double)g.gz ? g.gz - 1 : (int)c);
+  return clamp_floor((x - g.base0) * g.inv0, g.gz - 1);  // monotone in x: the runs rely on it
 }
 __device__ __forceinline__ unsigned first_bin(const BinGrid& g, int list, int cls, int side, int col) {
   return (unsigned)(((list * g.classes + cls) * g.sides + side) * g.cols + col) << g.zshift;
@@ -194,7 +193,7 @@ __device__ __forceinline__ void axis_stats(const double b[6], bool live, SceneSc
 // object's envelope (the union of the object's vertex boxes; one atomic per
 // object per warp) and the per-axis statistics that choose the sweep axis.
 // Faces and edges are boxes of these vertices, so this pass also finds
-// every non-finite coordinate.
+// every non-finite coordinate; such a vertex takes no further part.
 __global__ void __launch_bounds__(kThreads) envelope_kernel(const double* __restrict__ v_t0,
                                                             const double* __restrict__ v_t1,
                                                             const int32_t* __restrict__ v_obj, long long nv,
@@ -204,10 +203,11 @@ __global__ void __launch_bounds__(kThreads) envelope_kernel(const double* __rest
   const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
   double b[6] = {0, 0, 0, 0, 0, 0};
-  const bool live = g < nv;
+  bool live = g < nv;
   int o = -1;
   if (live) {
-    if (!swept_box<1>(v_t0, v_t1, nullptr, g, thickness, b)) atomicOr(&sc->error_word, 1ull);
+    live = swept_box<1>(v_t0, v_t1, nullptr, g, thickness, b);
+    if (!live) atomicOr(&sc->error_word, 1ull);
     o = v_obj[g];
   }
   if (cull_objects > 0) {
@@ -380,8 +380,8 @@ __global__ void grid_kernel(SceneScratch* sc, int budget, int two_body) {
 }
 
 // Every primitive's swept box (Swept*Box, :256-301), kept unless it is a
-// vertex in no face or (self pairs excluded) it lies outside every other
-// object's envelope.  Kept boxes are appended (one atomic per warp) to a
+// vertex in no face, has a non-finite coordinate or (self pairs excluded) lies
+// outside every other object's envelope.  Kept boxes are appended (one atomic per warp) to a
 // compact list of (box, primitive) entries that everything after works on;
 // their extents per list size the grid.  The extents are 32-bit keys reduced
 // by one instruction per warp and in shared memory per block: with 64-bit keys
@@ -419,9 +419,10 @@ __global__ void __launch_bounds__(kThreads, 4) cull_kernel(const double* __restr
     const long long i = g - L.off[l];
     const int o = L.obj[l][i];
     keep = !(l == 0 && o < 0);
-    if (l == 0) swept_box<1>(v_t0, v_t1, nullptr, i, thickness, b);
-    else if (l == 1) swept_box<3>(v_t0, v_t1, L.prim[1], i, thickness, b);
-    else swept_box<2>(v_t0, v_t1, L.prim[2], i, thickness, b);
+    const bool finite = l == 0   ? swept_box<1>(v_t0, v_t1, nullptr, i, thickness, b)
+                        : l == 1 ? swept_box<3>(v_t0, v_t1, L.prim[1], i, thickness, b)
+                                 : swept_box<2>(v_t0, v_t1, L.prim[2], i, thickness, b);
+    keep = keep && finite;
     if (keep && cull_objects > 0) {
       bool near_other = false;
       for (int q = 0; q < cull_objects && !near_other; ++q) {
@@ -436,7 +437,7 @@ __global__ void __launch_bounds__(kThreads, 4) cull_kernel(const double* __restr
     other = keep && o != 0 && o != 1;
   }
   if (__any_sync(kFull, other) && lane == 0) atomicOr(&sc->obj_other, 1u);
-  if (ordered) {  // nothing is culled: every entry in place (a vertex in no face marked)
+  if (ordered) {  // nothing is culled: every entry in place (one that is not kept is marked)
     if (g < L.off[3]) {
       double* dst = cbox + 6 * g;
 #pragma unroll
@@ -732,7 +733,7 @@ __global__ void __launch_bounds__(kThreads, P2C_SWEEP_BLOCKS)
           const unsigned bin = (ordinary ? span.x : large.x) + ((d1 * stride + k - d1 * n2) << zshift);
           const unsigned last = bin + (span.w >> 16);
           offset = B.start[bin + (span.w & 0xffffu)];
-          len = B.start[last] + B.count[last] - offset;
+          len = run_length(offset, B.start[last] + B.count[last]);
         }
         unsigned before = len;  // inclusive, then exclusive sum of the runs' lengths over the box's lanes
 #pragma unroll

@@ -115,7 +115,8 @@ __device__ __forceinline__ double dmax(double a, double b) { return (a < b) ? b 
 // Swept box of a primitive with K vertices (Extend/Expand/Swept*Box,
 // scene_object_envelope_native_ti_walltime.cpp:256-301): min/max over the
 // t0 and t1 positions, then +-thickness.  Returns false on a non-finite
-// coordinate.
+// coordinate: such a box may have no order (a coordinate that is NaN in both
+// frames leaves [inf, -inf]), so the broad phases report it and file none.
 template <int K>
 __device__ __forceinline__ bool swept_box(const double* __restrict__ v_t0, const double* __restrict__ v_t1,
                                           const int32_t* __restrict__ prim, long long i, double thickness,
@@ -145,16 +146,24 @@ __device__ __forceinline__ bool swept_box(const double* __restrict__ v_t0, const
   return finite;
 }
 
+// floor(c) within [0, last]; NaN (an infinite offset times a zero scale) is 0.
+__device__ __forceinline__ int clamp_floor(double c, int last) {
+  c = floor(c);
+  return !(c >= 0.0) ? 0 : (c >= (double)last ? last : (int)c);
+}
+
 __device__ __forceinline__ int column(double x, double base, double inv, int g) {
-  const double c = floor((x - base) * inv);
-  return c < 0.0 ? 0 : (c >= (double)g ? g - 1 : (int)c);
+  return clamp_floor((x - base) * inv, g - 1);
 }
 
 // Monotone (non-decreasing) in x: the sweep windows rely on it.
 __device__ __forceinline__ unsigned quantise(double x, const Grid& g) {
-  const double c = floor((x - g.base0) * g.scale0);
-  return c < 0.0 ? 0u : (c >= (double)g.qmax ? g.qmax : (unsigned)c);
+  return (unsigned)clamp_floor((x - g.base0) * g.scale0, (int)g.qmax);
 }
+
+// Entries of a run from first up to end: none when a box whose bounds are in
+// no order puts its end before its start.
+__device__ __forceinline__ unsigned run_length(unsigned first, unsigned end) { return end > first ? end - first : 0u; }
 
 // Where the partners of a scanning box can lie: the columns of their min
 // corners, and in each the quantised window [q(lo), q(hi)] of the partner list.

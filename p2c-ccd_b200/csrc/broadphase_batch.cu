@@ -181,13 +181,14 @@ __global__ void __launch_bounds__(kPrepThreads) prep_kernel(BatchBroad B) {
 // vert[s + 1])): its swept box joins its object's envelope (order keys, one
 // atomic per object and warp) and the scene's sums of extents, centres and
 // squared centres that choose the sweep axis.  Faces and edges are boxes of
-// these vertices, so the vertex pass also finds every non-finite coordinate.
+// these vertices, so the vertex pass also finds every non-finite coordinate;
+// such a vertex takes no further part.
 __global__ void __launch_bounds__(kThreads) envelope_kernel(BatchBroad B, unsigned long long V) {
   __shared__ double red[9][kThreads / 32];
   __shared__ int scene_lo, scene_hi, block_scene;
   const unsigned long long g = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
-  const bool live = g < V;
+  bool live = g < V;
   int s = -1, o = -1;
   double b[6] = {0, 0, 0, 0, 0, 0};
   if (threadIdx.x == 0) {
@@ -200,8 +201,9 @@ __global__ void __launch_bounds__(kThreads) envelope_kernel(BatchBroad B, unsign
     s = scene_from(B.off.vert, B.n, block_scene, g);
     const p2c_batch_scene& d = B.scenes[s];
     const long long i = (long long)(g - B.off.vert[s]);
-    if (!swept_box<1>(d.v_t0, d.v_t1, nullptr, i, d.thickness, b)) atomicOr(&B.sc[s].error_word, 1ull);
-    if (cull_count(d) > 0) o = d.v_obj[i];
+    live = swept_box<1>(d.v_t0, d.v_t1, nullptr, i, d.thickness, b);
+    if (!live) atomicOr(&B.sc[s].error_word, 1ull);
+    if (live && cull_count(d) > 0) o = d.v_obj[i];
   }
   // object envelopes: per (scene, object) one atomic per warp
   {
@@ -289,8 +291,8 @@ __device__ __forceinline__ void max_if_larger(unsigned long long* p, unsigned lo
 }
 
 // One thread per primitive: its swept box; kept unless it is a vertex in no
-// face or (self pairs excluded) it lies outside every other object's
-// envelope.  Kept boxes are appended (one atomic per warp) to a compact list
+// face, has a non-finite coordinate or (self pairs excluded) lies outside
+// every other object's envelope.  Kept boxes are appended (one atomic per warp) to a compact list
 // of (box, primitive) entries that everything after works on, and their
 // extents per (scene, list) size the column grids.
 // A block takes kCullSpan consecutive primitives: its start (the search for its
@@ -317,9 +319,10 @@ __global__ void __launch_bounds__(kThreads) cull_kernel(BatchBroad B, unsigned l
       const long long i = l == 0 ? loc : (l == 1 ? loc - d.nv : loc - d.nv - d.nf);
       const int o = (l == 0 ? d.v_obj : (l == 1 ? d.f_obj : d.e_obj))[i];
       keep = !(l == 0 && o < 0);
-      if (l == 0) swept_box<1>(d.v_t0, d.v_t1, nullptr, i, d.thickness, b);
-      else if (l == 1) swept_box<3>(d.v_t0, d.v_t1, d.faces, i, d.thickness, b);
-      else swept_box<2>(d.v_t0, d.v_t1, d.edges, i, d.thickness, b);
+      const bool finite = l == 0   ? swept_box<1>(d.v_t0, d.v_t1, nullptr, i, d.thickness, b)
+                          : l == 1 ? swept_box<3>(d.v_t0, d.v_t1, d.faces, i, d.thickness, b)
+                                   : swept_box<2>(d.v_t0, d.v_t1, d.edges, i, d.thickness, b);
+      keep = keep && finite;
       const int cull = cull_count(d);
       if (keep && cull > 0) {
         const BroadScratch& sc = B.sc[s];
