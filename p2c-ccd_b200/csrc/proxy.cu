@@ -411,8 +411,11 @@ __global__ void __launch_bounds__(kThreads, 4) sweep_kernel(ProxyLayout L, long 
   const int c2b = proxy_column(bhi, g.base2, g.inv2, g.g2);
   const int n2 = c2b - c2a + 1;
   int n_cells = (c1b - c1a + 1) * n2;
-  // past the end, or past the slab width hint (error word bit 8)
-  if (t / kSweepLanes >= n || (L.table_bits > 0 && (slab >> L.table_bits))) n_cells = 0;
+  // past the end, past the slab width hint (error word bit 8), or bounds in no
+  // order (bit 1): reversed columns would multiply to a positive count
+  if (t / kSweepLanes >= n || (L.table_bits > 0 && (slab >> L.table_bits)) ||
+      !(lo <= hi && alo <= ahi && blo <= bhi))
+    n_cells = 0;
   const unsigned q_lo = proxy_quantise(lo, g), q_hi = proxy_quantise(hi, g);
   // column-axis bounds rounded outward: a pair that overlaps in doubles
   // overlaps in these floats, so they reject most entries with one load
@@ -449,7 +452,7 @@ __global__ void __launch_bounds__(kThreads, 4) sweep_kernel(ProxyLayout L, long 
       } else {
         const unsigned long long key = (slab << 30) | ((unsigned long long)cell << 16);
         begin = (unsigned)lower_bound(K, n, key | q_lo);
-        len = (unsigned)lower_bound(K, n, (key | q_hi) + 1ull) - begin;
+        len = run_length(begin, (unsigned)lower_bound(K, n, (key | q_hi) + 1ull));
       }
     }
     unsigned before = len;  // inclusive, then exclusive sum of the windows over the box's lanes
