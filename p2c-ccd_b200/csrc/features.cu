@@ -42,10 +42,10 @@ struct FeatureLayout {
   unsigned long long* k2;        // n: (slab << 8 | type) of the lookup order
   unsigned long long* ko;        // n: (object << patch_bits | patch) of the lookup order
   unsigned* idx;                 // n: proxy index of the lookup order
-  // tables
+  // tables (a call uses them or the arrays above: they share the memory)
   unsigned long long* hash_key;  // packed tuples, ~0 empty
   unsigned* hash_first;          // their smallest proxy indices
-  unsigned hash_size;            // a power of two, at least 2 n
+  unsigned hash_size;            // a power of two, at least 2 n; 0 past kHashMost proxies
   unsigned* group_count;         // 2^kGroupBits: proxies of (object, slab)
   unsigned* slab_count;          // 2^kGroupBits
   unsigned* object_seen;         // 2^kGroupBits
@@ -55,6 +55,7 @@ struct FeatureLayout {
 };
 
 constexpr int kGroupBits = 14;
+constexpr size_t kHashMost = (size_t)1 << 30;  // twice as many entries are the largest table of 32-bit places
 
 FeatureLayout carve(void* base, long long n) {
   FeatureLayout L{};
@@ -67,6 +68,7 @@ FeatureLayout carve(void* base, long long n) {
   };
   const size_t N = (size_t)std::max(n, 1ll);
   L.acc = static_cast<unsigned long long*>(take(32));
+  const size_t shared = off;
   for (int k = 0; k < 2; ++k) {
     L.key[k] = static_cast<unsigned long long*>(take(8 * N));
     L.val[k] = static_cast<unsigned*>(take(4 * N));
@@ -74,19 +76,23 @@ FeatureLayout carve(void* base, long long n) {
   L.k2 = static_cast<unsigned long long*>(take(8 * N));
   L.ko = static_cast<unsigned long long*>(take(8 * N));
   L.idx = static_cast<unsigned*>(take(4 * N));
-  L.hash_size = 64;
-  while (L.hash_size < 2 * N) L.hash_size <<= 1;
-  L.hash_key = static_cast<unsigned long long*>(take(12 * (size_t)L.hash_size));
-  L.hash_first = reinterpret_cast<unsigned*>(L.hash_key == nullptr ? nullptr : L.hash_key + L.hash_size);
-  L.group_count = static_cast<unsigned*>(take((size_t)12 << kGroupBits));
-  L.slab_count = L.group_count == nullptr ? nullptr : L.group_count + (1 << kGroupBits);
-  L.object_seen = L.group_count == nullptr ? nullptr : L.group_count + (2 << kGroupBits);
   size_t t = 0;
   cub::DeviceRadixSort::SortPairs(nullptr, t, (const unsigned long long*)nullptr, (unsigned long long*)nullptr,
                                   (const unsigned*)nullptr, (unsigned*)nullptr, (int)N);
   L.tmp_bytes = t;
   L.tmp = take(t);
   L.total = off;
+  off = shared;
+  if (N <= kHashMost) {
+    L.hash_size = 64;
+    while (L.hash_size < 2 * N) L.hash_size <<= 1;
+    L.hash_key = static_cast<unsigned long long*>(take(12 * (size_t)L.hash_size));
+    L.hash_first = reinterpret_cast<unsigned*>(L.hash_key == nullptr ? nullptr : L.hash_key + L.hash_size);
+    L.group_count = static_cast<unsigned*>(take((size_t)12 << kGroupBits));
+    L.slab_count = L.group_count == nullptr ? nullptr : L.group_count + (1 << kGroupBits);
+    L.object_seen = L.group_count == nullptr ? nullptr : L.group_count + (2 << kGroupBits);
+  }
+  L.total = std::max(L.total, off);
   return L;
 }
 
@@ -588,7 +594,7 @@ int p2c_proposal_feature_rows(const p2c_proxy_scene* scene, const p2c_candidate_
   // Tables: two passes where the sorts are 22 launches (51,200 proxies: 15 us
   // against 128).  A word of 64 bits could equal the empty key; more (object,
   // slab) groups than 2^14 would take longer to sum on one block than to sort.
-  const bool hashed = packed && sb + 8 + ob + pb < 64 && sb + ob <= kGroupBits;
+  const bool hashed = packed && sb + 8 + ob + pb < 64 && sb + ob <= kGroupBits && L.hash_size != 0u;
   if (n > 0 && hashed) {
     P2C_CUDA(cudaMemsetAsync(L.hash_key, 0xff, 12 * (size_t)L.hash_size, s));
     P2C_CUDA(cudaMemsetAsync(L.group_count, 0, (size_t)12 << kGroupBits, s));
