@@ -485,10 +485,14 @@ __device__ bool run_engine(const P& prob, const CertParams& prm, int fetch1, int
         }
         SubtreeTask* tk = pools.tasks + (ticket & (pools.task_cap - 1ull));
         unsigned long long tag = 0;
-        if (lane == 0) tag = load_acquire(&tk->tag);
+        int all_done = 0;  // one lane's read for the warp: the lanes leave together
+        if (lane == 0) {
+          tag = load_acquire(&tk->tag);
+          all_done = tag == 0ull && volatile_load(&es->finalized.v) >= n_total;
+        }
         tag = __shfl_sync(FULL, tag, 0);
         if (tag == 0ull) {
-          if (volatile_load(&es->finalized.v) >= n_total) break;
+          if (__shfl_sync(FULL, all_done, 0)) break;
           __nanosleep(backoff);
           backoff = min(backoff * 2u, P2C_BACKOFF);
           P2C_PROF_MARK(3)
