@@ -374,7 +374,7 @@ struct CertParams {
   double eps_space;
   int max_depth;
   int fetch_limit;               // queries a warp keeps in flight (1..32; the engine's slots bound it)
-  unsigned long long budget_ns;  // device time budget of one launch (0 = none)
+  unsigned long long budget_ns;  // device time budget of one launch (device_budget_ns: never 0)
 };
 
 // Counters of one warp's loop (warp-uniform).

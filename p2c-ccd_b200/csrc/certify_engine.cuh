@@ -51,9 +51,9 @@
 // the distance in single precision that spared 95 % of the FP64 samples made
 // the loop longer, not shorter (cloth 445 -> 690 us), and was dropped.
 //
-// No wait in this engine is unbounded: every loop checks the launch's device
-// time budget (CertParams::budget_ns); on expiry the engine returns false and
-// the launcher reports P2C_ERR_TIMEOUT.
+// No wait in this engine is unbounded: the loop checks the launch's device
+// time budget (CertParams::budget_ns, never zero); on expiry the engine
+// returns false and the launcher reports P2C_ERR_TIMEOUT.
 #pragma once
 
 #include "certify_core.cuh"
@@ -371,7 +371,7 @@ __device__ bool run_engine(const P& prob, const CertParams& prm, int fetch1, int
 
   P2C_PROF_START()
   for (unsigned iter = 0;; ++iter) {
-    if ((iter & 63u) == 0u && prm.budget_ns != 0ull) {
+    if ((iter & 63u) == 0u) {
       int over = 0;
       if (lane == 0) over = (global_ns() - t_start) > prm.budget_ns;
       if (__shfl_sync(FULL, over, 0)) {
@@ -738,20 +738,30 @@ __device__ bool run_engine(const P& prob, const CertParams& prm, int fetch1, int
           if (more != 0u) atomicAdd(&A.outstanding, more);
         }
         __syncwarp();
+        bool lost = false;
         if (lane < count) {
           SubtreeTask* tk = pools.tasks + ((task + (unsigned long long)lane) & (pools.task_cap - 1ull));
-          // the taker of the ring's previous lap has long read the entry; wait for it all the same
+          // The taker of the ring's previous lap has long read the entry: the
+          // ring holds more than all warps can have published and not taken
+          // (certify_shape).  Wait for it all the same, and if the budget ends
+          // first fail the launch: a node written over would be lost.
 #pragma unroll 1
-          for (unsigned spin = 0; volatile_load(&tk->tag) != 0ull; ++spin) {
+          for (unsigned spin = 0; volatile_load(&tk->tag) != 0ull && !lost; ++spin) {
             __nanosleep(64);
-            if ((spin & 255u) == 255u && prm.budget_ns != 0ull && (global_ns() - t_start) > prm.budget_ns) break;
+            lost = (spin & 255u) == 255u && (global_ns() - t_start) > prm.budget_ns;
           }
-          tk->path = sh.nkey[e];
-          const unsigned long long tag = (((unsigned long long)sh.qidx[es_slot] << 24) |
-                                          ((unsigned long long)gi << 8) |
-                                          (unsigned long long)(sh.family[es_slot] - 1)) + 1ull;
-          __threadfence();  // the leader's record updates come before the tag
-          store_release(&tk->tag, tag);
+          if (!lost) {
+            tk->path = sh.nkey[e];
+            const unsigned long long tag = (((unsigned long long)sh.qidx[es_slot] << 24) |
+                                            ((unsigned long long)gi << 8) |
+                                            (unsigned long long)(sh.family[es_slot] - 1)) + 1ull;
+            __threadfence();  // the leader's record updates come before the tag
+            store_release(&tk->tag, tag);
+          }
+        }
+        if (__any_sync(FULL, lost)) {
+          ok = false;
+          break;
         }
         st.donations += (unsigned)count;
         bottom += (unsigned)count;
@@ -795,7 +805,7 @@ __device__ inline bool walk_tree(const Geo& g, int family, double T0, double T1,
   bool done = d0 <= prm.eps_space;  // the root collides at t0
   if (!done) d1 = sample(T1);
   for (unsigned k = 0; !done; ++k) {
-    if ((k & 63u) == 63u && prm.budget_ns != 0ull && global_ns() - t_start > prm.budget_ns) return false;
+    if ((k & 63u) == 63u && global_ns() - t_start > prm.budget_ns) return false;
     const double mid = mul(0.5, add(t0, t1));
     ops.add(2);
     if (depth > 0) st.nodes += 1;

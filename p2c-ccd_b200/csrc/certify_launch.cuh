@@ -2,6 +2,7 @@
 // every entry point that runs the warp certifier.
 #pragma once
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 
@@ -31,8 +32,10 @@ struct CertifyScratch {
 // not yet taken.  Task tags must read zero before each launch.
 constexpr unsigned long long kTreeAggCap = 8192;
 constexpr unsigned long long kTaskCap = 16384;
-static_assert((kTaskCap & (kTaskCap - 1ull)) == 0ull && kTaskCap >= P2C_OVERSUPPLY + 148ull * 16ull * P2C_EXPORT_LANES,
-              "the pool's ring holds every warp's unclaimed nodes");
+static_assert((kTaskCap & (kTaskCap - 1ull)) == 0ull, "ring places are taken by a mask");
+// Warps whose unclaimed nodes the ring holds (P2C_EXPORT_LANES each, 2,730
+// warps; 148 SMs run 2,368).
+constexpr unsigned long long kMostWarps = (kTaskCap - P2C_OVERSUPPLY) / P2C_EXPORT_LANES;
 #ifndef P2C_HELPERS_PER_SM
 #define P2C_HELPERS_PER_SM 8
 #endif
@@ -76,7 +79,7 @@ int certify_shape(K kernel, LaunchShape* shape) {
   int per_sm = 0;
   P2C_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kCertifyThreads, smem));
   if (per_sm < 1) per_sm = 1;
-  shape->grid = dev.sm_count * per_sm;
+  shape->grid = std::min(dev.sm_count * per_sm, (int)(kMostWarps / kCertifyWarps));
   shape->smem = smem;
   return P2C_OK;
 }
