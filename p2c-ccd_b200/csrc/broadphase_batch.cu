@@ -26,7 +26,8 @@
 //      sorted positions;
 //   6. one sweep of both families over each scene's own columns, appending pairs as
 //      (scene << w | packed pair), w the widest scene's packed pair, into a buffer of
-//      the scenes' summed capacities (scene s owns its capacity's slice);
+//      the scenes' summed capacities (scene s owns its capacity's slice); windows of
+//      large primitives are cut into pieces for a second launch;
 //   7. ONE ordering of all pairs by rows (pair_rows.cuh), straight into each scene's
 //      own buffer as (a << 32 | b), padded with ~0: every scene's list comes out
 //      exactly as p2c_scene_candidates with sorted pairs writes it.
@@ -111,6 +112,9 @@ struct BatchBroad {
   unsigned* cell_end;
   unsigned long long* pack[2];     // vf / ee pairs as found, each scene's in its capacity's slice
   unsigned long long* sweep_next;  // next boxes of the sweep
+  uint4* pieces;                   // queued pieces of long windows: box, first entry, end
+  unsigned long long* n_pieces;
+  unsigned long long piece_cap;    // pieces the queue holds
   int pair_bits[2];                // packed pair bits of the widest scene, per family
 };
 
@@ -593,10 +597,92 @@ struct ScenePairBuffer {
 constexpr int kSweepLanes = 8;
 constexpr unsigned kWholeRun = 8;  // a column of at most this many entries is walked without a search
 
-// Both families in one launch.  Vertex-face pairs: a vertex owns the pairs
-// whose face minimum is >= its minimum, a face the others.  Edge-edge pairs:
-// an edge owns the pairs whose partner minimum is larger (ties: larger index).
-// Bound by dependent loads.  Two lanes per box with a queue for long windows,
+// A window longer than kLongWindow goes to a queue in pieces of kPiece entries,
+// which a second launch spreads over the whole GPU.  A primitive that is large
+// against the others of its scene (a ground quad under a mesh) has all of them
+// in one window: walked by its eight lanes alone it sets the length of the
+// launch.  Candidates of a sheet of 96,800 triangles over one quad: 36,400 us
+// by the eight lanes, 714 with the queue; 64 uneven scenes, which hardly use
+// it, pay 3 us for its empty launch.  Windows from 128 / 256 / 512 entries on:
+// 698 / 714 / 717 us, but four self-colliding sheets over quads, where middling
+// windows abound, 4,030 / 567 / 559; pieces of 32 / 64 / 128 entries: 737 / 714 /
+// 720 and 4,080 / 567 / 582.  A full queue leaves a window to its lanes.
+#ifndef P2C_BATCH_LONG_WINDOW
+#define P2C_BATCH_LONG_WINDOW 256
+#endif
+#ifndef P2C_BATCH_PIECE
+#define P2C_BATCH_PIECE 64
+#endif
+constexpr unsigned kLongWindow = P2C_BATCH_LONG_WINDOW;
+constexpr unsigned kPiece = P2C_BATCH_PIECE;
+// One piece per eight primitives of the batch, within [4096, 2^20] (a small
+// batch keeps a small workspace).
+__host__ __device__ inline unsigned long long piece_cap_for(unsigned long long prims) {
+  const unsigned long long c = prims / 8;
+  return c < 4096ull ? 4096ull : (c > (1ull << 20) ? (1ull << 20) : c);
+}
+
+// A scanning box: its list, scene and primitive, and what its walk tests
+// first.  The exact bounds are read again for an entry that passes.
+struct ScanBox {
+  unsigned i;
+  int l, s, id, obj;
+  double lo, hi;
+  FBox pf;
+};
+
+// Entry j is a pair that the box owns.  Vertex-face pairs: a vertex owns the
+// pairs whose face minimum is >= its minimum, a face the others.  Edge-edge
+// pairs: an edge owns the pairs whose partner minimum is larger (ties: larger
+// index).
+__device__ __forceinline__ bool test_entry(const BatchBroad& B, const ScanBox& x, unsigned j, unsigned long long& key) {
+  const float4 qf = B.S.fb[j];
+  const double qlo = B.S.lo[j];
+  if (!(qlo >= x.lo && qlo <= x.hi && fmay_overlap(x.pf, qf))) return false;
+  const int qid = B.S.id[j];
+  const bool own = x.l == 0 || qlo > x.lo || (x.l == 2 && qid > x.id);
+  if (!own || !overlap3(box_at(B.S, (long long)x.i), qlo, B.S, j)) return false;
+  const p2c_batch_scene& d = B.scenes[x.s];
+  if (B.S.obj[j] == x.obj) {  // the reference's object rules
+    if (d.exclude_self) return false;
+    if (x.l == 2) {
+      const int32_t* ea = d.edges + 2 * (long long)x.id;
+      const int32_t* eb = d.edges + 2 * (long long)qid;
+      const int a0 = __ldg(ea), a1 = __ldg(ea + 1), b0 = __ldg(eb), b1 = __ldg(eb + 1);
+      if (a0 == b0 || a0 == b1 || a1 == b0 || a1 == b1) return false;
+    } else {
+      const int vtx = x.l == 0 ? x.id : qid;
+      const int32_t* fv = d.faces + 3 * (long long)(x.l == 0 ? qid : x.id);
+      if (__ldg(fv) == vtx || __ldg(fv + 1) == vtx || __ldg(fv + 2) == vtx) return false;
+    }
+  }
+  const int shift = max(1, bit_length_dev(x.l == 2 ? d.ne : d.nf));
+  const unsigned a = x.l == 2 ? (unsigned)min(x.id, qid) : (unsigned)(x.l == 0 ? x.id : qid);
+  const unsigned b = x.l == 2 ? (unsigned)max(x.id, qid) : (unsigned)(x.l == 0 ? qid : x.id);
+  key = ((unsigned long long)x.s << B.pair_bits[x.l == 2 ? 1 : 0]) | pair_key(a, b, shift);
+  return true;
+}
+
+// Queues the window [offset, offset + len) of box i, if it is long; the fuller
+// the queue, the longer it has to be, so that a scene with many middling
+// windows leaves room for the longest.
+__device__ __forceinline__ bool queue_window(uint4* pieces, unsigned long long* n_pieces, unsigned long long cap,
+                                             unsigned i, unsigned offset, unsigned len) {
+  if (len <= kLongWindow) return false;
+  const unsigned long long used = *reinterpret_cast<volatile unsigned long long*>(n_pieces);
+  if (len <= kLongWindow << min(8ull * used / cap, 8ull)) return false;
+  const unsigned n = (len + kPiece - 1u) / kPiece;
+  const unsigned long long at = atomicAdd(n_pieces, (unsigned long long)n);
+  if (at + n > cap) {
+    for (unsigned long long k = at; k < cap; ++k) pieces[k] = make_uint4(0u, 0u, 0u, 0u);  // empty
+    return false;
+  }
+  for (unsigned k = 0; k < n; ++k)
+    pieces[at + k] = make_uint4(i, offset + k * kPiece, offset + min(len, (k + 1u) * kPiece), 0u);
+  return true;
+}
+
+// Both families in one launch.  Bound by dependent loads.  Two lanes per box,
 // an atomic for every step that found a pair and four launches: 379 us for a
 // served group of eight scenes, 83 for 64 uneven scenes; now 178 and 63.
 __global__ void __launch_bounds__(kThreads, 4) sweep_kernel(BatchBroad B, int vf_on, int ee_on) {
@@ -613,43 +699,40 @@ __global__ void __launch_bounds__(kThreads, 4) sweep_kernel(BatchBroad B, int vf
     first = __shfl_sync(kFull, first, 0);
     if (first >= steps) break;
     for (unsigned t = first; t < min(first + take, steps); ++t) {
-      const unsigned i = t * kBoxes + (unsigned)sub;
-      bool live = i < n;
-      int l = 0, s = 0;
+      ScanBox x{t * kBoxes + (unsigned)sub, 0, 0, 0, 0, 0.0, 0.0, FBox{0.f, 0.f, 0.f, 0.f}};
+      bool live = x.i < n;
       if (live) {
-        const unsigned long long key = sorted_key(B, i);
-        l = (int)((key >> kBatchListShift) & 3ull);
-        s = (int)(key >> kBatchSceneShift);
-        live = l == 2 ? ee_on != 0 : (l <= 1 && vf_on != 0);
+        const unsigned long long key = sorted_key(B, x.i);
+        x.l = (int)((key >> kBatchListShift) & 3ull);
+        x.s = (int)(key >> kBatchSceneShift);
+        live = x.l == 2 ? ee_on != 0 : (x.l <= 1 && vf_on != 0);
       }
-      const int partner = l == 2 ? 2 : 1 - l;
-      int c1a = 0, c2a = 0, n2 = 1, columns = 0, id = 0, obj = 0;
+      const int partner = x.l == 2 ? 2 : 1 - x.l;
+      int c1a = 0, c2a = 0, n2 = 1, columns = 0;
       unsigned q_lo = 0, q_hi = 0;
-      double lo = 0.0, hi = 0.0;
-      FBox pf{0.f, 0.f, 0.f, 0.f};
       if (live) {
-        const Grid& g = B.sc[s].grid;
-        const Box6 pb = box_at(B.S, (long long)i);
+        const Grid& g = B.sc[x.s].grid;
+        const Box6 pb = box_at(B.S, (long long)x.i);
         Walker w;
         walker_init(w, g, pb.lo, pb.hi, pb.alo, pb.ahi, pb.blo, pb.bhi, g.reach1[partner], g.reach2[partner]);
-        id = B.S.id[i];
-        obj = B.S.obj[i];
-        lo = pb.lo;
-        hi = pb.hi;
-        pf = fbox_of(pb);
+        x.id = B.S.id[x.i];
+        x.obj = B.S.obj[x.i];
+        x.lo = pb.lo;
+        x.hi = pb.hi;
+        x.pf = fbox_of(pb);
         c1a = w.c1;
         c2a = w.c2_begin;
         n2 = w.c2_end - w.c2_begin + 1;
         columns = (w.c1_end - w.c1 + 1) * n2;
-        q_lo = w.q_lo + split_prefix(g, obj);
-        q_hi = w.q_hi + split_prefix(g, obj);
+        q_lo = w.q_lo + split_prefix(g, x.obj);
+        q_hi = w.q_hi + split_prefix(g, x.obj);
       }
-      const unsigned* begins = cell_table(B, B.cell_begin, s, partner);
-      const unsigned* ends = cell_table(B, B.cell_end, s, partner);
+      const unsigned* begins = cell_table(B, B.cell_begin, x.s, partner);
+      const unsigned* ends = cell_table(B, B.cell_end, x.s, partner);
       for (int c = member; __any_sync(kFull, c - member < columns); c += kSweepLanes) {
         unsigned offset = 0, len = 0;
         if (c < columns) {
-          const int cell = (c1a + c / n2) * B.sc[s].grid.g2 + c2a + c % n2;
+          const int cell = (c1a + c / n2) * B.sc[x.s].grid.g2 + c2a + c % n2;
           unsigned b = begins[cell], e = ends[cell];
           if (e - b > kWholeRun) {
             const unsigned end = e;
@@ -665,10 +748,11 @@ __global__ void __launch_bounds__(kThreads, 4) sweep_kernel(BatchBroad B, int vf
               if (B.S.q[m] <= q_hi) b = m + 1;
               else e = m;
             }
-            len = b - offset;
-          } else if (e > b) {
+            len = run_length(offset, b);
+            if (queue_window(B.pieces, B.n_pieces, B.piece_cap, x.i, offset, len)) len = 0u;
+          } else {
             offset = b;
-            len = e - b;
+            len = run_length(b, e);
           }
         }
         unsigned before = len;  // inclusive, then exclusive sum of the windows over the box's lanes
@@ -688,44 +772,47 @@ __global__ void __launch_bounds__(kThreads, 4) sweep_kernel(BatchBroad B, int vf
             if (at <= k) run += d;
           }
           const unsigned j = __shfl_sync(kFull, offset, run, kSweepLanes) + k;
-          bool found = false;
           unsigned long long key = 0;
-          if (k < entries) {
-            const float4 qf = B.S.fb[j];
-            const double qlo = B.S.lo[j];
-            if (qlo >= lo && qlo <= hi && fmay_overlap(pf, qf)) {
-              const int qid = B.S.id[j];
-              const bool own = l == 0 || qlo > lo || (l == 2 && qid > id);
-              if (own && overlap3(box_at(B.S, (long long)i), qlo, B.S, j)) {
-                const p2c_batch_scene& d = B.scenes[s];
-                found = true;
-                if (B.S.obj[j] == obj) {  // the reference's object rules
-                  if (d.exclude_self) {
-                    found = false;
-                  } else if (l == 2) {
-                    const int32_t* ea = d.edges + 2 * (long long)id;
-                    const int32_t* eb = d.edges + 2 * (long long)qid;
-                    const int a0 = __ldg(ea), a1 = __ldg(ea + 1), b0 = __ldg(eb), b1 = __ldg(eb + 1);
-                    found = !(a0 == b0 || a0 == b1 || a1 == b0 || a1 == b1);
-                  } else {
-                    const int vtx = l == 0 ? id : qid;
-                    const int32_t* fv = d.faces + 3 * (long long)(l == 0 ? qid : id);
-                    found = !(__ldg(fv) == vtx || __ldg(fv + 1) == vtx || __ldg(fv + 2) == vtx);
-                  }
-                }
-                if (found) {
-                  const int shift = max(1, bit_length_dev(l == 2 ? d.ne : d.nf));
-                  const unsigned a = l == 2 ? (unsigned)min(id, qid) : (unsigned)(l == 0 ? id : qid);
-                  const unsigned b = l == 2 ? (unsigned)max(id, qid) : (unsigned)(l == 0 ? qid : id);
-                  key = ((unsigned long long)s << B.pair_bits[l == 2 ? 1 : 0]) | pair_key(a, b, shift);
-                }
-              }
-            }
-          }
-          vfb.append(found && l != 2, key, B, 0);
-          eeb.append(found && l == 2, key, B, 1);
+          const bool found = k < entries && test_entry(B, x, j, key);
+          vfb.append(found && x.l != 2, key, B, 0);
+          eeb.append(found && x.l == 2, key, B, 1);
         }
       }
+    }
+  }
+  if (vfb.n != 0u) vfb.flush(vfb.n, B, 0);
+  if (eeb.n != 0u) eeb.flush(eeb.n, B, 1);
+}
+
+// The queued pieces, each by the lanes of one group.
+__global__ void __launch_bounds__(kThreads, 4) piece_kernel(BatchBroad B) {
+  __shared__ unsigned long long slots[2][kThreads / 32][96];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned member = (unsigned)lane & (kSweepLanes - 1), sub = (unsigned)lane / kSweepLanes;
+  constexpr unsigned kBoxes = 32 / kSweepLanes;
+  ScenePairBuffer vfb{slots[0][warp], 0u}, eeb{slots[1][warp], 0u};
+  const unsigned n = (unsigned)min(*B.n_pieces, B.piece_cap);
+  for (unsigned first = (blockIdx.x * (kThreads / 32) + (unsigned)warp) * kBoxes; first < n;
+       first += gridDim.x * (kThreads / 32) * kBoxes) {
+    uint4 piece = make_uint4(0u, 0u, 0u, 0u);
+    if (first + sub < n) piece = B.pieces[first + sub];
+    ScanBox x{piece.x, 0, 0, 0, 0, 0.0, 0.0, FBox{0.f, 0.f, 0.f, 0.f}};
+    if (piece.z > piece.y) {
+      const unsigned long long key = sorted_key(B, x.i);
+      const Box6 pb = box_at(B.S, (long long)x.i);
+      x.l = (int)((key >> kBatchListShift) & 3ull);
+      x.s = (int)(key >> kBatchSceneShift);
+      x.id = B.S.id[x.i];
+      x.obj = B.S.obj[x.i];
+      x.lo = pb.lo;
+      x.hi = pb.hi;
+      x.pf = fbox_of(pb);
+    }
+    for (unsigned j = piece.y + member; __any_sync(kFull, j - member < piece.z); j += kSweepLanes) {
+      unsigned long long key = 0;
+      const bool found = j < piece.z && test_entry(B, x, j, key);
+      vfb.append(found && x.l != 2, key, B, 0);
+      eeb.append(found && x.l == 2, key, B, 1);
     }
   }
   if (vfb.n != 0u) vfb.flush(vfb.n, B, 0);
@@ -858,8 +945,11 @@ Carve carve(void* base, const p2c_batch_scene* scenes_dev, int n, const Totals& 
   B.keys32[1] = reinterpret_cast<unsigned*>(B.keys[1]);
   B.key32 = 0;
   B.sorted_buf = 0;
-  B.n_keyed = static_cast<unsigned long long*>(take(8));
-  B.sweep_next = static_cast<unsigned long long*>(take(8));
+  B.n_keyed = static_cast<unsigned long long*>(take(24));  // and the two counters behind it
+  B.sweep_next = B.n_keyed + 1;
+  B.n_pieces = B.n_keyed + 2;
+  B.piece_cap = piece_cap_for(t.P);
+  B.pieces = static_cast<uint4*>(take(sizeof(uint4) * (size_t)B.piece_cap));
   B.vals[0] = static_cast<unsigned*>(take(4 * P));
   B.vals[1] = static_cast<unsigned*>(take(4 * P));
   B.S.lo = static_cast<double*>(take(8 * P));
@@ -934,8 +1024,7 @@ int launch_batch_candidates(const p2c_batch_scene* h, const p2c_batch_scene* dev
   P2C_CUDA(cudaMemsetAsync(B.sc, 0, sizeof(BroadScratch) * (size_t)n, s));
   P2C_CUDA(cudaMemsetAsync(B.cell_begin, 0, 4 * 3 * (size_t)t.cells, s));
   P2C_CUDA(cudaMemsetAsync(B.cell_end, 0, 4 * 3 * (size_t)t.cells, s));
-  P2C_CUDA(cudaMemsetAsync(B.n_keyed, 0, sizeof(unsigned long long), s));
-  P2C_CUDA(cudaMemsetAsync(B.sweep_next, 0, sizeof(unsigned long long), s));
+  P2C_CUDA(cudaMemsetAsync(B.n_keyed, 0, 3 * sizeof(unsigned long long), s));
   prep_kernel<<<1, kPrepThreads, 0, s>>>(B);
   P2C_CUDA(cudaGetLastError());
   const unsigned long long P = t.P;
@@ -981,11 +1070,14 @@ int launch_batch_candidates(const p2c_batch_scene* h, const p2c_batch_scene* dev
                     s>>>(B);
     P2C_CUDA(cudaGetLastError());
   }
-  if (P > 0) {
-    if (t.vf > 0 || t.ee > 0)
-      sweep_kernel<<<std::min(grid_for((long long)P * kSweepLanes, kThreads), resident_grid(sweep_kernel, info)), kThreads,
-                     0, s>>>(B, t.vf > 0 ? 1 : 0, t.ee > 0 ? 1 : 0);
+  if (P > 0 && (t.vf > 0 || t.ee > 0)) {
+    sweep_kernel<<<std::min(grid_for((long long)P * kSweepLanes, kThreads), resident_grid(sweep_kernel, info)), kThreads,
+                   0, s>>>(B, t.vf > 0 ? 1 : 0, t.ee > 0 ? 1 : 0);
     P2C_CUDA(cudaGetLastError());
+    if (P > kLongWindow) {
+      piece_kernel<<<resident_grid(piece_kernel, info), kThreads, 0, s>>>(B);
+      P2C_CUDA(cudaGetLastError());
+    }
   }
   const BatchRows vf{B.scenes, B.sc, B.pack[0], B.off.vf_cap, B.off.vert, n, B.pair_bits[0], 0, (long long)t.vf};
   const BatchRows ee{B.scenes, B.sc, B.pack[1], B.off.ee_cap, B.off.edge, n, B.pair_bits[1], 1, (long long)t.ee};
