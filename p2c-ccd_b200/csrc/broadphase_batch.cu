@@ -112,9 +112,9 @@ struct BatchBroad {
   unsigned* cell_end;
   unsigned long long* pack[2];     // vf / ee pairs as found, each scene's in its capacity's slice
   unsigned long long* sweep_next;  // next boxes of the sweep
-  uint4* pieces;                   // queued pieces of long windows: box, first entry, end
-  unsigned long long* n_pieces;
-  unsigned long long piece_cap;    // pieces the queue holds
+  uint4* pieces;                   // queues of pieces of long windows: box, first entry, end
+  unsigned long long* n_pieces;    // per queue
+  unsigned long long piece_cap;    // pieces a queue holds
   int pair_bits[2];                // packed pair bits of the widest scene, per family
 };
 
@@ -602,11 +602,13 @@ constexpr unsigned kWholeRun = 8;  // a column of at most this many entries is w
 // against the others of its scene (a ground quad under a mesh) has all of them
 // in one window: walked by its eight lanes alone it sets the length of the
 // launch.  Candidates of a sheet of 96,800 triangles over one quad: 36,400 us
-// by the eight lanes, 714 with the queue; 64 uneven scenes, which hardly use
-// it, pay 3 us for its empty launch.  Windows from 128 / 256 / 512 entries on:
-// 698 / 714 / 717 us, but four self-colliding sheets over quads, where middling
-// windows abound, 4,030 / 567 / 559; pieces of 32 / 64 / 128 entries: 737 / 714 /
-// 720 and 4,080 / 567 / 582.  A full queue leaves a window to its lanes.
+// by the eight lanes, 714 with the queues; 64 uneven scenes, which hardly use
+// them, pay 3 us for their empty launch.  Windows from 128 / 256 / 512 entries
+// on: 698 / 714 / 717 us; pieces of 32 / 64 / 128 entries: 737 / 714 / 720.
+// A full queue leaves a window to its lanes.  Windows are queued by length, one
+// queue for each factor of four, so that the many middling ones of a dense
+// scene never take the room of the longest (four self-colliding sheets over
+// quads: 4,030 us when they do, 567 when not).
 #ifndef P2C_BATCH_LONG_WINDOW
 #define P2C_BATCH_LONG_WINDOW 256
 #endif
@@ -615,11 +617,12 @@ constexpr unsigned kWholeRun = 8;  // a column of at most this many entries is w
 #endif
 constexpr unsigned kLongWindow = P2C_BATCH_LONG_WINDOW;
 constexpr unsigned kPiece = P2C_BATCH_PIECE;
-// One piece per eight primitives of the batch, within [4096, 2^20] (a small
-// batch keeps a small workspace).
+constexpr int kPieceQueues = 4;
+// All queues: one piece per eight primitives of the batch, within [4096, 2^20]
+// (a small batch keeps a small workspace).
 __host__ __device__ inline unsigned long long piece_cap_for(unsigned long long prims) {
   const unsigned long long c = prims / 8;
-  return c < 4096ull ? 4096ull : (c > (1ull << 20) ? (1ull << 20) : c);
+  return (c < 4096ull ? 4096ull : (c > (1ull << 20) ? (1ull << 20) : c)) / kPieceQueues;
 }
 
 // A scanning box: its list, scene and primitive, and what its walk tests
@@ -663,16 +666,15 @@ __device__ __forceinline__ bool test_entry(const BatchBroad& B, const ScanBox& x
   return true;
 }
 
-// Queues the window [offset, offset + len) of box i, if it is long; the fuller
-// the queue, the longer it has to be, so that a scene with many middling
-// windows leaves room for the longest.
+// Queues the window [offset, offset + len) of box i, if it is long and fits.
 __device__ __forceinline__ bool queue_window(uint4* pieces, unsigned long long* n_pieces, unsigned long long cap,
                                              unsigned i, unsigned offset, unsigned len) {
   if (len <= kLongWindow) return false;
-  const unsigned long long used = *reinterpret_cast<volatile unsigned long long*>(n_pieces);
-  if (len <= kLongWindow << min(8ull * used / cap, 8ull)) return false;
+  const int q = (len > 4u * kLongWindow) + (len > 16u * kLongWindow) + (len > 64u * kLongWindow);
+  if (*reinterpret_cast<volatile unsigned long long*>(n_pieces + q) >= cap) return false;
   const unsigned n = (len + kPiece - 1u) / kPiece;
-  const unsigned long long at = atomicAdd(n_pieces, (unsigned long long)n);
+  const unsigned long long at = atomicAdd(n_pieces + q, (unsigned long long)n);
+  pieces += (unsigned long long)q * cap;
   if (at + n > cap) {
     for (unsigned long long k = at; k < cap; ++k) pieces[k] = make_uint4(0u, 0u, 0u, 0u);  // empty
     return false;
@@ -791,28 +793,31 @@ __global__ void __launch_bounds__(kThreads, 4) piece_kernel(BatchBroad B) {
   const unsigned member = (unsigned)lane & (kSweepLanes - 1), sub = (unsigned)lane / kSweepLanes;
   constexpr unsigned kBoxes = 32 / kSweepLanes;
   ScenePairBuffer vfb{slots[0][warp], 0u}, eeb{slots[1][warp], 0u};
-  const unsigned n = (unsigned)min(*B.n_pieces, B.piece_cap);
-  for (unsigned first = (blockIdx.x * (kThreads / 32) + (unsigned)warp) * kBoxes; first < n;
-       first += gridDim.x * (kThreads / 32) * kBoxes) {
-    uint4 piece = make_uint4(0u, 0u, 0u, 0u);
-    if (first + sub < n) piece = B.pieces[first + sub];
-    ScanBox x{piece.x, 0, 0, 0, 0, 0.0, 0.0, FBox{0.f, 0.f, 0.f, 0.f}};
-    if (piece.z > piece.y) {
-      const unsigned long long key = sorted_key(B, x.i);
-      const Box6 pb = box_at(B.S, (long long)x.i);
-      x.l = (int)((key >> kBatchListShift) & 3ull);
-      x.s = (int)(key >> kBatchSceneShift);
-      x.id = B.S.id[x.i];
-      x.obj = B.S.obj[x.i];
-      x.lo = pb.lo;
-      x.hi = pb.hi;
-      x.pf = fbox_of(pb);
-    }
-    for (unsigned j = piece.y + member; __any_sync(kFull, j - member < piece.z); j += kSweepLanes) {
-      unsigned long long key = 0;
-      const bool found = j < piece.z && test_entry(B, x, j, key);
-      vfb.append(found && x.l != 2, key, B, 0);
-      eeb.append(found && x.l == 2, key, B, 1);
+  for (int q = kPieceQueues - 1; q >= 0; --q) {
+    const unsigned n = (unsigned)min(B.n_pieces[q], B.piece_cap);
+    const uint4* pieces = B.pieces + (unsigned long long)q * B.piece_cap;
+    for (unsigned first = (blockIdx.x * (kThreads / 32) + (unsigned)warp) * kBoxes; first < n;
+         first += gridDim.x * (kThreads / 32) * kBoxes) {
+      uint4 piece = make_uint4(0u, 0u, 0u, 0u);
+      if (first + sub < n) piece = pieces[first + sub];
+      ScanBox x{piece.x, 0, 0, 0, 0, 0.0, 0.0, FBox{0.f, 0.f, 0.f, 0.f}};
+      if (piece.z > piece.y) {
+        const unsigned long long key = sorted_key(B, x.i);
+        const Box6 pb = box_at(B.S, (long long)x.i);
+        x.l = (int)((key >> kBatchListShift) & 3ull);
+        x.s = (int)(key >> kBatchSceneShift);
+        x.id = B.S.id[x.i];
+        x.obj = B.S.obj[x.i];
+        x.lo = pb.lo;
+        x.hi = pb.hi;
+        x.pf = fbox_of(pb);
+      }
+      for (unsigned j = piece.y + member; __any_sync(kFull, j - member < piece.z); j += kSweepLanes) {
+        unsigned long long key = 0;
+        const bool found = j < piece.z && test_entry(B, x, j, key);
+        vfb.append(found && x.l != 2, key, B, 0);
+        eeb.append(found && x.l == 2, key, B, 1);
+      }
     }
   }
   if (vfb.n != 0u) vfb.flush(vfb.n, B, 0);
@@ -912,6 +917,7 @@ size_t sort_temp_bytes(const Totals& t) {
 struct Carve {
   BatchBroad B;
   RowScratch rows = {};
+  size_t zero_bytes = 0;  // from the scratch on
   void* tmp = nullptr;
   size_t tmp_bytes = 0;
   size_t total = 0;
@@ -934,7 +940,14 @@ Carve carve(void* base, const p2c_batch_scene* scenes_dev, int n, const Totals& 
   B.off.vf_cap = static_cast<unsigned long long*>(take(8 * (size_t)(n + 1)));
   B.off.ee_cap = static_cast<unsigned long long*>(take(8 * (size_t)(n + 1)));
   B.off.cell = static_cast<unsigned long long*>(take(8 * (size_t)(n + 1)));
+  const size_t zero_at = off;  // scratch, counters and column tables start at zero
   B.sc = static_cast<BroadScratch*>(take(sizeof(BroadScratch) * (size_t)n));
+  B.n_keyed = static_cast<unsigned long long*>(take(8 * (2 + kPieceQueues)));
+  B.sweep_next = B.n_keyed + 1;
+  B.n_pieces = B.n_keyed + 2;
+  B.cell_begin = static_cast<unsigned*>(take(4 * 3 * (size_t)t.cells));
+  B.cell_end = static_cast<unsigned*>(take(4 * 3 * (size_t)t.cells));
+  C.zero_bytes = off - zero_at;
   B.off.vert = static_cast<unsigned long long*>(take(8 * (size_t)(n + 1)));
   B.off.edge = static_cast<unsigned long long*>(take(8 * (size_t)(n + 1)));
   B.cbox = static_cast<double*>(take(48 * P));
@@ -945,11 +958,8 @@ Carve carve(void* base, const p2c_batch_scene* scenes_dev, int n, const Totals& 
   B.keys32[1] = reinterpret_cast<unsigned*>(B.keys[1]);
   B.key32 = 0;
   B.sorted_buf = 0;
-  B.n_keyed = static_cast<unsigned long long*>(take(24));  // and the two counters behind it
-  B.sweep_next = B.n_keyed + 1;
-  B.n_pieces = B.n_keyed + 2;
   B.piece_cap = piece_cap_for(t.P);
-  B.pieces = static_cast<uint4*>(take(sizeof(uint4) * (size_t)B.piece_cap));
+  B.pieces = static_cast<uint4*>(take(sizeof(uint4) * (size_t)(B.piece_cap * kPieceQueues)));
   B.vals[0] = static_cast<unsigned*>(take(4 * P));
   B.vals[1] = static_cast<unsigned*>(take(4 * P));
   B.S.lo = static_cast<double*>(take(8 * P));
@@ -962,8 +972,6 @@ Carve carve(void* base, const p2c_batch_scene* scenes_dev, int n, const Totals& 
   B.S.fb = static_cast<float4*>(take(16 * P));
   B.S.id = static_cast<int32_t*>(take(4 * P));
   B.S.obj = static_cast<int32_t*>(take(4 * P));
-  B.cell_begin = static_cast<unsigned*>(take(4 * 3 * (size_t)t.cells));
-  B.cell_end = static_cast<unsigned*>(take(4 * 3 * (size_t)t.cells));
   B.pack[0] = static_cast<unsigned long long*>(take(8 * (size_t)std::max<unsigned long long>(t.vf, 1ull)));
   B.pack[1] = static_cast<unsigned long long*>(take(8 * (size_t)std::max<unsigned long long>(t.ee, 1ull)));
   const long long caps[2] = {(long long)t.vf, (long long)t.ee};
@@ -1021,10 +1029,7 @@ int launch_batch_candidates(const p2c_batch_scene* h, const p2c_batch_scene* dev
   B.key32 = key_bits <= 32 ? 1 : 0;  // up to 256 scenes: 32-bit keys halve the key traffic of the sort
   B.pair_bits[0] = t.pair_bits[0];
   B.pair_bits[1] = t.pair_bits[1];
-  P2C_CUDA(cudaMemsetAsync(B.sc, 0, sizeof(BroadScratch) * (size_t)n, s));
-  P2C_CUDA(cudaMemsetAsync(B.cell_begin, 0, 4 * 3 * (size_t)t.cells, s));
-  P2C_CUDA(cudaMemsetAsync(B.cell_end, 0, 4 * 3 * (size_t)t.cells, s));
-  P2C_CUDA(cudaMemsetAsync(B.n_keyed, 0, 3 * sizeof(unsigned long long), s));
+  P2C_CUDA(cudaMemsetAsync(B.sc, 0, C.zero_bytes, s));
   prep_kernel<<<1, kPrepThreads, 0, s>>>(B);
   P2C_CUDA(cudaGetLastError());
   const unsigned long long P = t.P;
