@@ -86,13 +86,19 @@ struct RowLists {
 
 namespace {
 
+// Lanes of a warp that meet in a row add to its counter once: all pairs of a
+// primitive that is large against the others share one.
 template <class Source>
 __global__ void __launch_bounds__(kRowThreads) row_count_kernel(RowLists<Source> L) {
   const RowList<Source>& R = L.l[blockIdx.y];
-  for (long long i = (long long)blockIdx.x * kRowThreads + threadIdx.x; i < R.src.cap;
-       i += (long long)gridDim.x * kRowThreads) {
-    unsigned long long k;
-    if (R.src.load(i, k)) atomicAdd(R.row + R.src.row(k), 1u);
+  const int lane = threadIdx.x & 31;
+  for (long long i0 = (long long)blockIdx.x * kRowThreads; i0 < R.src.cap; i0 += (long long)gridDim.x * kRowThreads) {
+    const long long i = i0 + threadIdx.x;
+    unsigned long long k = 0ull;
+    const bool in = i < R.src.cap && R.src.load(i, k);
+    const unsigned row = in ? (unsigned)R.src.row(k) : 0xffffffffu;
+    const unsigned same = __match_any_sync(0xffffffffu, row);
+    if (in && lane == __ffs((int)same) - 1) atomicAdd(R.row + row, (unsigned)__popc(same));
   }
 }
 
@@ -100,10 +106,18 @@ template <class Source>
 __global__ void __launch_bounds__(kRowThreads) row_place_kernel(RowLists<Source> L) {
   const RowList<Source>& R = L.l[blockIdx.y];
   const unsigned base = R.base();
-  for (long long i = (long long)blockIdx.x * kRowThreads + threadIdx.x; i < R.src.cap;
-       i += (long long)gridDim.x * kRowThreads) {
-    unsigned long long k;
-    if (R.src.load(i, k)) R.placed[atomicAdd(R.row + R.src.row(k), 1u) - base] = k;
+  const int lane = threadIdx.x & 31;
+  for (long long i0 = (long long)blockIdx.x * kRowThreads; i0 < R.src.cap; i0 += (long long)gridDim.x * kRowThreads) {
+    const long long i = i0 + threadIdx.x;
+    unsigned long long k = 0ull;
+    const bool in = i < R.src.cap && R.src.load(i, k);
+    const unsigned row = in ? (unsigned)R.src.row(k) : 0xffffffffu;
+    const unsigned same = __match_any_sync(0xffffffffu, row);
+    const int leader = __ffs((int)same) - 1;
+    unsigned at = 0u;
+    if (in && lane == leader) at = atomicAdd(R.row + row, (unsigned)__popc(same));
+    at = __shfl_sync(0xffffffffu, at, leader) + (unsigned)__popc(same & ((1u << lane) - 1u));
+    if (in) R.placed[at - base] = k;
   }
 }
 
