@@ -602,13 +602,13 @@ constexpr unsigned kWholeRun = 8;  // a column of at most this many entries is w
 // against the others of its scene (a ground quad under a mesh) has all of them
 // in one window: walked by its eight lanes alone it sets the length of the
 // launch.  Candidates of a sheet of 96,800 triangles over one quad: 36,400 us
-// by the eight lanes, 714 with the queues; 64 uneven scenes, which hardly use
+// by the eight lanes, 530 with the queues; 64 uneven scenes, which hardly use
 // them, pay 3 us for their empty launch.  Windows from 128 / 256 / 512 entries
-// on: 698 / 714 / 717 us; pieces of 32 / 64 / 128 entries: 737 / 714 / 720.
+// on differ by 2 %, pieces of 32 / 64 / 128 entries by 3 %.
 // A full queue leaves a window to its lanes.  Windows are queued by length, one
 // queue for each factor of four, so that the many middling ones of a dense
 // scene never take the room of the longest (four self-colliding sheets over
-// quads: 4,030 us when they do, 567 when not).
+// quads: 4,030 us when they do, 560 when not).
 #ifndef P2C_BATCH_LONG_WINDOW
 #define P2C_BATCH_LONG_WINDOW 256
 #endif
@@ -618,11 +618,11 @@ constexpr unsigned kWholeRun = 8;  // a column of at most this many entries is w
 constexpr unsigned kLongWindow = P2C_BATCH_LONG_WINDOW;
 constexpr unsigned kPiece = P2C_BATCH_PIECE;
 constexpr int kPieceQueues = 4;
-// All queues: one piece per eight primitives of the batch, within [4096, 2^20]
+// A queue holds one piece per eight primitives of the batch, within [4096, 2^20]
 // (a small batch keeps a small workspace).
 __host__ __device__ inline unsigned long long piece_cap_for(unsigned long long prims) {
   const unsigned long long c = prims / 8;
-  return (c < 4096ull ? 4096ull : (c > (1ull << 20) ? (1ull << 20) : c)) / kPieceQueues;
+  return c < 4096ull ? 4096ull : (c > (1ull << 20) ? (1ull << 20) : c);
 }
 
 // A scanning box: its list, scene and primitive, and what its walk tests
@@ -667,20 +667,39 @@ __device__ __forceinline__ bool test_entry(const BatchBroad& B, const ScanBox& x
 }
 
 // Queues the window [offset, offset + len) of box i, if it is long and fits.
+// Of the last queue, whose windows have no largest length, a window takes at
+// most a kQueueShare-th of what is free, in longer pieces if need be: 30,000
+// triangles among 20 larger ones have 140 windows of 30,000 to 90,000 entries,
+// more than the queue holds in short pieces (28.4 ms then, 5.6 so).
+constexpr unsigned kQueueShare = 32;
+
 __device__ __forceinline__ bool queue_window(uint4* pieces, unsigned long long* n_pieces, unsigned long long cap,
                                              unsigned i, unsigned offset, unsigned len) {
   if (len <= kLongWindow) return false;
   const int q = (len > 4u * kLongWindow) + (len > 16u * kLongWindow) + (len > 64u * kLongWindow);
-  if (*reinterpret_cast<volatile unsigned long long*>(n_pieces + q) >= cap) return false;
-  const unsigned n = (len + kPiece - 1u) / kPiece;
-  const unsigned long long at = atomicAdd(n_pieces + q, (unsigned long long)n);
   pieces += (unsigned long long)q * cap;
-  if (at + n > cap) {
-    for (unsigned long long k = at; k < cap; ++k) pieces[k] = make_uint4(0u, 0u, 0u, 0u);  // empty
-    return false;
+  n_pieces += q;
+  unsigned long long at = *reinterpret_cast<volatile unsigned long long*>(n_pieces);
+  unsigned piece = kPiece, n = (len + kPiece - 1u) / kPiece;
+  if (q < kPieceQueues - 1) {
+    if (at >= cap) return false;
+    at = atomicAdd(n_pieces, (unsigned long long)n);
+    if (at + n > cap) {
+      for (unsigned long long k = at; k < cap; ++k) pieces[k] = make_uint4(0u, 0u, 0u, 0u);  // empty
+      return false;
+    }
+  } else {
+    for (unsigned long long seen = at;; at = seen) {  // ends: another window's success changes the count, never past cap
+      const unsigned most = (unsigned)(cap - at) / kQueueShare;
+      if (most == 0u) return false;
+      piece = max(kPiece, (len + most - 1u) / most);
+      n = (len + piece - 1u) / piece;
+      seen = atomicCAS(n_pieces, at, at + n);
+      if (seen == at) break;
+    }
   }
   for (unsigned k = 0; k < n; ++k)
-    pieces[at + k] = make_uint4(i, offset + k * kPiece, offset + min(len, (k + 1u) * kPiece), 0u);
+    pieces[at + k] = make_uint4(i, offset + k * piece, offset + min(len, (k + 1u) * piece), 0u);
   return true;
 }
 

@@ -72,6 +72,23 @@ def test_queue_of_pieces_fills(cuda_device):
     _pairs_equal(batch, cuda_device, exclude_self=False)
 
 
+def test_many_large_primitives(cuda_device):
+    """More windows of the longest kind (over 16,384 entries) than their queue
+    holds in short pieces."""
+    from p2cccd_b200 import scenes
+
+    g = np.random.default_rng(9)
+    small = np.repeat(g.uniform(-1.0, 1.0, (6000, 1, 3)), 3, axis=1).reshape(-1, 3)
+    small = small + g.normal(0.0, 1e-3, small.shape)
+    tri = lambda n: np.arange(3 * n, dtype=np.int32).reshape(-1, 3)  # noqa: E731
+    objs = []
+    for _ in range(30):
+        v = g.normal(0.0, 0.1, (3, 3))
+        objs.append((v - 10.0, v + 10.0, tri(1)))
+    objs.append((small, small + g.normal(0.0, 1e-3, small.shape), tri(6000)))
+    _pairs_equal([scenes.combine([(a, b, f, scenes.unique_edges(f)) for a, b, f in objs])], cuda_device)
+
+
 @pytest.mark.parametrize("n", [220])
 def test_large_primitive_does_not_set_the_time(cuda_device, n):
     """Walked by one group of lanes the quad's windows took 36 ms; as pieces
