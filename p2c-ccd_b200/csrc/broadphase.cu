@@ -1031,9 +1031,9 @@ int launch_broadphase(const p2c_scene& scene, unsigned long long* vf_out, long l
                         RankList{L.unsorted[1], ee_out, ee_cap, ee_shift}, vf_blocks, (const SceneScratch*)L.sc,
                         counts_dev));
   } else if (sort_out) {
-    const long long rows[2] = {scene.nv, scene.ne};
+    const long long rows[2] = {scene.nv, scene.ne}, most_in_row[2] = {scene.nf, scene.ne};
     rc = launch_pair_rows(L.rows, SceneRows{vf_out, &L.sc->vf_count, vf_cap, vf_shift},
-                          SceneRows{ee_out, &L.sc->ee_count, ee_cap, ee_shift}, rows, s);
+                          SceneRows{ee_out, &L.sc->ee_count, ee_cap, ee_shift}, rows, most_in_row, s);
     if (rc != P2C_OK) return rc;
   }
   if (!rank_sort)  // the rank sort writes the counts itself

@@ -905,6 +905,7 @@ __global__ void export_counts_kernel(BatchBroad B) {
 struct Totals {
   unsigned long long P = 0, V = 0, E = 0, vf = 0, ee = 0, cells = 0;
   int pair_bits[2] = {2, 2};  // widest packed pair of any scene: vf, ee
+  long long most_in_row[2] = {0, 0};  // most pairs of one vertex, of one edge
 };
 
 Totals totals_of(const p2c_batch_scene* h, int n) {
@@ -918,6 +919,8 @@ Totals totals_of(const p2c_batch_scene* h, int n) {
     t.ee += (unsigned long long)h[s].ee_cap;
     t.cells += (unsigned long long)cell_budget(np);
     t.pair_bits[0] = std::max(t.pair_bits[0], bit_length(h[s].nv) + std::max(1, bit_length(h[s].nf)));
+    t.most_in_row[0] = std::max<long long>(t.most_in_row[0], h[s].nf);
+    t.most_in_row[1] = std::max<long long>(t.most_in_row[1], h[s].ne);
     t.pair_bits[1] = std::max(t.pair_bits[1], bit_length(h[s].ne) + std::max(1, bit_length(h[s].ne)));
   }
   return t;
@@ -1106,7 +1109,7 @@ int launch_batch_candidates(const p2c_batch_scene* h, const p2c_batch_scene* dev
   const BatchRows vf{B.scenes, B.sc, B.pack[0], B.off.vf_cap, B.off.vert, n, B.pair_bits[0], 0, (long long)t.vf};
   const BatchRows ee{B.scenes, B.sc, B.pack[1], B.off.ee_cap, B.off.edge, n, B.pair_bits[1], 1, (long long)t.ee};
   const long long rows[2] = {(long long)t.V, (long long)t.E};
-  rc = launch_pair_rows(C.rows, vf, ee, rows, s);
+  rc = launch_pair_rows(C.rows, vf, ee, rows, t.most_in_row, s);
   if (rc != P2C_OK) return rc;
   export_counts_kernel<<<grid_for(n, 128), 128, 0, s>>>(B);
   P2C_CUDA(cudaGetLastError());

@@ -33,7 +33,6 @@
 // in order, and each total is the exact left-to-right sum formed from
 // composable pieces (the ordered fold below).  Every total is therefore the
 // reference's to the bit.
-#include <cooperative_groups.h>
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_select.cuh>
 #include <thrust/iterator/counting_iterator.h>
@@ -41,6 +40,7 @@
 #include <cmath>
 
 #include "p2c_internal.cuh"
+#include "run_merge.cuh"
 
 namespace p2c {
 namespace {
@@ -92,8 +92,9 @@ struct __align__(16) WalkRow {
 };
 
 struct Tile {
-  unsigned start, len;
+  unsigned start, len;  // len has kTileMerged set when the group has several
 };
+constexpr unsigned kTileMerged = 1u << 31;
 
 // One piece of kFoldChunk terms of a total: its sum (any order, to predict the
 // binade it is added in), that binade's last place, and the increments of the
@@ -275,11 +276,12 @@ __global__ void __launch_bounds__(kThreads) parse_kernel(ParseIn in, long long n
 //
 // Rows of a group lie together in index order; they are ordered by (key,
 // index).  Groups of up to 256 rows are sorted by one warp each in registers,
-// larger ones in tiles of 4096 by one block each, and the tiles are
-// merged pairwise by one cooperative launch (which returns at once when no
-// group is larger than a tile).  Each row's key is read once; the sort over
-// all rows by the 64-bit key that this stands in for was 8 radix passes:
-// 168 us for 1 M rows, the ordering kernels 52.
+// larger ones in tiles of 4096 by one block each, and the tiles are merged
+// eight at a time by a launch per round (which returns at once when no group is
+// larger than a tile; plain launches, so that a stream which owns part of the
+// SMs only will do).  Each row's key is read once; the sort over all rows by the
+// 64-bit key that this stands in for was 8 radix passes: 168 us for 1 M rows,
+// the ordering kernels 52.
 
 __device__ __forceinline__ bool entry_less(unsigned long long ka, unsigned ia, unsigned long long kb, unsigned ib) {
   return ka < kb || (ka == kb && ia < ib);
@@ -396,7 +398,8 @@ __global__ void __launch_bounds__(kThreads) order_small_kernel(long long n, unsi
       if (lane == 0) {
         const unsigned tiles = (len + kTileRows - 1) / kTileRows;
         const unsigned at = atomicAdd(&L.acc->n_tiles, tiles);
-        for (unsigned k = 0; k < tiles; ++k) L.tiles[at + k] = Tile{begin + k * kTileRows, min(kTileRows, len - k * kTileRows)};
+        for (unsigned k = 0; k < tiles; ++k)
+          L.tiles[at + k] = Tile{begin + k * kTileRows, min(kTileRows, len - k * kTileRows) | (tiles > 1u ? kTileMerged : 0u)};
         if (len > kTileRows) {
           const unsigned long long b = atomicAdd(&L.acc->big, (1ull << 32) | len);
           L.big_start[b >> 32] = begin;
@@ -413,97 +416,86 @@ __global__ void __launch_bounds__(kThreads) order_small_kernel(long long n, unsi
   }
 }
 
-// One block per tile; keys of tiles to be merged go along.
+struct OrderBuffer {
+  unsigned long long* key;
+  unsigned* idx;
+};
+// What a round reads: the last one writes (key[1], order), and they alternate.
+__device__ __forceinline__ OrderBuffer merge_buffer(const DenseLayout& L, unsigned* order, int rounds, int round) {
+  if (((rounds - round) & 1) == 0) return OrderBuffer{L.key[1], order};
+  return OrderBuffer{L.qkey[0], L.idx[1]};
+}
+
+// One block per tile; tiles to be merged go where the first round reads, with their keys.
 __global__ void __launch_bounds__(kTileThreads) order_tile_kernel(unsigned* order, DenseLayout L) {
   extern __shared__ __align__(16) unsigned char tile_raw[];
   unsigned long long* key = reinterpret_cast<unsigned long long*>(tile_raw);
   unsigned* idx = reinterpret_cast<unsigned*>(tile_raw + kTileRows * 8);
   const unsigned n = L.acc->n_tiles;
+  const OrderBuffer merged = merge_buffer(L, order, merge_rounds(kTileRows, L.acc->longest), 0);
   for (unsigned t = blockIdx.x; t < n; t += gridDim.x) {
     const Tile tile = L.tiles[t];
+    const unsigned len = tile.len & ~kTileMerged;
     unsigned size = 2u;
-    while (size < tile.len) size <<= 1;
+    while (size < len) size <<= 1;
     for (unsigned e = threadIdx.x; e < size; e += kTileThreads) {
-      const unsigned j = e < tile.len ? order[tile.start + e] : 0xffffffffu;
+      const unsigned j = e < len ? order[tile.start + e] : 0xffffffffu;
       idx[e] = j;
-      key[e] = e < tile.len ? L.key[0][j] : ~0ull;
+      key[e] = e < len ? L.key[0][j] : ~0ull;
     }
     __syncthreads();
     block_sort(key, idx, size);
-    for (unsigned e = threadIdx.x; e < tile.len; e += kTileThreads) {
-      order[tile.start + e] = idx[e];
-      L.key[1][tile.start + e] = key[e];
+    const bool merge = (tile.len & kTileMerged) != 0u;
+    for (unsigned e = threadIdx.x; e < len; e += kTileThreads) {
+      if (merge) merged.key[tile.start + e] = key[e];
+      (merge ? merged.idx : order)[tile.start + e] = idx[e];
     }
     __syncthreads();
   }
 }
 
-// Pairwise merges of the tiles of groups larger than one: every thread writes
-// kMergeOut consecutive places, from where the merge path crosses their first.
-constexpr int kMergeOut = 8;
-
-__global__ void __launch_bounds__(kThreads) order_merge_kernel(unsigned* order, DenseLayout L) {
+// One round over the groups of more than one tile (run_merge.cuh).
+__global__ void __launch_bounds__(kThreads) order_merge_kernel(unsigned* order, DenseLayout L, int round) {
+  pdl_wait();
+  pdl_trigger();
+  const int rounds = merge_rounds(kTileRows, L.acc->longest);
+  if (round >= rounds) return;
   const unsigned long long big = L.acc->big;
-  const unsigned n_big = (unsigned)(big >> 32), rows = (unsigned)big, longest = L.acc->longest;
-  if (n_big == 0u) return;  // the same in every block
-  cooperative_groups::grid_group grid = cooperative_groups::this_grid();
-  unsigned long long* key[2] = {L.key[1], L.qkey[0]};
-  unsigned* idx[2] = {order, L.idx[1]};
-  int src = 0;
-  const unsigned stride = gridDim.x * kThreads, t = blockIdx.x * kThreads + threadIdx.x;
-  for (unsigned long long width = kTileRows; width < longest; width *= 2ull) {
-    for (unsigned long long v0 = (unsigned long long)t * kMergeOut; v0 < rows;
-         v0 += (unsigned long long)stride * kMergeOut) {
-      const unsigned vend = (unsigned)min((unsigned long long)rows, v0 + kMergeOut);
-      unsigned v = (unsigned)v0;
-      while (v < vend) {  // pieces of one pair of runs of one group
-        unsigned lo = 0u, hi = n_big - 1u;
-        while (lo < hi) {
-          const unsigned mid = (lo + hi + 1u) >> 1;
-          if (L.big_at[mid] <= v) lo = mid;
-          else hi = mid - 1u;
-        }
-        const unsigned at = L.big_at[lo], len = (lo + 1u < n_big ? L.big_at[lo + 1u] : rows) - at;
-        const unsigned a = v - at;  // place in the group
-        const unsigned long long pair = (unsigned long long)a / (2ull * width) * (2ull * width);
-        const unsigned base = L.big_start[lo] + (unsigned)pair;
-        const unsigned left = (unsigned)min(width, (unsigned long long)len - pair);
-        const unsigned both = (unsigned)min(2ull * width, (unsigned long long)len - pair);
-        const unsigned right = both - left;
-        const unsigned d = a - (unsigned)pair, dend = min(both, d + (vend - v));
-        const unsigned long long *ka = key[src] + base, *kb = ka + left;
-        const unsigned *ia = idx[src] + base, *ib = ia + left;
-        unsigned x0 = d > right ? d - right : 0u, x1 = min(d, left);  // entries of the left run before place d
-        while (x0 < x1) {
-          const unsigned m = (x0 + x1) >> 1, o = d - 1u - m;
-          const bool left_first = ka[m] < kb[o] || (ka[m] == kb[o] && ia[m] < ib[o]);
-          if (left_first) x0 = m + 1u;
-          else x1 = m;
-        }
-        unsigned x = x0, y = d - x0;
-        for (unsigned p = d; p < dend; ++p) {
-          const bool take_left = y >= right || (x < left && (ka[x] < kb[y] || (ka[x] == kb[y] && ia[x] < ib[y])));
-          key[1 - src][base + p] = take_left ? ka[x] : kb[y];
-          idx[1 - src][base + p] = take_left ? ia[x] : ib[y];
-          if (take_left) ++x;
-          else ++y;
-        }
-        v += dend - d;
-      }
-    }
-    grid.sync();
-    src = 1 - src;
-  }
-  if (src == 0) return;
-  for (unsigned v = t; v < rows; v += stride) {
-    unsigned lo = 0u, hi = n_big - 1u;
-    while (lo < hi) {
-      const unsigned mid = (lo + hi + 1u) >> 1;
-      if (L.big_at[mid] <= v) lo = mid;
+  const unsigned n_big = (unsigned)(big >> 32), rows = (unsigned)big;
+  const OrderBuffer from = merge_buffer(L, order, rounds, round), to = merge_buffer(L, order, rounds, round + 1);
+  const unsigned width = merge_width(kTileRows, round);
+  for (unsigned v0 = blockIdx.x * kThreads; v0 < rows; v0 += gridDim.x * kThreads) {
+    const bool live = v0 + threadIdx.x < rows;
+    const unsigned v = min(v0 + threadIdx.x, rows - 1u);
+    unsigned g = 0u, hi = n_big - 1u;
+    while (g < hi) {
+      const unsigned mid = (g + hi + 1u) >> 1;
+      if (L.big_at[mid] <= v) g = mid;
       else hi = mid - 1u;
     }
-    const unsigned p = L.big_start[lo] + (v - L.big_at[lo]);
-    order[p] = L.idx[1][p];
+    const unsigned at = L.big_at[g], len = (g + 1u < n_big ? L.big_at[g + 1u] : rows) - at, a = v - at;
+    const unsigned own = a / width, run0 = own / kMergeRuns * kMergeRuns, first = L.big_start[g] + run0 * width;
+    const unsigned long long* key = from.key + first;
+    const unsigned* idx = from.idx + first;
+    const unsigned long long my_key = key[a - run0 * width];
+    const unsigned my_idx = idx[a - run0 * width];
+    unsigned n[kMergeRuns];
+#pragma unroll
+    for (unsigned k = 0; k < kMergeRuns; ++k) {
+      const unsigned long long begin = (unsigned long long)(run0 + k) * width;  // in the group
+      n[k] = run0 + k == own || begin >= len ? 0u : (unsigned)min((unsigned long long)width, len - begin);
+    }
+    const unsigned g0 = __shfl_sync(0xffffffffu, g, 0), own0 = __shfl_sync(0xffffffffu, own, 0);
+    const bool together = __all_sync(0xffffffffu, live && g == g0 && own == own0);
+    const unsigned place =
+        first + (a - own * width) +
+        entries_before(width, n, my_key, my_idx, together, [&](unsigned k, unsigned p, unsigned long long x, unsigned i) {
+          const unsigned long long other = key[k * width + p];
+          return other < x || (other == x && idx[k * width + p] < i);
+        });
+    if (!live) continue;
+    to.key[place] = my_key;
+    to.idx[place] = my_idx;
   }
 }
 
@@ -1152,11 +1144,9 @@ int p2c_dense_group_early_stop(int64_t n, const uint64_t* query_id_dev, const ui
         const int tiles = (int)std::min<long long>(n / kWarpRows + 1, info.sm_count * 4);
         order_tile_kernel<<<tiles, kTileThreads, smem, s>>>(order, L);
       }
-      if (n > (long long)kTileRows) {
-        void* args[] = {&order, &L};
-        P2C_CUDA(cudaLaunchCooperativeKernel((const void*)order_merge_kernel, dim3(info.sm_count), dim3(kThreads), args,
-                                             0, s));
-      }
+      for (int round = 0; round < merge_rounds(kTileRows, (unsigned long long)n); ++round)
+        P2C_CUDA(launch_pdl(order_merge_kernel, dim3((unsigned)info.sm_count * 4u), dim3(kThreads), 0, s, order, L,
+                            round));
     }
     group_kernel<<<grid, kThreads, 0, s>>>(order, n, config->representative_attempt_limit,
                                            config->interval_miss_penalty_scale, L);

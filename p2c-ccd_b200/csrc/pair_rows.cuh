@@ -4,8 +4,10 @@
 // A counting sort by a (count, scan, place) puts the pairs into rows, then
 // every row orders its own b: rows of up to 16 pairs count the smaller ones
 // pair by pair, rows of up to 1,024 are sorted by one warp each in registers,
-// longer ones in tiles of 8,192 by one block each, merged pairwise by one
-// cooperative launch that returns at once when there is nothing to merge.
+// longer ones in tiles of 8,192 by one block each, merged eight at a time by a
+// launch per round that returns at once when there is nothing to merge.  Plain
+// launches: a cooperative one, which could run all rounds, fails on a stream
+// that owns part of the SMs only.
 //
 // Bound by L2: each pair is read twice and placed once at random (an 8-byte
 // write to its row), which stays in the 126 MB L2 for the lists of a step.  A
@@ -14,11 +16,10 @@
 // places) 865 -> 473; a 624k-triangle cloth (3.1 M in 4.4 M) 327 -> 90.
 #pragma once
 
-#include <cooperative_groups.h>
-
 #include <cub/device/device_scan.cuh>
 
 #include "p2c_internal.cuh"
+#include "run_merge.cuh"
 
 namespace p2c {
 
@@ -26,7 +27,6 @@ constexpr int kRowThreads = 256;
 constexpr unsigned kRowCountMax = 16;    // pairs of a row ordered by counting
 constexpr unsigned kRowWarpMax = 1024;   // by a warp
 constexpr unsigned kRowTile = 8192;      // by a block
-constexpr int kRowMergeOut = 8;          // places a thread merges at once
 
 struct RowSpan {
   unsigned start, len;
@@ -232,13 +232,24 @@ __device__ __forceinline__ void row_warp_order(const RowList<Source>& R, RowSpan
   }
 }
 
+// Rounds that merge the longest row of both lists.
+template <class Source>
+__device__ __forceinline__ int row_rounds(const RowLists<Source>& L) {
+  return merge_rounds(kRowTile, max(L.l[0].ctr->longest, L.l[1].ctr->longest));
+}
+// Whether a round reads placed (otherwise the places of the same numbers in
+// the input).  The last one does: it stores, which may be over the input.
+__device__ __forceinline__ bool row_round_placed(int rounds, int round) { return ((rounds - 1 - round) & 1) == 0; }
+
 // Tiles of long rows, a block each; then rows of 17 to 1,024 pairs, a warp each.
-// Tiles of one-tile rows go out, those to be merged back to placed.
+// Tiles of one-tile rows go out, those to be merged where the first round reads.
 template <class Source>
 __global__ void __launch_bounds__(kRowThreads, 4) row_long_kernel(RowLists<Source> L) {
   __shared__ unsigned word[kRowTile];
   const RowList<Source>& R = L.l[blockIdx.y];
   const unsigned n_tiles = R.ctr->n_tiles;
+  const int rounds = n_tiles != 0u ? row_rounds(L) : 0;
+  unsigned long long* merged = row_round_placed(rounds, 0) ? R.placed : R.src.input();
   for (unsigned t = blockIdx.x; t < n_tiles; t += gridDim.x) {
     const RowSpan s = R.tiles[t];
     unsigned size = 2u;
@@ -267,7 +278,7 @@ __global__ void __launch_bounds__(kRowThreads, 4) row_long_kernel(RowLists<Sourc
     for (unsigned e = threadIdx.x; e < s.len; e += kRowThreads) {
       const unsigned long long key = (first & ~mask) | word[e];
       if (row_len <= kRowTile) R.src.store(s.start + e, key, R.row);
-      else R.placed[s.start + e] = key;
+      else merged[s.start + e] = key;
     }
     __syncthreads();
   }
@@ -303,63 +314,48 @@ __device__ __forceinline__ unsigned row_big(const RowList<Source>& R, unsigned n
   return lo;
 }
 
-// Pairwise merges of the tiles of rows longer than one, between placed and the
-// places of the same numbers in the input: every thread writes kRowMergeOut
-// consecutive places, from where the merge path crosses the first.
+// One round over the rows of more than one tile (run_merge.cuh).  Bound by the
+// latency of the searches and by scattered 8-byte writes, both in L2.  1.4 M
+// pairs in rows of up to 145,000, two rounds: 186 us, as much as four pairwise
+// rounds in one cooperative launch (176); 266 with every lane searching whole
+// runs.
 template <class Source>
-__global__ void __launch_bounds__(kRowThreads) row_merge_kernel(RowLists<Source> L) {
-  const unsigned longest = max(L.l[0].ctr->longest, L.l[1].ctr->longest);
-  if (longest == 0u) return;  // the same in every block
-  cooperative_groups::grid_group grid = cooperative_groups::this_grid();
-  const unsigned stride = gridDim.x * kRowThreads, t = blockIdx.x * kRowThreads + threadIdx.x;
-  int src = 0;
-  for (unsigned long long width = kRowTile; width < longest; width *= 2ull) {
-    for (int list = 0; list < 2; ++list) {
-      const RowList<Source>& R = L.l[list];
-      const unsigned long long big = R.ctr->big;
-      const unsigned n_big = (unsigned)(big >> 32), total = (unsigned)big;
-      const unsigned long long* from = src == 0 ? R.placed : R.src.input();
-      unsigned long long* to = src == 0 ? R.src.input() : R.placed;
-      for (unsigned long long v0 = (unsigned long long)t * kRowMergeOut; v0 < total;
-           v0 += (unsigned long long)stride * kRowMergeOut) {
-        const unsigned vend = (unsigned)min((unsigned long long)total, v0 + kRowMergeOut);
-        unsigned v = (unsigned)v0;
-        while (v < vend) {  // pieces of one pair of runs of one row
-          const unsigned r = row_big(R, n_big, v), at = R.big_at[r];
-          const unsigned len = (r + 1u < n_big ? R.big_at[r + 1u] : total) - at;
-          const unsigned long long pair = (unsigned long long)(v - at) / (2ull * width) * (2ull * width);
-          const unsigned first = R.big_start[r] + (unsigned)pair;
-          const unsigned left = (unsigned)min(width, (unsigned long long)len - pair);
-          const unsigned both = (unsigned)min(2ull * width, (unsigned long long)len - pair), right = both - left;
-          const unsigned d = v - at - (unsigned)pair, dend = min(both, d + (vend - v));
-          const unsigned long long *ka = from + first, *kb = ka + left;
-          unsigned x0 = d > right ? d - right : 0u, x1 = min(d, left);  // words of the left run before place d
-          while (x0 < x1) {
-            const unsigned m = (x0 + x1) >> 1;
-            if (ka[m] < kb[d - 1u - m]) x0 = m + 1u;
-            else x1 = m;
-          }
-          unsigned x = x0, y = d - x0;
-          for (unsigned p = d; p < dend; ++p) {
-            const bool take_left = y >= right || (x < left && ka[x] < kb[y]);
-            to[first + p] = take_left ? ka[x++] : kb[y++];
-          }
-          v += dend - d;
-        }
-      }
+__global__ void __launch_bounds__(kRowThreads) row_merge_kernel(RowLists<Source> L, int round) {
+  pdl_wait();
+  pdl_trigger();
+  const int rounds = row_rounds(L);
+  if (round >= rounds) return;
+  const RowList<Source>& R = L.l[blockIdx.y];
+  const unsigned long long big = R.ctr->big;
+  const unsigned n_big = (unsigned)(big >> 32), total = (unsigned)big;
+  const bool last = round == rounds - 1;
+  const unsigned long long* from = row_round_placed(rounds, round) ? R.placed : R.src.input();
+  unsigned long long* to = row_round_placed(rounds, round) ? R.src.input() : R.placed;
+  const unsigned width = merge_width(kRowTile, round);
+  for (unsigned long long v0 = (unsigned long long)blockIdx.x * kRowThreads; v0 < total;
+       v0 += (unsigned long long)gridDim.x * kRowThreads) {
+    const bool live = v0 + threadIdx.x < total;
+    const unsigned v = (unsigned)min(v0 + threadIdx.x, (unsigned long long)total - 1ull);
+    const unsigned r = row_big(R, n_big, v), at = R.big_at[r];
+    const unsigned len = (r + 1u < n_big ? R.big_at[r + 1u] : total) - at, a = v - at;
+    const unsigned own = a / width, run0 = own / kMergeRuns * kMergeRuns;
+    const unsigned first = R.big_start[r] + run0 * width;  // run0 * width <= a
+    const unsigned long long* runs = from + first;
+    const unsigned long long key = runs[a - run0 * width];
+    unsigned n[kMergeRuns];
+#pragma unroll
+    for (unsigned k = 0; k < kMergeRuns; ++k) {
+      const unsigned long long begin = (unsigned long long)(run0 + k) * width;  // in the row
+      n[k] = run0 + k == own || begin >= len ? 0u : (unsigned)min((unsigned long long)width, len - begin);
     }
-    grid.sync();
-    src = 1 - src;
-  }
-  for (int list = 0; list < 2; ++list) {
-    const RowList<Source>& R = L.l[list];
-    const unsigned long long big = R.ctr->big;
-    const unsigned n_big = (unsigned)(big >> 32), total = (unsigned)big;
-    const unsigned long long* from = src == 0 ? R.placed : R.src.input();
-    for (unsigned v = t; v < total; v += stride) {
-      const unsigned r = row_big(R, n_big, v), p = R.big_start[r] + (v - R.big_at[r]);
-      R.src.store(p, from[p], R.row);
-    }
+    const unsigned r0 = __shfl_sync(0xffffffffu, r, 0), own0 = __shfl_sync(0xffffffffu, own, 0);
+    const bool together = __all_sync(0xffffffffu, live && r == r0 && own == own0);
+    const unsigned place = a - own * width +
+                           entries_before(width, n, key, 0u, together, [&](unsigned k, unsigned p, unsigned long long x,
+                                                                           unsigned) { return runs[k * width + p] < x; });
+    if (!live) continue;
+    if (last) R.src.store(first + place, key, R.row);
+    else to[first + place] = key;
   }
 }
 
@@ -405,10 +401,11 @@ RowScratch carve_rows(long long rows, const long long pair_cap[2], Take take) {
   return s;
 }
 
-// Sorts both lists (one of capacity 0 takes no part).
+// Sorts both lists (one of capacity 0 takes no part).  most_in_row: pairs that
+// one row of each list can have.
 template <class Source>
 int launch_pair_rows(const RowScratch& w, const Source& first, const Source& second, const long long rows[2],
-                     cudaStream_t s) {
+                     const long long most_in_row[2], cudaStream_t s) {
   RowLists<Source> L;
   const Source* src[2] = {&first, &second};
   for (int k = 0; k < 2; ++k)
@@ -426,11 +423,10 @@ int launch_pair_rows(const RowScratch& w, const Source& first, const Source& sec
   row_place_kernel<<<blocks, kRowThreads, 0, s>>>(L);
   row_short_kernel<<<blocks, kRowThreads, 0, s>>>(L);
   row_long_kernel<<<dim3((unsigned)info.sm_count * 4u, 2), kRowThreads, 0, s>>>(L);
-  if (most > (long long)kRowTile) {
-    void* args[] = {&L};
-    P2C_CUDA(cudaLaunchCooperativeKernel((const void*)row_merge_kernel<Source>, dim3((unsigned)info.sm_count),
-                                         dim3(kRowThreads), args, 0, s));
-  }
+  const long long longest = std::max(std::min(first.cap, most_in_row[0]), std::min(second.cap, most_in_row[1]));
+  for (int round = 0; round < merge_rounds(kRowTile, (unsigned long long)longest); ++round)
+    P2C_CUDA(launch_pdl(row_merge_kernel<Source>, dim3((unsigned)info.sm_count * 4u, 2), dim3(kRowThreads), 0, s, L,
+                        round));
   P2C_CUDA(cudaGetLastError());
   return P2C_OK;
 }
