@@ -241,7 +241,7 @@ int p2c_certify_queries(const p2c_point_triangle* pt_dev, int64_t n_pt, const in
  * while a CUDA graph is captured, frame loops that forbid allocation, hosts that
  * own all device memory under a fixed budget.  No counterpart in the reference.
  * Same arguments and results as p2c_certify_queries without the workspace: the
- * scratch is a 1 MiB file-scope device array that every GPU loading this library
+ * scratch is a 1.44 MiB file-scope device array that every GPU loading this library
  * holds until exit, so at most P2C_STATIC_QUEUE_MAX_QUERIES work items per call
  * (larger queues return P2C_ERR_INVALID).  The first call on a device resolves
  * the array's device address (cudaGetSymbolAddress); make that first call before

@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(kCertifyThreads, kCertifyMinBlocks)
     f1 = (int)min(32ll, max(1ll, (prob.n(1) + warps - 1) / warps));
     f2 = (int)min(32ll, max(1ll, (prob.n(2) + warps - 1) / warps));
   }
-  const bool ok = run_engine<true>(prob, prm, f1, f2, sh, st, &sc->engine, pools, t_start);
+  const bool ok = run_engine(prob, prm, f1, f2, sh, st, &sc->engine, pools, t_start);
   flush_stats(st, ok, sc);
 }
 

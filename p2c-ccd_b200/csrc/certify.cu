@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(kCertifyThreads, kCertifyMinBlocks)
   EngineShared& sh = reinterpret_cast<EngineShared*>(smem_raw)[threadIdx.x >> 5];
   WarpStats st;
   const unsigned long long t_start = global_ns();
-  const bool ok = run_engine<true>(prob, prm, fetch_pt, fetch_ee, sh, st, &scratch->engine, pools, t_start);
+  const bool ok = run_engine(prob, prm, fetch_pt, fetch_ee, sh, st, &scratch->engine, pools, t_start);
   flush_stats(st, ok, scratch);
 }
 

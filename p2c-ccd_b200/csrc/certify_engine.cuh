@@ -19,7 +19,7 @@
 // deep tree shortens by up to five: a warp's instructions cost the same
 // whether one lane or all take part.
 //
-// Across warps (kExport): when some warp has nothing to do, a warp holding
+// Across warps: when some warp has nothing to do, a warp holding
 // more nodes than one iteration takes publishes its shallowest ones to a
 // global pool that idle warps drain, so one deep tree is bisected by many
 // warps.
@@ -341,7 +341,7 @@ __device__ __forceinline__ Outcome tree_outcome(unsigned long long coll_key, uns
 //   void load(int family, long long q, Geo&, double& T0, double& T1, int& bad) const;
 //   void finish(int family, long long q, const Outcome&) const;
 //   void invalid(int family, long long q, int bad, double T0, double T1) const;
-template <bool kExport, class P>
+template <class P>
 __device__ bool run_engine(const P& prob, const CertParams& prm, int fetch1, int fetch2,
                            EngineShared& sh, WarpStats& st, EngineState* es, const EnginePools& pools,
                            unsigned long long t_start) {
@@ -403,13 +403,13 @@ __device__ bool run_engine(const P& prob, const CertParams& prm, int fetch1, int
           prob.finish(sh.family[lane], sh.qidx[lane], tree_outcome(ck, mb, und, sh.T0[lane], sh.T1[lane]));
       }
       const unsigned finished = __ballot_sync(FULL, finish);
-      if (kExport && finished != 0u && lane == 0) atomicAdd(&es->finalized.v, (unsigned long long)__popc(finished));
+      if (finished != 0u && lane == 0) atomicAdd(&es->finalized.v, (unsigned long long)__popc(finished));
       free_mask |= done_mask;
       done_mask = 0u;
       __syncwarp();
     }
     P2C_PROF_MARK(9)
-    const bool read_pool = kExport && (iter & (P2C_HUNGRY_PERIOD - 1u)) == 0u;
+    const bool read_pool = (iter & (P2C_HUNGRY_PERIOD - 1u)) == 0u;
     if (read_pool) {  // read here, used at the end of the iteration
       published = volatile_load(&es->task_reserve.v);
       tickets = volatile_load(&es->task_head.v);
@@ -454,7 +454,7 @@ __device__ bool run_engine(const P& prob, const CertParams& prm, int fetch1, int
           }
         }
         const unsigned dropped = __ballot_sync(FULL, gone), got = __ballot_sync(FULL, fresh);
-        if (kExport && dropped != 0u && lane == 0) atomicAdd(&es->finalized.v, (unsigned long long)__popc(dropped));
+        if (dropped != 0u && lane == 0) atomicAdd(&es->finalized.v, (unsigned long long)__popc(dropped));
         if (got == 0u) continue;
         free_mask &= ~__reduce_or_sync(FULL, fresh ? (1u << s) : 0u);
         if (fresh) sh.batch[__popc(got & lt_mask)] = s;
@@ -470,7 +470,6 @@ __device__ bool run_engine(const P& prob, const CertParams& prm, int fetch1, int
         // ---- (B) no node and no query left: a node from the global pool ------
         // A ticket names the pool entry this warp gets; it polls that entry
         // alone, so waiting warps do not contend.
-        if (!kExport) break;
         if (!waiting) {
           if (!helper) {  // at most helper_cap idle warps stay to take nodes; the others leave
             int stay = 0;

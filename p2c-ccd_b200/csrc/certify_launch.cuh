@@ -59,12 +59,12 @@ struct LaunchShape {
   size_t smem = 0;
 };
 
+// The counters, and the tags of the pool's ring right behind them.
 inline cudaError_t reset_scratch(CertifyScratch* sc, cudaStream_t s, bool with_pools = false) {
-  cudaError_t e = cudaMemsetAsync(sc, 0, sizeof(CertifyScratch), s);
+  const size_t bytes = with_pools ? kScratchHeaderBytes + kTaskCap * sizeof(SubtreeTask) : sizeof(CertifyScratch);
+  const cudaError_t e = cudaMemsetAsync(sc, 0, bytes, s);
   if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(sc->invalid_key, 0xff, sizeof(sc->invalid_key), s);
-  if (e != cudaSuccess || !with_pools) return e;
-  return cudaMemsetAsync(pools_at(sc).tasks, 0, kTaskCap * sizeof(SubtreeTask), s);
+  return cudaMemsetAsync(sc->invalid_key, 0xff, sizeof(sc->invalid_key), s);
 }
 
 template <class K>

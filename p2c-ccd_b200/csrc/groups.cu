@@ -323,8 +323,7 @@ __global__ void __launch_bounds__(kCertifyThreads, kCertifyMinBlocks)
   const unsigned long long t_start = global_ns();
   const long long warps = (long long)gridDim.x * kCertifyWarps;
   const int fetch = (int)min(32ll, max(1ll, (prob.count() + warps - 1) / warps));
-  const bool ok = run_engine<true>(prob, prm, fetch, fetch, sh, st, &scratch->engine, pools,
-                                                t_start);
+  const bool ok = run_engine(prob, prm, fetch, fetch, sh, st, &scratch->engine, pools, t_start);
   flush_stats(st, ok, scratch);
 }
 

@@ -70,8 +70,7 @@ __global__ void __launch_bounds__(kCertifyThreads, kCertifyMinBlocks)
   const long long warps = (long long)gridDim.x * kCertifyWarps;
   const int fetch_vf = (int)min(32ll, max(1ll, (n_vf + warps - 1) / warps));
   const int fetch_ee = (int)min(32ll, max(1ll, (n_ee + warps - 1) / warps));
-  const bool ok = run_engine<true>(prob, prm, fetch_vf, fetch_ee, sh, st, &scratch->engine,
-                                                pools, t_start);
+  const bool ok = run_engine(prob, prm, fetch_vf, fetch_ee, sh, st, &scratch->engine, pools, t_start);
   flush_stats(st, ok, scratch);
   if (threadIdx.x == 0 && blockIdx.x == 0) {
     prob.agg->n_certified[0] = (unsigned long long)n_vf;
