@@ -499,20 +499,37 @@ __global__ void __launch_bounds__(kThreads) order_merge_kernel(unsigned* order, 
   }
 }
 
+// Asynchronous copy of a row to shared memory, and the wait for all but the
+// newest kAhead groups of them.
+constexpr int kAhead = 3;
+__device__ __forceinline__ void copy_row(WalkRow* to, const WalkRow* from) {
+  const unsigned dst = (unsigned)__cvta_generic_to_shared(to);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n\tcp.async.ca.shared.global [%2], [%3], 16;" ::"r"(dst),
+               "l"(from), "r"(dst + 16u), "l"(reinterpret_cast<const char*>(from) + 16)
+               : "memory");
+}
+__device__ __forceinline__ void commit_rows() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void wait_rows() { asm volatile("cp.async.wait_group %0;" ::"n"(kAhead) : "memory"); }
+
 // One warp per group: the walk of group_scheduler.cpp:116-232.  Rows are read
 // through the order; every slot of the group's terms is written.  Bound by the
 // chain of dependent additions of the two sums, so both run side by side over
-// all 32 lanes (rows that add nothing add +0.0): walk and the gather of sorted
-// costs before it took 99 us for 1 M rows, now 43.
+// all 32 lanes (rows that add nothing add +0.0), and by the rows' latency in
+// long groups, so the next three steps' rows are on their way to shared memory
+// while one is worked on: one group of a million rows 28.3 -> 14.2 ms, 1 M rows
+// in groups of up to 256 unchanged (their walk and the gather of sorted costs
+// before it took 99 us, now 43).
 __global__ void __launch_bounds__(kThreads, 4) group_kernel(const unsigned* order, long long n, unsigned limit,
                                                          double penalty, DenseLayout L) {
   __shared__ unsigned long long s_ctr[kNumCounters];
   __shared__ double2 s_add[kThreads / 32][32];
+  __shared__ WalkRow s_rows[kThreads / 32][kAhead + 1][32];
   if (threadIdx.x < kNumCounters) s_ctr[threadIdx.x] = 0;
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const unsigned G = (unsigned)L.acc->n_groups;
   double2* add = s_add[threadIdx.x >> 5];
+  WalkRow(*ahead)[32] = s_rows[threadIdx.x >> 5];
   unsigned c[kNumCounters] = {};  // none exceeds 2 n < 2^30
   // slots past the last group's: the compaction runs over 3 n
   for (long long i = 2 * n + G + (long long)blockIdx.x * kThreads + threadIdx.x; i < 3 * n;
@@ -529,23 +546,35 @@ __global__ void __launch_bounds__(kThreads, 4) group_kernel(const unsigned* orde
     unsigned rank = 0;
     unsigned calls = 0, fallback = 0, hits = 0, misses = 0;
     bool high_group = false;
+    // step k's rows go to place k mod kAhead + 1, each lane's to its own slot
+    unsigned moved = 0u, j[kAhead + 1];
+    auto fetch = [&](unsigned pos, unsigned row) {
+      if (pos < end) {
+        copy_row(&ahead[(pos - begin) / 32u % (kAhead + 1)][lane], L.rows + row);
+        moved += row != pos ? 1u : 0u;
+      }
+      commit_rows();
+    };
+#pragma unroll
+    for (int k = 0; k <= kAhead; ++k) j[k] = begin + 32u * k + lane < end ? order[begin + 32u * k + lane] : 0u;
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) fetch(begin + 32u * k + lane, j[k]);
+    unsigned next = j[kAhead];
     for (unsigned base = begin; base < end; base += 32) {
       const unsigned pos = base + lane;
       const int nvalid = (int)min(32u, end - base);
       const bool in = lane < nvalid;
+      fetch(pos + 32u * kAhead, next);
+      next = pos + 32u * (kAhead + 1) < end ? order[pos + 32u * (kAhead + 1)] : 0u;
+      wait_rows();
       double f = 0.0, nr = 0.0;
       unsigned fl = 0;
-      bool moved = false;
       if (in) {
-        const unsigned j = order[pos];
-        const WalkRow r = L.rows[j];
+        const WalkRow r = ahead[(base - begin) / 32u % (kAhead + 1)][lane];
         f = r.full;
         nr = r.narrow;
         fl = (unsigned)r.flags;
-        moved = j != pos;
       }
-      const unsigned m_moved = __ballot_sync(0xffffffffu, moved);
-      c[kReordered] += __popc(m_moved);
       const unsigned my_slot = slot0 + 2 * (pos - begin);
       truth = truth || __any_sync(0xffffffffu, fl & kColl);
       int from = 0;
@@ -637,6 +666,7 @@ __global__ void __launch_bounds__(kThreads, 4) group_kernel(const unsigned* orde
       __syncwarp();
       if (cost_here) gcost = (wbfp + extra0) + extra1;
     }
+    c[kReordered] += __reduce_add_sync(0xffffffffu, moved);
     if (lane == 0) {
       L.terms[slot0 + 2 * (end - begin)] = last_term;
       L.g_full[g] = gfull;
