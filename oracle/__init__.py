@@ -29,6 +29,12 @@ REF_SO = HERE / "_ref" / "libp2c_ref.so"
 REF_TOOL_SO = HERE / "_ref" / "libp2c_ref_tool.so"
 REF_CUDA_SO = HERE / "_ref" / "libp2c_ref_cuda.so"
 
+
+class ReferenceNotBuilt(FileNotFoundError):
+    """A library of the reference's own sources is absent: a test that needs it
+    is skipped (tests/conftest.py)."""
+
+
 TRAJ = np.dtype([("feature_id", "<i8"), ("position_t0", "<f8", (3,)), ("position_t1", "<f8", (3,))])
 PT = np.dtype([("point_id", "<i8"), ("triangle_id", "<i8"), ("point", TRAJ), ("triangle_v0", TRAJ),
                ("triangle_v1", TRAJ), ("triangle_v2", TRAJ)])
@@ -113,7 +119,7 @@ def ref_cuda() -> ctypes.CDLL:
     global _ref_cuda
     if _ref_cuda is None:
         if not REF_CUDA_SO.exists():
-            raise FileNotFoundError(f"{REF_CUDA_SO} is not built (reference CUDA sources or nvcc absent)")
+            raise ReferenceNotBuilt(f"{REF_CUDA_SO} is not built (reference CUDA sources or nvcc absent)")
         _ref_cuda = ctypes.CDLL(str(REF_CUDA_SO))
         C = _ref_cuda
         vp, i64, f64, ci = ctypes.c_void_p, ctypes.c_int64, ctypes.c_double, ctypes.c_int
@@ -147,7 +153,7 @@ def ref() -> ctypes.CDLL:
     global _ref
     if _ref is None:
         if not REF_SO.exists():
-            raise FileNotFoundError(f"{REF_SO} is not built (the reference sources were not available)")
+            raise ReferenceNotBuilt(f"{REF_SO} is not built (the reference sources were not available)")
         _ref = ctypes.CDLL(str(REF_SO))
         R = _ref
         vp, i64, f64, ci = ctypes.c_void_p, ctypes.c_int64, ctypes.c_double, ctypes.c_int
@@ -341,7 +347,7 @@ def ref_tool() -> ctypes.CDLL:
     global _ref_tool
     if _ref_tool is None:
         if not REF_TOOL_SO.exists():
-            raise FileNotFoundError(f"{REF_TOOL_SO} is not built (the reference sources were not available)")
+            raise ReferenceNotBuilt(f"{REF_TOOL_SO} is not built (the reference sources were not available)")
         T = ctypes.CDLL(str(REF_TOOL_SO))
         vp, i64, f64, ci, u64 = ctypes.c_void_p, ctypes.c_int64, ctypes.c_double, ctypes.c_int, ctypes.c_uint64
         T.ref_tool_last_error.restype = ctypes.c_char_p

@@ -17,6 +17,18 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA device (B200, sm_100a)")
 
 
+@pytest.hookimpl(wrapper=True)
+def pytest_runtest_call(item):
+    """A test that compares with the reference itself says so where the
+    reference's libraries are not built, whether or not it asked first."""
+    import oracle
+
+    try:
+        return (yield)
+    except oracle.ReferenceNotBuilt as e:
+        pytest.skip(str(e))
+
+
 @pytest.fixture(scope="session")
 def oracle_mod():
     import oracle
