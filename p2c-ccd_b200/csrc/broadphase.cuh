@@ -1,5 +1,5 @@
-// broadphase.cuh — scratch layout of the column-subdivided sweep-and-prune
-// (device side of p2c_scene_candidates).
+// broadphase.cuh — what the broad phases share (boxes, orders, prefilter, pair
+// staging) and the scratch and grid of the batched one (p2c_batch_candidates).
 #pragma once
 
 #include <cstdint>
@@ -12,13 +12,6 @@ namespace p2c {
 constexpr int kMaxCullObjects = 64;  // object-envelope culling up to this many objects
 constexpr int kMaxColumns = 128;     // columns per non-sweep axis (cell id < 2^14)
 constexpr int kCellBits = 14;
-// Width of the quantised sweep-axis minimum in a scene's sort key
-// (list << (14 + q) | cell << q | quantised min): 8 bits keep the key at 24
-// bits (3 radix passes) for scenes up to kSmallSceneQPrims primitives, 16
-// bits (4 passes) give larger scenes - dense flat sheets above all - tighter
-// sweep windows.  Chosen on the host from the primitive count.
-constexpr int kQBitsSmall = 8, kQBitsLarge = 16;
-constexpr long long kSmallSceneQPrims = 1000000;
 
 // Order-preserving maps to unsigned integers (radix-sortable keys).
 __device__ __forceinline__ unsigned long long order_key(double x) {
@@ -49,13 +42,6 @@ struct SortedBoxes {
   float4* fb;     // the non-sweep bounds rounded outward to float: (alo down, ahi up, blo down, bhi up)
   int32_t* id;    // primitive index in the scene
   int32_t* obj;   // object id
-  unsigned* cell_begin;  // [kMaxColumns^2] first entry of each column
-  unsigned* cell_end;    // [kMaxColumns^2] one past its last entry
-};
-
-struct BoxList {
-  long long n = 0;
-  SortedBoxes s{};
 };
 
 struct ListStats {
@@ -68,12 +54,11 @@ struct ListStats {
 struct Grid {
   int axis, a1, a2, g1, g2;
   unsigned qmax;                    // largest quantised value
-  int qbits;                        // width of the key's low field (scene keys)
   // Two-body split: with self pairs excluded and exactly two objects (ids 0
-  // and 1), the low field is (object << (qbits - 1)) | quantised min, so a
-  // column's entries of each object form their own sorted run and a box
-  // walks only the other object's run.  split_shift is qbits - 1 then, else
-  // -1 (the low field is the quantised min alone).
+  // and 1), the key's low field is (object << split_shift) | quantised min, so
+  // a column's entries of each object form their own sorted run and a box
+  // walks only the other object's run.  Otherwise split_shift is -1 (the low
+  // field is the quantised min alone).
   int split_shift;
   double base1, base2, inv1, inv2;  // column = floor((x - base) * inv)
   double base0, scale0;             // quantiser of the sweep axis: floor((x - base0) * scale0)
@@ -92,9 +77,6 @@ struct BroadScratch {
   unsigned long long ee_count;
   unsigned long long error_word;  // bit 0: non-finite coordinate
   unsigned long long obj_other;   // non-zero: a kept primitive's object id is neither 0 nor 1
-  unsigned long long keyed;       // single scene: boxes kept after culling (compact entries)
-  unsigned long long sweep_next[2];  // single scene: next slot of the vertex-face / edge-edge sweep
-  unsigned blocks_done;              // single scene: cull blocks finished (the last sizes the grid)
 };
 
 // Prefix of the partner object's run in a split low field (0 unsplit): a
@@ -106,7 +88,6 @@ __device__ __forceinline__ unsigned split_prefix(const Grid& g, int32_t obj) {
 __device__ __forceinline__ unsigned split_field(const Grid& g, int32_t obj, unsigned q) {
   return g.split_shift >= 0 ? ((unsigned)obj << g.split_shift) | q : q;
 }
-
 
 // ---- device helpers shared by the single-scene and batched sweeps ---------
 __device__ __forceinline__ double dmin(double a, double b) { return (b < a) ? b : a; }  // std::min

@@ -107,7 +107,7 @@ struct BatchBroad {
   int sorted_buf;            // which of keys / vals [0] or [1] holds the sorted entries
   unsigned long long* n_keyed;  // boxes kept after culling (the compact and sorted entries)
   unsigned* vals[2];
-  SortedBoxes S;             // P entries in sorted order (cell tables unused here)
+  SortedBoxes S;             // P entries in sorted order
   unsigned* cell_begin;      // 3 x total cells
   unsigned* cell_end;
   unsigned long long* pack[2];     // vf / ee pairs as found, each scene's in its capacity's slice
@@ -420,7 +420,6 @@ __global__ void grid_kernel(BatchBroad B) {
   g.axis = axis;
   g.a1 = axis == 0 ? 1 : 0;
   g.a2 = axis == 2 ? 1 : 2;
-  g.qbits = kBatchQBits;
   const p2c_batch_scene& d = B.scenes[s];
   const bool split = d.exclude_self && d.n_obj == 2 && sc.obj_other == 0ull;
   g.split_shift = split ? kBatchQBits - 1 : -1;
