@@ -815,9 +815,12 @@ __device__ __forceinline__ void export_counts(const SceneScratch* sc, unsigned l
 // (keys are unique), counted by eight threads per key over tiles of the list
 // in shared memory, on as many blocks as there are 32-key groups.  n^2
 // comparisons, but spread over the GPU: 3,700 edge pairs take 10.7 us where one
-// block's radix sort took 20.5 us (both with cold caches), and 16,384 keys,
-// the limit, still less than the radix sort's fill, six passes and unpack.
-constexpr long long kRankSortCap = 16384;
+// block's radix sort took 20.5 us (both with cold caches).  The line: all
+// candidates of a scene by ranks / by rows, both lists' buffers as large as the
+// larger list: 1,554 pairs 58 / 87 us, 3,770 89 / 91, 7,388 136 / 103, 18,629 251 / 122.
+// Buffers have room to spare (1.25 to 1.4 times and more), so 8,192 places hold
+// the lists that ranks suit.
+constexpr long long kRankSortCap = 8192;
 constexpr int kRankKeys = 32;
 constexpr int kRankTile = 2048;
 
