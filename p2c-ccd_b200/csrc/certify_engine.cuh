@@ -99,22 +99,38 @@ struct EnginePools {
 
 constexpr int kMaxTreeDepth = 63;  // leaf keys need one bit below the deepest level
 
-// Shape of the loop below (compile-time):
-//   P2C_ENGINE_SLOTS   queries a warp keeps in flight (at most 32);
-//   P2C_ENGINE_STACK   pending nodes a warp can hold (a power of two);
-//   P2C_ROOT_BATCH     queries fetched together (three root samples each);
-//   P2C_EXPORT_LANES   nodes one warp may publish to the pool per iteration;
+// Shape of the loop below (compile-time), with the times of other values, us a
+// pass after an L2 flush: 20,000 plain queries / two spheres of 40,960 triangles
+// / a 60,000-triangle cloth's self candidates / a 624k-triangle cloth's any-hit.
+// As set: 213 / 140 / 634 / 10,540; repeats differ by 1 % in the first, 0.2 % in
+// the others.
+//   P2C_ENGINE_SLOTS   queries a warp keeps in flight (at most 32).
+//                      8: 215 / 140 / 676 / 9,728; 32: 192 / 138 / 693 / 13,213
+//                      (three blocks an SM);
+//   P2C_ENGINE_STACK   pending nodes a warp can hold (a power of two).
+//                      512: 183 / 138 / 695 / 10,585 (three blocks an SM);
+//   P2C_ROOT_BATCH     queries fetched together (three root samples each).
+//                      5: 213 / 140 / 664 / 10,000;
+//   P2C_EXPORT_LANES   nodes one warp may publish to the pool per reading of its
+//                      counters.  1: 302 / 140 / 665 / 10,933; 3: 264 / 140 / 649 / 10,645;
 //   P2C_OVERSUPPLY     unclaimed nodes the pool may hold before warps stop
-//                      publishing;
-//   P2C_BACKOFF        longest sleep between two polls of an idle warp (ns);
-//   P2C_EXPORT_ABOVE   a warp publishes nodes beyond this many;
+//                      publishing.  64: 213 / 140 / 638 / 10,543;
+//   P2C_BACKOFF        longest sleep between two polls of an idle warp (ns).
+//                      64: 215 / 140 / 637 / 10,525; 1,024: 211 / 140 / 633 / 10,537;
+//   P2C_EXPORT_ABOVE   a warp publishes nodes beyond this many.
+//                      16: 219 / 140 / 644 / 10,614; 64: 207 / 140 / 631 / 10,507;
 //   P2C_FINISH_BATCH   finished queries a warp collects before it writes their
 //                      results together (their writes are chains of dependent
-//                      loads, stores and atomics);
+//                      loads, stores and atomics).
+//                      1: 215 / 140 / 695 / 10,846; 16: 215 / 140 / 639 / 9,500;
 //   P2C_GUIDED         a warp claims at most 1 / (P2C_GUIDED * warps) of the
-//                      queries left in a queue (and one more);
+//                      queries left in a queue (and one more).
+//                      2: 207 / 143 / 634 / 10,546; 4: 221 / 143 / 641 / 10,532;
 //   P2C_HUNGRY_PERIOD  iterations between reads of the pool's counters (a
-//                      power of two).
+//                      power of two).  1: 233 / 142 / 656 / 10,603; 8: 221 / 140 / 631 / 10,543.
+// P2C_HELPERS_PER_SM (certify_launch.cuh, 8): 2: 199 / 138 / 649 / 10,814; 16: 241 / 145 /
+// 648 / 10,617.  P2C_CERTIFY_BLOCKS (4): 3: 193 / 138 / 688 / 12,259; 5: 224 / 142 / 674 /
+// 11,001.  No value is best at all four; these lose least.
 #ifndef P2C_ENGINE_SLOTS
 #define P2C_ENGINE_SLOTS 16
 #endif
@@ -525,6 +541,8 @@ __device__ bool run_engine(const P& prob, const CertParams& prm, int fetch1, int
     P2C_PROF_COUNT(11)
     st.iters += 1u;
     const double eps_space = prm.eps_space;
+    // Up to ten nodes fill the lanes with their descendants; with groups up to
+    // four or six nodes only, two spheres take 149 or 143 us instead of 140.
     if (!roots && size > 10u) {
       // ---- (C) up to 32 nodes, one per lane -----------------------------------------
       const int count = max(1, min((int)min(size, 32u), (int)(kStack - 64u) - (int)size));  // room for a descent

@@ -386,7 +386,7 @@ __device__ __forceinline__ long long lower_bound(const unsigned long long* __res
 // pairs.  One lane walking each window, with an atomic for every step that
 // found a pair, took 209 us for 51,200 proxies with 280,000 hits; now 108.
 constexpr int kSweepLanes = 8;
-constexpr unsigned kWholeRun = 8;  // a column of at most this many entries is walked without a search
+constexpr unsigned kWholeRun = 8;  // a column of at most this many entries is walked without a search (as in the batch)
 
 __global__ void __launch_bounds__(kThreads, 4) sweep_kernel(ProxyLayout L, long long n, unsigned long long cap,
                                                          int rank_bits) {
