@@ -1069,7 +1069,7 @@ def run_b200(args) -> dict | None:
         bp_bytes = wl.broad_phase_bytes()
         broad_roof = {"bound": "hbm", "achieved": bp_bytes / (bp * 1e-3) / 1e9, "peak": hbm_peak, "unit": "GB/s",
                       "frac": bp_bytes / (bp * 1e-3) / 1e9 / hbm_peak, "traffic": None,
-                      "peak_source": hbm_src, "kernel": "candidate generation (boxes, sort, sweep)",
+                      "peak_source": hbm_src, "kernel": "candidate generation (boxes, bins or sort, sweep, pair order)",
                       "algorithmic_bytes_per_step": bp_bytes, "bytes_formula": "48V + 24F + 16E + 120(V+F+E) + 8P"}
         if hasattr(wl, "fused_ideal_bytes"):
             broad_roof["fused_ideal_bytes_per_step"] = wl.fused_ideal_bytes()
@@ -1574,7 +1574,7 @@ def run_proxy(args) -> dict | None:
                       frac=build_bytes / (build_ms * 1e-3) / 1e9 / hbm_peak, algorithmic_bytes_per_step=build_bytes,
                       bytes_per_unit="36 B per patch + 200 B per slab record read, 113 B per proxy written")
     feat_bytes = 528 * n_cand
-    feat_roof = dict(rl, kernel="proposal feature rows (density sorts, first-proxy lookup, rows_kernel)",
+    feat_roof = dict(rl, kernel="proposal feature rows (density counters, first-proxy lookup, rows_kernel)",
                      achieved=feat_bytes / (feat_ms * 1e-3) / 1e9, frac=feat_bytes / (feat_ms * 1e-3) / 1e9 / hbm_peak,
                      algorithmic_bytes_per_step=feat_bytes,
                      bytes_per_unit="80 B candidate + 2 x 96 B proxy read, 256 B row written per candidate")
@@ -1696,7 +1696,7 @@ def run_groups(args) -> dict | None:
     hbm_src = "of measured (MEASURED_PEAKS.json hbm_gbs)" if "hbm_gbs" in peaks else "of fallback (6.65 TB/s)"
     row_bytes = 128 * n  # query + candidate id, cost target, 8 trace doubles, 8 scores, 3 scores
     roofline = {"bound": "hbm", "peak": hbm_peak, "unit": "GB/s", "traffic": None, "peak_source": hbm_src,
-                "kernel": "whole replay (parse, two stable sorts, gather, group walk, ordered folds)",
+                "kernel": "whole replay (parse, sort by id, order inside groups, group walk, ordered totals)",
                 "achieved": row_bytes / (ms * 1e-3) / 1e9, "frac": row_bytes / (ms * 1e-3) / 1e9 / hbm_peak,
                 "algorithmic_bytes_per_step": row_bytes,
                 "bytes_per_unit": "128 B per candidate row read once",

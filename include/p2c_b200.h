@@ -290,7 +290,8 @@ size_t p2c_scene_candidates_workspace_bytes(int64_t nv, int64_t nf, int64_t ne, 
  * BuildVFCandidates / BuildEECandidates (tools/scene_object_envelope_native_
  * ti_walltime.cpp:603-699) with the same pair set.  Pairs are written as
  * (vertex << 32 | face) and (edge_lo << 32 | edge_hi); counts_dev[0..3] =
- * {vf pairs, ee pairs, error word (1: non-finite coordinate), sweep axis}.
+ * {vf pairs, ee pairs, error word (1: non-finite coordinate; the vertices,
+ * faces and edges that have one are in no pair), sweep axis}.
  * When a count exceeds its capacity only capacity pairs are kept and the
  * caller retries with a larger buffer (counts are the full totals).
  * sort_pairs = 1 sorts each list ascending, padding with ~0 up to its

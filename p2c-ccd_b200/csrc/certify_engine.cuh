@@ -35,17 +35,19 @@
 // collision are pruned: the recursion never reaches them.
 //
 // Bound by instruction issue and the latency of dependent FP64 chains, not by
-// memory: on a 624k-triangle cloth's edge-edge trees 600 instructions per 32
-// nodes, 57 % of the issue slots and 37 % of the FP64 pipe busy, DRAM idle, four
-// warps per scheduler (128 registers).  So a full iteration has a path of its
-// own without the groups' bookkeeping, the sample is one out-of-line function
-// for both paths, and all warps work on one family at a time: the code is 67 KB,
-// and instruction fetch stalls cost up to 20 % otherwise.  Against the engine
+// memory: on a 156k-triangle cloth's fallback trees (edge-edge) 51 % of the issue
+// slots and 31 % of the FP64 pipe are busy, DRAM idle, four warps per scheduler
+// (128 registers).  So a full iteration has a path of its own without the
+// groups' bookkeeping, the sample is one out-of-line function for both paths,
+// and all warps work on one family at a time: the code is 67 KB, and
+// instruction fetch stalls cost up to 20 % otherwise.  Against the engine
 // that tied a lane to a subtree and handed subtrees between lanes, on a B200:
 // two 40,960-triangle spheres 75 -> 33 us (12 iterations on the longest warp
 // instead of 27), 20,000 plain queries 365 -> 180 us, a 60,000-triangle cloth's
 // 295,000 self candidates 780 -> 420 us, a 624k-triangle cloth's 1.9 M any-hit
-// certificates 10.3 -> 8.5 ms, 64 uneven scenes 283 -> 190 us.  Idle warps hold a
+// certificates 10.3 -> 8.5 ms, 64 uneven scenes 283 -> 190 us; slower only where
+// each warp has one deep tree of the same size from the start (1,200 of 8,191
+// nodes 362 -> 459, of a launch that shares none).  Idle warps hold a
 // ticket each and poll their own pool entry: with one shared head that they
 // advanced by compare-and-swap the 20,000 queries took 1,200 us.  A bracket of
 // the distance in single precision that spared 95 % of the FP64 samples made
